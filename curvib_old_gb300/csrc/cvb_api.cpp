@@ -1706,9 +1706,15 @@ static int ensure_face_gram(cvb_ctx *ctx) {
   TRY(galloc(ctx, G, &gram, 9 * ctx->L[l].g.n()));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_face_gram(ctx->L[l].g, fm, gram, ctx->stream);
+  int *wild = nullptr, h_wild = 0;
+  TRY(dalloc(ctx, &wild, 1));
+  cudaMemsetAsync(wild, 0, sizeof(int), ctx->stream);
+  launch_face_gram(ctx->L[l].g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], gram, wild, ctx->stream);
+  cudaMemcpyAsync(&h_wild, wild, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+  dfree(ctx, wild);
   CKL();
   CK(cudaStreamSynchronize(ctx->stream));
+  G.gram_tame = h_wild == 0;
   G.gram = gram;
   return CVB_OK;
 }
@@ -1755,8 +1761,8 @@ static void momentum_ff1(cvb_ctx *ctx, double ren, int central, bool cart = true
     launch_contra2cart(F.g, ctx->cm[0], ctx->cm[1], ctx->cm[2], F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1,
                      -1, ctx->geo->c2c);
   launch_convection(F.g, ctx->uc_dev, ctx->ucat_dev, F.nvert, central != 0, ctx->conv_fp, ctx->conv_dev, ctx->stream);
-  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, 1. / ren,
-                 ctx->conv_fp, ctx->visc_dev, ctx->stream);
+  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
+                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, ctx->visc_dev, ctx->stream);
   launch_form_function1(F.g, F.nvert, ctx->p_dev, ctx->conv_dev, ctx->visc_dev, ctx->cm[0], ctx->cm[1], ctx->cm[2],
                         ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->rct_dev,
                         ctx->rhs_dev, ctx->stream);
@@ -1788,8 +1794,8 @@ int cvb_viscous(cvb_ctx *ctx, const double *ucat, double ren, double *visc) {
   TRY(ensure_face_gram(ctx));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, 1. / ren,
-                 ctx->conv_fp, ctx->visc_dev, ctx->stream);
+  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
+                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, ctx->visc_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(visc, ctx->visc_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -2729,7 +2735,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
         const double *fm[9];
         for (int q = 0; q < 9; q++) fm[q] = ctx->fm[level][q];
         launch_viscous(L.g, L.nvert, ctx->ucat_dev, fm, ctx->iaj[level], ctx->jaj[level], ctx->kaj[level],
-                       ctx->geo->gram, 1. / 300., ctx->conv_fp, ctx->visc_dev, ctx->stream);
+                       ctx->geo->gram, ctx->geo->gram_tame, 1. / 300., ctx->conv_fp, ctx->visc_dev, ctx->stream);
         break;
       }
       case CVB_KERNEL_MOMENTUM_RHS:

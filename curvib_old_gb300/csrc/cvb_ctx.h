@@ -32,6 +32,7 @@ struct Geometry {
   double *cm[3] = {};                     // finest: centre metrics csi, eta, zet (Cmpnts, [N][3])
   double *inv_aj = nullptr;               // finest: 1 / aj, for the range projection's sum of b / aj
   double *gram = nullptr;                 // finest, on first use: face metric products ([9][N], see k_face_gram)
+  bool gram_tame = false;                 // ... and whether they and the face metrics are in intmul.cuh's range
   double *c2c = nullptr;                  // finest, on first use: Contra2Cart's minors and determinant ([10][N])
   ~Geometry() {
     if (allocs.empty()) return;

@@ -309,9 +309,10 @@ void launch_metrics_divergence(const Geom &g, const double *csi, const double *e
 // face.  fm: the nine face-metric arrays (I, J, K x csi, eta, zet); fp: 9 N
 // doubles of scratch; rct: 3 N doubles of scratch.
 // gram: the 9 N face metric products of launch_face_gram (formed once per grid)
-void launch_face_gram(const Geom &g, const double *const *fm, double *gram, cudaStream_t s);
+void launch_face_gram(const Geom &g, const double *const *fm, const double *iaj, const double *jaj,
+                      const double *kaj, double *gram, int *wild, cudaStream_t s);
 void launch_viscous(const Geom &g, const double *nvert, const double *ucat, const double *const *fm,
-                    const double *iaj, const double *jaj, const double *kaj, const double *gram, double nu,
+                    const double *iaj, const double *jaj, const double *kaj, const double *gram, bool tame, double nu,
                     double *fp, double *visc, cudaStream_t s);
 void launch_form_function1(const Geom &g, const double *nvert, const double *p, const double *conv,
                            const double *visc, const double *csi, const double *eta, const double *zet,

@@ -5,7 +5,10 @@
 // (--fmad=false, build.py), so every product and sum rounds on its own in the
 // order the expressions are written -- the reference's C order -- and the
 // results equal the reference's bit for bit.
+#include <cmath>
+
 #include "cvb_internal.h"
+#include "intmul.cuh"
 #include "launch.cuh"
 
 namespace cvb {
@@ -59,54 +62,126 @@ struct FaceMetrics {
 
 }  // namespace
 
-// The viscous flux of every face (rhs.c:2056-2487): face d of cell P, between P
-// and P + e_d, into fp[(3 d + c) N + P]; the derivatives across the face's two
-// tangential directions are one-sided next to cells with nvert in (0.5, 7).
-__global__ void k_visc_faces(Geom g, const double *__restrict__ nv, const double *__restrict__ ucat, FaceMetrics M,
-                             const double *__restrict__ gram, double nu, double *__restrict__ fp) {
-  const size_t n = g.n();
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
-    const long P = (long)e;
-    const long st[3] = {1, g.mx, (long)g.mx * g.my};
-    const int q[3] = {i, j, k}, m[3] = {g.mx, g.my, g.mz};
-    for (int d = 0; d < 3; d++) {
-      bool in = q[d] <= m[d] - 2;
-      for (int t = 0; t < 3; t++)
-        if (t != d) in = in && q[t] >= 1 && q[t] <= m[t] - 2;
-      if (!in) continue;
-      const long sd = st[d];
-      double D[3][3];
-      for (int c = 0; c < 3; c++) D[d][c] = ucat[3 * (P + sd) + c] - ucat[3 * P + c];
-      for (int t = 0; t < 3; t++) {
-        if (t == d) continue;
-        const long s = st[t];
-        const bool up = visc_blocked(nv[P + s]) || visc_blocked(nv[P + sd + s]);
-        const bool dn = visc_blocked(nv[P - s]) || visc_blocked(nv[P + sd - s]);
-        for (int c = 0; c < 3; c++) {
+namespace {
+
+// One face of Viscous: the differences of ucat across face d of cell P into
+// D[t][c] (t the direction), one-sided along its two tangential directions
+// next to cells with nvert in (0.5, 7).
+__device__ __forceinline__ void visc_differences(const long (&st)[3], int d, long sd, long P,
+                                                 const double *__restrict__ nv, const double *__restrict__ ucat,
+                                                 double (&D)[3][3]) {
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    if (t == d) {
+#pragma unroll
+      for (int c = 0; c < 3; c++) D[t][c] = ucat[3 * (P + sd) + c] - ucat[3 * P + c];
+      continue;
+    }
+    const long s = st[t];
+    const bool up = visc_blocked(nv[P + s]) || visc_blocked(nv[P + sd + s]);
+    const bool dn = visc_blocked(nv[P - s]) || visc_blocked(nv[P + sd - s]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
 #define U(off) ucat[3 * (P + (off)) + c]
-          if (up) D[t][c] = scale_down<1>(U(sd) + U(0) - U(sd - s) - U(-s));
-          else if (dn) D[t][c] = scale_down<1>(U(sd + s) + U(s) - U(sd) - U(0));
-          else D[t][c] = scale_down<2>(U(sd + s) + U(s) - U(sd - s) - U(-s));
+      if (up) D[t][c] = scale_down<1>(U(sd) + U(0) - U(sd - s) - U(-s));
+      else if (dn) D[t][c] = scale_down<1>(U(sd + s) + U(s) - U(sd) - U(0));
+      else D[t][c] = scale_down<2>(U(sd + s) + U(s) - U(sd - s) - U(-s));
 #undef U
-        }
+    }
+  }
+}
+
+// The flux of face d of cell P from its differences, with FP64 multiplies.
+__device__ __noinline__ void visc_flux_fp64(const FaceMetrics &M, int d, long P, size_t n,
+                                            const double *__restrict__ gram, double nu, const double (&D)[3][3],
+                                            double (&v)[3]) {
+  const double *m0 = M.m[d][0] + 3 * P, *m1 = M.m[d][1] + 3 * P, *m2 = M.m[d][2] + 3 * P, *nd = M.m[d][d] + 3 * P;
+  const double *g = gram + (size_t)(3 * d) * n + P;
+  const double ajc = M.aj[d][P];
+  for (int c = 0; c < 3; c++) {
+    double r[3];
+    for (int q = 0; q < 3; q++) r[q] = D[0][q] * m0[c] + D[1][q] * m1[c] + D[2][q] * m2[c];
+    v[c] = 0;
+    v[c] += (g[0] * D[0][c] + g[n] * D[1][c] + g[2 * n] * D[2][c] + r[0] * nd[0] + r[1] * nd[1] + r[2] * nd[2]) *
+            ajc * (nu);
+  }
+}
+
+}  // namespace
+
+// The viscous flux of every face (rhs.c:2056-2487): face d of cell P, between P
+// and P + e_d, into fp[(3 d + c) N + P].  Bound by the FP64 pipe: of a face's
+// 105 operations (21 sums for the differences, 45 for r, 39 for the flux) the
+// 51 products go to the integer pipe (INT: intmul.cuh, for grids whose metrics
+// are in its range), beside the 54 sums, and the leading 0 + v of the
+// reference's accumulation, which only turns -0 into +0, to an integer compare.
+// A face with a value out of that range takes the FP64 multiplies.  Viscous on
+// the 192^3 box: 4.68 ms with FP64 multiplies, 2.83 ms so (the sums alone keep
+// the FP64 pipe busy for 1.9 ms).  Four blocks per SM (128 registers): three
+// (148 registers, nothing limited) 3.15 ms, five (spills) 2.88 ms.
+template <bool INT>
+__global__ void __launch_bounds__(128, 4) k_visc_faces(Geom g, const double *__restrict__ nv,
+                                                       const double *__restrict__ ucat,
+                                                       const __grid_constant__ FaceMetrics M,
+                                                       const double *__restrict__ gram, double nu,
+                                                       double *__restrict__ fp) {
+  const size_t n = g.n();
+  const long st[3] = {1, g.mx, (long)g.mx * g.my};
+  const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
+  const long P = (long)e;
+  // the directions one after another, not unrolled: three copies of the
+  // products' code would not fit the instruction cache
+#pragma unroll 1
+  for (int d = 0; d < 3; d++) {
+    const bool in = i <= g.mx - 2 && j <= g.my - 2 && k <= g.mz - 2 && (d == 0 || i >= 1) && (d == 1 || j >= 1) &&
+                    (d == 2 || k >= 1);
+    if (!in) continue;
+    double D[3][3], v[3];
+    visc_differences(st, d, d == 0 ? st[0] : d == 1 ? st[1] : st[2], P, nv, ucat, D);
+    bool fp64 = !INT;
+    if constexpr (INT) {
+      IntMulA Da[3][3];
+      IntMulB Nb[3];
+#pragma unroll
+      for (int t = 0; t < 3; t++)
+#pragma unroll
+        for (int c = 0; c < 3; c++) Da[t][c] = int_split_a(D[t][c], fp64);
+      {
+        IntMulB Gb[3];
+#pragma unroll
+        for (int t = 0; t < 3; t++) Gb[t] = int_split_b(gram[(size_t)(3 * d + t) * n + e]);
+#pragma unroll
+        for (int c = 0; c < 3; c++)
+          v[c] = int_mul(Da[0][c], Gb[0]) + int_mul(Da[1][c], Gb[1]) + int_mul(Da[2][c], Gb[2]);
       }
-      const double *mc = M.m[d][0] + 3 * P, *me = M.m[d][1] + 3 * P, *mz = M.m[d][2] + 3 * P;
-      const double *mm[3] = {mc, me, mz};
-      const double *nd = mm[d];
-      double gg[3];  // mm[a] . nd, from k_face_gram
-      for (int a = 0; a < 3; a++) gg[a] = gram[(size_t)(3 * d + a) * n + e];
-      double r[3][3];
-      for (int qq = 0; qq < 3; qq++)
-        for (int c = 0; c < 3; c++) r[qq][c] = D[0][qq] * mm[0][c] + D[1][qq] * mm[1][c] + D[2][qq] * mm[2][c];
-      const double ajc = M.aj[d][P];
+#pragma unroll
+      for (int t = 0; t < 3; t++) Nb[t] = int_split_b(M.m[d][d][3 * P + t]);
+      const IntMulB ajc = int_split_b(M.aj[d][P]), nub = int_split_b(nu);
+#pragma unroll
       for (int c = 0; c < 3; c++) {
-        double v = 0;
-        v += (gg[0] * D[0][c] + gg[1] * D[1][c] + gg[2] * D[2][c] + r[0][c] * nd[0] + r[1][c] * nd[1] +
-              r[2][c] * nd[2]) * ajc * (nu);
-        fp[(size_t)(3 * d + c) * n + e] = v;
+        IntMulB Mb[3];
+#pragma unroll
+        for (int t = 0; t < 3; t++) Mb[t] = int_split_b(M.m[d][t][3 * P + c]);
+        double s = c == 0 ? v[0] : c == 1 ? v[1] : v[2];
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+          const double r = int_mul(Da[0][t], Mb[0]) + int_mul(Da[1][t], Mb[1]) + int_mul(Da[2][t], Mb[2]);
+          s = s + int_mul(int_split_a(r, fp64), Nb[t]);
+        }
+        s = int_mul(int_split_a(s, fp64), ajc);
+        s = int_mul(int_split_a(s, fp64), nub);
+        // 0 + s
+        if (__double_as_longlong(s) == (long long)0x8000000000000000ULL) s = 0.;
+        if (c == 0) v[0] = s;
+        else if (c == 1) v[1] = s;
+        else v[2] = s;
       }
     }
+    if (fp64) visc_flux_fp64(M, d, P, n, gram, nu, D, v);
+#pragma unroll
+    for (int c = 0; c < 3; c++) fp[(size_t)(3 * d + c) * n + e] = v[c];
   }
 }
 
@@ -130,34 +205,57 @@ __global__ void k_visc_div(Geom g, const double *__restrict__ fp, double *__rest
 // N + P] = M[d][a] . M[d][d] at cell P (x, y, z products summed in that
 // order, as the two kernels wrote them).  They depend on the grid alone, so
 // they are formed once per grid and read back, the same values bit for bit.
-__global__ void k_face_gram(Geom g, FaceMetrics M, double *__restrict__ gram) {
+// *wild counts the metrics, Jacobians and products that intmul.cuh's products
+// do not take: neither zero nor within its range of exponents.
+__global__ void k_face_gram(Geom g, FaceMetrics M, double *__restrict__ gram, int *__restrict__ wild) {
   const size_t n = g.n();
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
+  const int m[3] = {g.mx, g.my, g.mz};
+  bool out = false;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    const int q[3] = {(int)(e % g.mx), (int)((e / g.mx) % g.my), (int)(e / ((size_t)g.mx * g.my))};
     for (int d = 0; d < 3; d++) {
+      bool face = q[d] <= m[d] - 2;  // a face k_visc_faces forms
+      for (int t = 0; t < 3; t++)
+        if (t != d) face = face && q[t] >= 1 && q[t] <= m[t] - 2;
+      auto look = [&](double v) {
+        if (face) int_split_a(v, out);
+      };
       const double *nd = M.m[d][d] + 3 * e;
       for (int a = 0; a < 3; a++) {
         const double *mm = M.m[d][a] + 3 * e;
-        gram[(size_t)(3 * d + a) * n + e] = mm[0] * nd[0] + mm[1] * nd[1] + mm[2] * nd[2];
+        const double v = mm[0] * nd[0] + mm[1] * nd[1] + mm[2] * nd[2];
+        gram[(size_t)(3 * d + a) * n + e] = v;
+        look(v);
+        for (int c = 0; c < 3; c++) look(mm[c]);
       }
+      look(M.aj[d][e]);
     }
+  }
+  if (out) atomicAdd(wild, 1);
 }
 
-void launch_face_gram(const Geom &g, const double *const *fm, double *gram, cudaStream_t s) {
+void launch_face_gram(const Geom &g, const double *const *fm, const double *iaj, const double *jaj,
+                      const double *kaj, double *gram, int *wild, cudaStream_t s) {
   FaceMetrics M;
   for (int d = 0; d < 3; d++)
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
-  k_face_gram<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, M, gram); count_launch();
+  M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
+  k_face_gram<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, M, gram, wild); count_launch();
 }
 
+// tame: the grid's metrics are all in intmul.cuh's range (k_face_gram).
 void launch_viscous(const Geom &g, const double *nvert, const double *ucat, const double *const *fm,
-                    const double *iaj, const double *jaj, const double *kaj, const double *gram, double nu, double *fp,
-                    double *visc, cudaStream_t s) {
+                    const double *iaj, const double *jaj, const double *kaj, const double *gram, bool tame, double nu,
+                    double *fp, double *visc, cudaStream_t s) {
   FaceMetrics M;
   for (int d = 0; d < 3; d++)
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
   const unsigned nb = blocks_for(g.n(), 128);
-  k_visc_faces<<<nb, 128, 0, s>>>(g, nvert, ucat, M, gram, nu, fp); count_launch();
+  const bool nu_tame = std::fabs(nu) >= std::ldexp(1., -510) && std::fabs(nu) < std::ldexp(1., 511);
+  if (tame && nu_tame) k_visc_faces<true><<<nb, 128, 0, s>>>(g, nvert, ucat, M, gram, nu, fp);
+  else k_visc_faces<false><<<nb, 128, 0, s>>>(g, nvert, ucat, M, gram, nu, fp);
+  count_launch();
   k_visc_div<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, fp, visc); count_launch();
 }
 

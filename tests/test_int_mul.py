@@ -1,0 +1,79 @@
+"""The integer-pipe product of the momentum kernels
+(curvib_old_gb300/csrc/intmul.cuh), restated here on integers and checked
+against the FP64 multiply bit for bit: significands at the edges of the
+rounding (ties, all ones, one bit), exponents at both ends of its range, and
+zeros of both signs."""
+import random
+import struct
+
+M32 = 0xFFFFFFFF
+
+
+def bits(x):
+    return struct.unpack("<Q", struct.pack("<d", x))[0]
+
+
+def value(b):
+    return struct.unpack("<d", struct.pack("<Q", b))[0]
+
+
+def split(x, shift):
+    b = bits(x)
+    h, l = b >> 32, b & M32
+    m = 0 if ((h & 0x7FFFFFFF) | l) == 0 else (h & 0xFFFFF) | 0x100000
+    s = ((m << 32 | l) << shift) & (2**64 - 1) if m else 0
+    return s & M32, s >> 32, h & 0xFFF00000
+
+
+def in_range(x):
+    h = bits(x) >> 32
+    return x == 0.0 or (((h & 0x7FFFFFFF) - (513 << 20)) & M32) < 1022 << 20
+
+
+def int_mul(x, y):
+    (al, ah, ase), (bl, bh, bse) = split(x, 5), split(y, 6)
+    t = al * bl
+    u = ah * bl + (t >> 32)
+    v = al * bh + u
+    assert u < 2**64 and v < 2**64
+    w = ah * bh + (v >> 32)
+    r, wl, wh = (v & M32) | ((t & M32) >> 11), w & M32, w >> 32
+    top = wh & 0x100000
+    if not top:
+        wh, wl, r = (wh << 1 | wl >> 31) & M32, (wl << 1 | r >> 31) & M32, r << 1 & M32
+    carry = (r + 0x7FFFFFFF + (wl & 1)) >> 32
+    lo = wl + carry
+    hi = (wh + (lo >> 32)) & M32
+    lo &= M32
+    if hi == 0:
+        return value(((ase ^ bse) & 0x80000000) << 32 | lo)
+    return value(((hi + ase + bse + top - (1024 << 20)) & M32) << 32 | lo)
+
+
+def significands(rng):
+    yield from (0, 1, 2, 3, 2**52 - 1, 2**52 - 2, 2**51, 2**51 + 1, 2**26, 2**26 + 1, 2**27 - 1, 0x5555555555555)
+    for _ in range(60):
+        b = rng.getrandbits(52)
+        yield b
+        yield b & ~((1 << rng.randrange(52)) - 1)  # few bits set: exact products and ties
+        yield b | ((1 << rng.randrange(52)) - 1)
+
+
+def test_product_is_the_rounded_one():
+    rng = random.Random(1)
+    ms = list(significands(rng))
+    ends = (513, 514, 1022, 1023, 1024, 1533, 1534)
+    for p in ms:
+        for q in ms:
+            x = value(rng.getrandbits(1) << 63 | rng.choice(ends) << 52 | p)
+            y = value(rng.getrandbits(1) << 63 | rng.choice(ends) << 52 | q)
+            assert in_range(x) and in_range(y)
+            assert bits(int_mul(x, y)) == bits(x * y), (x, y)
+    for z in (0.0, -0.0):
+        for x in (1.5, -2.0**-510, 2.0**511, 0.0, -0.0):
+            assert bits(int_mul(z, x)) == bits(z * x) and bits(int_mul(x, z)) == bits(x * z)
+
+
+def test_range():
+    assert all(in_range(x) for x in (0.0, -0.0, 2.0**-510, -(2.0**511), 1.9 * 2.0**511))
+    assert not any(in_range(x) for x in (2.0**-511, 5e-324, 2.0**512, float("inf"), float("-inf"), float("nan")))
