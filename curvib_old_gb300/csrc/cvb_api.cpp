@@ -1260,6 +1260,7 @@ void cvb_destroy(cvb_ctx *ctx) {
   free_all(ctx);
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
+  if (ctx->bc_ev) cudaEventDestroy(ctx->bc_ev);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -1998,7 +1999,7 @@ int cvb_set_inlet_nodes(cvb_ctx *ctx, const double *coor0, double cmx, double cm
 static int bc_buffers(cvb_ctx *ctx) {
   const Geom &g = ctx->L[ctx->nlevels - 1].g;
   const size_t n2 = (size_t)(g.mx - 2) * (g.my - 2);
-  if (!ctx->bc_scratch) TRY(dalloc(ctx, &ctx->bc_scratch, 2 * n2));
+  if (!ctx->bc_scratch) TRY(dalloc(ctx, &ctx->bc_scratch, n2));
   if (!ctx->bc_host) {
     if (cudaMallocHost((void **)&ctx->bc_host, sizeof(double) * 2 * n2) != cudaSuccess) {
       cudaGetLastError();
@@ -2006,6 +2007,7 @@ static int bc_buffers(cvb_ctx *ctx) {
       return fail(ctx, CVB_OOM, "pinned host buffer of %zu bytes failed", sizeof(double) * 2 * n2);
     }
   }
+  if (!ctx->bc_ev) CK(cudaEventCreateWithFlags(&ctx->bc_ev, cudaEventDisableTiming));
   return CVB_OK;
 }
 
@@ -2025,7 +2027,6 @@ struct BcSums {
   bool have_flux_in = false;
   double area = 0.;
   bool have_area = false;
-  int rc = CVB_OK;
 };
 
 // InflowFlux: the inlet face's ubcs and Ucont.z, and FluxInSum (summed once:
@@ -2045,37 +2046,42 @@ static int inflow_dev(cvb_ctx *ctx, const InletProfile &ip, BcSums &bs) {
   return CVB_OK;
 }
 
-// FormBCS's three passes; with an outlet each pass sums its flux on the host
-// and hands the kernel the ratio (bcs.c:4952-4956: FluxIn = FluxInSum +
-// FarFluxInSum (0: no far-field face) + FluxIntpSum).
+// FormBCS (k_form_ring says why one pass of the faces and edges stands for
+// its three).  With an outlet each pass's flux is summed on the host and its
+// kernel handed the ratio (bcs.c:4952-4956: FluxIn = FluxInSum + FarFluxInSum
+// (0: no far-field face) + FluxIntpSum); Contra2Cart of the planes the outlet
+// does not touch runs while the host adds the first pass's terms.
 static int form_bcs_dev(cvb_ctx *ctx, double flux_intp_sum, BcSums &bs) {
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   const Geom &g = F.g;
   const size_t n2 = (size_t)(g.mx - 2) * (g.my - 2);
-  std::function<void()> outlet;
-  if (ctx->H[ctx->nlevels - 1].d.bctype[5] == 4)
-    outlet = [ctx, &F, &g, n2, flux_intp_sum, &bs]() {
-      if (bs.rc) return;
-      launch_outlet_terms(g, F.nvert, ctx->cm[2], ctx->ucat_dev, ctx->bc_scratch, ctx->stream);
-      const size_t nt = bs.have_area ? n2 : 2 * n2;
-      if (cudaMemcpyAsync(ctx->bc_host, ctx->bc_scratch, sizeof(double) * nt, cudaMemcpyDeviceToHost, ctx->stream) !=
-              cudaSuccess ||
-          cudaStreamSynchronize(ctx->stream) != cudaSuccess) {
-        bs.rc = fail(ctx, CVB_CUDA_ERROR, "FormBCS outlet: %s", cudaGetErrorString(cudaGetLastError()));
-        return;
-      }
+  const double *csi = ctx->cm[0], *eta = ctx->cm[1], *zet = ctx->cm[2], *fac = ctx->geo->c2c;
+  if (ctx->H[ctx->nlevels - 1].d.bctype[5] == 4) {
+    auto plane = [&](bool apply, double ratio, bool terms, bool area) -> int {
+      launch_outlet_plane(g, csi, eta, zet, fac, F.nvert, apply, ratio, terms, area, ctx->uc_dev, ctx->ubcs_dev,
+                          ctx->ucat_dev, ctx->bc_host, ctx->stream);
+      CKL();
+      if (terms) CK(cudaEventRecord(ctx->bc_ev, ctx->stream));
+      return CVB_OK;
+    };
+    TRY(plane(false, 0., true, !bs.have_area));
+    launch_contra2cart(g, csi, eta, zet, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1, g.mz - 3, fac);
+    for (int pass = 0; pass < 3; pass++) {
+      CK(cudaEventSynchronize(ctx->bc_ev));
       const double flux_out = ordered_sum(ctx->bc_host, n2);
       if (!bs.have_area) {
         bs.area = ordered_sum(ctx->bc_host + n2, n2);
         bs.have_area = true;
       }
       const double flux_in = bs.flux_in + 0. + flux_intp_sum;
-      const double ratio = (flux_in - flux_out) / bs.area;
-      launch_outlet_apply(g, F.nvert, ctx->cm[2], ctx->ucat_dev, ratio, ctx->uc_dev, ctx->ubcs_dev, ctx->stream);
-    };
-  launch_form_bcs(g, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->geo->c2c, F.nvert, ctx->uc_dev, ctx->ubcs_dev,
-                  ctx->ucat_dev, ctx->p_dev, outlet, ctx->stream);
-  return bs.rc;
+      TRY(plane(true, (flux_in - flux_out) / bs.area, pass < 2, false));
+    }
+  } else {
+    launch_contra2cart(g, csi, eta, zet, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1, -1, fac);
+  }
+  launch_form_ring(g, ctx->ubcs_dev, ctx->ucat_dev, ctx->p_dev, ctx->stream);
+  CKL();
+  return CVB_OK;
 }
 
 int cvb_inflow_flux(cvb_ctx *ctx, double *ucont, double *ubcs, int inletprofile, double *flux_in_sum) {
@@ -2191,12 +2197,9 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   CK(cudaMemcpyAsync(ctx->p_dev, p, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->ubcs_dev, ubcs, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->stream));
   // InflowFlux (a wall k = 0 face: nothing), OutflowFlux (it only sums a flux
-  // nothing here reads), FormBCS
+  // nothing here reads), FormBCS.  The stages' InflowFlux is part of their
+  // update (k_imp_waxpy).
   BcSums bs;
-  auto boundary = [&]() -> int {
-    if (inlet) TRY(inflow_dev(ctx, uin, bs));
-    return form_bcs_dev(ctx, o->flux_intp_sum, bs);
-  };
   // Rhs starts at 0 (VecSet, implicitsolver.c:7140); CalcRHS leaves part of
   // its ring as it was
   CK(cudaMemsetAsync(ctx->rhs_dev, 0, sizeof(double) * n3, ctx->stream));
@@ -2209,7 +2212,8 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   };
   // before the loop (implicitsolver.c:7124-7148): the boundary conditions,
   // pUcont = Ucont, CalcRHS
-  TRY(boundary());
+  if (inlet) TRY(inflow_dev(ctx, uin, bs));
+  TRY(form_bcs_dev(ctx, o->flux_intp_sum, bs));
   CK(cudaMemcpyAsync(ctx->pu_dev, ctx->uc_dev, sizeof(double) * n3, cudaMemcpyDeviceToDevice, ctx->stream));
   calc_rhs();
   double normF0, normF1 = 1000., normdU1 = 1000., lambda = cfl;
@@ -2223,8 +2227,9 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
     pseudot++;
     for (int s = 0; s < 4; s++) {
       const double a = lambda * alfa[s] * dt * st;
-      launch_imp_waxpy(n3, a, ctx->rhs_dev, ctx->pu_dev, ctx->uc_dev, ctx->stream);
-      TRY(boundary());
+      launch_imp_waxpy(F.g, a, ctx->rhs_dev, ctx->pu_dev, F.nvert, inlet ? ctx->bc_scratch : nullptr, ctx->uc_dev,
+                       ctx->stream);
+      TRY(form_bcs_dev(ctx, o->flux_intp_sum, bs));
       calc_rhs();
     }
     normdU1 = normdU_bk;

@@ -108,8 +108,9 @@ struct cvb_ctx {
   std::vector<double> inlet_table;  // InletRead's uinr [101][1001] (profiles 0 and 5)
   double inlet_flux_in = 4.104388e-04;  // the reference's Flux_in (its initial value), profiles 3 and 6
   int inlet_ti = 0;                     // the time step profile 8 reads
-  double *bc_scratch = nullptr;            // InflowFlux / outlet: plane terms (device)
-  double *bc_host = nullptr;               // the same terms, pinned host memory, for the host's ordered sums
+  double *bc_scratch = nullptr;            // InflowFlux: plane terms (device)
+  double *bc_host = nullptr;               // the inlet's and outlet's terms, pinned host memory, for the host's ordered sums
+  cudaEvent_t bc_ev = nullptr;             // the outlet's terms are there
   double u_bc = 0.;                        // GhostNodeVelocity: the rheology plates' velocity (bcs.c's U_bc)
   double *ibm_cent = nullptr;  // cell centres of the last cvb_ibm_search that gave them
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

@@ -2,7 +2,6 @@
 // Grid layout everywhere: one level is the reference's DMDA box [mz][my][mx],
 // i fastest, boundary ring included (mx = IM+1 for IM nodes).
 #pragma once
-#include <functional>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -326,30 +325,27 @@ void launch_calc_rhs(const Geom &g, const double *nvert, const double *ucont, co
 void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi, const double *eta,
                                 const double *zet, double *ubcs, double *ucat, cudaStream_t s,
                                 const double *cent = nullptr, double u_bc = 0.);
-// FormBCS with walls on the x and y faces: its three passes of the outlet's
-// flux correction (outlet_pass, empty for a walled k = mz - 1 face; it
-// launches on s), Contra2Cart, the ghost faces' interior cells and the 12
-// edge averages of ucat and p
-void launch_form_bcs(const Geom &g, const double *csi, const double *eta, const double *zet, const double *fac,
-                     const double *nvert, double *ucont, double *ubcs, double *ucat, double *p,
-                     const std::function<void()> &outlet_pass, cudaStream_t s);
+// FormBCS with walls on the x and y faces: the ghost faces' interior cells and
+// the 12 edge averages of ucat and p, as its last pass leaves them
+void launch_form_ring(const Geom &g, const double *ubcs, double *ucat, double *p, cudaStream_t s);
+// The outlet's passes (bctype[5] 4) on the last interior k plane: with apply
+// the flux correction by ratio and Contra2Cart of the plane; with want_terms
+// (always without apply) its flux terms in the reference's loop order into
+// terms[0 .. n2), with want_area the area terms into terms[n2 .. 2 n2)
+void launch_outlet_plane(const Geom &g, const double *csi, const double *eta, const double *zet, const double *fac,
+                         const double *nvert, bool apply, double ratio, bool want_terms, bool want_area,
+                         double *ucont, double *ubcs, double *ucat, double *terms, cudaStream_t s);
 // InflowFlux on an inlet k = 0 face with a constant speed uin: ubcs and
 // Ucont.z there, and the face's flux terms in the reference's loop order into
 // terms ((mx - 2)(my - 2) doubles) for the host to add
 void launch_inflow(const Geom &g, const double *nvert, const double *zet, double uin, const double *coor0,
                    int profile, double cmy, double cmz, const double *uin_cell, double *ucont, double *ubcs,
                    double *terms, cudaStream_t s);
-// The outlet's flux correction (one FormBCS pass, bctype[5] 4): its flux and
-// area terms in the reference's loop order into terms[0 .. n2) and
-// terms[n2 .. 2 n2); then, with the ratio the host formed from their sums,
-// ubcs on the last face and Ucont.z of the last interior face
-void launch_outlet_terms(const Geom &g, const double *nvert, const double *zet, const double *ucat, double *terms,
-                         cudaStream_t s);
-void launch_outlet_apply(const Geom &g, const double *nvert, const double *zet, const double *ucat, double ratio,
-                         double *ucont, double *ubcs, cudaStream_t s);
-// ImpRK's stage update u = a rhs + pu, and its two infinity norms (|rhs|,
+// ImpRK's stage update u = a rhs + pu, with inflow (an inlet: launch_inflow's
+// terms) its Ucont.z on the inlet too; and its two infinity norms (|rhs|,
 // |pu - u|; pu null: |rhs| only) as bit patterns into out[0..1] (device)
-void launch_imp_waxpy(size_t n, double a, const double *rhs, const double *pu, double *u, cudaStream_t s);
+void launch_imp_waxpy(const Geom &g, double a, const double *rhs, const double *pu, const double *nvert,
+                      const double *inflow, double *u, cudaStream_t s);
 void launch_imp_norms(size_t n, const double *rhs, const double *pu, const double *u, unsigned long long *out,
                       cudaStream_t s);
 

@@ -125,6 +125,7 @@ __global__ void __launch_bounds__(128, 4) k_visc_faces(Geom g, const double *__r
                                                        const __grid_constant__ FaceMetrics M,
                                                        const double *__restrict__ gram, double nu,
                                                        double *__restrict__ fp) {
+  dep_sync();
   const size_t n = g.n();
   const long st[3] = {1, g.mx, (long)g.mx * g.my};
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
@@ -188,6 +189,7 @@ __global__ void __launch_bounds__(128, 4) k_visc_faces(Geom g, const double *__r
 // visc = the flux differences over each interior cell (rhs.c:2490-2511); 0 on
 // the ring (the reference's VecSet before the loops).
 __global__ void k_visc_div(Geom g, const double *__restrict__ fp, double *__restrict__ visc) {
+  dep_sync();
   const size_t n = g.n();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
@@ -253,10 +255,9 @@ void launch_viscous(const Geom &g, const double *nvert, const double *ucat, cons
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
   const unsigned nb = blocks_for(g.n(), 128);
   const bool nu_tame = std::fabs(nu) >= std::ldexp(1., -510) && std::fabs(nu) < std::ldexp(1., 511);
-  if (tame && nu_tame) k_visc_faces<true><<<nb, 128, 0, s>>>(g, nvert, ucat, M, gram, nu, fp);
-  else k_visc_faces<false><<<nb, 128, 0, s>>>(g, nvert, ucat, M, gram, nu, fp);
-  count_launch();
-  k_visc_div<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, fp, visc); count_launch();
+  if (tame && nu_tame) launch_dep(k_visc_faces<true>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
+  else launch_dep(k_visc_faces<false>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
+  launch_dep(k_visc_div, blocks_for(g.n(), 256), 256, 0, s, g, (const double *)fp, visc);
 }
 
 // ------------------------------------------------------------- FormFunction1
@@ -265,6 +266,7 @@ void launch_viscous(const Geom &g, const double *nvert, const double *ucat, cons
 __global__ void k_ff1_rct(Geom g, const double *__restrict__ conv, const double *__restrict__ visc,
                           const double *__restrict__ csi, const double *__restrict__ eta,
                           const double *__restrict__ zet, const double *__restrict__ aj, double *__restrict__ rct) {
+  dep_sync();
   const size_t n = g.n();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
@@ -326,6 +328,7 @@ __device__ __forceinline__ bool ff_dp(const double *__restrict__ nv, const doubl
 __global__ void k_ff1_faces(Geom g, const double *__restrict__ nv, const double *__restrict__ p,
                             const double *__restrict__ rct, FaceMetrics M, const double *__restrict__ gram,
                             double *__restrict__ rhs) {
+  dep_sync();
   const size_t n = g.n();
   const long st[3] = {1, g.mx, (long)g.mx * g.my};
   const int m[3] = {g.mx, g.my, g.mz};
@@ -381,8 +384,8 @@ void launch_form_function1(const Geom &g, const double *nvert, const double *p, 
   for (int d = 0; d < 3; d++)
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
-  k_ff1_rct<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, conv, visc, csi, eta, zet, aj, rct); count_launch();
-  k_ff1_faces<<<blocks_for(g.n(), 128), 128, 0, s>>>(g, nvert, p, rct, M, gram, rhs); count_launch();
+  launch_dep(k_ff1_rct, blocks_for(g.n(), 256), 256, 0, s, g, conv, visc, csi, eta, zet, aj, rct);
+  launch_dep(k_ff1_faces, blocks_for(g.n(), 128), 128, 0, s, g, nvert, p, (const double *)rct, M, gram, rhs);
 }
 
 // ------------------------------------------------------------------ CalcRHS
@@ -395,6 +398,7 @@ void launch_form_function1(const Geom &g, const double *nvert, const double *p, 
 __global__ void k_calc_rhs(Geom g, const double *__restrict__ nv, const double *__restrict__ uc,
                            const double *__restrict__ uo, const double *__restrict__ urm, int bdf2, double a,
                            int mz_end, double *__restrict__ rhs) {
+  dep_sync();
   const size_t n = g.n();
   const int mx = g.mx, my = g.my, mz = g.mz;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
@@ -437,18 +441,30 @@ __global__ void k_calc_rhs(Geom g, const double *__restrict__ nv, const double *
 
 void launch_calc_rhs(const Geom &g, const double *nvert, const double *ucont, const double *ucont_o,
                      const double *ucont_rm1, int bdf2, double neg_inv_dt, int mz_end, double *rhs, cudaStream_t s) {
-  k_calc_rhs<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, nvert, ucont, ucont_o, ucont_rm1, bdf2, neg_inv_dt, mz_end,
-                                                     rhs);
-  count_launch();
+  launch_dep(k_calc_rhs, blocks_for(g.n(), 256), 256, 0, s, g, nvert, ucont, ucont_o, ucont_rm1, bdf2, neg_inv_dt,
+             mz_end, rhs);
 }
 
 // ------------------------------------------------------------------- ImpRK
-// One Runge-Kutta stage's update (implicitsolver.c:7156, VecWAXPY):
-// u = a rhs + pu over every entry.
-__global__ void k_imp_waxpy(size_t n, double a, const double *__restrict__ rhs, const double *__restrict__ pu,
-                            double *__restrict__ u) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x)
-    u[e] = a * rhs[e] + pu[e];
+// One Runge-Kutta stage's update (implicitsolver.c:7156, VecWAXPY): u = a rhs
+// + pu over every entry; then, with inflow (an inlet on k = 0: k_inflow's
+// terms), what the InflowFlux that follows leaves in Ucont, its Ucont.z above
+// fluid cells.  The inlet's ubcs stay as the first InflowFlux of the call
+// left them: they depend on the grid, nvert and the profile alone.
+__global__ void __launch_bounds__(256) k_imp_waxpy(Geom g, double a, const double *__restrict__ rhs,
+                                                   const double *__restrict__ pu, const double *__restrict__ nv,
+                                                   const double *__restrict__ inflow, double *__restrict__ u) {
+  dep_sync();
+  const size_t n = 3 * g.n(), plane = (size_t)g.mx * g.my;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    double v = a * rhs[e] + pu[e];
+    if (inflow && e < 3 * plane && e % 3 == 2) {
+      const int q = (int)(e / 3), j = q / g.mx, i = q - j * g.mx;
+      if (i >= 1 && i <= g.mx - 2 && j >= 1 && j <= g.my - 2 && nv[q + plane] < 0.1)
+        v = inflow[(j - 1) * (g.mx - 2) + i - 1];
+    }
+    u[e] = v;
+  }
 }
 
 // The two infinity norms ImpRK takes after its stages (implicitsolver.c:
@@ -488,13 +504,13 @@ __global__ void __launch_bounds__(256) k_imp_norms(size_t n, const double *__res
   }
 }
 
-// ------------------------------------------------- InflowFlux, the outlet
+// ------------------------------------------------------------- InflowFlux
 // The reference adds a plane's flux and area terms one after another in its
 // (j, i) loop.  A chain of dependent FP64 adds is slow on this GPU (one
 // thread, about 70 cycles an add: 2.5 ms for a 192 x 192 plane), so the
-// kernels below write the terms, in that order, for the host to add; cells
-// the reference skips carry +0.0, which leaves a sum that started at +0.0 as
-// it was.
+// kernel below writes the terms, in that order, for the host to add (as
+// k_outlet_plane does); cells the reference skips carry +0.0, which leaves a
+// sum that started at +0.0 as it was.
 //
 // The shaped inlet speeds (bcs.c:152-192) at face cell (i, j): the mean of
 // its four nodes of the k = 0 node plane (coor0, [my][mx][3]) less the centre
@@ -556,62 +572,9 @@ void launch_inflow(const Geom &g, const double *nvert, const double *zet, double
   count_launch();
 }
 
-// The outlet (bcs.c:4914-4940): over the fluid cells of the last interior k
-// plane, the flux ucat . zet (x, y, z in order) and the area |zet| (x, y, z)
-// into terms[0 .. n) and terms[n .. 2n).
-__global__ void k_outlet_terms(Geom g, const double *__restrict__ nv, const double *__restrict__ zet,
-                               const double *__restrict__ ucat, double *__restrict__ terms) {
-  const int ni = g.mx - 2, n = ni * (g.my - 2);
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int i = 1 + t % ni, j = 1 + t / ni;
-  const size_t q = ((size_t)(g.mz - 2) * g.my + j) * g.mx + i;
-  double f = 0., a = 0.;
-  if (nv[q] < 0.1) {
-    const double *c = ucat + 3 * q, *z = zet + 3 * q;
-    f = c[0] * z[0] + c[1] * z[1] + c[2] * z[2];
-    a = __dsqrt_rn(z[0] * z[0] + z[1] * z[1] + z[2] * z[2]);
-  }
-  terms[t] = f;
-  terms[n + t] = a;
-}
-
-// The outlet's correction (bcs.c:4960-4992) with the ratio the host formed
-// from the sums: on the outlet's fluid cells ubcs of the last face = the ucat
-// next to it, and Ucont.z of the last interior face = ubcs . zet + ratio
-// |zet|.
-__global__ void k_outlet_apply(Geom g, const double *__restrict__ nv, const double *__restrict__ zet,
-                               const double *__restrict__ ucat, double ratio, double *__restrict__ uc,
-                               double *__restrict__ ub) {
-  const int ni = g.mx - 2, n = ni * (g.my - 2);
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const int i = 1 + t % ni, j = 1 + t / ni;
-  const size_t q = ((size_t)(g.mz - 2) * g.my + j) * g.mx + i, qb = q + (size_t)g.mx * g.my;
-  if (!(nv[q] < 0.1)) return;
-  const double *c = ucat + 3 * q, *z = zet + 3 * q;
-  double b[3];
-  for (int k = 0; k < 3; k++) b[k] = ub[3 * qb + k] = c[k];
-  uc[3 * q + 2] = (b[0] * z[0] + b[1] * z[1] + b[2] * z[2]) + ratio * __dsqrt_rn(z[0] * z[0] + z[1] * z[1] + z[2] * z[2]);
-}
-
-void launch_outlet_terms(const Geom &g, const double *nvert, const double *zet, const double *ucat, double *terms,
-                         cudaStream_t s) {
-  const int n = (g.mx - 2) * (g.my - 2);
-  k_outlet_terms<<<blocks_for(n, 256), 256, 0, s>>>(g, nvert, zet, ucat, terms);
-  count_launch();
-}
-
-void launch_outlet_apply(const Geom &g, const double *nvert, const double *zet, const double *ucat, double ratio,
-                         double *ucont, double *ubcs, cudaStream_t s) {
-  const int n = (g.mx - 2) * (g.my - 2);
-  k_outlet_apply<<<blocks_for(n, 256), 256, 0, s>>>(g, nvert, zet, ucat, ratio, ucont, ubcs);
-  count_launch();
-}
-
-void launch_imp_waxpy(size_t n, double a, const double *rhs, const double *pu, double *u, cudaStream_t s) {
-  k_imp_waxpy<<<blocks_for(n, 256), 256, 0, s>>>(n, a, rhs, pu, u);
-  count_launch();
+void launch_imp_waxpy(const Geom &g, double a, const double *rhs, const double *pu, const double *nvert,
+                      const double *inflow, double *u, cudaStream_t s) {
+  launch_dep(k_imp_waxpy, blocks_for(3 * g.n(), 256), 256, 0, s, g, a, rhs, pu, nvert, inflow, u);
 }
 
 void launch_imp_norms(size_t n, const double *rhs, const double *pu, const double *u, unsigned long long *out,

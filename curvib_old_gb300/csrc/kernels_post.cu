@@ -8,9 +8,8 @@
 // reference's order (no fused multiply-add), so results equal the reference's
 // bit for bit.  Arrays are the finest level's [mz][my][mx] box, Cmpnts
 // interleaved.
-#include <functional>
-
 #include "cvb_internal.h"
+#include "launch.cuh"
 
 namespace cvb {
 
@@ -86,18 +85,12 @@ __global__ void __launch_bounds__(256) k_c2c_factors(Geom g, const double *__res
   for (int q = 0; q < kC2cFactors; q++) fac[q * n + p] = f[q];
 }
 
+// Contra2Cart of interior cell p.
 template <bool FAC>
-__global__ void __launch_bounds__(256) k_contra2cart(Geom g, const double *__restrict__ csi,
-                                                     const double *__restrict__ eta, const double *__restrict__ zet,
-                                                     const double *__restrict__ fac,
-                                                     const double *__restrict__ nvert, const double *__restrict__ uc,
-                                                     double *__restrict__ ucat, int k0, int nk) {
-  const int ni = g.mx - 2, nj = g.my - 2;
-  const size_t cells = (size_t)ni * nj * nk, n = g.n();
-  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= cells) return;
-  const int i = 1 + (int)(t % ni), j = 1 + (int)((t / ni) % nj), k = k0 + (int)(t / ((size_t)ni * nj));
-  const size_t p = ((size_t)k * g.my + j) * g.mx + i;
+__device__ __forceinline__ void c2c_cell(const Geom &g, const double *__restrict__ csi, const double *__restrict__ eta,
+                                         const double *__restrict__ zet, const double *__restrict__ fac,
+                                         const double *__restrict__ nvert, const double *uc, double *ucat, size_t p) {
+  const size_t n = g.n();
   const double nv = nvert[p];
   if (!(nv < 0.1 || nv > 7.0)) return;
   const size_t pw = p - 1, ps = p - g.mx, pb = p - (size_t)g.mx * g.my;
@@ -123,6 +116,21 @@ __global__ void __launch_bounds__(256) k_contra2cart(Geom g, const double *__res
   ucat[3 * p + 2] = __ddiv_rn(d2, f[9]);
 }
 
+template <bool FAC>
+__global__ void __launch_bounds__(256) k_contra2cart(Geom g, const double *__restrict__ csi,
+                                                     const double *__restrict__ eta, const double *__restrict__ zet,
+                                                     const double *__restrict__ fac,
+                                                     const double *__restrict__ nvert, const double *__restrict__ uc,
+                                                     double *__restrict__ ucat, int k0, int nk) {
+  dep_sync();
+  const int ni = g.mx - 2, nj = g.my - 2;
+  const size_t cells = (size_t)ni * nj * nk;
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= cells) return;
+  const int i = 1 + (int)(t % ni), j = 1 + (int)((t / ni) % nj), k = k0 + (int)(t / ((size_t)ni * nj));
+  c2c_cell<FAC>(g, csi, eta, zet, fac, nvert, uc, ucat, ((size_t)k * g.my + j) * g.mx + i);
+}
+
 // Interior cells of the planes k0 .. k0 + nk - 1 (all interior planes by
 // default); fac: k_c2c_factors' arrays, or null to form the minors here.
 void launch_contra2cart(const Geom &g, const double *csi, const double *eta, const double *zet,
@@ -132,10 +140,9 @@ void launch_contra2cart(const Geom &g, const double *csi, const double *eta, con
   const size_t cells = (size_t)(g.mx - 2) * (g.my - 2) * nk;
   if (!cells) return;
   if (fac)
-    k_contra2cart<true><<<nblk(cells, 256), 256, 0, s>>>(g, csi, eta, zet, fac, nvert, ucont, ucat, k0, nk);
+    launch_dep(k_contra2cart<true>, nblk(cells, 256), 256, 0, s, g, csi, eta, zet, fac, nvert, ucont, ucat, k0, nk);
   else
-    k_contra2cart<false><<<nblk(cells, 256), 256, 0, s>>>(g, csi, eta, zet, fac, nvert, ucont, ucat, k0, nk);
-  count_launch();
+    launch_dep(k_contra2cart<false>, nblk(cells, 256), 256, 0, s, g, csi, eta, zet, fac, nvert, ucont, ucat, k0, nk);
 }
 
 void launch_c2c_factors(const Geom &g, const double *csi, const double *eta, const double *zet, double *fac,
@@ -273,7 +280,6 @@ struct GhostArgs {
   int bc[6];
   const double *csi, *eta, *zet;  // centre metrics
   double *ub, *u;                 // ubcs, ucat
-  double *p = nullptr;            // FormBCS: the pressure, averaged on the edges with ucat
   const double *cent = nullptr;   // the cell centres (an annulus face)
   double u_bc = 0.;               // the rheology plates' velocity (bcs.c's U_bc)
 };
@@ -326,15 +332,13 @@ __global__ void k_ghost_special(GhostArgs A) {
   ub[2] = ds(u[2], dm(un, nz));
 }
 
-// Non-periodic ghost faces of one axis, u = 2 ubcs - u(inner neighbour): the
-// whole face in GhostNodeVelocity (bcs.c:4015-4076), the face's interior cells
-// in FormBCS (interior != 0, bcs.c:5250-5318).
-__global__ void k_ghost_faces(GhostArgs A, int axis, int interior) {
+// Non-periodic ghost faces of one axis, u = 2 ubcs - u(inner neighbour), the
+// whole face (GhostNodeVelocity, bcs.c:4015-4076).
+__global__ void k_ghost_faces(GhostArgs A, int axis) {
   const Geom &g = A.g;
   const Face F{axis, (int)blockIdx.z};
   const int a = blockIdx.x * blockDim.x + threadIdx.x, b = blockIdx.y * blockDim.y + threadIdx.y;
   if (a >= F.na(g) || b >= F.nb(g)) return;
-  if (interior && (a < 1 || a > F.na(g) - 2 || b < 1 || b > F.nb(g) - 2)) return;
   const size_t p0 = F.at(g, a, b, 0), p1 = F.at(g, a, b, 1);
 #pragma unroll
   for (int c = 0; c < 3; c++) A.u[3 * p0 + c] = ds(dm(2.0, A.ub[3 * p0 + c]), A.u[3 * p1 + c]);
@@ -361,8 +365,7 @@ __global__ void k_ghost_ring(GhostArgs A, int axis, int whole) {
   for (int c = 0; c < 3; c++) A.u[3 * p0 + c] = A.u[3 * ps + c];
 }
 
-// The 12 edges of the box (bcs.c:4176-4283; FormBCS's, with p beside ucat,
-// bcs.c:5439-5570), each the mean of its two neighbours across the edge, in
+// The 12 edges of the box (bcs.c:4176-4283), each the mean of its two neighbours across the edge, in
 // the reference's order: one block, one edge after the other (edges share
 // corner cells).
 __global__ void k_ghost_edges(GhostArgs A) {
@@ -372,7 +375,6 @@ __global__ void k_ghost_edges(GhostArgs A) {
   auto avg = [&](size_t d, size_t a, size_t b) {
 #pragma unroll
     for (int c = 0; c < 3; c++) A.u[3 * d + c] = mean2(A.u[3 * a + c], A.u[3 * b + c]);
-    if (A.p) A.p[d] = mean2(A.p[a], A.p[b]);
   };
   for (int e = 0; e < 12; e++) {
     const int len = e < 8 ? ((e & 3) < 2 ? my : mx) : mz;
@@ -422,7 +424,7 @@ void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi,
   for (int axis = 0; axis < 3; axis++) {
     if (bc[2 * axis] == 7) continue;
     face_grid(g, axis, 2, grd, blk);
-    k_ghost_faces<<<grd, blk, 0, s>>>(A, axis, 0);
+    k_ghost_faces<<<grd, blk, 0, s>>>(A, axis);
     count_launch();
   }
   // first round: the three axes touch disjoint cells and read only interior
@@ -443,52 +445,134 @@ void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi,
   }
 }
 
+// ------------------------------------------------------------------- FormBCS
 // FormBCS (bcs.c:4436-5889) on a box with walls on its x and y faces and
 // walls, or an inlet and an outlet, on its k faces.  Its loop of three passes
-// (bcs.c:4483) each runs the outlet's flux correction (outlet_pass, before
-// Contra2Cart there), Contra2Cart, the ghost faces on the faces' interior cells
-// and the 12 edges of ucat and p.  Contra2Cart reads only ucont, and the faces
-// read only interior cells: with walls on the k faces, passes two and three
-// give the first pass's values there and only the edges, which read one
-// another's cells at the corners, change, so Contra2Cart and the faces run
-// once and the edges three times.  With an outlet, a pass changes Ucont.z of
-// the last interior k face only, so Contra2Cart runs on that plane alone in
-// passes two and three.
-void launch_form_bcs(const Geom &g, const double *csi, const double *eta, const double *zet, const double *fac,
-                     const double *nvert, double *ucont, double *ubcs, double *ucat, double *p,
-                     const std::function<void()> &outlet_pass, cudaStream_t s) {
-  GhostArgs A;
-  A.g = g;
-  for (int f = 0; f < 6; f++) A.bc[f] = 1;
-  A.csi = csi; A.eta = eta; A.zet = zet;
-  A.ub = ubcs;
-  A.u = ucat;
-  A.p = p;
-  dim3 grd, blk;
-  auto faces = [&]() {
-    for (int axis = 0; axis < 3; axis++) {
-      face_grid(g, axis, 2, grd, blk);
-      k_ghost_faces<<<grd, blk, 0, s>>>(A, axis, 1);
-      count_launch();
-    }
-  };
-  auto edges = [&]() {
-    k_ghost_edges<<<1, 256, 0, s>>>(A);
-    count_launch();
-  };
-  if (!outlet_pass) {
-    launch_contra2cart(g, csi, eta, zet, nvert, ucont, ucat, s, 1, -1, fac);
-    faces();
-    for (int pass = 0; pass < 3; pass++) edges();
+// (bcs.c:4483) each runs the outlet's flux correction, Contra2Cart, the ghost
+// faces on the faces' interior cells and the 12 edges of ucat and p.  What a
+// pass reads of the one before it is little:
+//  - the outlet's correction changes Ucont.z of the last interior k face, so
+//    Contra2Cart gives new values on that plane of cells alone, which is all
+//    the next pass's outlet flux reads (k_outlet_plane);
+//  - the ghost faces read interior cells, the edges' inner cells the ghost
+//    faces, and the corner cells, which the last four edges write last, the
+//    inner cells of the other edges from the same pass.  So the faces and
+//    edges of the last pass alone are the routine's result (k_form_ring).
+// One pass of one launch in place of three passes of four: at 32^3, where an
+// ImpRK stage is latency, the ring's share of a stage went from 80 us (three
+// passes of one block walking 12 edges, 19 us each, and of three faces'
+// kernels) to 4.
+
+// The ring cell of ucat on face (axis, high) whose inner neighbour is cell q
+// (q's index in memory; the ring cell one step along the axis from it).
+__device__ __forceinline__ double ring_face(const double *ub, const double *u, size_t q, long step, int c) {
+  return ds(dm(2.0, ub[3 * (q + step) + c]), u[3 * q + c]);
+}
+// The inner edge cell beside cell q: the mean of the two ring cells that are
+// one step from q along sa and along sb.
+__device__ __forceinline__ double ring_edge(const double *ub, const double *u, size_t q, long sa, long sb, int c) {
+  return mean2(ring_face(ub, u, q, sa, c), ring_face(ub, u, q, sb, c));
+}
+
+// blockIdx.y 0 .. 5: the interior cells of face 2 axis + side; 6 .. 17: the
+// cells of edge (v, a, b), along axis v at the sides a, b of the other two
+// (the corners with the edges along z).
+__global__ void __launch_bounds__(256) k_form_ring(Geom g, const double *__restrict__ ub, double *u, double *p) {
+  dep_sync();
+  const int ext[3] = {g.mx, g.my, g.mz};
+  const long st[3] = {1, g.mx, (long)g.mx * g.my};
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (blockIdx.y < 6) {
+    const int axis = blockIdx.y >> 1, hi = blockIdx.y & 1;
+    const int A = axis == 0 ? 1 : 0, B = axis == 2 ? 1 : 2;
+    const int na = ext[A] - 2, nb = ext[B] - 2;
+    if (t >= na * nb) return;
+    const size_t q = (size_t)(1 + t % na) * st[A] + (size_t)(1 + t / na) * st[B] + (hi ? ext[axis] - 2 : 1) * st[axis];
+    const long step = hi ? st[axis] : -st[axis];
+#pragma unroll
+    for (int c = 0; c < 3; c++) u[3 * (q + step) + c] = ring_face(ub, u, q, step, c);
     return;
   }
-  for (int pass = 0; pass < 3; pass++) {
-    outlet_pass();
-    if (pass == 0) launch_contra2cart(g, csi, eta, zet, nvert, ucont, ucat, s, 1, -1, fac);
-    else launch_contra2cart(g, csi, eta, zet, nvert, ucont, ucat, s, g.mz - 2, 1, fac);
-    faces();
-    edges();
+  const int e = blockIdx.y - 6, v = e >> 2, ha = e & 1, hb = (e >> 1) & 1;
+  const int A = v == 0 ? 1 : 0, B = v == 2 ? 1 : 2;
+  if (t >= ext[v]) return;
+  // the cell inside the edge along A and B, and the steps out of the box
+  const size_t qab = (ha ? ext[A] - 2 : 1) * st[A] + (hb ? ext[B] - 2 : 1) * st[B];
+  const long sa = ha ? st[A] : -st[A], sb = hb ? st[B] : -st[B];
+  if (t >= 1 && t <= ext[v] - 2) {
+    const size_t q = qab + (size_t)t * st[v];
+#pragma unroll
+    for (int c = 0; c < 3; c++) u[3 * (q + sa + sb) + c] = ring_edge(ub, u, q, sa, sb, c);
+    p[q + sa + sb] = mean2(p[q + sa], p[q + sb]);
+  } else if (v == 2) {
+    // a corner: the mean of the cells beside it on the edges along y (at the
+    // sides of x and z) and along x (at the sides of y and z)
+    const size_t q = qab + (t ? ext[2] - 2 : 1) * st[2];
+    const long sz = t ? st[2] : -st[2];
+#pragma unroll
+    for (int c = 0; c < 3; c++)
+      u[3 * (q + sa + sb + sz) + c] = mean2(ring_edge(ub, u, q, sa, sz, c), ring_edge(ub, u, q, sb, sz, c));
+    p[q + sa + sb + sz] = mean2(mean2(p[q + sa], p[q + sz]), mean2(p[q + sb], p[q + sz]));
   }
+}
+
+void launch_form_ring(const Geom &g, const double *ubcs, double *ucat, double *p, cudaStream_t s) {
+  const int big = g.mx * g.my > g.my * g.mz ? (g.mx * g.my > g.mx * g.mz ? g.mx * g.my : g.mx * g.mz)
+                                            : (g.my * g.mz > g.mx * g.mz ? g.my * g.mz : g.mx * g.mz);
+  launch_dep(k_form_ring, dim3(nblk(big, 256), 18), 256, 0, s, g, ubcs, ucat, p);
+}
+
+// One step of the outlet's passes on the last interior k plane.  APPLY: the
+// correction (bcs.c:4960-4992) with the ratio the host formed from the sums
+// -- on fluid cells ubcs of the last face = the ucat next to it and Ucont.z of
+// the last interior face = ubcs . zet + ratio |zet| -- then Contra2Cart of the
+// plane.  TERMS: the next pass's flux terms ucat . zet of the fluid cells
+// (bcs.c:4914-4940: x, y, z in order) into terms[0 .. n), AREA their |zet|
+// into terms[n .. 2n), in the reference's loop order for the host to add
+// (terms is pinned host memory: the host waits for the kernel, not for a copy).
+// Cells the reference skips carry +0.0.
+template <bool APPLY, bool TERMS, bool AREA>
+__global__ void __launch_bounds__(128) k_outlet_plane(Geom g, const double *__restrict__ csi,
+                                                      const double *__restrict__ eta, const double *__restrict__ zet,
+                                                      const double *__restrict__ fac, const double *__restrict__ nv,
+                                                      double ratio, double *uc, double *ub, double *ucat,
+                                                      double *terms) {
+  dep_sync();
+  const int ni = g.mx - 2, n = ni * (g.my - 2);
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= n) return;
+  const int i = 1 + t % ni, j = 1 + t / ni;
+  const size_t q = ((size_t)(g.mz - 2) * g.my + j) * g.mx + i, qb = q + (size_t)g.mx * g.my;
+  const bool fluid = nv[q] < 0.1;
+  const double *z = zet + 3 * q;
+  double *c = ucat + 3 * q;
+  double a = 0., f = 0.;
+  if (fluid && (APPLY || AREA)) a = __dsqrt_rn(da(da(dm(z[0], z[0]), dm(z[1], z[1])), dm(z[2], z[2])));
+  if (APPLY) {
+    if (fluid) {
+      ub[3 * qb] = c[0];
+      ub[3 * qb + 1] = c[1];
+      ub[3 * qb + 2] = c[2];
+      uc[3 * q + 2] = da(da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2])), dm(ratio, a));
+    }
+    c2c_cell<true>(g, csi, eta, zet, fac, nv, uc, ucat, q);
+  }
+  if (TERMS) {
+    if (fluid) f = da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2]));
+    terms[t] = f;
+    if (AREA) terms[n + t] = a;
+  }
+}
+
+void launch_outlet_plane(const Geom &g, const double *csi, const double *eta, const double *zet, const double *fac,
+                         const double *nvert, bool apply, double ratio, bool want_terms, bool want_area,
+                         double *ucont, double *ubcs, double *ucat, double *terms, cudaStream_t s) {
+  const int n = (g.mx - 2) * (g.my - 2);
+  auto go = [&](auto k) {
+    launch_dep(k, nblk(n, 128), 128, 0, s, g, csi, eta, zet, fac, nvert, ratio, ucont, ubcs, ucat, terms);
+  };
+  if (!apply) want_area ? go(k_outlet_plane<false, true, true>) : go(k_outlet_plane<false, true, false>);
+  else want_terms ? go(k_outlet_plane<true, true, false>) : go(k_outlet_plane<true, false, false>);
 }
 
 // ---------------------------------------------------------------------------
@@ -582,6 +666,7 @@ __device__ __forceinline__ bool conv_fluid(double n) { return conv_below(n, 0.1)
 __global__ void __launch_bounds__(256) k_conv_faces(Geom g, const double *__restrict__ ucont,
                                                    const double *__restrict__ ucat, const double *__restrict__ nv,
                                                    int central, double *__restrict__ fp) {
+  dep_sync();
   const size_t n = g.n(), plane = (size_t)g.mx * g.my;
   for (size_t pu = (size_t)blockIdx.x * blockDim.x + threadIdx.x; pu < n; pu += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(pu % g.mx), j = (int)((pu / g.mx) % g.my), k = (int)(pu / plane);
@@ -640,6 +725,7 @@ __global__ void __launch_bounds__(256) k_conv_faces(Geom g, const double *__rest
 // conv = fp1 - fp1_w + fp2 - fp2_s + fp3 - fp3_b per component, left to right
 // as the C; 0 on the ring.
 __global__ void __launch_bounds__(256) k_conv_diff(Geom g, const double *__restrict__ fp, double *__restrict__ conv) {
+  dep_sync();
   const size_t n = g.n(), plane = (size_t)g.mx * g.my;
   for (size_t p = (size_t)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(p % g.mx), j = (int)((p / g.mx) % g.my), k = (int)(p / plane);
@@ -660,10 +746,8 @@ void launch_convection(const Geom &g, const double *ucont, const double *ucat, c
                        double *fp, double *conv, cudaStream_t s) {
   const size_t n = g.n();
   const unsigned blocks = nblk(n, 256) < 152u * 8 ? nblk(n, 256) : 152u * 8;
-  k_conv_faces<<<blocks, 256, 0, s>>>(g, ucont, ucat, nvert, central, fp);
-  count_launch();
-  k_conv_diff<<<blocks, 256, 0, s>>>(g, fp, conv);
-  count_launch();
+  launch_dep(k_conv_faces, blocks, 256, 0, s, g, ucont, ucat, nvert, central, fp);
+  launch_dep(k_conv_diff, blocks, 256, 0, s, g, (const double *)fp, conv);
 }
 
 }  // namespace cvb
