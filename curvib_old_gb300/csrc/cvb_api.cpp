@@ -1570,6 +1570,7 @@ static int ghost_types_ok(cvb_ctx *ctx, const int *bc) {
 }
 
 static int ensure_c2c(cvb_ctx *ctx);
+static C2cFactors c2c_factors(const cvb_ctx *ctx) { return {ctx->geo->c2c, ctx->geo->c2c_tame}; }
 static int post_buffers(cvb_ctx *ctx, size_t n) {
   if (!ctx->ucat_dev) TRY(dalloc(ctx, &ctx->ucat_dev, 3 * n));
   if (!ctx->ubcs_dev) TRY(dalloc(ctx, &ctx->ubcs_dev, 3 * n));
@@ -1585,8 +1586,7 @@ int cvb_contra2cart(cvb_ctx *ctx, const double *ucont, double *ucat) {
   TRY(post_buffers(ctx, n));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  launch_contra2cart(F.g, ctx->cm[0], ctx->cm[1], ctx->cm[2], F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1,
-                     -1, ctx->geo->c2c);
+  launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(ucat, ctx->ucat_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1648,8 +1648,7 @@ int cvb_projection_cart(cvb_ctx *ctx, const double *phi, double dt, double st, d
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], F.nvert, ctx->w, dt, st, ctx->uc_dev, ctx->stream);
-  launch_contra2cart(F.g, ctx->cm[0], ctx->cm[1], ctx->cm[2], F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1,
-                     -1, ctx->geo->c2c);
+  launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   launch_ghost_node_velocity(F.g, bc, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev, ctx->ucat_dev, ctx->stream,
                              ctx->ibm_cent, ctx->u_bc);
   CKL();
@@ -1679,18 +1678,24 @@ int cvb_convection(cvb_ctx *ctx, const double *ucont, const double *ucat, int ce
   return CVB_OK;
 }
 
-// The grid's Contra2Cart factors (k_c2c_factors: the metric rows' minors and
-// determinant of every interior cell), formed on first use and kept with the
+// The grid's Contra2Cart factors (k_c2c_factors: the metric rows' minors,
+// determinant and its reciprocal of every interior cell), formed on first use and kept with the
 // grid's metrics.
 static int ensure_c2c(cvb_ctx *ctx) {
   Geometry &G = *ctx->geo;
   if (G.c2c) return CVB_OK;
   const int l = ctx->nlevels - 1;
   double *fac = nullptr;
-  TRY(galloc(ctx, G, &fac, 10 * ctx->L[l].g.n()));
-  launch_c2c_factors(ctx->L[l].g, ctx->cm[0], ctx->cm[1], ctx->cm[2], fac, ctx->stream);
+  TRY(galloc(ctx, G, &fac, 11 * ctx->L[l].g.n()));
+  int *wild = nullptr, h_wild = 0;
+  TRY(dalloc(ctx, &wild, 1));
+  cudaMemsetAsync(wild, 0, sizeof(int), ctx->stream);
+  launch_c2c_factors(ctx->L[l].g, ctx->cm[0], ctx->cm[1], ctx->cm[2], fac, wild, ctx->stream);
+  cudaMemcpyAsync(&h_wild, wild, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+  dfree(ctx, wild);
   CKL();
   CK(cudaStreamSynchronize(ctx->stream));
+  G.c2c_tame = h_wild == 0;
   G.c2c = fac;
   return CVB_OK;
 }
@@ -1737,7 +1742,6 @@ static int momentum_prepare(cvb_ctx *ctx, const char *who, const double *ucont, 
   TRY(post_buffers(ctx, n));
   if (!ctx->conv_dev) TRY(dalloc(ctx, &ctx->conv_dev, 3 * n));
   if (!ctx->conv_fp) TRY(dalloc(ctx, &ctx->conv_fp, 9 * n));
-  if (!ctx->visc_dev) TRY(dalloc(ctx, &ctx->visc_dev, 3 * n));
   if (!ctx->rct_dev) TRY(dalloc(ctx, &ctx->rct_dev, 3 * n));
   if (!ctx->rhs_dev) TRY(dalloc(ctx, &ctx->rhs_dev, 3 * n));
   TRY(ensure_face_gram(ctx));
@@ -1749,24 +1753,23 @@ static int momentum_prepare(cvb_ctx *ctx, const char *who, const double *ucont, 
 }
 
 // FormFunction1's kernels on the device copies: Contra2Cart, Convection,
-// Viscous, then the face values into rhs_dev.
+// Viscous, then the face values into rhs_dev; with calc, CalcRHS's.
 // cart = false: ucat's interior already holds Contra2Cart of the current
 // ucont (FormBCS ran it), so FormFunction1's own call would rewrite the same
 // values.
-static void momentum_ff1(cvb_ctx *ctx, double ren, int central, bool cart = true) {
+static void momentum_ff1(cvb_ctx *ctx, double ren, int central, const MomentumTime *calc, bool cart = true) {
   const int l = ctx->nlevels - 1;
   LevelDev &F = ctx->L[l];
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   if (cart)
-    launch_contra2cart(F.g, ctx->cm[0], ctx->cm[1], ctx->cm[2], F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1,
-                     -1, ctx->geo->c2c);
+    launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   launch_convection(F.g, ctx->uc_dev, ctx->ucat_dev, F.nvert, central != 0, ctx->conv_fp, ctx->conv_dev, ctx->stream);
   launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
-                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, ctx->visc_dev, ctx->stream);
-  launch_form_function1(F.g, F.nvert, ctx->p_dev, ctx->conv_dev, ctx->visc_dev, ctx->cm[0], ctx->cm[1], ctx->cm[2],
-                        ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->rct_dev,
-                        ctx->rhs_dev, ctx->stream);
+                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, nullptr, ctx->stream);
+  launch_form_function1(F.g, F.nvert, ctx->p_dev, ctx->conv_dev, ctx->conv_fp, ctx->cm[0], ctx->cm[1], ctx->cm[2],
+                        ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame,
+                        calc, ctx->rct_dev, ctx->rhs_dev, ctx->stream);
 }
 
 static int momentum_finish(cvb_ctx *ctx, double *ucat, double *rhs) {
@@ -1807,7 +1810,7 @@ int cvb_form_function1(cvb_ctx *ctx, const double *ucont, double *ucat, const do
                        double *rhs) {
   TRY(momentum_prepare(ctx, "FormFunction1", ucont, ucat, p, rhs));
   if (!(ren != 0.0)) return fail(ctx, CVB_BAD_INPUT, "FormFunction1: ren is 0");
-  momentum_ff1(ctx, ren, central);
+  momentum_ff1(ctx, ren, central, nullptr);
   return momentum_finish(ctx, ucat, rhs);
 }
 
@@ -1823,13 +1826,12 @@ int cvb_calc_rhs(cvb_ctx *ctx, const double *ucont, const double *ucont_o, const
   if (!ctx->urm_dev) TRY(dalloc(ctx, &ctx->urm_dev, 3 * n));
   CK(cudaMemcpyAsync(ctx->uo_dev, ucont_o, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->urm_dev, ucont_rm1, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  momentum_ff1(ctx, ren, central);
   // COEF_TIME_ACCURACY is 1.5 in the reference (variables.h:421): second-order
   // backward except on the first step
   const int bdf2 = (ti != tistart && ti != 1) ? 1 : 0;
   const int mz_end = ctx->H[l].d.bctype[5] == 8 ? F.g.mz - 2 : F.g.mz - 3;
-  launch_calc_rhs(F.g, F.nvert, ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end, ctx->rhs_dev,
-                  ctx->stream);
+  const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end};
+  momentum_ff1(ctx, ren, central, &calc);
   return momentum_finish(ctx, ucat, rhs);
 }
 
@@ -2055,17 +2057,17 @@ static int form_bcs_dev(cvb_ctx *ctx, double flux_intp_sum, BcSums &bs) {
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   const Geom &g = F.g;
   const size_t n2 = (size_t)(g.mx - 2) * (g.my - 2);
-  const double *csi = ctx->cm[0], *eta = ctx->cm[1], *zet = ctx->cm[2], *fac = ctx->geo->c2c;
+  const C2cFactors fac = c2c_factors(ctx);
   if (ctx->H[ctx->nlevels - 1].d.bctype[5] == 4) {
     auto plane = [&](bool apply, double ratio, bool terms, bool area) -> int {
-      launch_outlet_plane(g, csi, eta, zet, fac, F.nvert, apply, ratio, terms, area, ctx->uc_dev, ctx->ubcs_dev,
+      launch_outlet_plane(g, ctx->cm[2], fac, F.nvert, apply, ratio, terms, area, ctx->uc_dev, ctx->ubcs_dev,
                           ctx->ucat_dev, ctx->bc_host, ctx->stream);
       CKL();
       if (terms) CK(cudaEventRecord(ctx->bc_ev, ctx->stream));
       return CVB_OK;
     };
     TRY(plane(false, 0., true, !bs.have_area));
-    launch_contra2cart(g, csi, eta, zet, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1, g.mz - 3, fac);
+    launch_contra2cart(g, fac, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1, g.mz - 3);
     for (int pass = 0; pass < 3; pass++) {
       CK(cudaEventSynchronize(ctx->bc_ev));
       const double flux_out = ordered_sum(ctx->bc_host, n2);
@@ -2077,7 +2079,7 @@ static int form_bcs_dev(cvb_ctx *ctx, double flux_intp_sum, BcSums &bs) {
       TRY(plane(true, (flux_in - flux_out) / bs.area, pass < 2, false));
     }
   } else {
-    launch_contra2cart(g, csi, eta, zet, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream, 1, -1, fac);
+    launch_contra2cart(g, fac, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   }
   launch_form_ring(g, ctx->ubcs_dev, ctx->ucat_dev, ctx->p_dev, ctx->stream);
   CKL();
@@ -2181,7 +2183,6 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   TRY(post_buffers(ctx, n));
   if (!ctx->conv_dev) TRY(dalloc(ctx, &ctx->conv_dev, n3));
   if (!ctx->conv_fp) TRY(dalloc(ctx, &ctx->conv_fp, 9 * n));
-  if (!ctx->visc_dev) TRY(dalloc(ctx, &ctx->visc_dev, n3));
   if (!ctx->rct_dev) TRY(dalloc(ctx, &ctx->rct_dev, n3));
   if (!ctx->rhs_dev) TRY(dalloc(ctx, &ctx->rhs_dev, n3));
   if (!ctx->uo_dev) TRY(dalloc(ctx, &ctx->uo_dev, n3));
@@ -2205,11 +2206,8 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   CK(cudaMemsetAsync(ctx->rhs_dev, 0, sizeof(double) * n3, ctx->stream));
   const int bdf2 = (ti != tistart && ti != 1) ? 1 : 0;  // COEF_TIME_ACCURACY 1.5 (variables.h:421)
   const int mz_end = F.g.mz - 3;                        // no convective outflow on an all-wall box
-  auto calc_rhs = [&]() {
-    momentum_ff1(ctx, ren, central, false);
-    launch_calc_rhs(F.g, F.nvert, ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end, ctx->rhs_dev,
-                    ctx->stream);
-  };
+  const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end};
+  auto calc_rhs = [&]() { momentum_ff1(ctx, ren, central, &calc, false); };
   // before the loop (implicitsolver.c:7124-7148): the boundary conditions,
   // pUcont = Ucont, CalcRHS
   if (inlet) TRY(inflow_dev(ctx, uin, bs));
@@ -2726,8 +2724,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
       case CVB_KERNEL_RESIDUAL_F64: launch_residual<double>(L, L.r64, L.e64, L.t64, ctx->stream); break;
       case CVB_KERNEL_ZEBRA_F32: launch_zebra_half<float>(L, L.r32, L.e32, L.t32 + n, 1.3f, 1, false, ctx->stream); break;
       case CVB_KERNEL_CONTRA2CART:
-        launch_contra2cart(L.g, ctx->cm[0], ctx->cm[1], ctx->cm[2], L.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream,
-                           1, -1, ctx->geo->c2c);
+        launch_contra2cart(L.g, c2c_factors(ctx), L.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
         break;
       case CVB_KERNEL_GHOST_NODES:
         launch_ghost_node_velocity(L.g, ctx->H[level].d.bctype, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev,
@@ -2743,11 +2740,11 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
                        ctx->geo->gram, ctx->geo->gram_tame, 1. / 300., ctx->conv_fp, ctx->visc_dev, ctx->stream);
         break;
       }
-      case CVB_KERNEL_MOMENTUM_RHS:
-        momentum_ff1(ctx, 300., 0);
-        launch_calc_rhs(L.g, L.nvert, ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, 1, -1. / 2e-3, L.g.mz - 3, ctx->rhs_dev,
-                        ctx->stream);
+      case CVB_KERNEL_MOMENTUM_RHS: {
+        const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, 1, -1. / 2e-3, L.g.mz - 3};
+        momentum_ff1(ctx, 300., 0, &calc);
         break;
+      }
       default: launch_zebra_half<double>(L, L.r64, L.e64, L.t64 + n, 1.3, 1, false, ctx->stream); break;
     }
   };

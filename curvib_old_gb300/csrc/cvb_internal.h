@@ -288,13 +288,16 @@ struct IbmWork {
 // The search; tmp is one more [mz][my][mx] array.  The result is left in tmp.
 void launch_ibm_search(const IbmArgs &A, const IbmWork &W, double *tmp, cudaStream_t s);
 
-// fac: the grid's Contra2Cart factors (launch_c2c_factors, 10 N doubles), or
-// null to form them in the kernel
-void launch_contra2cart(const Geom &g, const double *csi, const double *eta, const double *zet,
-                        const double *nvert, const double *ucont, double *ucat, cudaStream_t s, int k0 = 1,
-                        int nk = -1, const double *fac = nullptr);
+// The grid's Contra2Cart factors (launch_c2c_factors, 11 N doubles) and whether
+// all of them are in intmul.cuh's range
+struct C2cFactors {
+  const double *fac;
+  bool tame;
+};
+void launch_contra2cart(const Geom &g, const C2cFactors &F, const double *nvert, const double *ucont, double *ucat,
+                        cudaStream_t s, int k0 = 1, int nk = -1);
 void launch_c2c_factors(const Geom &g, const double *csi, const double *eta, const double *zet, double *fac,
-                        cudaStream_t s);
+                        int *wild, cudaStream_t s);
 // max |div| and its first box index into out_v / out_i (device); pv / pi
 // hold 1024 partial pairs
 void launch_divergence(const Geom &g, const double *ucont, const double *aj, const double *nvert, double *pv,
@@ -313,12 +316,18 @@ void launch_face_gram(const Geom &g, const double *const *fm, const double *iaj,
 void launch_viscous(const Geom &g, const double *nvert, const double *ucat, const double *const *fm,
                     const double *iaj, const double *jaj, const double *kaj, const double *gram, bool tame, double nu,
                     double *fp, double *visc, cudaStream_t s);
+// CalcRHS's time term, on top of FormFunction1
+struct MomentumTime {
+  const double *ucont, *ucont_o, *ucont_rm1;
+  int bdf2;
+  double neg_inv_dt;
+  int mz_end;
+};
 void launch_form_function1(const Geom &g, const double *nvert, const double *p, const double *conv,
-                           const double *visc, const double *csi, const double *eta, const double *zet,
+                           const double *fp, const double *csi, const double *eta, const double *zet,
                            const double *aj, const double *const *fm, const double *iaj, const double *jaj,
-                           const double *kaj, const double *gram, double *rct, double *rhs, cudaStream_t s);
-void launch_calc_rhs(const Geom &g, const double *nvert, const double *ucont, const double *ucont_o,
-                     const double *ucont_rm1, int bdf2, double neg_inv_dt, int mz_end, double *rhs, cudaStream_t s);
+                           const double *kaj, const double *gram, bool tame, const MomentumTime *calc, double *rct,
+                           double *rhs, cudaStream_t s);
 // bc: the level's bctype[6]; the host has refused the types it does not cover.
 // cent: the cell centres ([N][3]) an annulus face needs; u_bc: the rheology
 // plates' velocity
@@ -332,9 +341,9 @@ void launch_form_ring(const Geom &g, const double *ubcs, double *ucat, double *p
 // the flux correction by ratio and Contra2Cart of the plane; with want_terms
 // (always without apply) its flux terms in the reference's loop order into
 // terms[0 .. n2), with want_area the area terms into terms[n2 .. 2 n2)
-void launch_outlet_plane(const Geom &g, const double *csi, const double *eta, const double *zet, const double *fac,
-                         const double *nvert, bool apply, double ratio, bool want_terms, bool want_area,
-                         double *ucont, double *ubcs, double *ucat, double *terms, cudaStream_t s);
+void launch_outlet_plane(const Geom &g, const double *zet, const C2cFactors &F, const double *nvert, bool apply,
+                         double ratio, bool want_terms, bool want_area, double *ucont, double *ubcs, double *ucat,
+                         double *terms, cudaStream_t s);
 // InflowFlux on an inlet k = 0 face with a constant speed uin: ubcs and
 // Ucont.z there, and the face's flux terms in the reference's loop order into
 // terms ((mx - 2)(my - 2) doubles) for the host to add

@@ -50,6 +50,14 @@ __device__ __forceinline__ IntMulB int_split_b(double x) {
   return {l << 6, __funnelshift_l(l, m, 6), h & 0xfff00000u};
 }
 
+__device__ __forceinline__ IntMulB int_split_b(double x, bool &out_of_range) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x);
+  const bool zero = ((h & 0x7fffffffu) | l) == 0;
+  out_of_range = out_of_range || (!zero && !int_mul_in_range(h));
+  const unsigned m = zero ? 0u : (h & 0xfffffu) | 0x100000u;
+  return {l << 6, __funnelshift_l(l, m, 6), h & 0xfff00000u};
+}
+
 // a * b rounded to nearest even.  The shifted significands A < 2^58, B < 2^59
 // give A B = S_a S_b 2^11 in [2^115, 2^117): bits 64 .. 116 are the 53-bit
 // significand of the result (one bit short where the product of the
@@ -77,6 +85,41 @@ __device__ __forceinline__ double int_mul(const IntMulA &a, const IntMulB &b) {
   // where the product was 2 or above) and the signs with them, modulo 2^32
   const unsigned se = hi + a.se + b.se + (top - (1024u << 20));
   return __hiloint2double(hi ? se : (a.se ^ b.se) & 0x80000000u, lo);
+}
+
+// 3 x rounded to nearest even: three times the significand has one or two bits
+// too many.  Other than normal numbers with a normal result and zeros go
+// through the multiply, out of line.
+static __device__ __noinline__ double triple_slow(double x) { return __dmul_rn(3., x); }
+__device__ __forceinline__ double int_triple(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e - 1u >= 2044u) return (b << 1) == 0 ? x : triple_slow(x);
+  const unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL, t = 3 * m;
+  const int s = t >> 54 ? 2 : 1;
+  const unsigned long long r = (t + (s - 1) + ((t >> s) & 1)) >> s;
+  return __longlong_as_double((long long)((b & 0x8000000000000000ULL) + r + ((unsigned long long)(e + s - 1) << 52)));
+}
+
+// x / y rounded to nearest even for a divisor used many times, from rcp = 1 / y
+// rounded to nearest: x rcp, then twice the residual x - y q added back through
+// rcp.  The residual of a quotient within an ulp is exact in one fused
+// multiply-add, and a quotient within an ulp so corrected with a correctly
+// rounded reciprocal is the correctly rounded one (P. W. Markstein,
+// "Computation of elementary functions on the IBM RISC System/6000 processor",
+// IBM J. Res. Dev. 34, 1990); x rcp itself may be off by more than an ulp, the
+// first correction makes it so.  Five FP64 operations.  For y and rcp within
+// int_mul's range and |x| within 2^-400 .. 2^400 (nothing over- or underflows
+// on the way), or x zero; other x take the division, out of line.
+static __device__ __noinline__ double quot_slow(double x, double y) { return __ddiv_rn(x, y); }
+__device__ __forceinline__ double quot_known(double x, double y, double rcp) {
+  const unsigned h = (unsigned)__double2hiint(x) & 0x7fffffffu;
+  if ((h | (unsigned)__double2loint(x)) == 0)
+    return __hiloint2double((__double2hiint(x) ^ __double2hiint(y)) & 0x80000000, 0);
+  if (h - (623u << 20) >= (800u << 20)) return quot_slow(x, y);
+  double q = __dmul_rn(x, rcp);
+  q = __fma_rn(__fma_rn(-y, q, x), rcp, q);
+  return __fma_rn(__fma_rn(-y, q, x), rcp, q);
 }
 
 }  // namespace cvb

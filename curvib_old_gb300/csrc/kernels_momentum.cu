@@ -47,12 +47,15 @@ __device__ __forceinline__ bool lt_01(double v) {
 // the result stays normal: K less in the exponent field; a zero stays itself;
 // subnormal results, inf and NaN go through the multiply, out of line.
 __device__ __noinline__ double scale_slow(double x, double f) { return x * f; }
-template <int K>
-__device__ __forceinline__ double scale_down(double x) {
+__device__ __forceinline__ double scale_down(double x, int K) {
   const long long b = __double_as_longlong(x), e = (b >> 52) & 0x7ff;
   if (e > K && e < 0x7ff) return __longlong_as_double(b - ((long long)K << 52));
   if ((b & 0x7fffffffffffffffLL) == 0) return x;
   return scale_slow(x, K == 1 ? 0.5 : 0.25);
+}
+template <int K>
+__device__ __forceinline__ double scale_down(double x) {
+  return scale_down(x, K);
 }
 
 struct FaceMetrics {
@@ -80,12 +83,13 @@ __device__ __forceinline__ void visc_differences(const long (&st)[3], int d, lon
     const long s = st[t];
     const bool up = visc_blocked(nv[P + s]) || visc_blocked(nv[P + sd + s]);
     const bool dn = visc_blocked(nv[P - s]) || visc_blocked(nv[P + sd - s]);
+    // one expression for the three forms, on the cells each takes
+    const long h = up ? 0 : s, l = !up && dn ? 0 : -s;
+    const int half = up || dn;
 #pragma unroll
     for (int c = 0; c < 3; c++) {
 #define U(off) ucat[3 * (P + (off)) + c]
-      if (up) D[t][c] = scale_down<1>(U(sd) + U(0) - U(sd - s) - U(-s));
-      else if (dn) D[t][c] = scale_down<1>(U(sd + s) + U(s) - U(sd) - U(0));
-      else D[t][c] = scale_down<2>(U(sd + s) + U(s) - U(sd - s) - U(-s));
+      D[t][c] = scale_down(U(sd + h) + U(h) - U(sd + l) - U(l), half ? 1 : 2);
 #undef U
     }
   }
@@ -186,19 +190,22 @@ __global__ void __launch_bounds__(128, 4) k_visc_faces(Geom g, const double *__r
   }
 }
 
-// visc = the flux differences over each interior cell (rhs.c:2490-2511); 0 on
-// the ring (the reference's VecSet before the loops).
+// Component c of visc at interior cell e: the flux differences over the cell
+// (rhs.c:2490-2511).
+__device__ __forceinline__ double visc_cell(const Geom &g, const double *__restrict__ fp, size_t e, int c) {
+  const size_t n = g.n(), w = e - 1, s = e - g.mx, b = e - (size_t)g.mx * g.my;
+  return fp[(size_t)c * n + e] - fp[(size_t)c * n + w] + fp[(size_t)(3 + c) * n + e] - fp[(size_t)(3 + c) * n + s] +
+         fp[(size_t)(6 + c) * n + e] - fp[(size_t)(6 + c) * n + b];
+}
+
+// visc, 0 on the ring (the reference's VecSet before the loops).
 __global__ void k_visc_div(Geom g, const double *__restrict__ fp, double *__restrict__ visc) {
   dep_sync();
   const size_t n = g.n();
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
     const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
     const bool in = i >= 1 && i <= g.mx - 2 && j >= 1 && j <= g.my - 2 && k >= 1 && k <= g.mz - 2;
-    const size_t w = e - 1, s = e - g.mx, b = e - (size_t)g.mx * g.my;
-    for (int c = 0; c < 3; c++)
-      visc[3 * e + c] = in ? (fp[(size_t)c * n + e] - fp[(size_t)c * n + w] + fp[(size_t)(3 + c) * n + e] -
-                              fp[(size_t)(3 + c) * n + s] + fp[(size_t)(6 + c) * n + e] - fp[(size_t)(6 + c) * n + b])
-                           : 0.0;
+    for (int c = 0; c < 3; c++) visc[3 * e + c] = in ? visc_cell(g, fp, e, c) : 0.0;
   }
 }
 
@@ -245,7 +252,13 @@ void launch_face_gram(const Geom &g, const double *const *fm, const double *iaj,
   k_face_gram<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, M, gram, wild); count_launch();
 }
 
-// tame: the grid's metrics are all in intmul.cuh's range (k_face_gram).
+// Whether v can be a right operand of int_mul.
+static bool int_mul_factor(double v) {
+  return std::fabs(v) >= std::ldexp(1., -510) && std::fabs(v) < std::ldexp(1., 511);
+}
+
+// tame: the grid's metrics are all in intmul.cuh's range (k_face_gram).  visc
+// null: the face fluxes fp alone.
 void launch_viscous(const Geom &g, const double *nvert, const double *ucat, const double *const *fm,
                     const double *iaj, const double *jaj, const double *kaj, const double *gram, bool tame, double nu,
                     double *fp, double *visc, cudaStream_t s) {
@@ -254,195 +267,266 @@ void launch_viscous(const Geom &g, const double *nvert, const double *ucat, cons
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
   const unsigned nb = blocks_for(g.n(), 128);
-  const bool nu_tame = std::fabs(nu) >= std::ldexp(1., -510) && std::fabs(nu) < std::ldexp(1., 511);
-  if (tame && nu_tame) launch_dep(k_visc_faces<true>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
+  if (tame && int_mul_factor(nu)) launch_dep(k_visc_faces<true>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
   else launch_dep(k_visc_faces<false>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
-  launch_dep(k_visc_div, blocks_for(g.n(), 256), 256, 0, s, g, (const double *)fp, visc);
+  if (visc) launch_dep(k_visc_div, blocks_for(g.n(), 256), 256, 0, s, g, (const double *)fp, visc);
 }
 
 // ------------------------------------------------------------- FormFunction1
 // rct: the contravariant form of rc = visc - conv at the cell centres
-// (rhs.c:2682-2700), interior cells; the ring stays 0 (a new vector).
-__global__ void k_ff1_rct(Geom g, const double *__restrict__ conv, const double *__restrict__ visc,
-                          const double *__restrict__ csi, const double *__restrict__ eta,
-                          const double *__restrict__ zet, const double *__restrict__ aj, double *__restrict__ rct) {
+// (rhs.c:2682-2700), interior cells; the ring stays 0 (a new vector).  visc is
+// formed here from Viscous's face fluxes fp (k_visc_div's differences), so it
+// is not written and read back.  Bound by the FP64 pipe: 33 sums a cell, the
+// 12 products on the integer pipe (INT).  At 192^3 0.49 ms, with k_visc_div
+// and FP64 products 0.66 ms.
+template <bool INT>
+__device__ __forceinline__ void rct_cell(const Geom &g, const double (&rc)[3], const double *__restrict__ csi,
+                                         const double *__restrict__ eta, const double *__restrict__ zet, double a,
+                                         long P, bool &fp64, double (&out)[3]) {
+  const long st[3] = {1, g.mx, (long)g.mx * g.my};
+  const double *m[3] = {csi, eta, zet};
+  IntMulA Rc[3];
+  if constexpr (INT)
+    for (int c = 0; c < 3; c++) Rc[c] = int_split_a(rc[c], fp64);
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    double mean[3];
+#pragma unroll
+    for (int c = 0; c < 3; c++) mean[c] = scale_down<1>(m[d][3 * P + c] + m[d][3 * (P - st[d]) + c]);
+    if constexpr (INT) {
+      const double s = int_mul(Rc[0], int_split_b(mean[0], fp64)) + int_mul(Rc[1], int_split_b(mean[1], fp64)) +
+                       int_mul(Rc[2], int_split_b(mean[2], fp64));
+      out[d] = int_mul(int_split_a(s, fp64), int_split_b(a, fp64));
+    } else {
+      out[d] = a * (mean[0] * rc[0] + mean[1] * rc[1] + mean[2] * rc[2]);
+    }
+  }
+}
+__device__ __noinline__ void rct_cell_fp64(const Geom &g, const double (&rc)[3], const double *__restrict__ csi,
+                                           const double *__restrict__ eta, const double *__restrict__ zet, double a,
+                                           long P, double (&out)[3]) {
+  bool unused = false;
+  rct_cell<false>(g, rc, csi, eta, zet, a, P, unused, out);
+}
+
+__global__ void __launch_bounds__(128) k_ff1_rct(const __grid_constant__ Geom g, const double *__restrict__ conv,
+                                                 const double *__restrict__ fp, const double *__restrict__ csi,
+                                                 const double *__restrict__ eta, const double *__restrict__ zet,
+                                                 const double *__restrict__ aj, double *__restrict__ rct) {
   dep_sync();
   const size_t n = g.n();
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
-    if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) {
-      rct[3 * e] = rct[3 * e + 1] = rct[3 * e + 2] = 0.0;
-      continue;
-    }
-    const long P = (long)e, sx = 1, sy = g.mx, sz = (long)g.mx * g.my;
+  const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
+  double out[3] = {0., 0., 0.};
+  if (i >= 1 && i <= g.mx - 2 && j >= 1 && j <= g.my - 2 && k >= 1 && k <= g.mz - 2) {
     double rc[3];
-    for (int c = 0; c < 3; c++) rc[c] = -1.0 * conv[3 * P + c] + visc[3 * P + c];
-    const double a = aj[P];
-    rct[3 * P + 0] = a * (scale_down<1>(csi[3 * P] + csi[3 * (P - sx)]) * rc[0] +
-                          scale_down<1>(csi[3 * P + 1] + csi[3 * (P - sx) + 1]) * rc[1] +
-                          scale_down<1>(csi[3 * P + 2] + csi[3 * (P - sx) + 2]) * rc[2]);
-    rct[3 * P + 1] = a * (scale_down<1>(eta[3 * P] + eta[3 * (P - sy)]) * rc[0] +
-                          scale_down<1>(eta[3 * P + 1] + eta[3 * (P - sy) + 1]) * rc[1] +
-                          scale_down<1>(eta[3 * P + 2] + eta[3 * (P - sy) + 2]) * rc[2]);
-    rct[3 * P + 2] = a * (scale_down<1>(zet[3 * P] + zet[3 * (P - sz)]) * rc[0] +
-                          scale_down<1>(zet[3 * P + 1] + zet[3 * (P - sz) + 1]) * rc[1] +
-                          scale_down<1>(zet[3 * P + 2] + zet[3 * (P - sz) + 2]) * rc[2]);
+#pragma unroll
+    for (int c = 0; c < 3; c++) rc[c] = -1.0 * conv[3 * e + c] + visc_cell(g, fp, e, c);
+    const double a = aj[e];
+    bool fp64 = false;
+    rct_cell<true>(g, rc, csi, eta, zet, a, (long)e, fp64, out);
+    if (fp64) rct_cell_fp64(g, rc, csi, eta, zet, a, (long)e, out);
   }
+#pragma unroll
+  for (int c = 0; c < 3; c++) rct[3 * e + c] = out[c];
 }
 
 namespace {
+
+// The sum of two nvert values (finite, >= 0): nearly all are +0, whose sum
+// needs no FP64 add.
+__device__ __noinline__ double nv_sum_slow(double a, double b) { return a + b; }
+__device__ __forceinline__ double nv_sum(double a, double b) {
+  if ((__double_as_longlong(a) | __double_as_longlong(b)) == 0) return 0.;
+  return nv_sum_slow(a, b);
+}
 
 // One tangential pressure derivative of face d of cell P (rhs.c:2803-2849 and
 // its siblings, walled boxes); false where the reference assigns nothing.
 __device__ __forceinline__ bool ff_dp(const double *__restrict__ nv, const double *__restrict__ p, long P, long sd,
                                       long s, int q, int m, double &val) {
-  const double up = nv[P + s] + nv[P + sd + s], dn = nv[P - s] + nv[P + sd - s];
-  if (q == m - 2 || gt_01(up)) {
-    if (lt_01(dn) && q != 1) {
-      val = scale_down<1>(p[P] + p[P + sd] - p[P - s] - p[P + sd - s]);
-      return true;
-    }
-    return false;
-  }
-  if (q == 1 || gt_01(dn)) {
-    if (lt_01(up)) {
-      val = scale_down<1>(p[P + s] + p[P + sd + s] - p[P] - p[P + sd]);
-      return true;
-    }
-    return false;
-  }
-  val = scale_down<2>(p[P + s] + p[P + sd + s] - p[P - s] - p[P + sd - s]);
+  const double up = nv_sum(nv[P + s], nv[P + sd + s]), dn = nv_sum(nv[P - s], nv[P + sd - s]);
+  // upper (the cells above are blocked or beyond the wall), lower, or central:
+  // one expression on the cells each takes
+  const bool upper = q == m - 2 || gt_01(up), lower = !upper && (q == 1 || gt_01(dn));
+  if (upper ? !(lt_01(dn) && q != 1) : lower && !lt_01(up)) return false;
+  const long h = upper ? 0 : s, l = lower ? 0 : -s;
+  val = scale_down(p[P + h] + p[P + sd + h] - p[P + l] - p[P + sd + l], upper || lower ? 1 : 2);
   return true;
 }
 
+// What the cell before (i, j, k) in the reference's loop order leaves in its
+// derivative variables dpde, dpdz: its z-section's (dpde from its branch, else
+// its y section's p[j+1] - p[j]); 0 before the first cell.  Its final dpdc is
+// assigned again by the next cell's x section before any use.
+__device__ __noinline__ void ff_previous(const Geom &g, const double *__restrict__ nv, const double *__restrict__ p,
+                                         int i, int j, int k, double &de, double &dz) {
+  de = dz = 0.0;
+  i--;
+  if (i < 1) { i = g.mx - 2; j--; }
+  if (j < 1) { j = g.my - 2; k--; }
+  if (k < 1) return;
+  const long sy = g.mx, sz = (long)g.mx * g.my, Q = ((long)k * g.my + j) * g.mx + i;
+  if (!ff_dp(nv, p, Q, sz, sy, j, g.my, de)) de = p[Q + sy] - p[Q];
+  dz = p[Q + sz] - p[Q];
+}
+
+// The pressure gradient through a face, (dp . gram) aj, with FP64 multiplies.
+__device__ __noinline__ double ff_gradient_fp64(double d0, double d1, double d2, const double *__restrict__ gr,
+                                                size_t n, double aj) {
+  return (d0 * gr[0] + d1 * gr[n] + d2 * gr[2 * n]) * aj;
+}
+// ... and the time term: 1.5 u - 2 u_o + 0.5 u_rm1 or u - u_o, times a, on
+// top of r.
+__device__ __noinline__ double ff_time_fp64(double r, double u, double uo, double urm, int bdf2, double a) {
+  double du;
+  if (bdf2) {
+    du = u;
+    du *= 1.5;
+    du += -2. * uo;
+    du += 0.5 * urm;
+  } else {
+    du = -1. * uo + u;
+  }
+  r += a * du;
+  return r;
+}
+
 }  // namespace
+
+// CalcRHS's part of k_ff1_faces.
+struct CalcRhsArgs {
+  const double *uc, *uo, *urm;  // Ucont, Ucont_o, Ucont_rm1
+  int bdf2;
+  double a;    // -1 / dt
+  int mz_end;  // mz - 3, or mz - 2 with a convective outflow (bctype[5] 8)
+};
 
 // The face values of FormFunction1 (rhs.c:2760-3222) and its blocked-face masks
 // (rhs.c:3225-3262) on the interior cells.  The reference keeps the three
 // derivative variables across its loop: where a branch assigns nothing the
 // value of the previous assignment stands.  Within a cell that is the previous
 // section's value; entering a cell it is what the previous cell in loop order
-// (k, j, i ascending over the interior) left -- its z-section pressure
-// derivatives, where its own branch or, failing that, its y-section assigned
-// dpde, and its dpdz = p[k+1] - p[k] -- and 0 before the first cell.
-__global__ void k_ff1_faces(Geom g, const double *__restrict__ nv, const double *__restrict__ p,
-                            const double *__restrict__ rct, FaceMetrics M, const double *__restrict__ gram,
-                            double *__restrict__ rhs) {
+// (k, j, i ascending over the interior) left (ff_previous).
+//
+// CALC: then CalcRHS (implicitsolver.c:6519-6713) in the same pass: rhs -= dU /
+// dt over every entry of the box (second-order backward dU = 1.5 u - 2 u_o +
+// 0.5 u_rm1, or u - u_o on the first step), the faces next to blocked cells
+// and the walls zeroed, the convective-outflow term on the last k face
+// (bctype[5] 8), then the reference's six boundary loops, which zero the ring
+// except on the box's last row in each direction.
+//
+// Bound by the FP64 pipe: 42 sums a cell; the 15 products go to the integer
+// pipe (INT: intmul.cuh; gram and the Jacobians in its range), the sums of
+// nvert and the previous cell's values are formed only where they are needed,
+// and the one-sided differences beside walls share the central ones' expression
+// (a warp of a row's end ran both).  At 192^3 0.74 ms with CalcRHS, in two
+// kernels with FP64 products 1.25 ms.  Eight blocks per SM (64 registers): six
+// 0.88 ms, seven 0.79 ms.
+template <bool INT, bool CALC>
+__global__ void __launch_bounds__(128, 8) k_ff1_faces(const __grid_constant__ Geom g, const double *__restrict__ nv,
+                                                   const double *__restrict__ p, const double *__restrict__ rct,
+                                                   const __grid_constant__ FaceMetrics M,
+                                                   const double *__restrict__ gram, CalcRhsArgs A,
+                                                   double *__restrict__ rhs) {
   dep_sync();
   const size_t n = g.n();
-  const long st[3] = {1, g.mx, (long)g.mx * g.my};
-  const int m[3] = {g.mx, g.my, g.mz};
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
-    if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) continue;
-    const long P = (long)e;
-    // the previous cell's end values
-    double dp[3] = {0.0, 0.0, 0.0};
-    {
-      int pi = i - 1, pj = j, pk = k;
-      if (pi < 1) { pi = g.mx - 2; pj = j - 1; }
-      if (pj < 1) { pj = g.my - 2; pk = k - 1; }
-      if (pk >= 1) {
-        const long Q = ((long)pk * g.my + pj) * g.mx + pi;
-        const int qq[3] = {pi, pj, pk};
-        // its z section: dpde from the branch, else its y section's p[j+1] - p[j]
-        double de;
-        if (!ff_dp(nv, p, Q, st[2], st[1], qq[1], m[1], de)) de = p[Q + st[1]] - p[Q];
-        dp[1] = de;
-        dp[2] = p[Q + st[2]] - p[Q];
-        // its final dpdc (the z section's branch, else the y section's, else
-        // its x section's p[i+1] - p[i]) is assigned again by this cell's x
-        // section before any use
-      }
-    }
-    const int q[3] = {i, j, k};
-    double out[3];
-    for (int d = 0; d < 3; d++) {
+  const int mx = g.mx, my = g.my, mz = g.mz;
+  const long st[3] = {1, mx, (long)mx * my};
+  const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (e >= n) return;
+  const int i = (int)(e % mx), j = (int)((e / mx) % my), k = (int)(e / ((size_t)mx * my));
+  const bool in = i >= 1 && i <= mx - 2 && j >= 1 && j <= my - 2 && k >= 1 && k <= mz - 2;
+  if (!CALC && !in) return;
+  const long P = (long)e;
+  const bool solid = in && gt_01(nv[P]);
+  double dp[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+  for (int d = 0; d < 3; d++) {
+    const long sd = d == 0 ? st[0] : d == 1 ? st[1] : st[2];
+    double v = 0.;
+    if (in) {
+#pragma unroll
       for (int t = 0; t < 3; t++) {
-        if (t == d) dp[t] = p[P + st[d]] - p[P];
-        else ff_dp(nv, p, P, st[d], st[t], q[t], m[t], dp[t]);
+        if (t == d) {
+          dp[t] = p[P + sd] - p[P];
+        } else if (!ff_dp(nv, p, P, sd, st[t], t == 0 ? i : t == 1 ? j : k, t == 0 ? mx : t == 1 ? my : mz, dp[t]) &&
+                   d == 0) {
+          double de, dz;
+          ff_previous(g, nv, p, i, j, k, de, dz);
+          dp[t] = t == 1 ? de : dz;
+        }
       }
       // (csi . nd, eta . nd, zet . nd) of face d, from k_face_gram
       const double *gr = gram + (size_t)(3 * d) * n + P;
-      double v = scale_down<1>(rct[3 * P + d] + rct[3 * (P + st[d]) + d]);
-      v -= (dp[0] * gr[0] + dp[1] * gr[n] + dp[2] * gr[2 * n]) * M.aj[d][P];
-      out[d] = v;
+      v = scale_down<1>(rct[3 * P + d] + rct[3 * (P + sd) + d]);
+      bool fp64 = !INT;
+      double gradient = 0.;
+      if constexpr (INT) {
+        const double s = int_mul(int_split_a(dp[0], fp64), int_split_b(gr[0])) +
+                         int_mul(int_split_a(dp[1], fp64), int_split_b(gr[n])) +
+                         int_mul(int_split_a(dp[2], fp64), int_split_b(gr[2 * n]));
+        gradient = int_mul(int_split_a(s, fp64), int_split_b(M.aj[d][P]));
+      }
+      if (fp64) gradient = ff_gradient_fp64(dp[0], dp[1], dp[2], gr, n, M.aj[d][P]);
+      v -= gradient;
+      if (solid || gt_01(nv[P + sd])) v = 0;
     }
-    if (gt_01(nv[P])) out[0] = out[1] = out[2] = 0;
-    if (gt_01(nv[P + st[0]])) out[0] = 0;
-    if (gt_01(nv[P + st[1]])) out[1] = 0;
-    if (gt_01(nv[P + st[2]])) out[2] = 0;
-    for (int c = 0; c < 3; c++) rhs[3 * P + c] = out[c];
+    const size_t q = 3 * e + d;
+    if constexpr (CALC) {
+      if (!in) v = rhs[q];
+      const double u = A.uc[q], uo = A.uo[q], urm = A.bdf2 ? A.urm[q] : 0.;
+      bool fp64 = !INT;
+      double r = v;
+      if constexpr (INT) {
+        double du;
+        if (A.bdf2) {
+          du = int_mul(int_split_a(u, fp64), int_split_b(1.5));
+          du += int_mul(int_split_a(uo, fp64), int_split_b(-2.));
+          du += scale_down<1>(urm);
+        } else {
+          du = -1. * uo + u;
+        }
+        r += int_mul(int_split_a(du, fp64), int_split_b(A.a));
+      }
+      if (fp64) r = ff_time_fp64(v, u, uo, urm, A.bdf2, A.a);
+      if (in) {
+        const int lim = d == 0 ? i - (mx - 3) : d == 1 ? j - (my - 3) : k - A.mz_end;
+        if (lim > 0 || gt_01(nv_sum(nv[P], nv[P + sd]))) r = 0.;
+        if (d == 2 && A.mz_end == mz - 2 && k == mz - 2) r += 0.8 * (u - A.uc[3 * (P - st[2]) + 2]);
+      }
+      // the six boundary loops (each covers its face minus the last row of the
+      // other two directions)
+      const bool kin = k < mz - 1, jin = j < my - 1, iin = i < mx - 1;
+      const bool all = ((i == 0 || i == mx - 1) && kin && jin) || ((j == 0 || j == my - 1) && kin && iin) ||
+                       ((k == 0 || k == mz - 1) && jin && iin);
+      const bool own = d == 0 ? i == mx - 2 && kin && jin : d == 1 ? j == my - 2 && kin && iin : k == mz - 2 && jin && iin;
+      v = all || own ? 0. : r;
+    }
+    rhs[q] = v;
   }
 }
 
+// FormFunction1 after its Contra2Cart, Convection (conv) and Viscous (fp, its
+// face fluxes); with calc, CalcRHS's part on top.
 void launch_form_function1(const Geom &g, const double *nvert, const double *p, const double *conv,
-                           const double *visc, const double *csi, const double *eta, const double *zet,
+                           const double *fp, const double *csi, const double *eta, const double *zet,
                            const double *aj, const double *const *fm, const double *iaj, const double *jaj,
-                           const double *kaj, const double *gram, double *rct, double *rhs, cudaStream_t s) {
+                           const double *kaj, const double *gram, bool tame, const MomentumTime *calc, double *rct,
+                           double *rhs, cudaStream_t s) {
   FaceMetrics M;
   for (int d = 0; d < 3; d++)
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
-  launch_dep(k_ff1_rct, blocks_for(g.n(), 256), 256, 0, s, g, conv, visc, csi, eta, zet, aj, rct);
-  launch_dep(k_ff1_faces, blocks_for(g.n(), 128), 128, 0, s, g, nvert, p, (const double *)rct, M, gram, rhs);
-}
-
-// ------------------------------------------------------------------ CalcRHS
-// After FormFunction1: rhs -= dU / dt over every entry (second-order backward
-// dU = 1.5 u - 2 u_o + 0.5 u_rm1, or u - u_o on the first step), the faces
-// next to blocked cells and the walls zeroed, the convective-outflow term on
-// the last k face (bctype[5] 8), then the reference's six boundary loops,
-// which zero the ring except on the box's last row in each direction
-// (implicitsolver.c:6519-6713).
-__global__ void k_calc_rhs(Geom g, const double *__restrict__ nv, const double *__restrict__ uc,
-                           const double *__restrict__ uo, const double *__restrict__ urm, int bdf2, double a,
-                           int mz_end, double *__restrict__ rhs) {
-  dep_sync();
-  const size_t n = g.n();
-  const int mx = g.mx, my = g.my, mz = g.mz;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const int i = (int)(e % mx), j = (int)((e / mx) % my), k = (int)(e / ((size_t)mx * my));
-    double r[3];
-    for (int c = 0; c < 3; c++) {
-      const size_t q = 3 * e + c;
-      double du;
-      if (bdf2) {
-        du = uc[q];
-        du *= 1.5;
-        du += -2. * uo[q];
-        du += scale_down<1>(urm[q]);
-      } else {
-        du = -1. * uo[q] + uc[q];
-      }
-      r[c] = rhs[q];
-      r[c] += a * du;
-    }
-    const bool in = i >= 1 && i <= mx - 2 && j >= 1 && j <= my - 2 && k >= 1 && k <= mz - 2;
-    if (in) {
-      const size_t sx = 1, sy = mx, sz = (size_t)mx * my;
-      if (gt_01(nv[e] + nv[e + sx]) || i > mx - 3) r[0] = 0.;
-      if (gt_01(nv[e] + nv[e + sy]) || j > my - 3) r[1] = 0.;
-      if (gt_01(nv[e] + nv[e + sz]) || k > mz_end) r[2] = 0.;
-      if (mz_end == mz - 2 && k == mz - 2) r[2] += 0.8 * (uc[3 * e + 2] - uc[3 * (e - sz) + 2]);
-    }
-    // the six boundary loops (each covers its face minus the last row of the
-    // other two directions)
-    const bool kin = k < mz - 1, jin = j < my - 1, iin = i < mx - 1;
-    const bool all = ((i == 0 || i == mx - 1) && kin && jin) || ((j == 0 || j == my - 1) && kin && iin) ||
-                     ((k == 0 || k == mz - 1) && jin && iin);
-    if (all) r[0] = r[1] = r[2] = 0;
-    if (i == mx - 2 && kin && jin) r[0] = 0;
-    if (j == my - 2 && kin && iin) r[1] = 0;
-    if (k == mz - 2 && jin && iin) r[2] = 0;
-    for (int c = 0; c < 3; c++) rhs[3 * e + c] = r[c];
-  }
-}
-
-void launch_calc_rhs(const Geom &g, const double *nvert, const double *ucont, const double *ucont_o,
-                     const double *ucont_rm1, int bdf2, double neg_inv_dt, int mz_end, double *rhs, cudaStream_t s) {
-  launch_dep(k_calc_rhs, blocks_for(g.n(), 256), 256, 0, s, g, nvert, ucont, ucont_o, ucont_rm1, bdf2, neg_inv_dt,
-             mz_end, rhs);
+  CalcRhsArgs A = {};
+  if (calc) A = {calc->ucont, calc->ucont_o, calc->ucont_rm1, calc->bdf2, calc->neg_inv_dt, calc->mz_end};
+  const unsigned nb = blocks_for(g.n(), 128);
+  launch_dep(k_ff1_rct, nb, 128, 0, s, g, conv, fp, csi, eta, zet, aj, rct);
+  auto go = [&](auto kern) { launch_dep(kern, nb, 128, 0, s, g, nvert, p, (const double *)rct, M, gram, A, rhs); };
+  const bool whole = tame && (!calc || int_mul_factor(calc->neg_inv_dt));
+  if (calc) whole ? go(k_ff1_faces<true, true>) : go(k_ff1_faces<false, true>);
+  else whole ? go(k_ff1_faces<true, false>) : go(k_ff1_faces<false, false>);
 }
 
 // ------------------------------------------------------------------- ImpRK

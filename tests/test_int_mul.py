@@ -77,3 +77,48 @@ def test_product_is_the_rounded_one():
 def test_range():
     assert all(in_range(x) for x in (0.0, -0.0, 2.0**-510, -(2.0**511), 1.9 * 2.0**511))
     assert not any(in_range(x) for x in (2.0**-511, 5e-324, 2.0**512, float("inf"), float("-inf"), float("nan")))
+
+
+def int_triple(x):
+    b = bits(x)
+    e = b >> 52 & 0x7FF
+    if not 1 <= e <= 2044:
+        return x if b << 1 & (2**64 - 1) == 0 else 3.0 * x
+    t = 3 * (b & (2**52 - 1) | 2**52)
+    s = 2 if t >> 54 else 1
+    r = (t + (s - 1) + (t >> s & 1)) >> s
+    return value(((b & 2**63) + r + ((e + s - 1) << 52)) & (2**64 - 1))
+
+
+def test_triple_is_the_rounded_one():
+    rng = random.Random(2)
+    for p in significands(rng):
+        for e in (0, 1, 2, 1023, 2043, 2044, 2045, 2046):
+            for sign in (0, 1):
+                x = value(sign << 63 | e << 52 | p)
+                assert bits(int_triple(x)) == bits(3.0 * x), x
+
+
+def rounded(q):
+    """A rational rounded to the nearest double, ties to even."""
+    return q.numerator / q.denominator  # Python's integer division rounds correctly
+
+
+def fma(a, b, c):
+    from fractions import Fraction
+    return rounded(Fraction(a) * Fraction(b) + Fraction(c))
+
+
+def test_quotient_is_the_rounded_one():
+    """quot_known: the quotient by a known divisor through its rounded reciprocal."""
+    rng = random.Random(3)
+    ms = list(significands(rng))
+    for p in ms:
+        for q in rng.sample(ms, 40):
+            x = value(rng.getrandbits(1) << 63 | rng.choice((623, 1000, 1023, 1422)) << 52 | p)
+            y = value(rng.getrandbits(1) << 63 | rng.choice((513, 1023, 1534)) << 52 | q)
+            rcp = 1.0 / y
+            r = x * rcp
+            r = fma(fma(-y, r, x), rcp, r)
+            r = fma(fma(-y, r, x), rcp, r)
+            assert bits(r) == bits(x / y), (x, y)
