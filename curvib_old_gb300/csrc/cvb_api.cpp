@@ -440,6 +440,20 @@ static int build_operators(cvb_ctx *ctx) {
     launch_split_coef(lv.g, lv.gf32, lv.ajf32, lv.code, lv.cs32, ctx->stream);
     CKL();
   }
+  // the rows of the one-thread-per-line relaxation
+  for (int l = 0; l < nl; l++) {
+    LevelDev &lv = ctx->L[l];
+    if (!lines_worth(lv.g)) continue;
+    const size_t S = SplitRow::count(lv.g);
+    if (!lv.lf64) TRY(dalloc(ctx, &lv.lf64, 3 * S));
+    if (lv.cross64 && lv.lw64) {
+      dfree(ctx, lv.lw64);
+      lv.lw64 = nullptr;
+    }
+    if (!lv.cross64 && !lv.lw64) TRY(dalloc(ctx, &lv.lw64, 7 * S));
+    launch_line_rows(lv.g, lv.w64, lv.line64, lv.lf64, lv.lw64, ctx->stream);
+    CKL();
+  }
   CK(cudaStreamSynchronize(ctx->stream));
   return CVB_OK;
 }
@@ -464,7 +478,8 @@ bool g_tune_loaded = false;
 
 // With CVB_TUNE_FILE set, measured choices persist in that text file (one
 // shape per line: mx my mz px py pz, the two cross-term flags and the
-// thirteen timings in microseconds), so a
+// fourteen timings in microseconds; lines of an earlier form, without the last,
+// are passed over and measured again), so a
 // later process -- a profiler run, say, whose own timings would be distorted --
 // makes the same choices.  Called with g_tune_mu held.
 void tune_file_load() {
@@ -476,10 +491,13 @@ void tune_file_load() {
   if (!f) return;
   ShapeKey k;
   cvb_ctx::Tune t;
-  while (std::fscanf(f, "%d %d %d %d %d %d %d %d %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf", &k.mx, &k.my,
-                     &k.mz, &k.px, &k.py, &k.pz, &k.c32, &k.c64, &t.us32[0], &t.us32[1], &t.us64[0], &t.us64[1],
-                     &t.zb32[0], &t.zb32[1], &t.zb64[0], &t.zb64[1], &t.zt32[0], &t.zt32[1], &t.zt32[2], &t.zw32[0],
-                     &t.zw32[1]) == 21) {
+  char line[1024];
+  while (std::fgets(line, sizeof line, f)) {
+    if (std::sscanf(line, "%d %d %d %d %d %d %d %d %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf", &k.mx,
+                    &k.my, &k.mz, &k.px, &k.py, &k.pz, &k.c32, &k.c64, &t.us32[0], &t.us32[1], &t.us64[0], &t.us64[1],
+                    &t.zb32[0], &t.zb32[1], &t.zb64[0], &t.zb64[1], &t.zt32[0], &t.zt32[1], &t.zt32[2], &t.zw32[0],
+                    &t.zw32[1], &t.zl64) != 22)
+      continue;
     t.level = 0;
     t.cells = (size_t)k.mx * k.my * k.mz;
     g_tune_cache.emplace(k, t);
@@ -491,9 +509,10 @@ void tune_file_append(const ShapeKey &k, const cvb_ctx::Tune &t) {
   if (!path || !*path) return;
   FILE *f = std::fopen(path, "a");
   if (!f) return;
-  std::fprintf(f, "%d %d %d %d %d %d %d %d %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f\n", k.mx,
-               k.my, k.mz, k.px, k.py, k.pz, k.c32, k.c64, t.us32[0], t.us32[1], t.us64[0], t.us64[1], t.zb32[0],
-               t.zb32[1], t.zb64[0], t.zb64[1], t.zt32[0], t.zt32[1], t.zt32[2], t.zw32[0], t.zw32[1]);
+  std::fprintf(f,
+               "%d %d %d %d %d %d %d %d %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f\n",
+               k.mx, k.my, k.mz, k.px, k.py, k.pz, k.c32, k.c64, t.us32[0], t.us32[1], t.us64[0], t.us64[1], t.zb32[0],
+               t.zb32[1], t.zb64[0], t.zb64[1], t.zt32[0], t.zt32[1], t.zt32[2], t.zw32[0], t.zw32[1], t.zl64);
   std::fclose(f);
 }
 }  // namespace
@@ -531,6 +550,8 @@ static int autotune_sweeps(cvb_ctx *ctx) {
       const int rps[3] = {4, 8, 16};
       for (int v = 0; v < 3; v++)
         if (t.zt32[v] > 0.0 && t.zt32[v] < best) { best = t.zt32[v]; L.ztma32 = rps[v]; }
+      // FP64 with one thread per line, on the same rule
+      L.zlines64 = L.lf64 && t.zl64 > 0.0 && t.zl64 < 0.97 * (L.zfuse64 ? t.zb64[1] : t.zb64[0]);
     };
     {
       std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -568,6 +589,7 @@ static int autotune_sweeps(cvb_ctx *ctx) {
         (prec == 0 ? t.us32 : t.us64)[v] = 1e3 * ms / reps;
       }
     L.ztma32 = 0;
+    L.zlines64 = 0;
     // zebra sweep (both colours): two kernels per half-sweep, then one (in place
     // without cross terms, else out of place through t)
     for (int prec = 0; prec < 2; prec++)
@@ -605,6 +627,23 @@ static int autotune_sweeps(cvb_ctx *ctx) {
       t.zw32[v] = 1e3 * ms / reps;
     }
     L.ztw32 = 0;
+    // the FP64 zebra sweep with one thread per line
+    t.zl64 = 0.0;
+    if (L.lf64) {
+      L.zlines64 = 1;
+      const int reps = 5;
+      for (int q = 0; q <= reps; q++) {
+        if (q == 1) CK(cudaEventRecord(ctx->ev0, ctx->stream));
+        launch_zebra_sweep<double>(L, L.r64, L.e64, L.t64, L.t64 + n, 1.3, false, ctx->stream);
+      }
+      CK(cudaEventRecord(ctx->ev1, ctx->stream));
+      CK(cudaEventSynchronize(ctx->ev1));
+      CKL();
+      float ms = 0;
+      CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
+      t.zl64 = 1e3 * ms / reps;
+      L.zlines64 = 0;
+    }
     // the FP32 zebra sweep with TMA-staged tiles, each chunk size
     for (int v = 0; v < 3; v++) {
       t.zt32[v] = 0.0;
@@ -2645,7 +2684,7 @@ int cvb_tuning_report(cvb_ctx *ctx, char *buf, int len) {
   std::string o = "{\"line_sweep\": [";
   for (size_t q = 0; q < ctx->tune.size(); q++) {
     const auto &t = ctx->tune[q];
-    char row[768];
+    char row[1024];
     const LevelDev &L = ctx->L[t.level];
     char z32[16];
     if (L.ztma32) snprintf(z32, sizeof z32, "tma%d", L.ztma32);
@@ -2655,11 +2694,11 @@ int cvb_tuning_report(cvb_ctx *ctx, char *buf, int len) {
              "\"f64\": {\"fused_us\": %.2f, \"split_us\": %.2f, \"choice\": \"%s\"}, "
              "\"zebra_f32\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"split4_us\": %.2f, \"fused4_us\": %.2f, "
              "\"tma4_us\": %.2f, \"tma8_us\": %.2f, \"tma16_us\": %.2f, \"choice\": \"%s\"}, "
-             "\"zebra_f64\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"choice\": \"%s\"}}",
+             "\"zebra_f64\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"lines_us\": %.2f, \"choice\": \"%s\"}}",
              q ? ", " : "", t.level, t.cells, t.us32[0], t.us32[1], L.sweep32 ? "split" : "fused", t.us64[0],
              t.us64[1], L.sweep64 ? "split" : "fused", t.zb32[0], t.zb32[1], t.zw32[0], t.zw32[1], t.zt32[0],
              t.zt32[1], t.zt32[2], z32,
-             t.zb64[0], t.zb64[1], L.zfuse64 ? "fused" : "split");
+             t.zb64[0], t.zb64[1], t.zl64, L.zlines64 ? "lines" : L.zfuse64 ? "fused" : "split");
     o += row;
   }
   o += "]}";

@@ -29,7 +29,6 @@ namespace {
 
 constexpr int kMaxSlots = 1024;
 constexpr int kMaxLevels = 16;
-constexpr int kMaxFusedRows = 400;
 constexpr size_t kMaxSmem = 200 * 1024;
 
 enum PState { P_NEW, P_ITER };

@@ -97,6 +97,9 @@ struct LevelDev {
   float *cs32;           // levels without FP32 cross terms: g11, g22, g33, aj and the code (its bits)
                          // in colour-split rows ([5][SplitRow::count]) for the zebra residual; else null
   double *line64;        // ... in FP64
+  // colour-split rows for the one-thread-per-line relaxation (kernels_lines.cu; null: the level does not
+  // try it): m, beta, -c of each row, and without cross terms the seven weights times -m
+  double *lf64, *lw64;
   // work vectors of this level (the finest level's b/x live in the solver)
   double *r64, *e64, *t64;  // FP64 V-cycle vectors
   float *r32, *e32, *t32;   // FP32 V-cycle vectors
@@ -108,6 +111,7 @@ struct LevelDev {
                             // (in place without cross terms, else out of place)
   int ztma32;               // FP32 zebra half-sweep with TMA-staged tiles (kernels_tma.cu): the
                             // row pairs per chunk (4, 8, 16) the autotuner chose, 0 off
+  int zlines64;             // FP64 zebra half-sweep with one thread per line (kernels_lines.cu), chosen at set-up
   int ztw32;                // lines per block of the FP32 zebra line-solve tiles (4 or 8; 0: 8)
   // coarsest level only: the densely inverted cells (first cm of cidx) and the
   // identity ones (the rest of cidx)
@@ -134,6 +138,9 @@ __host__ __device__ inline bool zebra_fusable(const LevelDev &L) {
   return !has_cross<T>(L) && (!L.g.px || (L.g.mx & 1) == 0) && (!L.g.pz || (L.g.mz & 1) == 0);
 }
 
+
+// The longest lines the tile and line kernels take (their shared memory).
+constexpr int kMaxFusedRows = 400;
 
 // --- kernel launchers (defined in the .cu files) ---------------------------
 // setup
@@ -357,5 +364,22 @@ void launch_imp_waxpy(const Geom &g, double a, const double *rhs, const double *
                       const double *inflow, double *u, cudaStream_t s);
 void launch_imp_norms(size_t n, const double *rhs, const double *pu, const double *u, unsigned long long *out,
                       cudaStream_t s);
+
+// --- FP64 y-line relaxation, one thread per line (kernels_lines.cu)
+// Tiles of 32 lines of one colour in a plane, and the fewest tiles of a colour
+// in a level that tries it: two for each of 152 SMs.
+inline int line_tiles_x(const Geom &g) { return ((g.mx - 1) / 2 + 31) / 32; }
+constexpr int kLineTiles = 304;
+inline bool lines_worth(const Geom &g) {
+  return g.my - 2 <= kMaxFusedRows && (long long)line_tiles_x(g) * (g.mz - 2) >= kLineTiles;
+}
+// lf (and, with lw, the scaled weights of a level without cross terms) from
+// the level's weights and Thomas factors
+void launch_line_rows(const Geom &g, const double *w64, const double *line64, double *lf, double *lw, cudaStream_t s);
+// one colour: fused, a half-sweep of x in place (xnew == x) for the right-hand
+// side r (zebra_fusable levels); else the line solves of the residual r
+// (rsplit: in colour-split rows), x null for a zero guess
+void launch_lines(const LevelDev &L, bool fused, const double *r, const double *x, double *xnew, double omega,
+                  int color, int rsplit, cudaStream_t s);
 
 }  // namespace cvb

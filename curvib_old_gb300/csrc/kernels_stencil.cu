@@ -183,7 +183,6 @@ __global__ void k_line_thomas(Geom g, const T *__restrict__ fac, const T *__rest
   }
 }
 
-static const int kMaxFusedRows = 400;
 static const size_t kMaxSmem = 200 * 1024;
 
 // Sweep variants: fused (residual inside the tile kernel) or split (a full-
@@ -275,9 +274,13 @@ static void zebra_fused(const LevelDev &L, const T *b, const T *xin, T *xout, T 
   else zebra_fused_tw<T, sizeof(T) == 4 ? kSolveTW32 : kSolveTW64>(L, b, xin, xout, omega, color, s);
 }
 template <typename T>
+static bool lines_chosen(const LevelDev &L) {
+  return sizeof(T) == 8 && L.zlines64 != 0;
+}
+template <typename T>
 static bool fused_ok(const LevelDev &L) {
   constexpr int TW = sizeof(T) == 4 ? kSolveTW32 : kSolveTW64;
-  const bool chosen = sizeof(T) == 4 ? L.zfuse32 != 0 : L.zfuse64 != 0;
+  const bool chosen = !lines_chosen<T>(L) && (sizeof(T) == 4 ? L.zfuse32 != 0 : L.zfuse64 != 0);
   return chosen && L.g.my <= kMaxFusedRows && line_solve_smem<T, TW>(L.g) <= kMaxSmem;
 }
 
@@ -294,12 +297,24 @@ void launch_zebra_half(const LevelDev &L, const T *b, T *x, T *res, T omega, int
     zebra_fused<T>(L, b, x, x, omega, color, s);
     return;
   }
+  if constexpr (sizeof(T) == 8) {
+    if (lines_chosen<T>(L) && (zero || zebra_fusable<T>(L))) {
+      launch_lines(L, !zero, b, zero ? nullptr : x, x, omega, color, 0, s);
+      return;
+    }
+  }
   const T *r = b;
   if (!zero) {
     dim3 grd(color_plane_blocks(L.g), 1, L.g.mz - 2);
     if (has_cross<T>(L)) launch_dep(k_resid_color<T, true>, grd, kFlat, 0, s, L, x, b, res, color);
     else launch_dep(k_resid_color<T, false>, grd, kFlat, 0, s, L, x, b, res, color);
     r = res;
+  }
+  if constexpr (sizeof(T) == 8) {
+    if (lines_chosen<T>(L)) {
+      launch_lines(L, false, r, x, x, omega, color, 1, s);
+      return;
+    }
   }
   if (sizeof(T) == 4 && L.ztw32 == 4) line_solve<T, 4>(L, r, zero ? nullptr : x, x, omega, s, color, zero ? 0 : 1);
   else line_solve<T, TW>(L, r, zero ? nullptr : x, x, omega, s, color, zero ? 0 : 1);
