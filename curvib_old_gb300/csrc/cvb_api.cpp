@@ -143,6 +143,7 @@ static void free_all(cvb_ctx *ctx) {
   ctx->cm[0] = ctx->cm[1] = ctx->cm[2] = nullptr;
   ctx->nvert_tmp = nullptr;
   ctx->Minv = nullptr;
+  ctx->minv_len = 0;
   ctx->cidx = nullptr;
   ctx->b = ctx->x = ctx->w = ctx->r = nullptr;
   for (int q = 0; q <= kMaxRestart; q++) ctx->V[q] = nullptr;
@@ -214,40 +215,6 @@ static int check_desc(cvb_ctx *ctx, const cvb_level_desc &d, int level, bool fin
 // Largest coarsest box (ring included) solved by a dense inverse unless the
 // options say otherwise: 18^3 = 5832 holds a 16^3-cell coarsest level.
 constexpr int kCoarseDenseMaxDefault = 6000;
-// Largest coarsest block inverted on the host; larger ones go to the device.
-constexpr int kHostInverseMax = 384;
-
-// Gauss-Jordan inverse with partial pivoting (coarsest level, n <= kHostInverseMax).
-static bool dense_inverse(std::vector<double> &A, int n, std::vector<double> &Inv) {
-  Inv.assign((size_t)n * n, 0.0);
-  for (int i = 0; i < n; i++) Inv[(size_t)i * n + i] = 1.0;
-  for (int c = 0; c < n; c++) {
-    int piv = c;
-    double best = std::fabs(A[(size_t)c * n + c]);
-    for (int r = c + 1; r < n; r++) {
-      double v = std::fabs(A[(size_t)r * n + c]);
-      if (v > best) { best = v; piv = r; }
-    }
-    if (!(best > 0.0)) return false;
-    if (piv != c) {
-      for (int q = 0; q < n; q++) {
-        std::swap(A[(size_t)c * n + q], A[(size_t)piv * n + q]);
-        std::swap(Inv[(size_t)c * n + q], Inv[(size_t)piv * n + q]);
-      }
-    }
-    double inv = 1.0 / A[(size_t)c * n + c];
-    for (int q = 0; q < n; q++) { A[(size_t)c * n + q] *= inv; Inv[(size_t)c * n + q] *= inv; }
-    for (int r = 0; r < n; r++) {
-      if (r == c) continue;
-      double f = A[(size_t)r * n + c];
-      if (f == 0.0) continue;
-      double *ar = &A[(size_t)r * n], *ac = &A[(size_t)c * n];
-      double *ir = &Inv[(size_t)r * n], *ic = &Inv[(size_t)c * n];
-      for (int q = 0; q < n; q++) { ar[q] -= f * ac[q]; ir[q] -= f * ic[q]; }
-    }
-  }
-  return true;
-}
 
 // Rows of the coarsest operator, made nonsingular: M = A + sum_r u_r v_r^T with
 // v_r the indicator of fluid region r and u_r = s v_r.  A's left null vector on
@@ -299,60 +266,62 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
   const int m = (int)idx.size();
   for (size_t p = 0; p < n; p++)
     if (pos[p] < 0) idx.push_back((int)p);
-  std::vector<double> A((size_t)m * m, 0.0);
+  // what the device needs to form M: the cells' order, the inverted rows'
+  // regions (-1: an identity row) and their neighbours' columns
+  std::vector<int> tab(idx);
+  tab.resize(n + (size_t)m + (size_t)m * NSLOT, 0);
+  int *reg = tab.data() + n, *col = reg + m, cnt[2] = {0, 0}, nfl = 0;
   double diag_sum = 0.0;
-  int nfl = 0;
   for (int r = 0; r < m; r++) {
-    size_t p = (size_t)idx[r];
-    if (!fluid[p]) { A[(size_t)r * m + r] = 1.0; continue; }
-    for (int q = 0; q < NSLOT; q++) A[(size_t)r * m + pos[cols[p * NSLOT + q]]] += w[(size_t)q * n + p];
-    diag_sum += std::fabs(A[(size_t)r * m + r]);
+    const size_t p = (size_t)idx[r];
+    reg[r] = region[p];
+    if (!fluid[p]) continue;
+    double diag = 0.0;
+    for (int q = 0; q < NSLOT; q++) {
+      const int c = pos[cols[p * NSLOT + q]];
+      col[(size_t)r * NSLOT + q] = c;
+      if (c == r) diag += w[(size_t)q * n + p];
+    }
+    diag_sum += std::fabs(diag);
+    cnt[region[p]]++;
     nfl++;
   }
-  if (nfl > 0) {
-    double s = diag_sum / nfl;
-    for (int reg = 0; reg < 2; reg++) {
-      int cnt = 0;
-      for (int r = 0; r < m; r++) cnt += region[idx[r]] == reg;
-      if (!cnt) continue;
-      double sv = s / cnt;
-      for (int r = 0; r < m; r++) {
-        if (region[idx[r]] != reg) continue;
-        for (int q = 0; q < m; q++)
-          if (region[idx[q]] == reg) A[(size_t)r * m + q] += sv;
-      }
-    }
+  double sv[2] = {0.0, 0.0};
+  for (int q = 0; q < 2; q++)
+    if (cnt[q]) sv[q] = diag_sum / nfl / cnt[q];
+  // the inverse stays where it was while it fits, so that captured V-cycles
+  // stay valid when a body moves
+  const size_t need = std::max((size_t)m * m, (size_t)1);
+  if (ctx->Minv && ctx->minv_len < need) {
+    dfree(ctx, ctx->Minv);
+    ctx->Minv = nullptr;
   }
-  if (ctx->Minv) dfree(ctx, ctx->Minv);
-  if (ctx->cidx) dfree(ctx, ctx->cidx);
-  ctx->Minv = nullptr;
-  ctx->cidx = nullptr;
-  TRY(dalloc(ctx, &ctx->Minv, std::max((size_t)m * m, (size_t)1)));
-  TRY(dalloc(ctx, &ctx->cidx, n));
-  if (m > kHostInverseMax) {
-    // thousands of unknowns (a 16^3 coarsest level): Gauss-Jordan on the device
-    double *dA = nullptr, *dwork = nullptr;
-    int *iwork = nullptr;
-    TRY(dalloc(ctx, &dA, (size_t)m * m));
-    int rc = dalloc(ctx, &dwork, 2 * (size_t)m);
+  if (!ctx->Minv) {
+    TRY(dalloc(ctx, &ctx->Minv, need));
+    ctx->minv_len = need;
+  }
+  if (!ctx->cidx) TRY(dalloc(ctx, &ctx->cidx, n));
+  CK(cudaMemcpyAsync(ctx->cidx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
+  if (m > 0) {
+    double *dA = nullptr;
+    int *dtab = nullptr, *iwork = nullptr;
+    const size_t nd = dense_inverse_doubles(m);
+    int rc = dalloc(ctx, &dA, (size_t)m * m + nd);
+    if (rc == CVB_OK) rc = dalloc(ctx, &dtab, tab.size());
     if (rc == CVB_OK) rc = dalloc(ctx, &iwork, 2 * (size_t)m + 1);
     bool ok = false;
-    if (rc == CVB_OK && cudaMemcpyAsync(dA, A.data(), sizeof(double) * m * m, cudaMemcpyHostToDevice,
-                                        ctx->stream) == cudaSuccess)
-      ok = device_dense_inverse(dA, m, ctx->Minv, iwork, iwork + m, dwork, dwork + m, iwork + 2 * m, ctx->stream);
+    if (rc == CVB_OK && cudaMemcpyAsync(dtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice,
+                                        ctx->stream) == cudaSuccess) {
+      launch_coarse_matrix(m, (int)n, dtab, dtab + n, dtab + n + m, sv[0], sv[1], C.w64, dA, ctx->stream);
+      ok = device_dense_inverse(dA, m, ctx->Minv, iwork, iwork + m, dA + (size_t)m * m, iwork + 2 * m, ctx->stream);
+    }
     if (iwork) dfree(ctx, iwork);
-    if (dwork) dfree(ctx, dwork);
-    dfree(ctx, dA);
+    if (dtab) dfree(ctx, dtab);
+    if (dA) dfree(ctx, dA);
     if (rc != CVB_OK) return rc;
     CK(cudaGetLastError());
     if (!ok) return fail(ctx, CVB_BAD_INPUT, "coarsest operator is singular after regularisation");
-  } else if (m > 0) {
-    std::vector<double> Inv;
-    if (!dense_inverse(A, m, Inv)) return fail(ctx, CVB_BAD_INPUT, "coarsest operator is singular after regularisation");
-    CK(cudaMemcpyAsync(ctx->Minv, Inv.data(), sizeof(double) * m * m, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
   }
-  CK(cudaMemcpyAsync(ctx->cidx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   C.cidx = ctx->cidx;
   C.cm = m;
@@ -1087,10 +1056,38 @@ static int solve_resident(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats
 // nvert holds the reference's cell codes (0 fluid, 1..2 immersed boundary, 3+
 // solid, ibm.c:4332-4438): finite and non-negative.
 static int check_nvert(cvb_ctx *ctx, const double *v, size_t n) {
-  for (size_t p = 0; p < n; p++)
-    if (!std::isfinite(v[p]) || v[p] < 0.0)
-      return fail(ctx, CVB_BAD_INPUT, "nvert[%zu] = %g is not a cell code (finite, >= 0)", p, v[p]);
+  // by bit patterns, a block at a time (a loop the compiler can vectorise):
+  // below +inf's, or -0
+  for (size_t p0 = 0; p0 < n; p0 += 4096) {
+    const size_t p1 = std::min(n, p0 + 4096);
+    unsigned bad = 0;
+    for (size_t p = p0; p < p1; p++) {
+      uint64_t b;
+      std::memcpy(&b, v + p, sizeof b);
+      bad |= (b >= 0x7ff0000000000000ULL) & (b != 0x8000000000000000ULL);
+    }
+    if (!bad) continue;
+    for (size_t p = p0; p < p1; p++)
+      if (!std::isfinite(v[p]) || v[p] < 0.0)
+        return fail(ctx, CVB_BAD_INPUT, "nvert[%zu] = %g is not a cell code (finite, >= 0)", p, v[p]);
+  }
   return CVB_OK;
+}
+
+static unsigned long long next_setup_id() {
+  static std::atomic<unsigned long long> setups{0};
+  return ++setups;
+}
+
+// Whether the kernels of a V-cycle get the same arguments on both levels.
+static bool same_launches(const LevelDev &a, const LevelDev &b) {
+  auto key = [](const LevelDev &L) {
+    return std::make_tuple(std::make_tuple(L.nvert, L.code, L.w64, L.gf32, L.ajf32, L.wgt32, L.line32, L.cs32, L.line64,
+                                           L.lf64, L.lw64, L.r64, L.e64, L.t64),
+                           std::make_tuple(L.r32, L.e32, L.t32, L.sweep32, L.sweep64, L.cross32, L.cross64, L.zfuse32,
+                                           L.zfuse64, L.ztma32, L.zlines64, L.ztw32, L.cidx, L.cm, L.gate));
+  };
+  return key(a) == key(b);
 }
 
 static int setup_problem(cvb_ctx *ctx, const double *nvert_box) {
@@ -1161,8 +1158,7 @@ static int setup_problem(cvb_ctx *ctx, const double *nvert_box) {
   TRY(build_coarse(ctx, &def));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->setup_ms[4] = ms_since(t);
-  static std::atomic<unsigned long long> setups{0};
-  ctx->setup_id = ++setups;
+  ctx->setup_id = next_setup_id();
   ctx->ready = true;
   return CVB_OK;
 }
@@ -1433,7 +1429,20 @@ int cvb_set_nvert(cvb_ctx *ctx, const double *nvert_finest) {
   std::vector<double> h;
   const double *v = box_view(df, nvert_finest, 1, h);
   TRY(check_nvert(ctx, v, (size_t)df.mx * df.my * df.mz));
-  drop_vcycle_graphs(ctx);
+  // the captured V-cycles stay valid where every argument of their kernels is
+  // what it was (a body that moves keeps the arrays, and as a rule the sweeps
+  // and the size of the coarsest block); a set-up that fails drops them
+  struct Graphs {
+    cvb_ctx *c;
+    bool keep = false;
+    ~Graphs() {
+      if (!keep) drop_vcycle_graphs(c);
+    }
+  } graphs{ctx};
+  const std::vector<LevelDev> was = ctx->L;
+  const double *minv_was = ctx->Minv;
+  const bool dense_was = ctx->coarse_dense;
+  ctx->setup_id = next_setup_id();
   CK(cudaMemcpyAsync(ctx->L[ctx->nlevels - 1].nvert, v, sizeof(double) * ctx->L[ctx->nlevels - 1].g.n(),
                      cudaMemcpyHostToDevice, ctx->stream));
   using clk = std::chrono::steady_clock;
@@ -1452,6 +1461,8 @@ int cvb_set_nvert(cvb_ctx *ctx, const double *nvert_finest) {
   TRY(build_coarse(ctx, &def));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->setup_ms[4] = ms_since(t);
+  graphs.keep = ctx->Minv == minv_was && ctx->coarse_dense == dense_was;
+  for (int l = 0; l < ctx->nlevels; l++) graphs.keep = graphs.keep && same_launches(was[l], ctx->L[l]);
   return CVB_OK;
 }
 

@@ -244,12 +244,18 @@ __device__ __forceinline__ double quot_newton(double b, double a) {
   r = fma(r, fma(-a, r, 1.0), r);
   return b * r;
 }
-// coarsest solve e = M^-1 r on C.cidx[0..C.cm), e = r on the other cells
 // In-place Gauss-Jordan inverse of the n x n row-major A on the device into
 // out (kernels_setup.cu); false for a singular matrix.  Work arrays: perm and
-// colmap n ints, prow and fcol n doubles, status one int.
-bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *prow, double *fcol,
-                          int *status, cudaStream_t s);
+// colmap n ints, work dense_inverse_doubles(n) doubles, status one int.
+size_t dense_inverse_doubles(int n);
+bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *work, int *status,
+                          cudaStream_t s);
+// The coarsest level's m x m matrix over the cells idx[0 .. m) of its n:
+// region[r] the row's fluid region (-1: an identity row), cols[19 r ..] its
+// neighbours' columns, sv0 / sv1 added over each region's block
+void launch_coarse_matrix(int m, int n, const int *idx, const int *region, const int *cols, double sv0, double sv1,
+                          const double *w64, double *A, cudaStream_t s);
+// coarsest solve e = M^-1 r on C.cidx[0..C.cm), e = r on the other cells
 void launch_dense_apply(const LevelDev &C, const double *Minv, const double *r, double *e, cudaStream_t s,
                         const int *gate = nullptr);
 void launch_dense_apply_f32(const LevelDev &C, const double *Minv, const float *r, float *e, cudaStream_t s,

@@ -353,82 +353,203 @@ void launch_nvert_restrict(const Geom &fine, const double *nvf, const Geom &coar
 namespace cvb {
 
 // ------------------------------------------------------------------ dense inverse
-// Gauss-Jordan inversion in place with partial pivoting, one column per step,
-// for the coarsest level's matrix when it is too large to invert on the host
-// in reasonable time (thousands of unknowns).  Step c: k_gj_pivot (one block)
-// picks the row of largest |A[r][c]| at or below c (the first of equal ones),
-// swaps it into row c, and stages the scaled pivot row (A[c][q] / A[c][c], with
-// 1 / A[c][c] in column c, the inverse's column) and the multipliers A[r][c];
-// k_gj_elim then updates every row from the staged copies, so no thread reads
-// what another writes.  The row swaps become column swaps of the result,
-// undone by k_gj_unpermute from the composed column map.
-constexpr int kGjThreads = 1024;
+// Gauss-Jordan inversion in place with partial pivoting, kGjW columns per step,
+// for the coarsest level's matrix.  Step c0 takes the columns c0 .. c0 + w - 1:
+//  - k_gj_panel (one block): LU elimination of those columns' rows from c0 down,
+//    in shared memory, picks the pivot rows (the largest entry, the first of
+//    equal ones, as column by column); the rows are swapped into place, the
+//    pivot block D inverted, and the columns (the multipliers F) and the pivot
+//    rows (B, the unit matrix in the panel's own columns) staged, so that no
+//    thread of the next kernel reads what another writes;
+//  - k_gj_update: R = D^-1 B replaces the pivot rows, and every other row
+//    becomes its own (zero in the panel's columns) minus F R.
+// The row swaps become column swaps of the result, undone by k_gj_unpermute
+// from the composed column map.
+//
+// The update is bound by the FP64 pipe (n^3 multiply-adds in all), the panel by
+// its n dependent steps on one SM.  Set-up of the coarsest solver, all in: 216
+// unknowns 0.9 ms (3.8 inverted on the host), 990 5.9 ms, 4,096 167 ms (23.2 and
+// 531 ms with one column a step: 2 n launches, n passes over the matrix, and
+// the matrix formed on the host).
+constexpr int kGjThreads = 1024, kGjW = 8, kGjTile = 64;
+// Panels of kGjW columns (64 bytes a row) of up to this many rows fit in shared
+// memory; beyond, w shrinks.
+constexpr int kGjSmemRows = 3200;
 
-__global__ void __launch_bounds__(kGjThreads) k_gj_pivot(double *__restrict__ A, int n, int c, int *__restrict__ perm,
-                                                         double *__restrict__ prow, double *__restrict__ fcol,
-                                                         int *__restrict__ status) {
-  if (*status) return;
-  __shared__ double sv[kGjThreads / 32];
-  __shared__ int si[kGjThreads / 32];
-  __shared__ int s_piv;
-  double best = -1.0;
-  int bi = n;
-  for (int r = c + threadIdx.x; r < n; r += blockDim.x) {
-    double v = fabs(A[(size_t)r * n + c]);
-    if (v > best) { best = v; bi = r; }  // NaN never wins
-  }
+// The better pivot of two (magnitude as a bit pattern, row): the larger, the
+// first of equal ones.  Magnitudes order as their patterns; a NaN counts as 0.
+__device__ __forceinline__ unsigned long long gj_magnitude(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v) & 0x7fffffffffffffffULL;
+  return b > 0x7ff0000000000000ULL ? 0 : b;
+}
+__device__ __forceinline__ void gj_better(unsigned long long &best, int &row, unsigned long long v, int r) {
+  if (v > best || (v == best && r < row)) { best = v; row = r; }
+}
+__device__ __forceinline__ void gj_warp_best(unsigned long long &best, int &row) {
   for (int o = 16; o > 0; o >>= 1) {
-    double ov = __shfl_down_sync(0xffffffffu, best, o);
-    int oi = __shfl_down_sync(0xffffffffu, bi, o);
-    if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+    const unsigned long long v = __shfl_down_sync(0xffffffffu, best, o);
+    const int r = __shfl_down_sync(0xffffffffu, row, o);
+    gj_better(best, row, v, r);
   }
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) { sv[wid] = best; si[wid] = bi; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double b = sv[0];
-    int i = si[0];
-    for (int w = 1; w < (int)(blockDim.x / 32); w++)
-      if (sv[w] > b || (sv[w] == b && si[w] < i)) { b = sv[w]; i = si[w]; }
-    if (!(b > 0.0) || i >= n) {
-      *status = 1;
-      i = -1;
-    } else {
-      perm[c] = i;
-    }
-    s_piv = i;
-  }
-  __syncthreads();
-  const int p = s_piv;
-  if (p < 0) return;
-  if (p != c)
-    for (int q = threadIdx.x; q < n; q += blockDim.x) {
-      double a = A[(size_t)c * n + q];
-      A[(size_t)c * n + q] = A[(size_t)p * n + q];
-      A[(size_t)p * n + q] = a;
-    }
-  __syncthreads();
-  const double inv = 1.0 / A[(size_t)c * n + c];
-  for (int q = threadIdx.x; q < n; q += blockDim.x)
-    prow[q] = q == c ? inv : __dmul_rn(A[(size_t)c * n + q], inv);
-  for (int r = threadIdx.x; r < n; r += blockDim.x) fcol[r] = r == c ? 0.0 : A[(size_t)r * n + c];
 }
 
-__global__ void k_gj_elim(double *__restrict__ A, int n, int c, const double *__restrict__ prow,
-                          const double *__restrict__ fcol, const int *__restrict__ status) {
+__global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A, int n, int c0, int w,
+                                                         int *__restrict__ perm, double *__restrict__ F,
+                                                         double *__restrict__ B, double *__restrict__ Dinv,
+                                                         int *__restrict__ status) {
+  extern __shared__ double S[];  // the panel's columns from row c0 down, [w][m | 1]
+  __shared__ unsigned long long sv[kGjThreads / 32];
+  __shared__ int si[kGjThreads / 32];
+  __shared__ int piv[kGjW];
+  __shared__ double rcp[kGjW];
+  __shared__ double D[kGjW][2 * kGjW];
+  dep_sync();
   if (*status) return;
-  const size_t nn = (size_t)n * n;
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < nn; e += (size_t)gridDim.x * blockDim.x) {
-    int r = (int)(e / n), q = (int)(e % n);
-    if (r == c) {
-      A[e] = prow[q];
-      continue;
-    }
-    double f = fcol[r];
-    if (f == 0.0) continue;  // column c of this row is already 0
-    double a = q == c ? 0.0 : A[e];
-    A[e] = __dsub_rn(a, __dmul_rn(f, prow[q]));
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, m = n - c0, mp = m | 1;
+  for (int e = t; e < m * kGjW; e += kGjThreads) {
+    const int r = e / kGjW, q = e % kGjW;
+    if (q < w) S[q * mp + r] = A[(size_t)(c0 + r) * n + c0 + q];
   }
+  __syncthreads();
+  unsigned long long best = 0;
+  int row = m;
+  for (int r = t; r < m; r += kGjThreads) gj_better(best, row, gj_magnitude(S[r]), r);
+  for (int s = 0; s < w; s++) {
+    gj_warp_best(best, row);
+    if (lane == 0) { sv[wid] = best; si[wid] = row; }
+    __syncthreads();
+    if (wid == 0) {
+      best = sv[lane];
+      row = si[lane];
+      gj_warp_best(best, row);
+      if (lane == 0) {
+        piv[s] = best > 0 ? row : -1;
+        if (best > 0) rcp[s] = 1.0 / S[s * mp + row];
+      }
+    }
+    __syncthreads();
+    const int p = piv[s];
+    if (p < 0) {
+      if (t == 0) *status = 1;
+      return;
+    }
+    if (p != s) {
+      if (t < w) {
+        const double v = S[t * mp + s];
+        S[t * mp + s] = S[t * mp + p];
+        S[t * mp + p] = v;
+      }
+      __syncthreads();
+    }
+    // eliminate, and look for the next column's pivot on the way
+    best = 0;
+    row = m;
+    if (s + 1 < w)
+      for (int r = s + 1 + t; r < m; r += kGjThreads) {
+        const double f = -S[s * mp + r] * rcp[s];
+        for (int q = s + 1; q < w; q++) {
+          const double v = fma(f, S[q * mp + s], S[q * mp + r]);
+          S[q * mp + r] = v;
+          if (q == s + 1) gj_better(best, row, gj_magnitude(v), r);
+        }
+      }
+    __syncthreads();
+  }
+  if (t < w) perm[c0 + t] = c0 + piv[t];
+  bool moved = false;
+  for (int s = 0; s < w; s++) moved = moved || piv[s] != s;
+  if (moved) {
+    for (int q = t; q < n; q += kGjThreads)
+      for (int s = 0; s < w; s++) {
+        const int p = piv[s];
+        if (p == s) continue;
+        const double v = A[(size_t)(c0 + s) * n + q];
+        A[(size_t)(c0 + s) * n + q] = A[(size_t)(c0 + p) * n + q];
+        A[(size_t)(c0 + p) * n + q] = v;
+      }
+    __syncthreads();
+  }
+  for (int e = t; e < n * kGjW; e += kGjThreads) {
+    const int r = e / kGjW, q = e % kGjW;
+    F[e] = q < w ? A[(size_t)r * n + c0 + q] : 0.0;
+  }
+  for (int s = 0; s < kGjW; s++)
+    for (int q = t; q < n; q += kGjThreads)
+      B[(size_t)s * n + q] =
+          q >= c0 && q < c0 + w ? (q - c0 == s ? 1.0 : 0.0) : s < w ? A[(size_t)(c0 + s) * n + q] : 0.0;
+  // D and its inverse: Gauss-Jordan beside the unit matrix, in the order of the
+  // pivots just found, whose reciprocals are at hand; the unit matrix beyond w
+  const int r = t / (2 * kGjW), q = t % (2 * kGjW);
+  const bool mine = t < kGjW * 2 * kGjW;
+  double d = 0.0;
+  if (mine) {
+    d = q < kGjW ? (r < w && q < w ? A[(size_t)(c0 + r) * n + c0 + q] : (r == q ? 1.0 : 0.0))
+                 : (q - kGjW == r ? 1.0 : 0.0);
+    D[r][q] = d;
+  }
+  __syncthreads();
+  for (int s = 0; s < w; s++) {
+    if (mine) {
+      const double pr = D[s][q] * rcp[s];
+      d = r == s ? pr : fma(-D[r][s], pr, d);
+    }
+    __syncthreads();
+    if (mine) D[r][q] = d;
+    __syncthreads();
+  }
+  if (t < kGjW * kGjW) Dinv[t] = D[t / kGjW][kGjW + t % kGjW];
+}
+
+// A 64 x 64 tile per block, 4 x 4 entries a thread (columns 16 apart).
+__global__ void __launch_bounds__(256) k_gj_update(double *__restrict__ A, int n, int c0, int w,
+                                                   const double *__restrict__ F, const double *__restrict__ B,
+                                                   const double *__restrict__ Dinv, const int *__restrict__ status) {
+  __shared__ double sR[kGjW][kGjTile], sF[kGjTile][kGjW + 1], sD[kGjW * kGjW];
+  dep_sync();
+  if (*status) return;
+  const int t = threadIdx.x, q0 = blockIdx.x * kGjTile, r0 = blockIdx.y * kGjTile;
+  if (t < kGjW * kGjW) sD[t] = Dinv[t];
+  for (int e = t; e < kGjTile * kGjW; e += 256) {
+    const int r = e / kGjW;
+    sF[r][e % kGjW] = r0 + r < n ? F[(size_t)r0 * kGjW + e] : 0.0;
+  }
+  __syncthreads();
+  for (int e = t; e < kGjW * kGjTile; e += 256) {
+    const int s = e / kGjTile, q = e % kGjTile;
+    double v = 0.0;
+    if (q0 + q < n)
+      for (int u = 0; u < kGjW; u++) v = fma(sD[s * kGjW + u], B[(size_t)u * n + q0 + q], v);
+    sR[s][q] = v;
+  }
+  __syncthreads();
+  const int tx = t % 16, ty = t / 16;
+  double acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const int r = r0 + ty * 4 + a, q = q0 + tx + 16 * b;
+      acc[a][b] = r < n && q < n && !(q >= c0 && q < c0 + w) ? A[(size_t)r * n + q] : 0.0;
+    }
+#pragma unroll
+  for (int s = 0; s < kGjW; s++) {
+    double f[4], p[4];
+#pragma unroll
+    for (int a = 0; a < 4; a++) f[a] = sF[ty * 4 + a][s];
+#pragma unroll
+    for (int b = 0; b < 4; b++) p[b] = sR[s][tx + 16 * b];
+#pragma unroll
+    for (int a = 0; a < 4; a++)
+#pragma unroll
+      for (int b = 0; b < 4; b++) acc[a][b] = fma(-f[a], p[b], acc[a][b]);
+  }
+#pragma unroll
+  for (int a = 0; a < 4; a++)
+#pragma unroll
+    for (int b = 0; b < 4; b++) {
+      const int r = r0 + ty * 4 + a, q = q0 + tx + 16 * b;
+      if (r < n && q < n) A[(size_t)r * n + q] = r >= c0 && r < c0 + w ? sR[r - c0][tx + 16 * b] : acc[a][b];
+    }
 }
 
 __global__ void k_gj_unpermute(const double *__restrict__ A, int n, const int *__restrict__ colmap,
@@ -440,16 +561,31 @@ __global__ void k_gj_unpermute(const double *__restrict__ A, int n, const int *_
   }
 }
 
+size_t dense_inverse_doubles(int n) { return 2 * (size_t)kGjW * n + kGjW * kGjW; }
+
 // Inverts the n x n row-major A (device, overwritten) into out (device).
-// perm / colmap are n ints, prow / fcol n doubles, status one int (device).
-// Returns false if a pivot column was all zero (a singular matrix).
-bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *prow, double *fcol,
-                          int *status, cudaStream_t s) {
+// perm / colmap are n ints, work dense_inverse_doubles(n) doubles, status one
+// int (device).  Returns false if a pivot column was all zero (a singular
+// matrix).
+bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *work, int *status,
+                          cudaStream_t s) {
+  static bool attr = false;
+  if (!attr) {
+    cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmemRows * kGjW * 8);
+    attr = true;
+  }
+  double *F = work, *B = F + (size_t)kGjW * n, *Dinv = B + (size_t)kGjW * n;
   cudaMemsetAsync(status, 0, sizeof(int), s);
-  const unsigned eb = (unsigned)std::min<size_t>(((size_t)n * n + 255) / 256, (size_t)152 * 16);
-  for (int c = 0; c < n; c++) {
-    k_gj_pivot<<<1, kGjThreads, 0, s>>>(A, n, c, perm, prow, fcol, status); count_launch();
-    k_gj_elim<<<eb, 256, 0, s>>>(A, n, c, prow, fcol, status); count_launch();
+  const unsigned tiles = (n + kGjTile - 1) / kGjTile;
+  for (int c0 = 0; c0 < n;) {
+    int w = kGjW;
+    while (w > 1 && (long long)((n - c0) | 1) * w > (long long)kGjSmemRows * kGjW) w--;
+    if (w > n - c0) w = n - c0;
+    launch_dep(k_gj_panel, 1, kGjThreads, sizeof(double) * (size_t)((n - c0) | 1) * w, s, A, n, c0, w, perm, F, B, Dinv,
+               status);
+    launch_dep(k_gj_update, dim3(tiles, tiles), 256, 0, s, A, n, c0, w, (const double *)F, (const double *)B,
+               (const double *)Dinv, (const int *)status);
+    c0 += w;
   }
   int h_status = 0;
   std::vector<int> h_perm(n), map(n);
@@ -461,8 +597,46 @@ bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap,
   for (int q = 0; q < n; q++) map[q] = q;
   for (int c = n - 1; c >= 0; c--) std::swap(map[c], map[h_perm[c]]);
   cudaMemcpyAsync(colmap, map.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s);
+  const unsigned eb = (unsigned)std::min<size_t>(((size_t)n * n + 255) / 256, (size_t)152 * 16);
   k_gj_unpermute<<<eb, 256, 0, s>>>(A, n, colmap, out); count_launch();
   return cudaStreamSynchronize(s) == cudaSuccess;
+}
+
+// The coarsest level's dense matrix: row r of the m inverted cells idx[r] holds
+// the level's 19 weights at its neighbours' columns (cols; -1: a neighbour that
+// is not inverted, whose weight is zero) and sv0 / sv1 more at every column of
+// its own fluid region; a row with no region is an identity row.
+__global__ void __launch_bounds__(256) k_coarse_fill(int m, const int *__restrict__ region, double sv0, double sv1,
+                                                     double *__restrict__ A) {
+  dep_sync();
+  const size_t mm = (size_t)m * m;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < mm; e += (size_t)gridDim.x * blockDim.x) {
+    const int r = (int)(e / m), q = (int)(e % m), reg = region[r];
+    A[e] = reg >= 0 && reg == region[q] ? (reg ? sv1 : sv0) : 0.0;
+  }
+}
+__global__ void __launch_bounds__(128) k_coarse_rows(int m, int n, const int *__restrict__ idx,
+                                                     const int *__restrict__ region, const int *__restrict__ cols,
+                                                     const double *__restrict__ w, double *__restrict__ A) {
+  dep_sync();
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= m) return;
+  if (region[r] < 0) {
+    A[(size_t)r * m + r] = 1.0;
+    return;
+  }
+  const int p = idx[r];
+  for (int q = 0; q < NSLOT; q++) {
+    const int c = cols[r * NSLOT + q];
+    if (c >= 0) A[(size_t)r * m + c] += w[(size_t)q * n + p];
+  }
+}
+void launch_coarse_matrix(int m, int n, const int *idx, const int *region, const int *cols, double sv0, double sv1,
+                          const double *w64, double *A, cudaStream_t s) {
+  const size_t mm = (size_t)m * m;
+  launch_dep(k_coarse_fill, dim3((unsigned)std::min<size_t>((mm + 255) / 256, (size_t)152 * 16)), 256, 0, s, m, region,
+             sv0, sv1, A);
+  launch_dep(k_coarse_rows, dim3((m + 127) / 128), 128, 0, s, m, n, idx, region, cols, w64, A);
 }
 
 }  // namespace cvb
