@@ -1558,7 +1558,7 @@ int cvb_poisson_solver_mg(cvb_ctx *ctx, double *ucont, double fis, int immersed,
   TRY(cvb_volume_flux_rev(ctx, ucont, fis, immersed, &flux, &area));
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   const size_t n = F.g.n();
-  launch_poisson_rhs(F.g, ctx->uc_dev, ctx->aj64[ctx->nlevels - 1], F.nvert, dt, st, ctx->b, ctx->partial, ctx->stream);
+  launch_poisson_rhs(F.g, ctx->uc_dev, ctx->aj64[ctx->nlevels - 1], F.nvert, dt, st, ctx->b, nullptr, ctx->stream);
   CKL();
   cvb_solve_opts def;
   if (!o) { cvb_solve_opts_default(&def); o = &def; }
@@ -1586,10 +1586,19 @@ int cvb_update_pressure(cvb_ctx *ctx, double *p, double *phi) {
   return CVB_OK;
 }
 
+static int ensure_face_gram(cvb_ctx *ctx);
+// The face metric products for the projection, which does without where there is
+// no room for them.
+static int want_face_gram(cvb_ctx *ctx) {
+  const int rc = ensure_face_gram(ctx);
+  return rc == CVB_OOM ? CVB_OK : rc;
+}
+
 int cvb_projection(cvb_ctx *ctx, const double *phi, double dt, double st, double *ucont) {
   if (!ctx) return CVB_BAD_INPUT;
   if (!ctx->ready) return fail(ctx, CVB_NOT_SETUP, "cvb_setup_hierarchy has not run");
   if (!phi || !ucont) return fail(ctx, CVB_BAD_INPUT, "phi/ucont is NULL");
+  TRY(want_face_gram(ctx));
   int l = ctx->nlevels - 1;
   LevelDev &F = ctx->L[l];
   size_t n = F.g.n();
@@ -1597,7 +1606,8 @@ int cvb_projection(cvb_ctx *ctx, const double *phi, double dt, double st, double
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], F.nvert, ctx->w, dt, st, ctx->uc_dev, ctx->stream);
+  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame, F.nvert, F.code,
+                    ctx->w, dt, st, ctx->uc_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(ucont, ctx->uc_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1691,13 +1701,15 @@ int cvb_projection_cart(cvb_ctx *ctx, const double *phi, double dt, double st, d
   LevelDev &F = ctx->L[l];
   const size_t n = F.g.n();
   TRY(post_buffers(ctx, n));
+  TRY(want_face_gram(ctx));
   CK(cudaMemcpyAsync(ctx->w, phi, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->ubcs_dev, ubcs, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], F.nvert, ctx->w, dt, st, ctx->uc_dev, ctx->stream);
+  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame, F.nvert, F.code,
+                    ctx->w, dt, st, ctx->uc_dev, ctx->stream);
   launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   launch_ghost_node_velocity(F.g, bc, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev, ctx->ucat_dev, ctx->stream,
                              ctx->ibm_cent, ctx->u_bc);

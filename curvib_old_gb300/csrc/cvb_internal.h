@@ -271,8 +271,8 @@ void launch_ib_correct(const Geom &g, double *ucont, const double *csi, const do
                        double flux_intp_sum, int flg, cudaStream_t s);
 void launch_update_pressure(const Geom &g, double *p, double *phi, cudaStream_t s);
 void launch_projection(const Geom &g, const double *const *fm /*I,J,K csi/eta/zet*/, const double *iaj,
-                       const double *jaj, const double *kaj, const double *nvert, const double *phi,
-                       double dt, double st, double *ucont, cudaStream_t s);
+                       const double *jaj, const double *kaj, const double *gram, bool tame, const double *nvert,
+                       const uint32_t *code, const double *phi, double dt, double st, double *ucont, cudaStream_t s);
 // Immersed-body classification (kernels_ibm.cu).  The body's bounding box is
 // cut into kIbmBuckets^3 buckets (ibm.c:4213); a ray from a cell centre walks
 // one bucket column upward.

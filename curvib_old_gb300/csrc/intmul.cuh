@@ -101,6 +101,27 @@ __device__ __forceinline__ double int_triple(double x) {
   return __longlong_as_double((long long)((b & 0x8000000000000000ULL) + r + ((unsigned long long)(e + s - 1) << 52)));
 }
 
+// x 2^-K (K = 1, 2) as the FP64 multiply gives it: K less in the exponent field
+// while the result stays normal; a zero stays itself; subnormal results, inf
+// and NaN go through the multiply, out of line.
+static __device__ __noinline__ double scale_slow(double x, double f) { return __dmul_rn(x, f); }
+__device__ __forceinline__ double scale_down(double x, int K) {
+  const long long b = __double_as_longlong(x), e = (b >> 52) & 0x7ff;
+  if (e > K && e < 0x7ff) return __longlong_as_double(b - ((long long)K << 52));
+  if ((b & 0x7fffffffffffffffLL) == 0) return x;
+  return scale_slow(x, K == 1 ? 0.5 : 0.25);
+}
+template <int K>
+__device__ __forceinline__ double scale_down(double x) {
+  return scale_down(x, K);
+}
+
+// Whether v can be a right operand of int_mul (host).
+inline bool int_mul_factor(double v) {
+  const double a = v < 0 ? -v : v;
+  return a >= 0x1p-510 && a < 0x1p511;
+}
+
 // x / y rounded to nearest even for a divisor used many times, from rcp = 1 / y
 // rounded to nearest: x rcp, then twice the residual x - y q added back through
 // rcp.  The residual of a quotient within an ulp is exact in one fused

@@ -5,8 +5,6 @@
 // (--fmad=false, build.py), so every product and sum rounds on its own in the
 // order the expressions are written -- the reference's C order -- and the
 // results equal the reference's bit for bit.
-#include <cmath>
-
 #include "cvb_internal.h"
 #include "intmul.cuh"
 #include "launch.cuh"
@@ -41,21 +39,6 @@ __device__ __forceinline__ bool gt_01(double v) {
 __device__ __forceinline__ bool lt_01(double v) {
   const long long b = __double_as_longlong(v);
   return b < kBits01 && !(b > kBitsNegInf && b < 0);
-}
-
-// x * 2^-K (K = 1, 2) as the FP64 multiply gives it, on the integer pipe while
-// the result stays normal: K less in the exponent field; a zero stays itself;
-// subnormal results, inf and NaN go through the multiply, out of line.
-__device__ __noinline__ double scale_slow(double x, double f) { return x * f; }
-__device__ __forceinline__ double scale_down(double x, int K) {
-  const long long b = __double_as_longlong(x), e = (b >> 52) & 0x7ff;
-  if (e > K && e < 0x7ff) return __longlong_as_double(b - ((long long)K << 52));
-  if ((b & 0x7fffffffffffffffLL) == 0) return x;
-  return scale_slow(x, K == 1 ? 0.5 : 0.25);
-}
-template <int K>
-__device__ __forceinline__ double scale_down(double x) {
-  return scale_down(x, K);
 }
 
 struct FaceMetrics {
@@ -250,11 +233,6 @@ void launch_face_gram(const Geom &g, const double *const *fm, const double *iaj,
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
   k_face_gram<<<blocks_for(g.n(), 256), 256, 0, s>>>(g, M, gram, wild); count_launch();
-}
-
-// Whether v can be a right operand of int_mul.
-static bool int_mul_factor(double v) {
-  return std::fabs(v) >= std::ldexp(1., -510) && std::fabs(v) < std::ldexp(1., 511);
 }
 
 // tame: the grid's metrics are all in intmul.cuh's range (k_face_gram).  visc

@@ -49,3 +49,32 @@ def test_products_match_oracle(grid, values):
         assert rc == 0 and _same(u_g, u_o) and _same(r_g, r_o)
     finally:
         ctx.close()
+
+
+@pytest.mark.parametrize("values", ["plain", "edge"])
+@pytest.mark.parametrize("dt,st", [(1e-3, 1.0), (0.7, 0.3), (2.0**-520, 1.0), (1e-3, 2.0**515)])
+@pytest.mark.parametrize("name", ["box_sphere", "triply_periodic"])
+def test_projection_and_rhs_match_oracle(name, dt, st, values):
+    """PoissonRHS and Projection with ordinary and extreme time factors; the
+    fluxes and pressures ordinary or with values beside and beyond the range."""
+    from curvib_old_gb300.solver import PoissonContext
+    c = build(name)
+    rng = np.random.default_rng(7)
+    uc, phi = c["ucont"].copy(), rng.standard_normal(c["nvert"].shape)
+    if values == "edge":
+        for a in (phi, uc):
+            at = rng.choice(a.size, a.size // 40, replace=False)
+            a.ravel()[at] = rng.choice(EDGE, at.size)
+    P = types.SimpleNamespace(metrics=c["metrics"], nvert=c["nvert"], ucont=uc, bctype=c["bctype"], semi=c["semi"])
+    ctx = PoissonContext().setup(P)
+    try:
+        L = O.OLevel(c["metrics"][-1], c["nvert"], c["bctype"], c["semi"])
+        with np.errstate(all="ignore"):
+            b_o, _ = O.poisson_rhs(L, uc, dt, st)
+            b_g, _ = ctx.poisson_rhs(uc, dt, st)
+            _, phi_o, uc_o = O.update_and_project(L, np.zeros_like(phi), phi, uc, dt, st)
+            _, phi_g = ctx.update_pressure(np.zeros_like(phi), phi)
+            uc_g = ctx.projection(phi_g, dt, st, uc)
+        assert _same(b_g, b_o) and _same(phi_g, phi_o) and _same(uc_g, uc_o)
+    finally:
+        ctx.close()

@@ -122,3 +122,13 @@ def test_quotient_is_the_rounded_one():
             r = fma(fma(-y, r, x), rcp, r)
             r = fma(fma(-y, r, x), rcp, r)
             assert bits(r) == bits(x / y), (x, y)
+
+
+def test_quotient_by_three_halves_is_the_rounded_one():
+    """The projection's division by 1.5: one correction."""
+    rng = random.Random(4)
+    ms = list(significands(rng)) + [rng.getrandbits(52) for _ in range(20000)]
+    for p in ms:
+        x = value(rng.getrandbits(1) << 63 | rng.choice((623, 1022, 1023, 1422)) << 52 | p)
+        r = x * (2.0 / 3.0)
+        assert bits(fma(fma(-1.5, r, x), 2.0 / 3.0, r)) == bits(x / 1.5), x
