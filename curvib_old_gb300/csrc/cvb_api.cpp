@@ -1296,6 +1296,9 @@ void cvb_destroy(cvb_ctx *ctx) {
   if (ctx->ev0) cudaEventDestroy(ctx->ev0);
   if (ctx->ev1) cudaEventDestroy(ctx->ev1);
   if (ctx->bc_ev) cudaEventDestroy(ctx->bc_ev);
+  if (ctx->side_ev) cudaEventDestroy(ctx->side_ev);
+  if (ctx->main_ev) cudaEventDestroy(ctx->main_ev);
+  if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
 }
@@ -1482,6 +1485,68 @@ int cvb_get_nvert(cvb_ctx *ctx, int level, double *nvert, int *mns) {
   return CVB_OK;
 }
 
+}  // extern "C"
+
+namespace {
+// Host copies beside the context's kernels, on its second stream: what a call
+// needs late is copied in, and what it is done with early is copied out, while
+// its kernels run.  The stream starts after everything queued on the context's
+// (the buffers' allocations among it) and is drained before the call returns,
+// on every path, so that host arrays and buffers outlive their copies.  A copy
+// of pageable memory holds the host: kernels it should run beside are launched
+// before it.
+struct SideCopies {
+  cvb_ctx *ctx;
+  explicit SideCopies(cvb_ctx *c) : ctx(c) {}
+  SideCopies(const SideCopies &) = delete;
+  ~SideCopies() {
+    if (ctx->side) cudaStreamSynchronize(ctx->side);
+  }
+  int begin() {
+    if (!ctx->side) CK(cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+    if (!ctx->side_ev) CK(cudaEventCreateWithFlags(&ctx->side_ev, cudaEventDisableTiming));
+    if (!ctx->main_ev) CK(cudaEventCreateWithFlags(&ctx->main_ev, cudaEventDisableTiming));
+    return after_kernels();
+  }
+  // the copies that follow wait for the kernels launched so far
+  int after_kernels() {
+    CK(cudaEventRecord(ctx->main_ev, ctx->stream));
+    CK(cudaStreamWaitEvent(ctx->side, ctx->main_ev, 0));
+    return CVB_OK;
+  }
+  // the kernels that follow wait for the copies queued so far
+  int before_kernels() {
+    CK(cudaEventRecord(ctx->side_ev, ctx->side));
+    CK(cudaStreamWaitEvent(ctx->stream, ctx->side_ev, 0));
+    return CVB_OK;
+  }
+  int in(double *dev, const double *host, size_t count) {
+    CK(cudaMemcpyAsync(dev, host, sizeof(double) * count, cudaMemcpyHostToDevice, ctx->side));
+    return CVB_OK;
+  }
+  int out(double *host, const double *dev, size_t count) {
+    CK(cudaMemcpyAsync(host, dev, sizeof(double) * count, cudaMemcpyDeviceToHost, ctx->side));
+    return CVB_OK;
+  }
+  int finish() {
+    CK(cudaStreamSynchronize(ctx->side));
+    return CVB_OK;
+  }
+};
+
+// VolumeFlux_rev's correction of uc_dev.
+int volume_flux_dev(cvb_ctx *ctx, double fis, int flg) {
+  LevelDev &F = ctx->L[ctx->nlevels - 1];
+  launch_ib_sums(F.g, ctx->uc_dev, ctx->area3, nullptr, nullptr, F.nvert, ctx->partial, ctx->stream);
+  launch_finish_sums(ctx->partial, 2, reduce_blocks(), ctx->sums, ctx->stream);
+  launch_ib_correct(F.g, ctx->uc_dev, ctx->area3, nullptr, nullptr, F.nvert, ctx->sums, fis, flg, ctx->stream);
+  CKL();
+  return CVB_OK;
+}
+}  // namespace
+
+extern "C" {
+
 int cvb_volume_flux_rev(cvb_ctx *ctx, double *ucont, double fis, int flg, double *flux, double *area) {
   if (!ctx) return CVB_BAD_INPUT;
   if (!ctx->ready) return fail(ctx, CVB_NOT_SETUP, "cvb_setup_hierarchy has not run");
@@ -1489,9 +1554,7 @@ int cvb_volume_flux_rev(cvb_ctx *ctx, double *ucont, double fis, int flg, double
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   size_t n = F.g.n();
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  launch_ib_sums(F.g, ctx->uc_dev, ctx->area3, nullptr, nullptr, F.nvert, ctx->partial, ctx->stream);
-  launch_finish_sums(ctx->partial, 2, reduce_blocks(), ctx->sums, ctx->stream);
-  launch_ib_correct(F.g, ctx->uc_dev, ctx->area3, nullptr, nullptr, F.nvert, ctx->sums, fis, flg, ctx->stream);
+  TRY(volume_flux_dev(ctx, fis, flg));
   launch_ib_sums(F.g, ctx->uc_dev, ctx->area3, nullptr, nullptr, F.nvert, ctx->partial, ctx->stream);
   CKL();
   double fa[2];
@@ -1554,10 +1617,16 @@ int cvb_poisson_solver_mg(cvb_ctx *ctx, double *ucont, double fis, int immersed,
                           const cvb_solve_opts *o, cvb_solve_stats *stats) {
   if (!ctx) return CVB_BAD_INPUT;
   if (!phi || !(dt != 0.0) || !(st != 0.0)) return fail(ctx, CVB_BAD_INPUT, "bad PoissonSolver_MG arguments");
-  double flux, area;
-  TRY(cvb_volume_flux_rev(ctx, ucont, fis, immersed, &flux, &area));
+  if (!ctx->ready) return fail(ctx, CVB_NOT_SETUP, "cvb_setup_hierarchy has not run");
+  if (!ucont) return fail(ctx, CVB_BAD_INPUT, "ucont is NULL");
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   const size_t n = F.g.n();
+  SideCopies side(ctx);
+  CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
+  TRY(volume_flux_dev(ctx, fis, immersed));
+  // the corrected fluxes go out while the solve runs
+  TRY(side.begin());
+  TRY(side.out(ucont, ctx->uc_dev, 3 * n));
   launch_poisson_rhs(F.g, ctx->uc_dev, ctx->aj64[ctx->nlevels - 1], F.nvert, dt, st, ctx->b, nullptr, ctx->stream);
   CKL();
   cvb_solve_opts def;
@@ -1567,6 +1636,7 @@ int cvb_poisson_solver_mg(cvb_ctx *ctx, double *ucont, double fis, int immersed,
   if (rc == CVB_OK || rc == CVB_NOT_CONVERGED)
     CK(cudaMemcpyAsync(phi, ctx->x, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
+  TRY(side.finish());
   return rc;
 }
 
@@ -1581,7 +1651,8 @@ int cvb_update_pressure(cvb_ctx *ctx, double *p, double *phi) {
   launch_update_pressure(F.g, ctx->p_dev, ctx->w, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(p, ctx->p_dev, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(phi, ctx->w, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
+  if (F.g.px || F.g.py || F.g.pz)  // only the periodic images change phi
+    CK(cudaMemcpyAsync(phi, ctx->w, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   return CVB_OK;
 }
@@ -1702,23 +1773,31 @@ int cvb_projection_cart(cvb_ctx *ctx, const double *phi, double dt, double st, d
   const size_t n = F.g.n();
   TRY(post_buffers(ctx, n));
   TRY(want_face_gram(ctx));
+  SideCopies side(ctx);
   CK(cudaMemcpyAsync(ctx->w, phi, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->ubcs_dev, ubcs, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
+  TRY(side.begin());  // after the copies in: they would share the link
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame, F.nvert, F.code,
                     ctx->w, dt, st, ctx->uc_dev, ctx->stream);
+  CK(cudaEventRecord(ctx->main_ev, ctx->stream));  // uc_dev is final
+  TRY(side.in(ctx->ucat_dev, ucat, 3 * n));
+  TRY(side.before_kernels());
   launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
-  launch_ghost_node_velocity(F.g, bc, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev, ctx->ucat_dev, ctx->stream,
-                             ctx->ibm_cent, ctx->u_bc);
+  TRY(side.in(ctx->ubcs_dev, ubcs, 3 * n));
+  TRY(side.before_kernels());
+  const bool ubcs_written =
+      launch_ghost_node_velocity(F.g, bc, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev, ctx->ucat_dev, ctx->stream,
+                                 ctx->ibm_cent, ctx->u_bc);
   CKL();
-  CK(cudaMemcpyAsync(ucont, ctx->uc_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(ubcs, ctx->ubcs_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(ucat, ctx->ucat_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamWaitEvent(ctx->side, ctx->main_ev, 0));
+  TRY(side.out(ucont, ctx->uc_dev, 3 * n));
+  TRY(side.after_kernels());
+  if (ubcs_written) TRY(side.out(ubcs, ctx->ubcs_dev, 3 * n));
+  TRY(side.out(ucat, ctx->ucat_dev, 3 * n));
   CK(cudaStreamSynchronize(ctx->stream));
-  return CVB_OK;
+  return side.finish();
 }
 
 int cvb_convection(cvb_ctx *ctx, const double *ucont, const double *ucat, int central, double *conv) {
@@ -1787,9 +1866,9 @@ static int ensure_face_gram(cvb_ctx *ctx) {
   return CVB_OK;
 }
 
-// Device inputs of FormFunction1 / CalcRHS on the finest level: ucont, ucat,
-// p and the incoming rhs copied in (NULL ucont / ucat: the device copies the
-// last projection left), the scratch allocated on first use.
+// Device inputs of FormFunction1 / CalcRHS on the finest level: ucont and ucat
+// copied in (NULL: the device copies the last projection left), the scratch
+// allocated on first use.
 static int momentum_prepare(cvb_ctx *ctx, const char *who, const double *ucont, const double *ucat, const double *p,
                             const double *rhs) {
   if (!ctx) return CVB_BAD_INPUT;
@@ -1809,17 +1888,17 @@ static int momentum_prepare(cvb_ctx *ctx, const char *who, const double *ucont, 
   TRY(ensure_face_gram(ctx));
   if (ucont) CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   if (ucat) CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->p_dev, p, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->rhs_dev, rhs, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   return CVB_OK;
 }
 
-// FormFunction1's kernels on the device copies: Contra2Cart, Convection,
-// Viscous, then the face values into rhs_dev; with calc, CalcRHS's.
+// FormFunction1's kernels on the device copies: the first half Contra2Cart,
+// Convection and Viscous's faces (of ucont and ucat), the second the face values
+// into rhs_dev, with calc CalcRHS's (which also read p, rhs_dev's ring and
+// calc's fluxes).
 // cart = false: ucat's interior already holds Contra2Cart of the current
 // ucont (FormBCS ran it), so FormFunction1's own call would rewrite the same
 // values.
-static void momentum_ff1(cvb_ctx *ctx, double ren, int central, const MomentumTime *calc, bool cart = true) {
+static void momentum_faces(cvb_ctx *ctx, double ren, int central, bool cart = true) {
   const int l = ctx->nlevels - 1;
   LevelDev &F = ctx->L[l];
   const double *fm[9];
@@ -1829,18 +1908,43 @@ static void momentum_ff1(cvb_ctx *ctx, double ren, int central, const MomentumTi
   launch_convection(F.g, ctx->uc_dev, ctx->ucat_dev, F.nvert, central != 0, ctx->conv_fp, ctx->conv_dev, ctx->stream);
   launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
                  ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, nullptr, ctx->stream);
+}
+static void momentum_rhs(cvb_ctx *ctx, const MomentumTime *calc) {
+  const int l = ctx->nlevels - 1;
+  LevelDev &F = ctx->L[l];
+  const double *fm[9];
+  for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   launch_form_function1(F.g, F.nvert, ctx->p_dev, ctx->conv_dev, ctx->conv_fp, ctx->cm[0], ctx->cm[1], ctx->cm[2],
                         ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame,
                         calc, ctx->rct_dev, ctx->rhs_dev, ctx->stream);
 }
 
-static int momentum_finish(cvb_ctx *ctx, double *ucat, double *rhs) {
+// FormFunction1 or (calc) CalcRHS from host arrays once ucont and ucat are on
+// their way in: p, the incoming rhs and calc's fluxes (uo, urm on the host) come
+// in while Contra2Cart, Convection and Viscous run, and ucat goes out beside the
+// last kernels.  CalcRHS at 192^3 from pinned arrays: 11.5 ms with the copies
+// before and after the kernels, 8.2 so (5.3 ms of kernels).
+static int momentum_call(cvb_ctx *ctx, double ren, int central, const MomentumTime *calc, const double *uo,
+                         const double *urm, const double *p, double *ucat, double *rhs) {
   const size_t n = ctx->L[ctx->nlevels - 1].g.n();
+  SideCopies side(ctx);
+  TRY(side.begin());  // after the copies in: they would share the link
+  momentum_faces(ctx, ren, central);
   CKL();
+  TRY(side.in(ctx->p_dev, p, n));
+  TRY(side.in(ctx->rhs_dev, rhs, 3 * n));
+  if (calc) {
+    TRY(side.in(ctx->uo_dev, uo, 3 * n));
+    if (calc->bdf2) TRY(side.in(ctx->urm_dev, urm, 3 * n));
+  }
+  TRY(side.before_kernels());
+  TRY(side.after_kernels());
+  momentum_rhs(ctx, calc);
+  CKL();
+  if (ucat) TRY(side.out(ucat, ctx->ucat_dev, 3 * n));
   CK(cudaMemcpyAsync(rhs, ctx->rhs_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  if (ucat) CK(cudaMemcpyAsync(ucat, ctx->ucat_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  return CVB_OK;
+  return side.finish();
 }
 
 int cvb_viscous(cvb_ctx *ctx, const double *ucat, double ren, double *visc) {
@@ -1872,8 +1976,7 @@ int cvb_form_function1(cvb_ctx *ctx, const double *ucont, double *ucat, const do
                        double *rhs) {
   TRY(momentum_prepare(ctx, "FormFunction1", ucont, ucat, p, rhs));
   if (!(ren != 0.0)) return fail(ctx, CVB_BAD_INPUT, "FormFunction1: ren is 0");
-  momentum_ff1(ctx, ren, central, nullptr);
-  return momentum_finish(ctx, ucat, rhs);
+  return momentum_call(ctx, ren, central, nullptr, nullptr, nullptr, p, ucat, rhs);
 }
 
 int cvb_calc_rhs(cvb_ctx *ctx, const double *ucont, const double *ucont_o, const double *ucont_rm1, double *ucat,
@@ -1886,15 +1989,12 @@ int cvb_calc_rhs(cvb_ctx *ctx, const double *ucont, const double *ucont_o, const
   const size_t n = F.g.n();
   if (!ctx->uo_dev) TRY(dalloc(ctx, &ctx->uo_dev, 3 * n));
   if (!ctx->urm_dev) TRY(dalloc(ctx, &ctx->urm_dev, 3 * n));
-  CK(cudaMemcpyAsync(ctx->uo_dev, ucont_o, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->urm_dev, ucont_rm1, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   // COEF_TIME_ACCURACY is 1.5 in the reference (variables.h:421): second-order
   // backward except on the first step
   const int bdf2 = (ti != tistart && ti != 1) ? 1 : 0;
   const int mz_end = ctx->H[l].d.bctype[5] == 8 ? F.g.mz - 2 : F.g.mz - 3;
   const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end};
-  momentum_ff1(ctx, ren, central, &calc);
-  return momentum_finish(ctx, ucat, rhs);
+  return momentum_call(ctx, ren, central, &calc, ucont_o, ucont_rm1, p, ucat, rhs);
 }
 
 // --- InflowFlux, FormBCS and ImpRK --------------------------------------------
@@ -2269,7 +2369,10 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   const int bdf2 = (ti != tistart && ti != 1) ? 1 : 0;  // COEF_TIME_ACCURACY 1.5 (variables.h:421)
   const int mz_end = F.g.mz - 3;                        // no convective outflow on an all-wall box
   const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, bdf2, -1. / dt, mz_end};
-  auto calc_rhs = [&]() { momentum_ff1(ctx, ren, central, &calc, false); };
+  auto calc_rhs = [&]() {
+    momentum_faces(ctx, ren, central, false);
+    momentum_rhs(ctx, &calc);
+  };
   // before the loop (implicitsolver.c:7124-7148): the boundary conditions,
   // pUcont = Ucont, CalcRHS
   if (inlet) TRY(inflow_dev(ctx, uin, bs));
@@ -2804,7 +2907,8 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
       }
       case CVB_KERNEL_MOMENTUM_RHS: {
         const MomentumTime calc = {ctx->uc_dev, ctx->uo_dev, ctx->urm_dev, 1, -1. / 2e-3, L.g.mz - 3};
-        momentum_ff1(ctx, 300., 0, &calc);
+        momentum_faces(ctx, 300., 0);
+        momentum_rhs(ctx, &calc);
         break;
       }
       default: launch_zebra_half<double>(L, L.r64, L.e64, L.t64 + n, 1.3, 1, false, ctx->stream); break;

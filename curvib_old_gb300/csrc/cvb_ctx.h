@@ -116,6 +116,9 @@ struct cvb_ctx {
   double u_bc = 0.;                        // GhostNodeVelocity: the rheology plates' velocity (bcs.c's U_bc)
   double *ibm_cent = nullptr;  // cell centres of the last cvb_ibm_search that gave them
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+  // a second stream for host copies beside the kernels (SideCopies), on first use
+  cudaStream_t side = nullptr;
+  cudaEvent_t side_ev = nullptr, main_ev = nullptr;
   bool ready = false;
   // changes with every set-up of the operators (process-wide counter): the
   // batch engine's captured V-cycles are valid for one value

@@ -343,8 +343,8 @@ void launch_form_function1(const Geom &g, const double *nvert, const double *p, 
                            double *rhs, cudaStream_t s);
 // bc: the level's bctype[6]; the host has refused the types it does not cover.
 // cent: the cell centres ([N][3]) an annulus face needs; u_bc: the rheology
-// plates' velocity
-void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi, const double *eta,
+// plates' velocity.  Returns whether any face's type writes ubcs
+bool launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi, const double *eta,
                                 const double *zet, double *ubcs, double *ucat, cudaStream_t s,
                                 const double *cent = nullptr, double u_bc = 0.);
 // FormBCS with walls on the x and y faces: the ghost faces' interior cells and

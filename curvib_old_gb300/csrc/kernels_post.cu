@@ -434,7 +434,7 @@ static void face_grid(const Geom &g, int axis, int faces, dim3 &grd, dim3 &blk) 
   grd = dim3(nblk(na, 32), nblk(nb, 8), faces);
 }
 
-void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi, const double *eta,
+bool launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi, const double *eta,
                                 const double *zet, double *ubcs, double *ucat, cudaStream_t s, const double *cent,
                                 double u_bc) {
   GhostArgs A;
@@ -473,6 +473,7 @@ void launch_ghost_node_velocity(const Geom &g, const int *bc, const double *csi,
     k_ghost_ring<<<grd, blk, 0, s>>>(A, axis, 1);
     count_launch();
   }
+  return special;
 }
 
 // ------------------------------------------------------------------- FormBCS
