@@ -147,10 +147,12 @@ static void free_all(cvb_ctx *ctx) {
   ctx->cidx = nullptr;
   ctx->b = ctx->x = ctx->w = ctx->r = nullptr;
   for (int q = 0; q <= kMaxRestart; q++) ctx->V[q] = nullptr;
-  for (int q = 0; q < kMaxRestart; q++) { ctx->Z64[q] = nullptr; ctx->Z32[q] = nullptr; }
+  for (int q = 0; q < kMaxRestart; q++) ctx->Z64[q] = nullptr;
+  ctx->Z32 = nullptr;
   ctx->b32 = nullptr;
-  ctx->dV = nullptr; ctx->dZ64 = nullptr; ctx->dZ32 = nullptr;
-  ctx->partial = ctx->sums = ctx->hdev = nullptr;
+  ctx->dV = nullptr; ctx->dZ64 = nullptr;
+  ctx->partial = ctx->sums = nullptr;
+  ctx->red_counter = nullptr;
   ctx->uc_dev = ctx->p_dev = nullptr;
   ctx->ucat_dev = ctx->ubcs_dev = nullptr;
   ctx->conv_dev = ctx->conv_fp = nullptr;
@@ -841,28 +843,48 @@ static int reduce_to_host(cvb_ctx *ctx, int nv, double *out) {
   return CVB_OK;
 }
 
-static int norm2(cvb_ctx *ctx, const double *v, size_t n, double *out) {
-  // dot(v, v) with the multi-dot kernel; its one-entry pointer table is dV[kMaxRestart + 1]
-  CK(cudaMemcpyAsync(ctx->dV + kMaxRestart + 1, &v, sizeof(double *), cudaMemcpyHostToDevice, ctx->stream));
-  launch_multidot(ctx->dV + kMaxRestart + 1, 1, v, n, ctx->partial, ctx->stream);
-  CKL();
-  double s;
-  TRY(reduce_to_host(ctx, 1, &s));
-  *out = std::sqrt(s);
-  return CVB_OK;
-}
+// The solver's scalars on the device: the dots, a norm (its square, 1 / its root)
+// and a mean; and in pinned host memory what the host reads of them.
+static double *dev_dots(cvb_ctx *ctx) { return ctx->sums; }
+static double *dev_norm(cvb_ctx *ctx) { return ctx->sums + kMaxRestart + 2; }
+static double *dev_mean(cvb_ctx *ctx) { return ctx->sums + kMaxRestart + 4; }
 
 static int fluid_mean_zero(cvb_ctx *ctx, int level, double *x) {
   LevelDev &L = ctx->L[level];
-  launch_fluid_mean_partial(L.g, L.code, x, ctx->partial, ctx->stream);
-  launch_finish_sums(ctx->partial, 2, reduce_blocks(), ctx->sums, ctx->stream);
-  launch_add_fluid_const(L.g, L.code, x, ctx->sums, 1, ctx->stream);
+  launch_fluid_mean(L.g, L.code, x, nullptr, -1.0, ctx->partial, ctx->red_counter, dev_mean(ctx), ctx->stream);
+  launch_add_fluid_const(L.g, L.code, x, dev_mean(ctx), 1, ctx->stream);
   CKL();
   return CVB_OK;
 }
 
-// Projects b onto range(A): b -= aj * (sum_fluid b/aj) / n_fluid on fluid cells.
-static int project_rhs(cvb_ctx *ctx, double *b, double *removed);
+static int ensure_scalars(cvb_ctx *ctx) {
+  if (!ctx->kry_host) CK(cudaMallocHost((void **)&ctx->kry_host, sizeof(double) * (kMaxRestart + 4)));
+  if (!ctx->kry_ev) CK(cudaEventCreateWithFlags(&ctx->kry_ev, cudaEventDisableTiming));
+  return CVB_OK;
+}
+static int norm2(cvb_ctx *ctx, const double *v, size_t n, double *out) {
+  launch_norm(v, n, ctx->partial, ctx->red_counter, dev_norm(ctx), ctx->kry_host, ctx->stream);
+  CKL();
+  CK(cudaStreamSynchronize(ctx->stream));
+  *out = std::sqrt(ctx->kry_host[0]);
+  return CVB_OK;
+}
+
+// The right-hand side's norm, with `project` after its projection onto range(A):
+// b -= aj * (sum_fluid b/aj) / n_fluid on fluid cells (*removed: the mean).
+static int rhs_norm(cvb_ctx *ctx, bool project, double *bnorm, double *removed) {
+  LevelDev &F = ctx->L[ctx->nlevels - 1];
+  if (!project) return norm2(ctx, ctx->b, F.g.n(), bnorm);
+  launch_fluid_mean(F.g, F.code, ctx->b, ctx->inv_aj, 1.0, ctx->partial, ctx->red_counter, dev_mean(ctx),
+                    ctx->stream);
+  launch_remove_mean(F.g, F.code, ctx->aj64[ctx->nlevels - 1], ctx->b, dev_mean(ctx), ctx->partial, ctx->red_counter,
+                     dev_norm(ctx), ctx->kry_host, ctx->stream);
+  CKL();
+  CK(cudaStreamSynchronize(ctx->stream));
+  *removed = ctx->kry_host[0];
+  *bnorm = std::sqrt(ctx->kry_host[1]);
+  return CVB_OK;
+}
 
 static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
   LevelDev &F = ctx->L[ctx->nlevels - 1];
@@ -870,8 +892,12 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
   cudaStream_t s = ctx->stream;
   const bool mixed = o->precision == CVB_PRECISION_MIXED;
   const int m = std::min(std::max(o->restart, 1), kMaxRestart);
+  BasisList V, Z;
+  for (int q = 0; q <= m; q++) V.v[q] = ctx->V[q];
+  for (int q = 0; q < m; q++) Z.v[q] = ctx->Z64[q];
+  TRY(ensure_scalars(ctx));
   double bnorm;
-  TRY(norm2(ctx, ctx->b, n, &bnorm));
+  TRY(rhs_norm(ctx, o->project_rhs != 0, &bnorm, &st->rhs_projected));
   st->rhs_norm = bnorm;
   if (!std::isfinite(bnorm)) return fail(ctx, CVB_NAN_DETECTED, "right-hand side is not finite");
   if (bnorm == 0.0) {
@@ -901,11 +927,10 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
     if (!std::isfinite(beta)) return fail(ctx, CVB_NAN_DETECTED, "residual became %g", beta);
     if (beta <= target) { status = CVB_OK; break; }
     if (total >= o->max_it) break;
-    // V[0] = r / beta (k_scale divides by the device scalar)
-    CK(cudaMemcpyAsync(ctx->hdev, &beta, sizeof(double), cudaMemcpyHostToDevice, s));
-    // in mixed precision the scaling also writes the V-cycle's FP32 input
+    // V[0] = r / beta, by the reciprocal that the norm left on the device; in mixed
+    // precision the scaling also writes the V-cycle's FP32 input
     float *in32 = mixed ? ctx->b32 : nullptr;
-    launch_scale(ctx->V[0], rcur, ctx->hdev, n, s, nullptr, in32);
+    launch_scale(ctx->V[0], rcur, dev_norm(ctx) + 1, n, in32, s);
     CKL();
     for (int q = 0; q <= m; q++) gv[q] = 0.0;
     gv[0] = beta;
@@ -917,9 +942,10 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
         // ctx->b32 holds V[j] in FP32 (written by the scaling that formed V[j])
         // FP32 V-cycle; its result is widened once into the FP64 basis so the
         // FP64 operator and the final update read it without per-use conversions
-        // (a conversion costs an FP64-pipe instruction on this part)
-        TRY(vcycle_graph<float>(ctx, o, 0, ctx->b32, ctx->Z32[0]));
-        launch_f32_to_f64(ctx->Z32[0], ctx->Z64[j], n, s);
+        // (the operator on the FP32 vector, widening on the integer pipe and
+        // keeping an FP32 basis, took 73 us at 4.4 M cells against 62 + 9)
+        TRY(vcycle_graph<float>(ctx, o, 0, ctx->b32, ctx->Z32));
+        launch_f32_to_f64(ctx->Z32, ctx->Z64[j], n, s);
         launch_apply<double>(F, ctx->Z64[j], ctx->w, s);
       } else {
         TRY(vcycle_graph<double>(ctx, o, j, ctx->V[j], ctx->Z64[j]));
@@ -935,30 +961,24 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
       // save a pass, but on a basis whose orthogonality classical Gram-Schmidt
       // has eroded it is off by far more than rounding, and FGMRES then needed
       // 32 iterations instead of 6 on the channel.
+      // The event is recorded before the scaling, so the host works beside it.
       double h[kMaxRestart + 2], h2[kMaxRestart + 1], nw2;
-      double *dsum = ctx->sums, *dnorm = ctx->sums + kMaxRestart + 2;
-      launch_multidot(ctx->dV, j + 1, ctx->w, n, ctx->partial, s, 1);
-      launch_finish_sums(ctx->partial, j + 2, reduce_blocks(), dsum, s);
-      launch_multiaxpy_norm(ctx->w, ctx->dV, dsum, j + 1, n, ctx->partial, s);
-      launch_finish_sums(ctx->partial, 1, reduce_blocks(), dnorm, s);
-      launch_scale_sqrt(ctx->V[j + 1], ctx->w, dnorm, n, s, in32);
-      CKL();
-      CK(cudaMemcpyAsync(h, dsum, sizeof(double) * (j + 2), cudaMemcpyDeviceToHost, s));
-      CK(cudaMemcpyAsync(&nw2, dnorm, sizeof(double), cudaMemcpyDeviceToHost, s));
-      CK(cudaStreamSynchronize(s));
-      const double w_before = h[j + 1];
-      for (int q = 0; q <= j; q++) h2[q] = 0.0;
-      if (o->cgs_refine && nw2 < 0.25 * w_before) {
-        launch_multidot(ctx->dV, j + 1, ctx->w, n, ctx->partial, s);
-        launch_finish_sums(ctx->partial, j + 1, reduce_blocks(), dsum, s);
-        launch_multiaxpy_norm(ctx->w, ctx->dV, dsum, j + 1, n, ctx->partial, s);
-        launch_finish_sums(ctx->partial, 1, reduce_blocks(), dnorm, s);
-        launch_scale_sqrt(ctx->V[j + 1], ctx->w, dnorm, n, s, in32);
+      auto gram_schmidt = [&](double *hq) -> int {
+        launch_dots(V, j + 1, ctx->w, n, ctx->partial, ctx->red_counter, dev_dots(ctx), s);
+        launch_orthogonalise(ctx->w, V, dev_dots(ctx), j + 1, n, ctx->partial, ctx->red_counter, dev_norm(ctx),
+                             ctx->kry_host, s);
+        CK(cudaEventRecord(ctx->kry_ev, s));
+        launch_scale(ctx->V[j + 1], ctx->w, dev_norm(ctx) + 1, n, in32, s);
         CKL();
-        CK(cudaMemcpyAsync(h2, dsum, sizeof(double) * (j + 1), cudaMemcpyDeviceToHost, s));
-        CK(cudaMemcpyAsync(&nw2, dnorm, sizeof(double), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-      }
+        CK(cudaEventSynchronize(ctx->kry_ev));
+        std::copy(ctx->kry_host, ctx->kry_host + j + 1, hq);
+        nw2 = ctx->kry_host[j + 1];
+        return CVB_OK;
+      };
+      TRY(gram_schmidt(h));
+      double w_before = nw2;  // |w|^2 before: Pythagoras is enough for the question asked of it
+      for (int q = 0; q <= j; q++) w_before += h[q] * h[q], h2[q] = 0.0;
+      if (o->cgs_refine && nw2 < 0.25 * w_before) TRY(gram_schmidt(h2));
       for (int q = 0; q <= j; q++) H[q][j] = h[q] + h2[q];
       double hn = std::sqrt(nw2);
       H[j + 1][j] = hn;
@@ -987,8 +1007,9 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
       for (int c2 = q + 1; c2 < j; c2++) t -= H[q][c2] * yv[c2];
       yv[q] = t / H[q][q];
     }
-    CK(cudaMemcpyAsync(ctx->hdev, yv, sizeof(double) * j, cudaMemcpyHostToDevice, s));
-    launch_axpy_z(ctx->x, nullptr, ctx->dZ64, ctx->hdev, j, n, s);
+    BasisWeights y;
+    std::copy(yv, yv + j, y.y);
+    launch_axpy_z(ctx->x, Z, y, j, n, s);
     launch_residual<double>(F, ctx->b, ctx->x, ctx->r, s);
     CKL();
     TRY(norm2(ctx, ctx->r, n, &beta));
@@ -1006,22 +1027,6 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
   return CVB_OK;
 }
 
-static int project_rhs(cvb_ctx *ctx, double *b, double *removed) {
-  int l = ctx->nlevels - 1;
-  LevelDev &F = ctx->L[l];
-  launch_fluid_ratio_partial(F.g, F.code, b, ctx->inv_aj, ctx->partial, ctx->stream);
-  launch_finish_sums(ctx->partial, 2, reduce_blocks(), ctx->sums, ctx->stream);
-  launch_remove_aj_mean(F.g, F.code, ctx->aj64[l], b, ctx->sums, ctx->stream);
-  CKL();
-  double h[2];
-  CK(cudaMemcpyAsync(h, ctx->sums, sizeof(double) * 2, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
-  // h = {sum b/aj, fluid count}; the removed part is aj * mean(b/aj) on fluid cells
-  double c = h[1] > 0 ? h[0] / h[1] : 0.0;
-  *removed = c;
-  return CVB_OK;
-}
-
 static int solve_resident(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
   if (!ctx->ready) return fail(ctx, CVB_NOT_SETUP, "cvb_setup_hierarchy has not run");
   cvb_solve_opts def;
@@ -1034,7 +1039,6 @@ static int solve_resident(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats
   if (!st) st = &local;
   std::memset(st, 0, sizeof(*st));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
-  if (o->project_rhs) TRY(project_rhs(ctx, ctx->b, &st->rhs_projected));
   int rc = fgmres(ctx, o, st);
   cudaEventRecord(ctx->ev1, ctx->stream);
   cudaEventSynchronize(ctx->ev1);
@@ -1139,11 +1143,11 @@ static int setup_problem(cvb_ctx *ctx, const double *nvert_box) {
   TRY(dalloc(ctx, &ctx->uc_dev, 3 * n)); TRY(dalloc(ctx, &ctx->p_dev, n));
   TRY(dalloc(ctx, &ctx->dV, kMaxRestart + 2));
   TRY(dalloc(ctx, &ctx->dZ64, kMaxRestart));
-  TRY(dalloc(ctx, &ctx->dZ32, kMaxRestart));
   int nb = reduce_blocks();
   TRY(dalloc(ctx, &ctx->partial, (size_t)nb * (kMaxRestart + 2)));
   TRY(dalloc(ctx, &ctx->sums, 2 * (kMaxRestart + 2)));
-  TRY(dalloc(ctx, &ctx->hdev, kMaxRestart + 2));
+  TRY(dalloc(ctx, &ctx->red_counter, 1));
+  CK(cudaMemsetAsync(ctx->red_counter, 0, sizeof(unsigned), ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
   ctx->setup_ms[1] = ms_since(t);
   t = clk::now();
@@ -1298,6 +1302,8 @@ void cvb_destroy(cvb_ctx *ctx) {
   if (ctx->bc_ev) cudaEventDestroy(ctx->bc_ev);
   if (ctx->side_ev) cudaEventDestroy(ctx->side_ev);
   if (ctx->main_ev) cudaEventDestroy(ctx->main_ev);
+  if (ctx->kry_ev) cudaEventDestroy(ctx->kry_ev);
+  if (ctx->kry_host) cudaFreeHost(ctx->kry_host);
   if (ctx->side) cudaStreamDestroy(ctx->side);
   if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -1409,11 +1415,10 @@ int cvb_ensure_basis(cvb_ctx *ctx, int m, bool mixed) {
     if (!ctx->V[q]) { TRY(dalloc(ctx, &ctx->V[q], n)); changed = true; }
   for (int q = 0; q < m; q++)
     if (!ctx->Z64[q]) { TRY(dalloc(ctx, &ctx->Z64[q], n)); changed = true; }
-  if (mixed && !ctx->Z32[0]) { TRY(dalloc(ctx, &ctx->Z32[0], n)); changed = true; }
+  if (mixed && !ctx->Z32) TRY(dalloc(ctx, &ctx->Z32, n));
   if (changed) {
     CK(cudaMemcpyAsync(ctx->dV, ctx->V, sizeof(double *) * (kMaxRestart + 1), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->dZ64, ctx->Z64, sizeof(double *) * kMaxRestart, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->dZ32, ctx->Z32, sizeof(float *) * kMaxRestart, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
   }
   return CVB_OK;

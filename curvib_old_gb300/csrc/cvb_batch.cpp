@@ -640,8 +640,8 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
       const LevelDev *dLs = dlev(bt, p->slot);
       if (f32) {
         conv.add(task(nullptr, c->V[j], nullptr, c->b32, gate, elem_blocks(n), 0, (int)n), elem_blocks(n));
-        gen_vcycle<float>(vs, c, dLs, nl - 1, 0, c->b32, c->Z32[0], bt->opts, gate);
-        widen.add(task(nullptr, c->Z32[0], nullptr, c->Z64[j], gate, elem_blocks(n), 0, (int)n), elem_blocks(n));
+        gen_vcycle<float>(vs, c, dLs, nl - 1, 0, c->b32, c->Z32, bt->opts, gate);
+        widen.add(task(nullptr, c->Z32, nullptr, c->Z64[j], gate, elem_blocks(n), 0, (int)n), elem_blocks(n));
       } else {
         gen_vcycle<double>(vs, c, dLs, nl - 1, 0, c->V[j], c->Z64[j], bt->opts, gate);
       }

@@ -88,12 +88,14 @@ struct cvb_ctx {
   double *b = nullptr, *x = nullptr, *w = nullptr, *r = nullptr;
   double *V[cvb::kMaxRestart + 1] = {};
   double *Z64[cvb::kMaxRestart] = {};
-  float *Z32[cvb::kMaxRestart] = {};
+  float *Z32 = nullptr;  // the FP32 V-cycle's output
   float *b32 = nullptr;
   double **dV = nullptr;  // device copies of the pointer tables
   double **dZ64 = nullptr;
-  float **dZ32 = nullptr;
-  double *partial = nullptr, *sums = nullptr, *hdev = nullptr;
+  double *partial = nullptr, *sums = nullptr;
+  unsigned *red_counter = nullptr;  // blocks that have stored their partial sums (zero between kernels)
+  double *kry_host = nullptr;       // the solver's scalars as the host reads them (pinned, on first use)
+  cudaEvent_t kry_ev = nullptr;
   double *uc_dev = nullptr, *p_dev = nullptr;
   double *ucat_dev = nullptr, *ubcs_dev = nullptr;  // Contra2Cart / GhostNodeVelocity (allocated on first use)
   double *conv_dev = nullptr, *conv_fp = nullptr;    // Convection: result and face fluxes (allocated on first use)
@@ -134,6 +136,6 @@ struct cvb_ctx {
   std::vector<Tune> tune;
 };
 
-// Allocates the finest level's FGMRES basis V[0..m], Z[0..m-1] (and the FP32
-// V-cycle output in mixed precision) if missing, and refreshes the device tables.
+// Allocates the finest level's FGMRES basis V[0..m], Z[0..m-1] and the FP32
+// V-cycle output of mixed precision if missing, and refreshes the device tables.
 int cvb_ensure_basis(cvb_ctx *ctx, int m, bool mixed);

@@ -192,45 +192,51 @@ template <typename T>
 void launch_prolong_add(const LevelDev &C, const LevelDev &F, const T *xc, T *xf, cudaStream_t s);
 
 // mixed-precision glue: FP64 operator on an FP32-stored vector
-void launch_apply64_from32(const LevelDev &L, const float *x, double *y, cudaStream_t s);
-void launch_f64_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate = nullptr);
-void launch_f32_to_f64(const float *a, double *b, size_t n, cudaStream_t s, const int *gate = nullptr);
+void launch_f32_to_f64(const float *a, double *b, size_t n, cudaStream_t s);
 
 // Krylov support (deterministic two-stage reductions)
 int reduce_blocks();
 int sm_count();
-void launch_multidot(const double *const *V, int nv, const double *w, size_t n, double *partial,
-                     cudaStream_t s, int self = 0, const int *gate = nullptr);
-void launch_multidot_f32(const float *const *V, int nv, const double *w, size_t n, double *partial,
-                         cudaStream_t s);
+// Pointers and weights of a Krylov basis, by value in a kernel's parameters.
+constexpr int kMaxBasis = 65;
+struct BasisList {
+  const double *v[kMaxBasis];
+};
+struct BasisWeights {
+  double y[kMaxBasis];
+};
+// The reductions below finish in their last block (partial: reduce_blocks()
+// doubles a sum; *counter zero before and after) and leave their scalars on the
+// device: out[0 .. nv) the dots with V; a norm's out[0] its square and out[1] its
+// reciprocal, the square also in pinned host memory.
+void launch_dots(const BasisList &V, int nv, const double *w, size_t n, double *partial, unsigned *counter, double *out,
+                 cudaStream_t s);
 void launch_finish_sums(const double *partial, int nv, int nblocks, double *out, cudaStream_t s,
                         const int *gate = nullptr);
-void launch_multiaxpy_norm(double *w, const double *const *V, const double *h_dev, int nv, size_t n,
-                           double *partial, cudaStream_t s, const int *gate = nullptr);
-// dst = src / *scal_dev (and, with dst32, its FP32 copy)
-void launch_scale(double *dst, const double *src, const double *scal_dev, size_t n, cudaStream_t s,
-                  const int *gate = nullptr, float *dst32 = nullptr);
-// dst = src / sqrt(*sq_dev) (and, with dst32, its FP32 copy)
-void launch_scale_sqrt(double *dst, const double *src, const double *sq_dev, size_t n, cudaStream_t s,
-                       float *dst32 = nullptr, const int *gate = nullptr);
+// w -= sum h_q V_q and the norm of w; host[0 .. nv) = h, host[nv] = |w|^2
+void launch_orthogonalise(double *w, const BasisList &V, const double *h, int nv, size_t n, double *partial,
+                          unsigned *counter, double *out, double *host, cudaStream_t s);
+void launch_norm(const double *v, size_t n, double *partial, unsigned *counter, double *out, double *host,
+                 cudaStream_t s);
+// dst = src * *rcp (and, with dst32, its FP32 copy)
+void launch_scale(double *dst, const double *src, const double *rcp, size_t n, float *dst32, cudaStream_t s);
 // cs[5][SplitRow::count] = g11, g22, g33 (gf32 slots 0, 4, 8), aj and the code's
 // bits, each cell at its colour-split position
 void launch_split_coef(const Geom &g, const float *gf32, const float *ajf32, const uint32_t *code, float *cs,
                        cudaStream_t s);
 // out = 1 / a, element by element (correctly rounded)
 void launch_reciprocal(const double *a, double *out, size_t n, cudaStream_t s);
-void launch_axpy_z(double *x, const float *const *Z32, const double *const *Z64, const double *y_dev,
-                   int nz, size_t n, cudaStream_t s);
-void launch_fluid_mean_partial(const Geom &g, const uint32_t *code, const double *x, double *partial,
-                               cudaStream_t s);
-void launch_add_fluid_const(const Geom &g, const uint32_t *code, double *x, const double *sumcnt,
-                            int zero_outside, cudaStream_t s);
-// range projection of a right-hand side: sums of b/aj (b times the stored 1/aj)
-// and counts over fluid cells, then b -= aj * sum/count there
-void launch_fluid_ratio_partial(const Geom &g, const uint32_t *code, const double *b, const double *inv_aj,
-                                double *partial, cudaStream_t s);
-void launch_remove_aj_mean(const Geom &g, const uint32_t *code, const double *aj, double *b, const double *sums,
-                           cudaStream_t s);
+void launch_axpy_z(double *x, const BasisList &Z, const BasisWeights &y, int nz, size_t n, cudaStream_t s);
+// the mean over the fluid cells of x, or with inv_aj of x inv_aj, over sign,
+// into *out (device); x += *shift there
+void launch_fluid_mean(const Geom &g, const uint32_t *code, const double *x, const double *inv_aj, double sign,
+                       double *partial, unsigned *counter, double *out, cudaStream_t s);
+void launch_add_fluid_const(const Geom &g, const uint32_t *code, double *x, const double *shift, int zero_outside,
+                            cudaStream_t s);
+// range projection of a right-hand side, b -= aj *mean on the fluid cells, and
+// the norm of the result; host[0] = *mean, host[1] = |b|^2
+void launch_remove_mean(const Geom &g, const uint32_t *code, const double *aj, double *b, const double *mean,
+                        double *partial, unsigned *counter, double *out, double *host, cudaStream_t s);
 // b / a for the range projection's sum: an FP32 reciprocal refined by two
 // Newton-Raphson steps in FP64 (r <- r + r (1 - a r)), within a unit or so in
 // the last place of the quotient, at a fraction of an FP64 division's cost on

@@ -122,6 +122,27 @@ inline bool int_mul_factor(double v) {
   return a >= 0x1p-510 && a < 0x1p511;
 }
 
+// (double)f and (float)v on the integer pipe (a conversion costs an FP64 operation):
+// the same bits for zeros and numbers with a normal result, others go through the
+// conversion, out of line.
+static __device__ __noinline__ double widen_slow(float f) { return (double)f; }
+__device__ __forceinline__ double int_widen(float f) {
+  const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u && m) return widen_slow(f);
+  const unsigned h = (((unsigned)((int)u >> 3)) & 0x8fffffffu) + (896u << 20);
+  return __hiloint2double((int)(m ? h : u), (int)(u << 29));
+}
+static __device__ __noinline__ float narrow_slow(double v) { return (float)v; }
+__device__ __forceinline__ float int_narrow(double v) {
+  const unsigned h = (unsigned)__double2hiint(v), l = (unsigned)__double2loint(v), e = (h >> 20) & 0x7ffu;
+  if (e - 897u < 254u - 1u) {  // a rounding up stays finite
+    const unsigned m = __funnelshift_l(l, h & 0x7fffffffu, 3) - (896u << 23), rest = l << 3;
+    // up where the rest is above half a unit, or is half and m odd
+    return __uint_as_float((h & 0x80000000u) | (m + (rest > 0x80000000u || (rest == 0x80000000u && (m & 1)))));
+  }
+  return ((h & 0x7fffffffu) | l) == 0 ? __uint_as_float(h) : narrow_slow(v);
+}
+
 // x / y rounded to nearest even for a divisor used many times, from rcp = 1 / y
 // rounded to nearest: x rcp, then twice the residual x - y q added back through
 // rcp.  The residual of a quotient within an ulp is exact in one fused

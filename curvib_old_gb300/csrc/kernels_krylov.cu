@@ -4,6 +4,7 @@
 // depend on timing or on what else shares the GPU.
 #include <algorithm>
 
+#include "intmul.cuh"
 #include "launch.cuh"
 
 namespace cvb {
@@ -12,7 +13,7 @@ static long long g_launches = 0;
 void count_launch(int n) { __atomic_add_fetch(&g_launches, (long long)n, __ATOMIC_RELAXED); }
 long long launch_count() { return __atomic_load_n(&g_launches, __ATOMIC_RELAXED); }
 
-static const int kRedThreads = 256;
+static const int kRedThreads = 256;  // the reductions' kernels: four blocks an SM, all resident
 static int g_red_blocks = 0;
 
 int sm_count() {
@@ -31,97 +32,113 @@ int reduce_blocks() {
   return g_red_blocks;
 }
 
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&acc)[NV], double *partial, int nblocks, int base) {
-  __shared__ double sh[NV][kRedThreads / 32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+// ------------------------------------------------------------ reductions
+// A kernel's NR sums over all its blocks.  Each thread's terms go through shared
+// memory, a warp per sum, into partial[q][block]; the last block to arrive adds
+// the partials, a warp per sum, and only its threads see the totals (tot, true
+// returned).  The trees are fixed by the grid, so the totals do not depend on the
+// order of arrival.  Few FP64 additions (12 a sum and warp-pair of a block, where
+// a shuffle tree per warp makes 40): they share the pipe that bounds these
+// kernels.  *counter is zero between launches.
+template <int NR>
+struct ReduceSmem {
+  double v[NR][kRedThreads];
+  double tot[NR];
+  int last;
+};
+__device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
-  for (int q = 0; q < NV; q++) {
-    double v = acc[q];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  return v;
+}
+template <int NR>
+__device__ __forceinline__ bool reduce_all(ReduceSmem<NR> &sm, const double (&acc)[NR], double *partial,
+                                           unsigned *counter) {
+  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, nb = gridDim.x;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) sh[q][wid] = v;
+  for (int q = 0; q < NR; q++) sm.v[q][t] = acc[q];
+  __syncthreads();
+  for (int q = wid; q < NR; q += kRedThreads / 32) {
+    double v = sm.v[q][lane];
+#pragma unroll
+    for (int u = 1; u < kRedThreads / 32; u++) v += sm.v[q][lane + 32 * u];
+    v = warp_sum(v);
+    if (lane == 0) {
+      __stcg(partial + (size_t)q * nb + blockIdx.x, v);
+      __threadfence();
+    }
   }
   __syncthreads();
-  if (threadIdx.x < NV) {
+  if (t == 0) sm.last = atomicAdd(counter, 1u) == (unsigned)nb - 1u;
+  __syncthreads();
+  if (!sm.last) return false;
+  __threadfence();
+  for (int q = wid; q < NR; q += kRedThreads / 32) {
     double v = 0.0;
-#pragma unroll
-    for (int w = 0; w < kRedThreads / 32; w++) v += sh[threadIdx.x][w];
-    partial[(size_t)(base + threadIdx.x) * nblocks + blockIdx.x] = v;
+    for (int b = lane; b < nb; b += 32) v += __ldcg(partial + (size_t)q * nb + b);
+    v = warp_sum(v);
+    if (lane == 0) sm.tot[q] = v;
   }
-}
-
-// partial[q][block] = sum over this block's elements of V_q[i] * w[i] for NV
-// vectors starting at `base`; with `self` the w.w sum goes to row `self_row`.
-// The vector count is a template parameter: predicated-off products would still
-// occupy the FP64 pipe, which bounds this kernel on this part.
-template <typename TV, int NV, bool SELF>
-__global__ void __launch_bounds__(kRedThreads) k_multidot(const TV *const *V, int base, const double *__restrict__ w,
-                                                           size_t n, double *partial, int self_row,
-                                                           const int *gate) {
-  dep_sync();
-  if (gated(gate)) return;
-  double acc[NV + 1];
-#pragma unroll
-  for (int q = 0; q <= NV; q++) acc[q] = 0.0;
-  const TV *v[NV];
-#pragma unroll
-  for (int q = 0; q < NV; q++) v[q] = V[base + q];
-  for (size_t p = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p < n; p += (size_t)gridDim.x * kRedThreads) {
-    double wp = w[p];
-#pragma unroll
-    for (int q = 0; q < NV; q++) acc[q] = fma((double)v[q][p], wp, acc[q]);
-    if (SELF) acc[NV] = fma(wp, wp, acc[NV]);
-  }
-  __shared__ double sh[NV + 1][kRedThreads / 32];
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int NR = SELF ? NV + 1 : NV;
-#pragma unroll
-  for (int q = 0; q < NR; q++) {
-    double x = acc[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[q][wid] = x;
-  }
+  if (t == 0) *counter = 0;
   __syncthreads();
-  if (threadIdx.x < NR) {
-    double x = 0.0;
+  return true;
+}
+
+// Two cells a thread at least, so that a small problem's last block has few partials.
+static unsigned red_grid(size_t n) {
+  return (unsigned)std::min<size_t>(reduce_blocks(), (n + 2 * kRedThreads - 1) / (2 * kRedThreads));
+}
+
+// out[base + q] = V_{base + q} . w for NV vectors.  The vector count is a
+// template parameter: predicated-off products would still occupy the FP64 pipe,
+// which bounds this kernel on this part (six vectors on 4.4 M cells: 45 us of it).
+template <int NV>
+__global__ void __launch_bounds__(kRedThreads, 4) k_dots(const __grid_constant__ BasisList V, int base,
+                                                      const double *__restrict__ w, size_t n, double *partial,
+                                                      unsigned *counter, double *__restrict__ out) {
+  dep_sync();
+  constexpr int U = NV <= 2 ? 4 : NV <= 4 ? 2 : 1;
+  __shared__ ReduceSmem<NV> sm;
+  double acc[NV];
 #pragma unroll
-    for (int ww = 0; ww < kRedThreads / 32; ww++) x += sh[threadIdx.x][ww];
-    int row = (SELF && threadIdx.x == NV) ? self_row : base + threadIdx.x;
-    partial[(size_t)row * gridDim.x + blockIdx.x] = x;
+  for (int q = 0; q < NV; q++) acc[q] = 0.0;
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  size_t p = blockIdx.x * (size_t)kRedThreads + threadIdx.x;
+  for (; p + (U - 1) * step < n; p += U * step) {
+    double v[U][NV], wp[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      wp[u] = w[p + u * step];
+#pragma unroll
+      for (int q = 0; q < NV; q++) v[u][q] = V.v[base + q][p + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int q = 0; q < NV; q++) acc[q] = fma(v[u][q], wp[u], acc[q]);
   }
+  for (; p < n; p += step) {
+    const double wp = w[p];
+#pragma unroll
+    for (int q = 0; q < NV; q++) acc[q] = fma(V.v[base + q][p], wp, acc[q]);
+  }
+  if (reduce_all<NV>(sm, acc, partial, counter) && threadIdx.x < NV) out[base + threadIdx.x] = sm.tot[threadIdx.x];
 }
 
-template <typename TV, bool SELF>
-static void multidot_chunk(const TV *const *V, int base, int cnt, const double *w, size_t n, double *partial,
-                           int self_row, cudaStream_t s, const int *gate = nullptr) {
-  int nb = reduce_blocks();
-  switch (cnt) {
-    case 1: launch_dep(k_multidot<TV, 1, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 2: launch_dep(k_multidot<TV, 2, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 3: launch_dep(k_multidot<TV, 3, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 4: launch_dep(k_multidot<TV, 4, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 5: launch_dep(k_multidot<TV, 5, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 6: launch_dep(k_multidot<TV, 6, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    case 7: launch_dep(k_multidot<TV, 7, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-    default: launch_dep(k_multidot<TV, 8, SELF>, nb, kRedThreads, 0, s, V, base, w, n, partial, self_row, gate); break;
-  }
+template <int NV>
+static void dots_chunk(const BasisList &V, int base, int cnt, const double *w, size_t n, double *partial,
+                       unsigned *counter, double *out, cudaStream_t s) {
+  if (cnt == NV)
+    launch_dep(k_dots<NV>, red_grid(n), kRedThreads, 0, s, V, base, w, n, partial, counter, out);
+  else if constexpr (NV > 1)
+    dots_chunk<NV - 1>(V, base, cnt, w, n, partial, counter, out, s);
 }
-
-// Dots of w with V_0..V_{nv-1} in chunks of up to 8 vectors (each chunk reads w
-// once more); with `self`, w.w lands in row nv of the partials.
-void launch_multidot(const double *const *V, int nv, const double *w, size_t n, double *partial, cudaStream_t s,
-                     int self, const int *gate) {
-  for (int base = 0; base < nv; base += 8) {
-    int cnt = nv - base < 8 ? nv - base : 8;
-    if (self && base == 0) multidot_chunk<double, true>(V, base, cnt, w, n, partial, nv, s, gate);
-    else multidot_chunk<double, false>(V, base, cnt, w, n, partial, nv, s, gate);
-  }
-}
-void launch_multidot_f32(const float *const *V, int nv, const double *w, size_t n, double *partial, cudaStream_t s) {
+// Dots of w with V_0..V_{nv-1} into out, in chunks of up to 8 vectors (each chunk
+// reads w once more).
+void launch_dots(const BasisList &V, int nv, const double *w, size_t n, double *partial, unsigned *counter, double *out,
+                 cudaStream_t s) {
   for (int base = 0; base < nv; base += 8)
-    multidot_chunk<float, false>(V, base, nv - base < 8 ? nv - base : 8, w, n, partial, nv, s);
+    dots_chunk<8>(V, base, std::min(nv - base, 8), w, n, partial, counter, out, s);
 }
 
 // out[q] = sum_b partial[q][b], one block per q, fixed tree.
@@ -145,51 +162,118 @@ void launch_finish_sums(const double *partial, int nv, int nblocks, double *out,
   launch_dep(k_finish, nv, kRedThreads, 0, s, partial, nblocks, out, gate);
 }
 
-// w -= sum_q h[q] V_q ; partial[block] = sum of w^2 over the block.
-__global__ void __launch_bounds__(kRedThreads) k_multiaxpy_norm(double *__restrict__ w, const double *const *V,
-                                                                 const double *__restrict__ h, int nv, size_t n,
-                                                                 double *partial, const int *gate) {
-  dep_sync();
-  if (gated(gate)) return;
-  __shared__ double hs[64];
-  if (threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
-  __syncthreads();
-  double acc = 0.0;
-  for (size_t p = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p < n; p += (size_t)gridDim.x * kRedThreads) {
-    double v = w[p];
-    for (int q = 0; q < nv; q++) v = fma(-hs[q], V[q][p], v);
-    w[p] = v;
-    acc = fma(v, v, acc);
+// What a norm's kernel leaves: out[0] = the sum of squares, out[1] = 1 / its root;
+// the sum, after nh other scalars h, also in pinned host memory.
+__device__ __forceinline__ void store_norm(double sum, double *out, const double *h, int nh, double *host) {
+  const int t = threadIdx.x;
+  if (t == 0) {
+    out[0] = sum;
+    out[1] = 1.0 / sqrt(sum);
+    host[nh] = sum;
   }
-  double a1[1] = {acc};
-  block_reduce_store<1>(a1, partial, gridDim.x, 0);
-}
-void launch_multiaxpy_norm(double *w, const double *const *V, const double *h_dev, int nv, size_t n,
-                           double *partial, cudaStream_t s, const int *gate) {
-  launch_dep(k_multiaxpy_norm, reduce_blocks(), kRedThreads, 0, s, w, V, h_dev, nv, n, partial, gate);
+  for (int q = t; q < nh; q += kRedThreads) host[q] = h[q];
 }
 
-// dst = src / *scal, or src / sqrt(*scal); with dst32 also its FP32 copy (the
-// next V-cycle's input in mixed precision)
-template <bool SQRT>
-__global__ void k_scale(double *__restrict__ dst, const double *__restrict__ src, const double *__restrict__ scal,
-                        size_t n, const int *gate, float *__restrict__ dst32) {
+// w -= sum_q h[q] V_q for 8 * octets + NR vectors, and the norm of w.  The
+// remainder is a template parameter for the same reason as k_dots's count; each
+// octet's loads come before its products.
+template <int NR>
+__global__ void __launch_bounds__(kRedThreads, 4) k_orthogonalise(double *__restrict__ w,
+                                                               const __grid_constant__ BasisList V,
+                                                               const double *__restrict__ h, int octets, size_t n,
+                                                               double *partial, unsigned *counter, double *out,
+                                                               double *host) {
   dep_sync();
-  if (gated(gate)) return;
-  double inv = 1.0 / (SQRT ? sqrt(*scal) : *scal);
+  __shared__ ReduceSmem<1> sm;
+  __shared__ double hs[kMaxBasis];
+  const int nv = 8 * octets + NR;
+  if (threadIdx.x < nv) hs[threadIdx.x] = h[threadIdx.x];
+  __syncthreads();
+  constexpr int U = NR <= 3 ? 2 : 1;
+  double acc[1] = {0.0};
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  for (size_t p0 = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p0 < n; p0 += U * step) {
+    double x[U][NR], v[U];
+    const bool two = U > 1 && p0 + step < n;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const size_t p = u && two ? p0 + step : p0;
+      v[u] = w[p];
+#pragma unroll
+      for (int q = 0; q < NR; q++) x[u][q] = V.v[q][p];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      if (u && !two) break;
+      const size_t p = p0 + u * step;
+#pragma unroll
+      for (int q = 0; q < NR; q++) v[u] = fma(-hs[q], x[u][q], v[u]);
+      for (int o = 0; o < octets; o++) {
+        const int b = NR + 8 * o;
+        double y[8];
+#pragma unroll
+        for (int q = 0; q < 8; q++) y[q] = V.v[b + q][p];
+#pragma unroll
+        for (int q = 0; q < 8; q++) v[u] = fma(-hs[b + q], y[q], v[u]);
+      }
+      w[p] = v[u];
+      acc[0] = fma(v[u], v[u], acc[0]);
+    }
+  }
+  if (reduce_all<1>(sm, acc, partial, counter)) store_norm(sm.tot[0], out, hs, nv, host);
+}
+template <int NR>
+static void orthogonalise(double *w, const BasisList &V, const double *h, int nv, size_t n, double *partial,
+                          unsigned *counter, double *out, double *host, cudaStream_t s) {
+  const int r = (nv - 1) % 8 + 1;
+  if (r == NR)
+    launch_dep(k_orthogonalise<NR>, red_grid(n), kRedThreads, 0, s, w, V, h, nv / 8 - (NR == 8), n, partial, counter,
+               out, host);
+  else if constexpr (NR > 1)
+    orthogonalise<NR - 1>(w, V, h, nv, n, partial, counter, out, host, s);
+}
+void launch_orthogonalise(double *w, const BasisList &V, const double *h, int nv, size_t n, double *partial,
+                          unsigned *counter, double *out, double *host, cudaStream_t s) {
+  orthogonalise<8>(w, V, h, nv, n, partial, counter, out, host, s);
+}
+
+// The norm of v.
+__global__ void __launch_bounds__(kRedThreads, 4) k_norm(const double *__restrict__ v, size_t n, double *partial,
+                                                      unsigned *counter, double *out, double *host) {
+  dep_sync();
+  __shared__ ReduceSmem<1> sm;
+  double acc[1] = {0.0};
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  for (size_t p0 = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p0 < n; p0 += 4 * step) {
+    double x[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) x[u] = p0 + u * step < n ? v[p0 + u * step] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (p0 + u * step < n) acc[0] = fma(x[u], x[u], acc[0]);
+  }
+  if (reduce_all<1>(sm, acc, partial, counter)) store_norm(sm.tot[0], out, nullptr, 0, host);
+}
+void launch_norm(const double *v, size_t n, double *partial, unsigned *counter, double *out, double *host,
+                 cudaStream_t s) {
+  launch_dep(k_norm, red_grid(n), kRedThreads, 0, s, v, n, partial, counter, out, host);
+}
+
+// dst = src *rcp (a norm's reciprocal), and with dst32 its FP32 copy (the next
+// V-cycle's input in mixed precision): one FP64 operation a cell, the
+// conversion on the integer pipe.
+__global__ void __launch_bounds__(256) k_scale(double *__restrict__ dst, const double *__restrict__ src,
+                                               const double *__restrict__ rcp, size_t n, float *__restrict__ dst32) {
+  dep_sync();
+  const double inv = *rcp;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
     const double v = src[p] * inv;
     dst[p] = v;
-    if (dst32) dst32[p] = (float)v;
+    if (dst32) dst32[p] = int_narrow(v);
   }
 }
-void launch_scale(double *dst, const double *src, const double *scal_dev, size_t n, cudaStream_t s,
-                  const int *gate, float *dst32) {
-  launch_dep(k_scale<false>, reduce_blocks(), 256, 0, s, dst, src, scal_dev, n, gate, dst32);
-}
-void launch_scale_sqrt(double *dst, const double *src, const double *sq_dev, size_t n, cudaStream_t s,
-                       float *dst32, const int *gate) {
-  launch_dep(k_scale<true>, reduce_blocks(), 256, 0, s, dst, src, sq_dev, n, gate, dst32);
+void launch_scale(double *dst, const double *src, const double *rcp, size_t n, float *dst32, cudaStream_t s) {
+  launch_dep(k_scale, (unsigned)((n + 1023) / 1024), 256, 0, s, dst, src, rcp, n, dst32);
 }
 
 __global__ void k_reciprocal(const double *__restrict__ a, double *__restrict__ out, size_t n) {
@@ -201,100 +285,139 @@ void launch_reciprocal(const double *a, double *out, size_t n, cudaStream_t s) {
   launch_dep(k_reciprocal, reduce_blocks(), 256, 0, s, a, out, n);
 }
 
-// x += sum_q y[q] Z_q (Z stored FP32 in mixed mode, FP64 in plain mode)
-__global__ void k_axpy_z(double *__restrict__ x, const float *const *Z32, const double *const *Z64,
-                         const double *__restrict__ y, int nz, size_t n) {
+// x += sum_q y[q] Z_q for 8 * octets + NR vectors
+template <int NR>
+__global__ void __launch_bounds__(256) k_axpy_z(double *__restrict__ x, const __grid_constant__ BasisList Z,
+                                                const __grid_constant__ BasisWeights y, int octets, size_t n) {
   dep_sync();
-  __shared__ double ys[64];
-  if (threadIdx.x < nz) ys[threadIdx.x] = y[threadIdx.x];
-  __syncthreads();
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
+    double z[NR];
     double v = x[p];
-    if (Z32)
-      for (int q = 0; q < nz; q++) v = fma(ys[q], (double)Z32[q][p], v);
-    else
-      for (int q = 0; q < nz; q++) v = fma(ys[q], Z64[q][p], v);
+#pragma unroll
+    for (int q = 0; q < NR; q++) z[q] = Z.v[q][p];
+#pragma unroll
+    for (int q = 0; q < NR; q++) v = fma(y.y[q], z[q], v);
+    for (int o = 0; o < octets; o++) {
+      const int b = NR + 8 * o;
+      double u[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) u[q] = Z.v[b + q][p];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v = fma(y.y[b + q], u[q], v);
+    }
     x[p] = v;
   }
 }
-void launch_axpy_z(double *x, const float *const *Z32, const double *const *Z64, const double *y_dev, int nz,
-                   size_t n, cudaStream_t s) {
-  launch_dep(k_axpy_z, reduce_blocks(), 256, 0, s, x, Z32, Z64, y_dev, nz, n);
+template <int NR>
+static void axpy_z(double *x, const BasisList &Z, const BasisWeights &y, int nz, size_t n, cudaStream_t s) {
+  if ((nz - 1) % 8 + 1 == NR)
+    launch_dep(k_axpy_z<NR>, (unsigned)((n + 1023) / 1024), 256, 0, s, x, Z, y, nz / 8 - (NR == 8), n);
+  else if constexpr (NR > 1)
+    axpy_z<NR - 1>(x, Z, y, nz, n, s);
+}
+void launch_axpy_z(double *x, const BasisList &Z, const BasisWeights &y, int nz, size_t n, cudaStream_t s) {
+  axpy_z<8>(x, Z, y, nz, n, s);
 }
 
-// Null space (PoissonNullSpaceFunction, poisson.c:411-558): sums and counts of x
-// over interior fluid cells (nvert < 0.1).
-__global__ void __launch_bounds__(kRedThreads) k_fluid_sum(Geom g, const uint32_t *__restrict__ code,
-                                                           const double *__restrict__ x, double *partial) {
+// ------------------------------------------------------------ null space, range
+// The mean over the interior fluid cells (nvert < 0.1) of x (the null space,
+// PoissonNullSpaceFunction, poisson.c:411-558), or of b / aj as b times the
+// stored 1 / aj (the range projection), times `sign`, into *out: counted in an
+// integer, four cells a step, so that a cell costs one FP64 operation.
+template <bool RATIO>
+__global__ void __launch_bounds__(kRedThreads, 4) k_fluid_mean(size_t n, const uint32_t *__restrict__ code,
+                                                            const double *__restrict__ x,
+                                                            const double *__restrict__ inv_aj, double sign,
+                                                            double *partial, unsigned *counter, double *out) {
   dep_sync();
+  __shared__ ReduceSmem<2> sm;
   double acc[2] = {0.0, 0.0};
-  size_t n = g.n();
-  for (size_t p = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p < n; p += (size_t)gridDim.x * kRedThreads) {
-    if (code[p] & CODE_FLUID) {
-      acc[0] += x[p];
-      acc[1] += 1.0;
+  unsigned cnt = 0;
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  for (size_t p0 = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p0 < n; p0 += 4 * step) {
+    uint32_t c[4];
+    double v[4], a[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const size_t p = p0 + u * step;
+      c[u] = p < n ? code[p] : 0;
+      v[u] = p < n ? x[p] : 0.0;
+      a[u] = RATIO && p < n ? inv_aj[p] : 0.0;
     }
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (c[u] & CODE_FLUID) {
+        acc[0] = RATIO ? fma(v[u], a[u], acc[0]) : acc[0] + v[u];
+        cnt++;
+      }
   }
-  block_reduce_store<2>(acc, partial, gridDim.x, 0);
+  acc[1] = (double)cnt;
+  if (reduce_all<2>(sm, acc, partial, counter) && threadIdx.x == 0)
+    *out = sm.tot[1] > 0.0 ? sm.tot[0] / (sign * sm.tot[1]) : 0.0;
 }
-void launch_fluid_mean_partial(const Geom &g, const uint32_t *code, const double *x, double *partial,
-                               cudaStream_t s) {
-  launch_dep(k_fluid_sum, reduce_blocks(), kRedThreads, 0, s, g, code, x, partial);
+void launch_fluid_mean(const Geom &g, const uint32_t *code, const double *x, const double *inv_aj, double sign,
+                       double *partial, unsigned *counter, double *out, cudaStream_t s) {
+  if (inv_aj)
+    launch_dep(k_fluid_mean<true>, red_grid(g.n()), kRedThreads, 0, s, g.n(), code, x, inv_aj, sign, partial, counter,
+               out);
+  else
+    launch_dep(k_fluid_mean<false>, red_grid(g.n()), kRedThreads, 0, s, g.n(), code, x, inv_aj, sign, partial, counter,
+               out);
 }
-// x += -sum/count on interior fluid cells; with zero_outside the ring and the
+
+// x += *shift on interior fluid cells; with zero_outside the ring and the
 // non-fluid cells are set to zero.
-__global__ void k_add_fluid_const(Geom g, const uint32_t *__restrict__ code, double *__restrict__ x,
-                                  const double *__restrict__ sc, int zero_outside) {
+__global__ void __launch_bounds__(256) k_add_fluid_const(size_t n, const uint32_t *__restrict__ code,
+                                                         double *__restrict__ x, const double *__restrict__ shift,
+                                                         int zero_outside) {
   dep_sync();
-  double shift = sc[1] > 0.0 ? sc[0] / (-1.0 * sc[1]) : 0.0;
-  size_t n = g.n();
+  const double c0 = *shift;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
     const uint32_t c = code[p];
-    if (c & CODE_FLUID) x[p] += shift;
+    if (c & CODE_FLUID) x[p] += c0;
     if (zero_outside && (c & CODE_IDENTITY)) x[p] = 0.0;  // the ring and nvert > 0.1
   }
 }
-void launch_add_fluid_const(const Geom &g, const uint32_t *code, double *x, const double *sumcnt, int zero_outside,
+void launch_add_fluid_const(const Geom &g, const uint32_t *code, double *x, const double *shift, int zero_outside,
                             cudaStream_t s) {
-  launch_dep(k_add_fluid_const, reduce_blocks(), 256, 0, s, g, code, x, sumcnt, zero_outside);
+  launch_dep(k_add_fluid_const, (unsigned)((g.n() + 1023) / 1024), 256, 0, s, g.n(), code, x, shift, zero_outside);
 }
 
-// The range projection's sums over the fluid cells: of b / aj, as b times the
-// stored 1 / aj (the FP64 pipe is this part's bound, and a division costs
-// several of its instructions), and the cell count, counted in an integer.
-__global__ void __launch_bounds__(kRedThreads) k_fluid_ratio(Geom g, const uint32_t *__restrict__ code,
-                                                             const double *__restrict__ b,
-                                                             const double *__restrict__ inv_aj, double *partial) {
+// The range projection b -= aj *mean on the fluid cells, and the norm of what is
+// left (the mean goes to the host with it).
+__global__ void __launch_bounds__(kRedThreads, 4) k_remove_mean(size_t n, const uint32_t *__restrict__ code,
+                                                             const double *__restrict__ aj, double *__restrict__ b,
+                                                             const double *__restrict__ mean, double *partial,
+                                                             unsigned *counter, double *out, double *host) {
   dep_sync();
-  double acc[2] = {0.0, 0.0};
-  unsigned cnt = 0;
-  size_t n = g.n();
-  for (size_t p = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p < n; p += (size_t)gridDim.x * kRedThreads) {
-    if (code[p] & CODE_FLUID) {
-      acc[0] = fma(b[p], inv_aj[p], acc[0]);
-      cnt++;
+  __shared__ ReduceSmem<1> sm;
+  const double c0 = *mean;
+  double acc[1] = {0.0};
+  const size_t step = (size_t)gridDim.x * kRedThreads;
+  for (size_t p0 = blockIdx.x * (size_t)kRedThreads + threadIdx.x; p0 < n; p0 += 4 * step) {
+    uint32_t c[4];
+    double v[4], a[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const size_t p = p0 + u * step;
+      c[u] = p < n ? code[p] : 0;
+      v[u] = p < n ? b[p] : 0.0;
+      a[u] = p < n ? aj[p] : 0.0;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      if (c[u] & CODE_FLUID) {
+        v[u] -= a[u] * c0;
+        b[p0 + u * step] = v[u];
+      }
+      if (p0 + u * step < n) acc[0] = fma(v[u], v[u], acc[0]);
     }
   }
-  acc[1] = (double)cnt;
-  block_reduce_store<2>(acc, partial, gridDim.x, 0);
+  if (reduce_all<1>(sm, acc, partial, counter)) store_norm(sm.tot[0], out, mean, 1, host);
 }
-void launch_fluid_ratio_partial(const Geom &g, const uint32_t *code, const double *b, const double *inv_aj,
-                                double *partial, cudaStream_t s) {
-  launch_dep(k_fluid_ratio, reduce_blocks(), kRedThreads, 0, s, g, code, b, inv_aj, partial);
-}
-__global__ void k_remove_aj_mean(Geom g, const uint32_t *__restrict__ code, const double *__restrict__ aj,
-                                 double *__restrict__ b, const double *__restrict__ sums) {
-  dep_sync();
-  double c = sums[1] > 0.0 ? sums[0] / sums[1] : 0.0;
-  size_t n = g.n();
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    if (code[p] & CODE_FLUID)
-      b[p] -= aj[p] * c;
-  }
-}
-void launch_remove_aj_mean(const Geom &g, const uint32_t *code, const double *aj, double *b, const double *sums,
-                           cudaStream_t s) {
-  launch_dep(k_remove_aj_mean, reduce_blocks(), 256, 0, s, g, code, aj, b, sums);
+void launch_remove_mean(const Geom &g, const uint32_t *code, const double *aj, double *b, const double *mean,
+                        double *partial, unsigned *counter, double *out, double *host, cudaStream_t s) {
+  launch_dep(k_remove_mean, red_grid(g.n()), kRedThreads, 0, s, g.n(), code, aj, b, mean, partial, counter, out, host);
 }
 
 // Coarsest level: e = Minv r with a dense FP64 inverse over the cells idx[0..m),

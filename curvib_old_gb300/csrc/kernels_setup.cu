@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "intmul.cuh"
 #include "launch.cuh"
 
 namespace cvb {
@@ -292,18 +293,22 @@ __global__ void k_to_f32(const double *__restrict__ a, float *__restrict__ b, si
 void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate) {
   launch_dep(k_to_f32, dim3(nblk(n, 256) < 4096 ? nblk(n, 256) : 4096), 256, 0, s, a, b, n, gate);
 }
-void launch_f64_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate) {
-  launch_to_f32(a, b, n, s, gate);
-}
-
-__global__ void k_to_f64(const float *__restrict__ a, double *__restrict__ b, size_t n, const int *gate) {
+// The FP32 V-cycle's result as the FP64 basis vector: the widening on the integer
+// pipe, four cells a thread (17 + 35 MB on 4.4 M cells).
+__global__ void __launch_bounds__(256) k_to_f64(const float *__restrict__ a, double *__restrict__ b, size_t n) {
   dep_sync();
-  if (gated(gate)) return;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
-    b[p] = (double)a[p];
+  const size_t p = 4 * (blockIdx.x * (size_t)blockDim.x + threadIdx.x);
+  if (p + 4 <= n) {  // both arrays are whole allocations: aligned
+    const float4 f = *reinterpret_cast<const float4 *>(a + p);
+    double2 *o = reinterpret_cast<double2 *>(b + p);
+    o[0] = make_double2(int_widen(f.x), int_widen(f.y));
+    o[1] = make_double2(int_widen(f.z), int_widen(f.w));
+  } else {
+    for (size_t q = p; q < n; q++) b[q] = int_widen(a[q]);
+  }
 }
-void launch_f32_to_f64(const float *a, double *b, size_t n, cudaStream_t s, const int *gate) {
-  launch_dep(k_to_f64, dim3(nblk(n, 256) < 4096 ? nblk(n, 256) : 4096), 256, 0, s, a, b, n, gate);
+void launch_f32_to_f64(const float *a, double *b, size_t n, cudaStream_t s) {
+  launch_dep(k_to_f64, nblk((n + 3) / 4, 256), 256, 0, s, a, b, n);
 }
 
 // MyNvertRestriction (poisson.c:1662-1773): a coarse cell is blocked (1) when the

@@ -54,9 +54,6 @@ template <>
 void launch_residual<double>(const LevelDev &L, const double *b, const double *x, double *r, cudaStream_t s) {
   apply64<double>(L, x, b, r, s);
 }
-void launch_apply64_from32(const LevelDev &L, const float *x, double *y, cudaStream_t s) {
-  apply64<float>(L, x, nullptr, y, s);
-}
 template <>
 void launch_apply<float>(const LevelDev &L, const float *x, float *y, cudaStream_t s) {
   apply32(L, x, nullptr, y, s);

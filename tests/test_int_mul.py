@@ -132,3 +132,43 @@ def test_quotient_by_three_halves_is_the_rounded_one():
         x = value(rng.getrandbits(1) << 63 | rng.choice((623, 1022, 1023, 1422)) << 52 | p)
         r = x * (2.0 / 3.0)
         assert bits(fma(fma(-1.5, r, x), 2.0 / 3.0, r)) == bits(x / 1.5), x
+
+
+def widen(u):
+    """The double, or None where the kernel leaves the value to the conversion."""
+    m = u & 0x7FFFFFFF
+    if (m - 0x00800000) & M32 >= 0x7F000000 and m:
+        return None
+    h = (((u - (u >> 31 << 32)) >> 3) & 0x8FFFFFFF) + (896 << 20)
+    return value((h if m else u) << 32 | (u << 29 & M32))
+
+
+def narrow(v):
+    """The FP32 bits, or None where the kernel leaves the value to the conversion."""
+    b = bits(v)
+    h, l = b >> 32, b & M32
+    e = h >> 20 & 0x7FF
+    if (e - 897) & M32 < 253:
+        m = ((h & 0x7FFFFFFF) << 3 & M32 | l >> 29) - (896 << 23) & M32
+        rest = l << 3 & M32
+        return (h & 0x80000000) | (m + (rest > 0x80000000 or (rest == 0x80000000 and m & 1)))
+    return h if (h & 0x7FFFFFFF) | l == 0 else None
+
+
+def test_conversions_are_the_rounded_ones():
+    import numpy as np
+    rng = random.Random(5)
+    for p in list(significands(rng)) + [rng.getrandbits(24) << 28 for _ in range(200)]:
+        for e in (0, 1, 896, 897, 898, 1022, 1023, 1149, 1150, 1151, 2047):
+            for sign in (0, 1):
+                v = value(sign << 63 | e << 52 | p)
+                n = narrow(v)
+                assert (n is not None) == (897 <= e <= 1149 or v == 0.0)
+                if n is not None:
+                    assert n == int(np.float32(v).view(np.uint32)), v
+    for u in [rng.getrandbits(32) for _ in range(20000)] + [0, 1 << 31, 1 << 23, 0x7F7FFFFF, 0x807FFFFF, 1]:
+        f = float(np.uint32(u).view(np.float32))
+        if 0 < u & 0x7FFFFFFF < 0x00800000 or u & 0x7FFFFFFF >= 0x7F800000:
+            assert widen(u) is None, u
+        else:
+            assert bits(widen(u)) == bits(f), u
