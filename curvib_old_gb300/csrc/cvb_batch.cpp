@@ -308,8 +308,8 @@ static void gen_vcycle_zebra(VSink &vs, cvb_ctx *ctx, const LevelDev *dLs, int l
   const int cgx = plane_blocks(C.g);
   vs.add(key_desc(depth, 101), OK_RESTRICT, task(dLv, res, nullptr, bc, gate, cgx, 1), cgx * C.g.mz);
   gen_vcycle<T>(vs, ctx, dLs, l - 1, depth + 1, bc, ec, o, gate);
-  vs.add(key_asc(depth, 0), OK_PROLONG, task(dLv, ec, nullptr, x, gate, plane_blocks(L.g), 1),
-         plane_blocks(L.g) * L.g.mz);
+  const ProlongGrid pg = ProlongGrid::of(L);
+  vs.add(key_asc(depth, 0), OK_PROLONG, task(dLv, ec, nullptr, x, gate, pg.gx, 1), pg.gx * pg.gz);
   for (int q = 0; q < o.post_sweeps; q++)
     gen_zebra_sweep<T>(vs, key_asc(depth, 1 + 10 * q), key_asc(depth, 2 + 10 * q), key_asc(depth, 4 + 10 * q),
                        key_asc(depth, 5 + 10 * q), L, dLv, b, x, tmp, false, gate);
@@ -342,8 +342,8 @@ static void gen_vcycle(VSink &vs, cvb_ctx *ctx, const LevelDev *dLs, int l, int 
   const int cgx = plane_blocks(C.g);
   vs.add(key_desc(depth, 101), OK_RESTRICT, task(dLv, res, nullptr, bc, gate, cgx, 1), cgx * C.g.mz);
   gen_vcycle<T>(vs, ctx, dLs, l - 1, depth + 1, bc, ec, o, gate);
-  vs.add(key_asc(depth, 0), OK_PROLONG, task(dLv, ec, nullptr, x, gate, plane_blocks(L.g), 1),
-         plane_blocks(L.g) * L.g.mz);
+  const ProlongGrid pg = ProlongGrid::of(L);
+  vs.add(key_asc(depth, 0), OK_PROLONG, task(dLv, ec, nullptr, x, gate, pg.gx, 1), pg.gx * pg.gz);
   for (int q = 0; q < o.post_sweeps; q++) {
     gen_sweep<T>(vs, key_asc(depth, 1 + 2 * q), key_asc(depth, 2 + 2 * q), L, dLv, b, x, x2, false, gate);
     std::swap(x, x2);

@@ -87,29 +87,35 @@ __device__ __forceinline__ double int_mul(const IntMulA &a, const IntMulB &b) {
   return __hiloint2double(hi ? se : (a.se ^ b.se) & 0x80000000u, lo);
 }
 
-// 3 x rounded to nearest even: three times the significand has one or two bits
-// too many.  Other than normal numbers with a normal result and zeros go
-// through the multiply, out of line.
-static __device__ __noinline__ double triple_slow(double x) { return __dmul_rn(3., x); }
-__device__ __forceinline__ double int_triple(double x) {
+// 3 x and 9 x rounded to nearest even: the significand's multiple has one or two
+// (three or four) bits too many.  Other than normal numbers with a normal result
+// and zeros go through the multiply, out of line.
+static __device__ __noinline__ double times_slow(double x, double k) { return __dmul_rn(k, x); }
+template <int K>
+__device__ __forceinline__ double int_times(double x) {
+  static_assert(K == 3 || K == 9, "");
+  constexpr int S = K == 3 ? 1 : 3;
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
   const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
-  if (e - 1u >= 2044u) return (b << 1) == 0 ? x : triple_slow(x);
-  const unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL, t = 3 * m;
-  const int s = t >> 54 ? 2 : 1;
-  const unsigned long long r = (t + (s - 1) + ((t >> s) & 1)) >> s;
+  if (e - 1u >= 2045u - S) return (b << 1) == 0 ? x : times_slow(x, K);
+  const unsigned long long m = (b & 0xfffffffffffffULL) | 0x10000000000000ULL, t = K * m;
+  const int s = t >> (53 + S) ? S + 1 : S;
+  const unsigned long long r = (t + ((1u << (s - 1)) - 1) + ((t >> s) & 1)) >> s;
   return __longlong_as_double((long long)((b & 0x8000000000000000ULL) + r + ((unsigned long long)(e + s - 1) << 52)));
 }
+__device__ __forceinline__ double int_triple(double x) { return int_times<3>(x); }
 
-// x 2^-K (K = 1, 2) as the FP64 multiply gives it: K less in the exponent field
-// while the result stays normal; a zero stays itself; subnormal results, inf
-// and NaN go through the multiply, out of line.
-static __device__ __noinline__ double scale_slow(double x, double f) { return __dmul_rn(x, f); }
+// x 2^-K as the FP64 multiply gives it: K less in the exponent field while the
+// result stays normal; a zero stays itself; subnormal results, inf and NaN go
+// through the multiply, out of line.
+static __device__ __noinline__ double scale_slow(double x, int K) {
+  return __dmul_rn(x, __longlong_as_double((long long)(1023 - K) << 52));
+}
 __device__ __forceinline__ double scale_down(double x, int K) {
   const long long b = __double_as_longlong(x), e = (b >> 52) & 0x7ff;
   if (e > K && e < 0x7ff) return __longlong_as_double(b - ((long long)K << 52));
   if ((b & 0x7fffffffffffffffLL) == 0) return x;
-  return scale_slow(x, K == 1 ? 0.5 : 0.25);
+  return scale_slow(x, K);
 }
 template <int K>
 __device__ __forceinline__ double scale_down(double x) {

@@ -439,8 +439,8 @@ __global__ void __launch_bounds__(256) k_dense(const double *__restrict__ M, con
     __syncthreads();
   }
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  const int tw = gridDim.x * nw;
-  for (int row = blockIdx.x * nw + (threadIdx.x >> 5); row < n; row += tw) {
+  // rows dealt out block by block: every SM gets the same number of them
+  for (int row = (threadIdx.x >> 5) * gridDim.x + blockIdx.x; row < n; row += gridDim.x * nw) {
     if (row >= m) {
       if (lane == 0) e[idx[row]] = r[idx[row]];
       continue;

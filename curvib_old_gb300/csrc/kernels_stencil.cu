@@ -342,7 +342,7 @@ template void launch_zebra_half<double>(const LevelDev &, const double *, double
 // zero_c, when set, is zeroed over the coarse grid in the same pass (the next
 // level's correction, which its V-cycle updates in place).
 template <typename T>
-__global__ void k_restrict(const __grid_constant__ LevelDev F, const __grid_constant__ LevelDev C,
+__global__ void __launch_bounds__(kFlat) k_restrict(const __grid_constant__ LevelDev F, const __grid_constant__ LevelDev C,
                            const T *__restrict__ xf, T *__restrict__ xc, T *__restrict__ zero_c) {
   dep_sync();
   if (gated(F.gate)) return;
@@ -354,7 +354,7 @@ __global__ void k_restrict(const __grid_constant__ LevelDev F, const __grid_cons
 }
 
 template <typename T>
-__global__ void k_prolong_add(const __grid_constant__ LevelDev C, const __grid_constant__ LevelDev F,
+__global__ void __launch_bounds__(kFlat) k_prolong_add(const __grid_constant__ LevelDev C, const __grid_constant__ LevelDev F,
                               const T *__restrict__ xc, T *__restrict__ xf) {
   dep_sync();
   if (gated(F.gate)) return;
@@ -367,7 +367,8 @@ void launch_restrict(const LevelDev &F, const LevelDev &C, const T *xf, T *xc, c
 }
 template <typename T>
 void launch_prolong_add(const LevelDev &C, const LevelDev &F, const T *xc, T *xf, cudaStream_t s) {
-  launch_dep(k_prolong_add<T>, dim3(plane_blocks(F.g), 1, F.g.mz), kFlat, 0, s, C, F, xc, xf);
+  const ProlongGrid g = ProlongGrid::of(F);
+  launch_dep(k_prolong_add<T>, dim3(g.gx, 1, g.gz), kFlat, 0, s, C, F, xc, xf);
 }
 template void launch_restrict<float>(const LevelDev &, const LevelDev &, const float *, float *, cudaStream_t,
                                      float *);

@@ -172,3 +172,17 @@ def test_conversions_are_the_rounded_ones():
             assert widen(u) is None, u
         else:
             assert bits(widen(u)) == bits(f), u
+
+
+def test_ninefold_is_the_rounded_one():
+    rng = random.Random(6)
+    for p in list(significands(rng)) + [rng.getrandbits(52) for _ in range(5000)]:
+        for e in (0, 1, 2, 1023, 2041, 2042, 2043, 2046):
+            x = value(rng.getrandbits(1) << 63 | e << 52 | p)
+            b = bits(x)
+            if not 1 <= e <= 2042:
+                continue  # zeros as they are, the others by the multiply
+            t = 9 * (b & (2**52 - 1) | 2**52)
+            s = 4 if t >> 56 else 3
+            r = (t + (1 << (s - 1)) - 1 + (t >> s & 1)) >> s
+            assert bits(9.0 * x) == ((b & 2**63) + r + ((e + s - 1) << 52)) & (2**64 - 1), x
