@@ -733,6 +733,24 @@ void coarse_solve<double>(cvb_ctx *ctx, const double *b, double *x, const cvb_so
 template <typename T>
 static void vcycle(cvb_ctx *ctx, int l, const T *b, T *out, const cvb_solve_opts *o, bool zeroed = false);
 
+// The finest of the small levels that a V-cycle takes in the tail kernels
+// (kernels_tail.cu), 0: none.
+template <typename T>
+static int tail_top(cvb_ctx *ctx, const cvb_solve_opts *o) {
+  if (o->smoother != CVB_SMOOTHER_ZEBRA || !ctx->coarse_dense) return 0;
+  return tail_levels<T>(ctx->L.data(), ctx->nlevels);
+}
+template <typename T>
+static void vcycle_tail(cvb_ctx *ctx, int top, const cvb_solve_opts *o) {
+  T *v[kTailLevels + 1][4];
+  for (int l = 0; l <= top; l++)
+    for (int q = 0; q < 4; q++) v[l][q] = vptr<T>(ctx->L[l], q);
+  const int pre = std::max(o->pre_sweeps, 1);
+  launch_tail<T>(ctx->L.data(), v, top, pre, o->post_sweeps, (T)o->omega, false, ctx->stream);
+  coarse_solve<T>(ctx, v[0][0], v[0][1], o);
+  launch_tail<T>(ctx->L.data(), v, top, pre, o->post_sweeps, (T)o->omega, true, ctx->stream);
+}
+
 // The V-cycle with zebra smoothing: x (= out) is updated in place, each sweep
 // one half-sweep per color.  zeroed: x is already zero (the restriction into
 // this level cleared it).
@@ -748,7 +766,8 @@ static void vcycle_zebra(cvb_ctx *ctx, int l, const T *b, T *x, const cvb_solve_
   for (int q = 0; q < pre; q++) launch_zebra_sweep<T>(L, b, x, tmp, res, omega, q == 0, s);
   launch_residual<T>(L, b, x, res, s);
   T *bc = vptr<T>(C, 0), *ec = vptr<T>(C, 1);
-  const bool clear = l - 1 > 0;  // the coarsest solve writes all of ec itself
+  // the coarsest solve and the tail write all of ec themselves
+  const bool clear = l - 1 > 0 && l - 1 != tail_top<T>(ctx, o);
   launch_restrict<T>(L, C, res, bc, s, clear ? ec : nullptr);
   vcycle<T>(ctx, l - 1, bc, ec, o, clear);
   launch_prolong_add<T>(C, L, ec, x, s);
@@ -760,6 +779,7 @@ template <typename T>
 static void vcycle(cvb_ctx *ctx, int l, const T *b, T *out, const cvb_solve_opts *o, bool zeroed) {
   cudaStream_t s = ctx->stream;
   if (l == 0) { coarse_solve<T>(ctx, b, out, o); return; }
+  if (l == tail_top<T>(ctx, o)) { vcycle_tail<T>(ctx, l, o); return; }
   if (o->smoother == CVB_SMOOTHER_ZEBRA) { vcycle_zebra<T>(ctx, l, b, out, o, zeroed); return; }
   LevelDev &L = ctx->L[l], &C = ctx->L[l - 1];
   size_t n = L.g.n();

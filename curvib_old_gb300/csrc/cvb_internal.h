@@ -394,4 +394,15 @@ void launch_line_rows(const Geom &g, const double *w64, const double *line64, do
 void launch_lines(const LevelDev &L, bool fused, const double *r, const double *x, double *xnew, double omega,
                   int color, int rsplit, cudaStream_t s);
 
+// --- a V-cycle's small levels in two kernels (kernels_tail.cu)
+constexpr int kTailLevels = 3;
+// how many of the levels 1, 2, ... they take (below the finest level)
+template <typename T>
+int tail_levels(const LevelDev *L, int nlevels);
+// v: each level's right-hand side, correction, scratch and residual; up false:
+// from the right-hand side of level n to that of level 0; up true: from level 0's
+// correction to level n's
+template <typename T>
+void launch_tail(const LevelDev *L, T *const (*v)[4], int n, int pre, int post, T omega, bool up, cudaStream_t s);
+
 }  // namespace cvb
