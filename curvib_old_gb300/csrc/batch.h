@@ -39,11 +39,11 @@ struct TaskList {
 struct KState {
   double H[(kBatchRestart + 1) * kBatchRestart];  // column j at H[j*(m+1) ...]
   double cs[kBatchRestart], sn[kBatchRestart], g[kBatchRestart + 1], y[kBatchRestart];
-  double beta;        // ||r|| at the start of the cycle
+  double rbeta;       // 1 / ||r|| at the start of the cycle: the scale of V_0
   double bnorm;       // ||b|| (after the range projection)
   double target;      // max(rtol*bnorm, atol)
   double est;         // |g_{j+1}|: the residual estimate of the current iterate
-  double hn;          // ||w|| after orthogonalisation: the scale of the next basis vector
+  double rhn;         // 1 / ||w|| after orthogonalisation: the scale of the next basis vector
   double removed;     // range projection: fluid mean of b/aj that was removed
   int m;              // restart length
   int max_it;
@@ -81,6 +81,7 @@ struct BProblem {
   BFlags *fl;
   const LevelDev *F;         // finest level (device copy)
   const double *aj;          // finest aj (FP64)
+  const double *inv_aj;      // and its reciprocals
 };
 
 // Reduction blocks of a problem of n cells: fixed by n alone, so a problem's
@@ -108,7 +109,7 @@ void glaunch_zebra_fused(const TaskList &tl, bool f32, float omega32, double ome
 void glaunch_zero(const TaskList &tl, bool f32, cudaStream_t s);
 // dense coarsest solve: a = r, b = Minv, c = e, p0 = n
 void glaunch_dense(const TaskList &tl, bool f32, cudaStream_t s);
-// element-wise: a = src, c = dst, p0 = n; kind 0 copy f32, 1 copy f64, 2 f64->f32, 3 f32->f64
+// element-wise: a = src, c = dst, p0 = n; kind 0 copy f32, 1 copy f64, 2 f32->f64
 void glaunch_elementwise(const TaskList &tl, int kind, cudaStream_t s);
 
 // Krylov phases over problems: p0 = problem index into P (device array).

@@ -58,7 +58,7 @@ struct Done {
 
 // Sink of the ops of one round, grouped by schedule key and kernel kind.
 enum OpKind {
-  OK_RES32, OK_RES64, OK_RESTRICT, OK_PROLONG, OK_SWEEP, OK_SOLVE, OK_DENSE, OK_COPY, OK_CONV, OK_WIDEN,
+  OK_RES32, OK_RES64, OK_RESTRICT, OK_PROLONG, OK_SWEEP, OK_SOLVE, OK_DENSE, OK_COPY,
   OK_ZERO, OK_RESC, OK_ZFUSED,
   // line solves of levels whose lines have 1, 2, 4 or 8 rows per lane: one
   // launch each, so each runs the kernel specialised for its layout
@@ -376,8 +376,6 @@ static void run_program(cvb_batch *bt, std::map<long long, std::array<Lists, OK_
           case OK_SOLVE_R8: glaunch_line_solve(ob.tl, f32, w32, w64, ob.smem, 8, s); break;
           case OK_DENSE: glaunch_dense(ob.tl, f32, s); break;
           case OK_COPY: glaunch_elementwise(ob.tl, f32 ? 0 : 1, s); break;
-          case OK_CONV: glaunch_elementwise(ob.tl, 2, s); break;
-          case OK_WIDEN: glaunch_elementwise(ob.tl, 3, s); break;
           case OK_ZERO: glaunch_zero(ob.tl, f32, s); break;
           case OK_RESC: glaunch_resid_color(ob.tl, f32, s); break;
           case OK_ZFUSED: glaunch_zebra_fused(ob.tl, f32, w32, w64, ob.smem, s); break;
@@ -464,16 +462,11 @@ static const LevelDev *dlev(cvb_batch *bt, int slot) { return bt->dL + (size_t)s
 static size_t fine_cells(cvb_ctx *c) { return c->L[c->nlevels - 1].g.n(); }
 
 // Multidot tasks of w with V[0..nv) (+ w.w into self_row when self_row >= 0).
-static void add_multidot(Lists &ls, const Prob &p, const double *w, int nv, int self_row, const int *gate) {
+// dots of w with nv basis vectors, or (nv = 0) its norm
+static void add_multidot(Lists &ls, const Prob &p, const double *w, int nv, const int *gate) {
   const int nb = batch_reduce_blocks(fine_cells(p.ctx));
-  if (nv == 0) {
-    ls.add(task(nullptr, w, nullptr, nullptr, gate, 0, 0, p.slot, 0, self_row), nb);
-    return;
-  }
-  for (int base = 0; base < nv; base += 8) {
-    int cnt = std::min(8, nv - base);
-    ls.add(task(nullptr, w, nullptr, nullptr, gate, 0, 0, p.slot, base | (cnt << 8), base == 0 ? self_row : -1), nb);
-  }
+  for (int base = 0; base == 0 || base < nv; base += 8)
+    ls.add(task(nullptr, w, nullptr, nullptr, gate, 0, 0, p.slot, base | (std::min(8, nv - base) << 8)), nb);
 }
 static void add_finish(Lists &ls, const Prob &p, int row0, int rows, const int *gate) {
   ls.add(task(nullptr, nullptr, nullptr, nullptr, gate, rows, 0, p.slot, row0), rows);
@@ -523,6 +516,7 @@ static int admit(cvb_batch *bt, Prob &p) {
   P.ks = dks(bt, p.slot); P.fl = dfl(bt, p.slot);
   P.F = dlev(bt, p.slot) + (c->nlevels - 1);
   P.aj = c->aj64[c->nlevels - 1];
+  P.inv_aj = c->inv_aj;
   BCK(cudaMemcpyAsync(dprob(bt, p.slot), &P, sizeof P, cudaMemcpyHostToDevice, bt->stream));
   BFlags f;
   std::memset(&f, 0, sizeof f);
@@ -556,7 +550,7 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
         rem.add(task(nullptr, nullptr, nullptr, nullptr, nog, elem_blocks(n), 0, p->slot), elem_blocks(n));
         proj_slots.push_back(p->slot);
       }
-      add_multidot(norm, *p, p->ctx->b, 0, kNormRow, nog);
+      add_multidot(norm, *p, p->ctx->b, 0, nog);
       add_finish(finn, *p, kNormRow, 1, nog);
     }
     launch_lists(ratio, glaunch_fluid_ratio, bt);
@@ -606,9 +600,10 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
                 *gnot = &dfl(bt, p->slot)->notfin;
       const int gx = plane_blocks(F.g);
       res.add(task(dlev(bt, p->slot) + (c->nlevels - 1), c->x, c->b, c->r, gfin, gx, 1), gx * F.g.mz);
-      add_multidot(norm, *p, c->r, 0, kNormRow, gfin);
+      add_multidot(norm, *p, c->r, 0, gfin);
       add_finish(finn, *p, kNormRow, 1, gfin);
-      scale.add(task(nullptr, c->r, &dks(bt, p->slot)->beta, c->V[0], ggate, elem_blocks(n), 0, (int)n),
+      scale.add(task(f32 ? (const LevelDev *)c->b32 : nullptr, c->r, &dks(bt, p->slot)->rbeta, c->V[0], ggate,
+                     elem_blocks(n), 0, (int)n),
                 elem_blocks(n));
       fsum.add(task(nullptr, nullptr, nullptr, nullptr, gnot, 0, 0, p->slot), batch_reduce_blocks(n));
       add_finish(fin01, *p, 0, 2, gnot);
@@ -628,7 +623,7 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
   if (!iterating.empty()) {
     std::map<long long, std::array<Lists, OK_COUNT>> prog;
     VSink vs{&prog};
-    Lists conv, widen, apply, mdot, fin, maxpy, finn, scale;
+    Lists widen, apply, mdot, fin, maxpy, finn, scale;
     std::vector<int> slots;
     for (Prob *p : iterating) {
       cvb_ctx *c = p->ctx;
@@ -639,7 +634,7 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
       const int *gate = &dfl(bt, p->slot)->gate;
       const LevelDev *dLs = dlev(bt, p->slot);
       if (f32) {
-        conv.add(task(nullptr, c->V[j], nullptr, c->b32, gate, elem_blocks(n), 0, (int)n), elem_blocks(n));
+        // b32 holds V[j] in FP32, written by the scaling that formed V[j]
         gen_vcycle<float>(vs, c, dLs, nl - 1, 0, c->b32, c->Z32, bt->opts, gate);
         widen.add(task(nullptr, c->Z32, nullptr, c->Z64[j], gate, elem_blocks(n), 0, (int)n), elem_blocks(n));
       } else {
@@ -647,17 +642,17 @@ static int issue_round(cvb_batch *bt, std::vector<Prob *> &starting, std::vector
       }
       const int gx = plane_blocks(F.g);
       apply.add(task(dLs + (nl - 1), c->Z64[j], nullptr, c->w, gate, gx, 1), gx * F.g.mz);
-      add_multidot(mdot, *p, c->w, j + 1, j + 1, gate);
-      add_finish(fin, *p, 0, j + 2, gate);
+      add_multidot(mdot, *p, c->w, j + 1, gate);
+      add_finish(fin, *p, 0, j + 1, gate);
       maxpy.add(task(nullptr, nullptr, nullptr, nullptr, gate, 0, 0, p->slot, j + 1), batch_reduce_blocks(n));
       add_finish(finn, *p, kNormRow, 1, gate);
-      scale.add(task(nullptr, c->w, &dks(bt, p->slot)->hn, c->V[j + 1], gate, elem_blocks(n), 0, (int)n),
+      scale.add(task(f32 ? (const LevelDev *)c->b32 : nullptr, c->w, &dks(bt, p->slot)->rhn, c->V[j + 1], gate,
+                     elem_blocks(n), 0, (int)n),
                 elem_blocks(n));
       slots.push_back(p->slot);
     }
-    for (OpBatch &ob : conv.v) glaunch_elementwise(ob.tl, 2, s);
     run_vcycles(bt, prog, f32, iterating);
-    for (OpBatch &ob : widen.v) glaunch_elementwise(ob.tl, 3, s);
+    for (OpBatch &ob : widen.v) glaunch_elementwise(ob.tl, 2, s);
     launch_lists2(apply, glaunch_residual64, bt);
     launch_lists(mdot, glaunch_multidot, bt);
     launch_lists(fin, glaunch_finish, bt);

@@ -237,19 +237,7 @@ void launch_add_fluid_const(const Geom &g, const uint32_t *code, double *x, cons
 // the norm of the result; host[0] = *mean, host[1] = |b|^2
 void launch_remove_mean(const Geom &g, const uint32_t *code, const double *aj, double *b, const double *mean,
                         double *partial, unsigned *counter, double *out, double *host, cudaStream_t s);
-// b / a for the range projection's sum: an FP32 reciprocal refined by two
-// Newton-Raphson steps in FP64 (r <- r + r (1 - a r)), within a unit or so in
-// the last place of the quotient, at a fraction of an FP64 division's cost on
-// this part (whose FP64 rate is low); a plain division where the FP32
-// reciprocal cannot represent 1/a.
-__device__ __forceinline__ double quot_newton(double b, double a) {
-  const float af = (float)a;
-  double r = (double)__frcp_rn(af);
-  if (!(r != 0.0 && r * 0.0 == 0.0)) return b / a;
-  r = fma(r, fma(-a, r, 1.0), r);
-  r = fma(r, fma(-a, r, 1.0), r);
-  return b * r;
-}
+
 // In-place Gauss-Jordan inverse of the n x n row-major A on the device into
 // out (kernels_setup.cu); false for a singular matrix.  Work arrays: perm and
 // colmap n ints, work dense_inverse_doubles(n) doubles, status one int.

@@ -192,7 +192,8 @@ __global__ void kg_elem(const __grid_constant__ TaskList tl) {
   TD *c = (TD *)K.c;
   const size_t n = (size_t)K.p0;
   for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < n; p += (size_t)K.gx * 256)
-    c[p] = (TD)a[p];
+    if constexpr (sizeof(TS) == 4 && sizeof(TD) == 8) c[p] = int_widen(a[p]);
+    else c[p] = (TD)a[p];
 }
 
 void glaunch_residual32(const TaskList &tl, cudaStream_t s) {
@@ -274,7 +275,6 @@ void glaunch_elementwise(const TaskList &tl, int kind, cudaStream_t s) {
   switch (kind) {
     case 0: launch_dep(kg_elem<float, float>, tl.nblocks, 256, 0, s, tl); break;
     case 1: launch_dep(kg_elem<double, double>, tl.nblocks, 256, 0, s, tl); break;
-    case 2: launch_dep(kg_elem<double, float>, tl.nblocks, 256, 0, s, tl); break;
     default: launch_dep(kg_elem<float, double>, tl.nblocks, 256, 0, s, tl); break;
   }
 }
@@ -301,60 +301,72 @@ __device__ __forceinline__ void block_store(double (&acc)[NR], double *partial, 
   }
 }
 
-template <int NV, bool SELF>
-__device__ __forceinline__ void multidot_body(const BProblem &P, const double *w, int base, int self_row, int lb) {
-  constexpr int NR = NV + (SELF ? 1 : 0);
-  double acc[NR > 0 ? NR : 1];
+// The vector count is a template parameter: predicated-off products would still
+// occupy the FP64 pipe, which bounds these kernels.
+template <int NV>
+__device__ __forceinline__ void multidot_body(const BProblem &P, const double *w, int base, int lb) {
+  double acc[NV];
+  int rows[NV];
+  const double *v[NV];
 #pragma unroll
-  for (int q = 0; q < NR; q++) acc[q] = 0.0;
-  const double *v[NV > 0 ? NV : 1];
+  for (int q = 0; q < NV; q++) acc[q] = 0.0, rows[q] = base + q, v[q] = P.V[base + q];
+  const size_t n = P.n, step = (size_t)P.nb * kRed;
+  constexpr int U = NV <= 2 ? 4 : NV <= 4 ? 2 : 1;
+  size_t p = (size_t)lb * kRed + threadIdx.x;
+  for (; p + (U - 1) * step < n; p += U * step) {
+    double x[U][NV], wp[U];
 #pragma unroll
-  for (int q = 0; q < NV; q++) v[q] = P.V[base + q];
-  const size_t n = P.n;
-  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < n; p += (size_t)P.nb * kRed) {
-    double wp = w[p];
+    for (int u = 0; u < U; u++) {
+      wp[u] = w[p + u * step];
+#pragma unroll
+      for (int q = 0; q < NV; q++) x[u][q] = v[q][p + u * step];
+    }
+#pragma unroll
+    for (int u = 0; u < U; u++)
+#pragma unroll
+      for (int q = 0; q < NV; q++) acc[q] = fma(x[u][q], wp[u], acc[q]);
+  }
+  for (; p < n; p += step) {
+    const double wp = w[p];
 #pragma unroll
     for (int q = 0; q < NV; q++) acc[q] = fma(v[q][p], wp, acc[q]);
-    if (SELF) acc[NV] = fma(wp, wp, acc[NV]);
   }
-  int rows[NR > 0 ? NR : 1];
+  block_store<NV>(acc, P.partial, P.nb, lb, rows);
+}
+__device__ __forceinline__ void norm_body(const BProblem &P, const double *w, int lb) {
+  double acc[1] = {0.0};
+  const int rows[1] = {kNormRow};
+  const size_t n = P.n, step = (size_t)P.nb * kRed;
+  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < n; p += 4 * step) {
+    double x[4];
 #pragma unroll
-  for (int q = 0; q < NV; q++) rows[q] = base + q;
-  if (SELF) rows[NV] = self_row;
-  block_store<NR>(acc, P.partial, P.nb, lb, rows);
+    for (int u = 0; u < 4; u++) x[u] = p + u * step < n ? w[p + u * step] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 4; u++)
+      if (p + u * step < n) acc[0] = fma(x[u], x[u], acc[0]);
+  }
+  block_store<1>(acc, P.partial, P.nb, lb, rows);
 }
 
-__global__ void __launch_bounds__(kRed) kg_multidot(const __grid_constant__ TaskList tl, const BProblem *__restrict__ PP) {
+// p1 = base | count << 8: the dots of a with that many basis vectors; count 0: its norm
+__global__ void __launch_bounds__(kRed, 4) kg_multidot(const __grid_constant__ TaskList tl,
+                                                       const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
   const BProblem P = PP[K.p0];
   const double *w = (const double *)K.a;
-  const int base = K.p1 & 0xff, cnt = (K.p1 >> 8) & 0xff, self_row = K.pad;
-  const int lb = blockIdx.x - K.block0;
-  if (self_row >= 0) {
-    switch (cnt) {
-      case 0: multidot_body<0, true>(P, w, base, self_row, lb); break;
-      case 1: multidot_body<1, true>(P, w, base, self_row, lb); break;
-      case 2: multidot_body<2, true>(P, w, base, self_row, lb); break;
-      case 3: multidot_body<3, true>(P, w, base, self_row, lb); break;
-      case 4: multidot_body<4, true>(P, w, base, self_row, lb); break;
-      case 5: multidot_body<5, true>(P, w, base, self_row, lb); break;
-      case 6: multidot_body<6, true>(P, w, base, self_row, lb); break;
-      case 7: multidot_body<7, true>(P, w, base, self_row, lb); break;
-      default: multidot_body<8, true>(P, w, base, self_row, lb); break;
-    }
-  } else {
-    switch (cnt) {
-      case 1: multidot_body<1, false>(P, w, base, 0, lb); break;
-      case 2: multidot_body<2, false>(P, w, base, 0, lb); break;
-      case 3: multidot_body<3, false>(P, w, base, 0, lb); break;
-      case 4: multidot_body<4, false>(P, w, base, 0, lb); break;
-      case 5: multidot_body<5, false>(P, w, base, 0, lb); break;
-      case 6: multidot_body<6, false>(P, w, base, 0, lb); break;
-      case 7: multidot_body<7, false>(P, w, base, 0, lb); break;
-      default: multidot_body<8, false>(P, w, base, 0, lb); break;
-    }
+  const int base = K.p1 & 0xff, lb = blockIdx.x - K.block0;
+  switch (K.p1 >> 8) {
+    case 0: norm_body(P, w, lb); break;
+    case 1: multidot_body<1>(P, w, base, lb); break;
+    case 2: multidot_body<2>(P, w, base, lb); break;
+    case 3: multidot_body<3>(P, w, base, lb); break;
+    case 4: multidot_body<4>(P, w, base, lb); break;
+    case 5: multidot_body<5>(P, w, base, lb); break;
+    case 6: multidot_body<6>(P, w, base, lb); break;
+    case 7: multidot_body<7>(P, w, base, lb); break;
+    default: multidot_body<8>(P, w, base, lb); break;
   }
 }
 void glaunch_multidot(const TaskList &tl, const BProblem *P, cudaStream_t s) {
@@ -385,45 +397,76 @@ void glaunch_finish(const TaskList &tl, const BProblem *P, cudaStream_t s) {
   launch_dep(kg_finish, tl.nblocks, kRed, 0, s, tl, P);
 }
 
-// w -= sum_{q < nv} sums[q] V_q ; partial[kNormRow][lb] = sum of w^2 over the block
-__global__ void __launch_bounds__(kRed) kg_multiaxpy_norm(const __grid_constant__ TaskList tl,
-                                                          const BProblem *__restrict__ PP) {
+// w -= sum_{q < nv} sums[q] V_q ; partial[kNormRow][lb] = sum of w^2 over the block.
+// NR + 8 octets = nv vectors, loads before products.
+template <int NR>
+__device__ __forceinline__ void multiaxpy_body(const BProblem &P, const double *hs, int octets, int lb) {
+  double acc[1] = {0.0};
+  const int rows[1] = {kNormRow};
+  double *w = P.w;
+  const double *v0[NR];
+#pragma unroll
+  for (int q = 0; q < NR; q++) v0[q] = P.V[q];
+  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < P.n; p += (size_t)P.nb * kRed) {
+    double x[NR], v = w[p];
+#pragma unroll
+    for (int q = 0; q < NR; q++) x[q] = v0[q][p];
+#pragma unroll
+    for (int q = 0; q < NR; q++) v = fma(-hs[q], x[q], v);
+    for (int b = NR; b < NR + 8 * octets; b += 8) {
+      double y[8];
+#pragma unroll
+      for (int q = 0; q < 8; q++) y[q] = P.V[b + q][p];
+#pragma unroll
+      for (int q = 0; q < 8; q++) v = fma(-hs[b + q], y[q], v);
+    }
+    w[p] = v;
+    acc[0] = fma(v, v, acc[0]);
+  }
+  block_store<1>(acc, P.partial, P.nb, lb, rows);
+}
+__global__ void __launch_bounds__(kRed, 4) kg_multiaxpy_norm(const __grid_constant__ TaskList tl,
+                                                             const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
   const BProblem P = PP[K.p0];
-  const int nv = K.p1, lb = blockIdx.x - K.block0;
+  const int nv = K.p1, lb = blockIdx.x - K.block0, o = (nv - 1) / 8;
   __shared__ double hs[kBatchRestart + 1];
   if (threadIdx.x < nv) hs[threadIdx.x] = P.sums[threadIdx.x];
   __syncthreads();
-  double acc = 0.0;
-  double *w = P.w;
-  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < P.n; p += (size_t)P.nb * kRed) {
-    double v = w[p];
-    for (int q = 0; q < nv; q++) v = fma(-hs[q], P.V[q][p], v);
-    w[p] = v;
-    acc = fma(v, v, acc);
+  switch (nv - 8 * o) {
+    case 1: multiaxpy_body<1>(P, hs, o, lb); break;
+    case 2: multiaxpy_body<2>(P, hs, o, lb); break;
+    case 3: multiaxpy_body<3>(P, hs, o, lb); break;
+    case 4: multiaxpy_body<4>(P, hs, o, lb); break;
+    case 5: multiaxpy_body<5>(P, hs, o, lb); break;
+    case 6: multiaxpy_body<6>(P, hs, o, lb); break;
+    case 7: multiaxpy_body<7>(P, hs, o, lb); break;
+    default: multiaxpy_body<8>(P, hs, o, lb); break;
   }
-  double a1[1] = {acc};
-  int rows[1] = {kNormRow};
-  block_store<1>(a1, P.partial, P.nb, lb, rows);
 }
 void glaunch_multiaxpy_norm(const TaskList &tl, const BProblem *P, cudaStream_t s) {
   if (!tl.n) return;
   launch_dep(kg_multiaxpy_norm, tl.nblocks, kRed, 0, s, tl, P);
 }
 
-// dst = src / *scal
-__global__ void kg_scale(const __grid_constant__ TaskList tl) {
+// c = a *b (the reciprocal of a norm) and, where L holds one, an FP32 copy (the
+// next V-cycle's input)
+__global__ void __launch_bounds__(256) kg_scale(const __grid_constant__ TaskList tl) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
-  const double inv = 1.0 / *(const double *)K.b;
+  const double inv = *(const double *)K.b;
   const double *a = (const double *)K.a;
   double *c = (double *)K.c;
+  float *c32 = (float *)K.L;
   const size_t n = (size_t)K.p0;
-  for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < n; p += (size_t)K.gx * 256)
-    c[p] = a[p] * inv;
+  for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < n; p += (size_t)K.gx * 256) {
+    const double v = a[p] * inv;
+    c[p] = v;
+    if (c32) c32[p] = int_narrow(v);
+  }
 }
 void glaunch_scale(const TaskList &tl, cudaStream_t s) {
   if (!tl.n) return;
@@ -442,7 +485,15 @@ __global__ void kg_update(const __grid_constant__ TaskList tl, const BProblem *_
   __syncthreads();
   for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < P.n; p += (size_t)K.gx * 256) {
     double v = P.x[p];
-    for (int q = 0; q < nz; q++) v = fma(ys[q], P.Z[q][p], v);
+    int q = 0;
+    for (; q + 4 <= nz; q += 4) {
+      double z[4];
+#pragma unroll
+      for (int u = 0; u < 4; u++) z[u] = P.Z[q + u][p];
+#pragma unroll
+      for (int u = 0; u < 4; u++) v = fma(ys[q + u], z[u], v);
+    }
+    for (; q < nz; q++) v = fma(ys[q], P.Z[q][p], v);
     P.x[p] = v;
   }
 }
@@ -454,63 +505,62 @@ void glaunch_update(const TaskList &tl, const BProblem *P, cudaStream_t s) {
 // Null space (PoissonNullSpaceFunction, poisson.c:411-558) on the finest level:
 // sums and counts of x over interior fluid cells into partial rows 0, 1.
 __device__ __forceinline__ bool fluid_cell(const uint32_t *code, size_t p) { return (code[p] & CODE_FLUID) != 0; }
+template <bool RATIO>
+__device__ __forceinline__ void fluid_sum_body(const BProblem &P, int lb) {
+  const uint32_t *cd = P.F->code;
+  double acc[2] = {0.0, 0.0};
+  unsigned cnt = 0;  // the cells are counted on the integer pipe
+  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < P.n; p += (size_t)P.nb * kRed)
+    if (fluid_cell(cd, p)) {
+      if (RATIO) acc[0] = fma(P.b[p], P.inv_aj[p], acc[0]);
+      else acc[0] += P.x[p];
+      cnt++;
+    }
+  acc[1] = (double)cnt;
+  const int rows[2] = {0, 1};
+  block_store<2>(acc, P.partial, P.nb, lb, rows);
+}
 __global__ void __launch_bounds__(kRed) kg_fluid_sum(const __grid_constant__ TaskList tl, const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
-  const BProblem P = PP[K.p0];
-  const Geom g = P.F->g;
-  const uint32_t *cd = P.F->code;
-  const int lb = blockIdx.x - K.block0;
-  double acc[2] = {0.0, 0.0};
-  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < P.n; p += (size_t)P.nb * kRed)
-    if (fluid_cell(cd, p)) {
-      acc[0] += P.x[p];
-      acc[1] += 1.0;
-    }
-  int rows[2] = {0, 1};
-  block_store<2>(acc, P.partial, P.nb, lb, rows);
+  fluid_sum_body<false>(PP[K.p0], blockIdx.x - K.block0);
+}
+// sums[0] / (sign sums[1]), the mean over the fluid cells: one division a block
+__device__ __forceinline__ double fluid_mean(const BProblem &P, double sign) {
+  __shared__ double m;
+  if (threadIdx.x == 0) m = P.sums[1] > 0.0 ? P.sums[0] / (sign * P.sums[1]) : 0.0;
+  __syncthreads();
+  return m;
 }
 __global__ void kg_add_fluid_const(const __grid_constant__ TaskList tl, const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
   const BProblem P = PP[K.p0];
-  const Geom g = P.F->g;
   const uint32_t *cd = P.F->code;
-  const double shift = P.sums[1] > 0.0 ? P.sums[0] / (-1.0 * P.sums[1]) : 0.0;
+  const double shift = fluid_mean(P, -1.0);
   for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < P.n; p += (size_t)K.gx * 256) {
     if (fluid_cell(cd, p)) P.x[p] += shift;
     else P.x[p] = 0.0;
   }
 }
-// range projection of b: sums of b/aj and counts over fluid cells (rows 0, 1)
+// range projection of b: sums of b/aj (by the stored reciprocals, as a single
+// solve does) and counts over fluid cells (rows 0, 1)
 __global__ void __launch_bounds__(kRed) kg_fluid_ratio(const __grid_constant__ TaskList tl,
                                                        const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
-  const BProblem P = PP[K.p0];
-  const Geom g = P.F->g;
-  const uint32_t *cd = P.F->code;
-  const int lb = blockIdx.x - K.block0;
-  double acc[2] = {0.0, 0.0};
-  for (size_t p = (size_t)lb * kRed + threadIdx.x; p < P.n; p += (size_t)P.nb * kRed)
-    if (fluid_cell(cd, p)) {
-      acc[0] += quot_newton(P.b[p], P.aj[p]);
-      acc[1] += 1.0;
-    }
-  int rows[2] = {0, 1};
-  block_store<2>(acc, P.partial, P.nb, lb, rows);
+  fluid_sum_body<true>(PP[K.p0], blockIdx.x - K.block0);
 }
 __global__ void kg_remove_aj_mean(const __grid_constant__ TaskList tl, const BProblem *__restrict__ PP) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
   if (gated(K.gate)) return;
   const BProblem P = PP[K.p0];
-  const Geom g = P.F->g;
   const uint32_t *cd = P.F->code;
-  const double c = P.sums[1] > 0.0 ? P.sums[0] / P.sums[1] : 0.0;
+  const double c = fluid_mean(P, 1.0);
   for (size_t p = (size_t)(blockIdx.x - K.block0) * 256 + threadIdx.x; p < P.n; p += (size_t)K.gx * 256)
     if (fluid_cell(cd, p)) P.b[p] -= P.aj[p] * c;
 }
@@ -610,7 +660,7 @@ __global__ void k_cycle_start(const __grid_constant__ ProbList pl, const BProble
     fl->fin = 1;
     return;
   }
-  ks->beta = beta;
+  ks->rbeta = 1.0 / beta;
   ks->j = 0;
   for (int q = 0; q <= ks->m; q++) ks->g[q] = 0.0;
   ks->g[0] = beta;
@@ -637,7 +687,7 @@ __global__ void k_arnoldi(const __grid_constant__ ProbList pl, const BProblem *_
   for (int q = 0; q <= j; q++) Hc[q] = P.sums[q];
   const double hn = sqrt(P.sums[kNormRow]);
   Hc[j + 1] = hn;
-  ks->hn = hn;
+  ks->rhn = 1.0 / hn;
   for (int q = 0; q < j; q++) {
     double t = ks->cs[q] * Hc[q] + ks->sn[q] * Hc[q + 1];
     Hc[q + 1] = -ks->sn[q] * Hc[q] + ks->cs[q] * Hc[q + 1];
