@@ -45,53 +45,70 @@ void launch_gcoef(const Geom &g, const double *const *m, const double *iaj, cons
                                            iaj, jaj, kaj, g9); count_launch();
 }
 
-// The cross-derivative form of poisson.c:793-1324: s_up/s_dn are the nvert sums
-// of the two cells beside the face one step up/down the cross direction.
-__device__ __forceinline__ int cross_branch(double s_up, double s_dn, int c, int m, int per) {
-  if ((c == m - 2 && !per) || s_up > 0.1) return (s_dn < 0.1 && (c != 1 || per)) ? 2 : 0;
-  if ((c == 1 && !per) || s_dn > 0.1) return (s_up < 0.1) ? 3 : 0;
+// The cross-derivative form of poisson.c:793-1324 from the nvert sums of the two
+// cells beside the face one step up/down the cross direction (against 0.1).
+struct NvSum {
+  bool gt, lt;
+  __device__ __forceinline__ NvSum(double s) : gt(s > 0.1), lt(s < 0.1) {}
+};
+__device__ __forceinline__ int cross_branch(NvSum up, NvSum dn, int c, int m, int per) {
+  if ((c == m - 2 && !per) || up.gt) return (dn.lt && (c != 1 || per)) ? 2 : 0;
+  if ((c == 1 && !per) || dn.gt) return up.lt ? 3 : 0;
   return 1;
 }
 
-__global__ void k_codes(Geom g, const double *__restrict__ nv, uint32_t *__restrict__ code) {
-  size_t n = g.n();
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    int i = (int)(p % g.mx), j = (int)((p / g.mx) % g.my), k = (int)(p / ((size_t)g.mx * g.my));
-    uint32_t c = 0;
-    const int mx = g.mx, my = g.my, mz = g.mz;
-    auto NV = [&](int a, int b, int d) { return nv[g.id(a, b, d)]; };
-    bool inj = j >= 1 && j <= my - 2, ink = k >= 1 && k <= mz - 2, ini = i >= 1 && i <= mx - 2;
+// Bound by the FP64 pipe where sums are formed and compared (24 of each a cell); a
+// cell whose 19 values are all zero, the bulk of a flow, takes neither: its sums are
+// zero.
+__global__ void __launch_bounds__(256) k_codes(Geom g, const double *__restrict__ nv, uint32_t *__restrict__ code) {
+  const int n = (int)g.n(), p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int mx = g.mx, my = g.my, mz = g.mz, pl = mx * my;
+  const int k = p / pl, j = (p - k * pl) / mx, i = p - k * pl - j * mx;
+  const bool inj = j >= 1 && j <= my - 2, ink = k >= 1 && k <= mz - 2, ini = i >= 1 && i <= mx - 2;
+  uint32_t c = 0;
+  auto form = [&](auto NV) {
     // upper-face cross branches, for every face some interior row can use
     if (inj && ink && i <= mx - 2) {  // E face of (i,j,k)
-      c |= (uint32_t)cross_branch(NV(i, j + 1, k) + NV(i + 1, j + 1, k), NV(i, j - 1, k) + NV(i + 1, j - 1, k), j, my, g.py) << 8;
-      c |= (uint32_t)cross_branch(NV(i, j, k + 1) + NV(i + 1, j, k + 1), NV(i, j, k - 1) + NV(i + 1, j, k - 1), k, mz, g.pz) << 10;
+      c |= (uint32_t)cross_branch(NV(0, 1, 0) + NV(1, 1, 0), NV(0, -1, 0) + NV(1, -1, 0), j, my, g.py) << 8;
+      c |= (uint32_t)cross_branch(NV(0, 0, 1) + NV(1, 0, 1), NV(0, 0, -1) + NV(1, 0, -1), k, mz, g.pz) << 10;
     }
     if (ini && ink && j <= my - 2) {  // N face
-      c |= (uint32_t)cross_branch(NV(i + 1, j, k) + NV(i + 1, j + 1, k), NV(i - 1, j, k) + NV(i - 1, j + 1, k), i, mx, g.px) << 12;
-      c |= (uint32_t)cross_branch(NV(i, j, k + 1) + NV(i, j + 1, k + 1), NV(i, j, k - 1) + NV(i, j + 1, k - 1), k, mz, g.pz) << 14;
+      c |= (uint32_t)cross_branch(NV(1, 0, 0) + NV(1, 1, 0), NV(-1, 0, 0) + NV(-1, 1, 0), i, mx, g.px) << 12;
+      c |= (uint32_t)cross_branch(NV(0, 0, 1) + NV(0, 1, 1), NV(0, 0, -1) + NV(0, 1, -1), k, mz, g.pz) << 14;
     }
     if (ini && inj && k <= mz - 2) {  // T face
-      c |= (uint32_t)cross_branch(NV(i + 1, j, k) + NV(i + 1, j, k + 1), NV(i - 1, j, k) + NV(i - 1, j, k + 1), i, mx, g.px) << 16;
-      c |= (uint32_t)cross_branch(NV(i, j + 1, k) + NV(i, j + 1, k + 1), NV(i, j - 1, k) + NV(i, j - 1, k + 1), j, my, g.py) << 18;
+      c |= (uint32_t)cross_branch(NV(1, 0, 0) + NV(1, 0, 1), NV(-1, 0, 0) + NV(-1, 0, 1), i, mx, g.px) << 16;
+      c |= (uint32_t)cross_branch(NV(0, 1, 0) + NV(0, 1, 1), NV(0, -1, 0) + NV(0, -1, 1), j, my, g.py) << 18;
     }
-    if (!(ini && inj && ink) || NV(i, j, k) > 0.1) {
+    if (!(ini && inj && ink) || NvSum(NV(0, 0, 0)).gt) {
       c |= CODE_IDENTITY;
     } else {
-      const double thr = 0.1;
       const int x_end = g.px ? mx - 1 : mx - 2, x_str = g.px ? 0 : 1;
       const int y_end = g.py ? my - 1 : my - 2, y_str = g.py ? 0 : 1;
       const int z_end = g.pz ? mz - 1 : mz - 2, z_str = g.pz ? 0 : 1;
-      if (NV(i + 1, j, k) < thr && i != x_end) c |= CODE_ACT_E;
-      if (NV(i - 1, j, k) < thr && i != x_str) c |= CODE_ACT_W;
-      if (NV(i, j + 1, k) < thr && j != y_end) c |= CODE_ACT_N;
-      if (NV(i, j - 1, k) < thr && j != y_str) c |= CODE_ACT_S;
-      if (NV(i, j, k + 1) < thr && k != z_end) c |= CODE_ACT_T;
-      if (NV(i, j, k - 1) < thr && k != z_str) c |= CODE_ACT_B;
+      if (NvSum(NV(1, 0, 0)).lt && i != x_end) c |= CODE_ACT_E;
+      if (NvSum(NV(-1, 0, 0)).lt && i != x_str) c |= CODE_ACT_W;
+      if (NvSum(NV(0, 1, 0)).lt && j != y_end) c |= CODE_ACT_N;
+      if (NvSum(NV(0, -1, 0)).lt && j != y_str) c |= CODE_ACT_S;
+      if (NvSum(NV(0, 0, 1)).lt && k != z_end) c |= CODE_ACT_T;
+      if (NvSum(NV(0, 0, -1)).lt && k != z_str) c |= CODE_ACT_B;
     }
-    if (NV(i, j, k) > 0.1) c |= CODE_BLOCKED;
-    if (ini && inj && ink && NV(i, j, k) < 0.1) c |= CODE_FLUID;
-    code[p] = c;
+    if (NvSum(NV(0, 0, 0)).gt) c |= CODE_BLOCKED;
+    if (ini && inj && ink && NvSum(NV(0, 0, 0)).lt) c |= CODE_FLUID;
+  };
+  bool open = ini && inj && ink;
+  if (open) {
+    const int o[19] = {0,       1,      -1,     mx,      -mx,     pl,      -pl,     1 + mx,  1 - mx, -1 + mx,
+                       -1 - mx, 1 + pl, 1 - pl, -1 + pl, -1 - pl, mx + pl, mx - pl, pl - mx, -pl - mx};
+    long long any = 0;
+#pragma unroll
+    for (int m = 0; m < 19; m++) any |= __double_as_longlong(nv[p + o[m]]);
+    open = (any << 1) == 0;
   }
+  if (open) form([](int, int, int) { return 0.0; });
+  else form([&](int a, int b, int d) { return nv[p + a + b * mx + d * pl]; });
+  code[p] = c;
 }
 
 __global__ void k_weight32(size_t n, const double *__restrict__ nv, float *__restrict__ w) {
@@ -168,7 +185,7 @@ void launch_split_coef(const Geom &g, const float *gf32, const float *ajf32, con
 // One cross term into vol[] in the reference's order (see add_cross in the oracle).
 __device__ __forceinline__ void add_cross(double *vol, int br, double gg, bool up, int P, int Q, int Pu,
                                           int Qu, int Pd, int Qd) {
-  double h = __dmul_rn(gg, 0.5), q = __dmul_rn(gg, 0.25);
+  const double h = scale_down<1>(gg), q = scale_down<2>(gg);
   if (br == 2) {
     if (up) { vol[P] = __dadd_rn(vol[P], h); vol[Q] = __dadd_rn(vol[Q], h); vol[Pd] = __dsub_rn(vol[Pd], h); vol[Qd] = __dsub_rn(vol[Qd], h); }
     else { vol[P] = __dsub_rn(vol[P], h); vol[Q] = __dsub_rn(vol[Q], h); vol[Pd] = __dadd_rn(vol[Pd], h); vol[Qd] = __dadd_rn(vol[Qd], h); }
@@ -183,7 +200,8 @@ __device__ __forceinline__ void add_cross(double *vol, int br, double gg, bool u
 
 // The 19 matrix entries of one row, accumulated exactly as PoissonLHSNew does
 // (poisson.c:789-1327), so the stored weights equal the reference's assembled
-// matrix bit for bit.
+// matrix bit for bit.  Bound by the FP64 pipe, which keeps the sums; the products
+// are on the integer pipe (intmul.cuh).
 __global__ void k_weights(Geom g, const double *__restrict__ g9, const double *__restrict__ aj,
                           const uint32_t *__restrict__ code, double *__restrict__ w) {
   size_t n = g.n();
@@ -194,7 +212,7 @@ __global__ void k_weights(Geom g, const double *__restrict__ g9, const double *_
       for (int m = 0; m < NSLOT; m++) w[(size_t)m * n + p] = (m == CP) ? 1.0 : 0.0;
       continue;
     }
-    int i = (int)(p % g.mx), j = (int)((p / g.mx) % g.my), k = (int)(p / ((size_t)g.mx * g.my));
+    const int i = (int)p % g.mx, j = (int)p / g.mx % g.my, k = (int)p / (g.mx * g.my);
     double vol[NSLOT];
 #pragma unroll
     for (int m = 0; m < NSLOT; m++) vol[m] = 0.0;
@@ -231,9 +249,18 @@ __global__ void k_weights(Geom g, const double *__restrict__ g9, const double *_
       add_cross(vol, code_branch(cb, 2, 1), G(7, pb), false, CP, BP, NP, BN, SP, BS);
       vol[CP] = __dsub_rn(vol[CP], G(8, pb)); vol[BP] = __dadd_rn(vol[BP], G(8, pb));
     }
-    double a = -aj[p];
+    const double a = -aj[p];
+    bool wild = false;
+    const IntMulB ab = int_split_b(a, wild);
+    double r[NSLOT];
 #pragma unroll
-    for (int m = 0; m < NSLOT; m++) w[(size_t)m * n + p] = __dmul_rn(vol[m], a);
+    for (int m = 0; m < NSLOT; m++) r[m] = int_mul(int_split_a(vol[m], wild), ab);
+    if (wild) {
+#pragma unroll
+      for (int m = 0; m < NSLOT; m++) r[m] = __dmul_rn(vol[m], a);
+    }
+#pragma unroll
+    for (int m = 0; m < NSLOT; m++) w[(size_t)m * n + p] = r[m];
   }
 }
 
@@ -245,43 +272,61 @@ void launch_weights(const Geom &g, const double *g9, const double *aj, const dou
 
 // Thomas factors of the in-line (j) part of each row: a_j = w[SP], m_j, c'_j.
 // Couplings that wrap around a periodic y seam stay outside the line solve.
-__global__ void k_line_factors(Geom g, const double *__restrict__ w, double *__restrict__ l64,
-                               float *__restrict__ l32) {
-  size_t n = g.n();
+//
+// A thread a line, a chain of one division a row: bound by that chain's latency, so
+// rows are read four ahead of it and written four at a time.
+__global__ void __launch_bounds__(32) k_line_factors(Geom g, const double *__restrict__ w, double *__restrict__ l64,
+                                                     float *__restrict__ l32) {
+  const size_t n = g.n();
   const LineFac F = LineFac::of(g);
-  const int Q = F.Q;
-  int lines = g.mx * g.mz;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < lines; t += gridDim.x * blockDim.x) {
-    int i = t % g.mx, k = t / g.mx;
-    const size_t base = F.line(i, k);
-    double cprev = 0.0;
-    for (int j = 0; j < g.my; j++) {
-      size_t p = g.id(i, j, k);
-      double a = w[(size_t)SP * n + p], b = w[(size_t)CP * n + p], c = w[(size_t)NP * n + p];
-      if (j == 0 || j == g.my - 1) { a = 0.0; c = 0.0; b = 1.0; }
-      if (g.py && j == 1) a = 0.0;
-      if (g.py && j == g.my - 2) c = 0.0;
-      double m = b - a * cprev;
-      // an empty row (a fluid cell cut off from all its neighbours) has no
-      // pivot: the sweep leaves it unchanged instead of dividing by zero
-      double minv = m != 0.0 ? 1.0 / m : 0.0;
-      double cp = c * minv;
-      if (j >= 1 && j <= g.my - 2) {
-        const size_t q = base + (j - 1);
-        l64[q] = a; l64[Q + q] = minv; l64[2 * Q + q] = cp;
-        l32[q] = (float)a; l32[Q + q] = (float)minv; l32[2 * Q + q] = (float)cp;
-      }
-      cprev = cp;
+  const int Q = F.Q, t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= g.mx * g.mz) return;
+  const int i = t % g.mx, k = t / g.mx;
+  const size_t base = F.line(i, k), col = g.id(i, 1, k);
+  double an[4], bn[4], cn[4], cprev = 0.0;
+  auto read = [&](int q0) {
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const bool in = q0 + u < g.my - 2;
+      const size_t p = col + (size_t)(in ? q0 + u : 0) * g.mx;
+      an[u] = in ? w[(size_t)SP * n + p] : 0.0;
+      bn[u] = in ? w[(size_t)CP * n + p] : 0.0;
+      cn[u] = in ? w[(size_t)NP * n + p] : 0.0;
     }
-    for (int q = g.my - 2; q < Q; q++)  // padding of the runs
-      for (int r = 0; r < 3; r++) { l64[base + r * Q + q] = 0.0; l32[base + r * Q + q] = 0.0f; }
+  };
+  read(0);
+  for (int q0 = 0; q0 < Q; q0 += 4) {
+    double a[4], b[4], c[4], minv[4], cp[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) a[u] = an[u], b[u] = bn[u], c[u] = cn[u];
+    if (q0 + 4 < Q) read(q0 + 4);
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int j = q0 + u + 1;
+      if (g.py && j == 1) a[u] = 0.0;
+      if (g.py && j == g.my - 2) c[u] = 0.0;
+      const double m = b[u] - a[u] * cprev;
+      // an empty row (a fluid cell cut off from all its neighbours) has no
+      // pivot: the sweep leaves it unchanged instead of dividing by zero; the
+      // rows beyond the line (a = b = c = 0) pad the run with zeros likewise
+      minv[u] = m != 0.0 ? 1.0 / m : 0.0;
+      cprev = cp[u] = c[u] * minv[u];
+    }
+    const double *v[3] = {a, minv, cp};
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      const size_t q = base + (size_t)r * Q + q0;
+      reinterpret_cast<double2 *>(l64 + q)[0] = make_double2(v[r][0], v[r][1]);
+      reinterpret_cast<double2 *>(l64 + q)[1] = make_double2(v[r][2], v[r][3]);
+      *reinterpret_cast<float4 *>(l32 + q) = make_float4((float)v[r][0], (float)v[r][1], (float)v[r][2], (float)v[r][3]);
+    }
   }
 }
 
 void launch_line_factors(const Geom &g, const double *w64, double *line64, float *line32,
                          cudaStream_t s) {
   int lines = g.mx * g.mz;
-  k_line_factors<<<nblk(lines, 128), 128, 0, s>>>(g, w64, line64, line32); count_launch();
+  k_line_factors<<<nblk(lines, 32), 32, 0, s>>>(g, w64, line64, line32); count_launch();
 }
 
 __global__ void k_to_f32(const double *__restrict__ a, float *__restrict__ b, size_t n, const int *gate) {
