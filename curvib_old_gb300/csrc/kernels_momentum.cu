@@ -117,12 +117,13 @@ __global__ void __launch_bounds__(128, 4) k_visc_faces(Geom g, const double *__r
   const long st[3] = {1, g.mx, (long)g.mx * g.my};
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
+  const int pl = g.mx * g.my, k = (int)e / pl, j = ((int)e - k * pl) / g.mx, i = (int)e - k * pl - j * g.mx;
   const long P = (long)e;
+  const FaceDirs dirs = FaceDirs::of_block();
   // the directions one after another, not unrolled: three copies of the
   // products' code would not fit the instruction cache
 #pragma unroll 1
-  for (int d = 0; d < 3; d++) {
+  for (int d = dirs.first; d < dirs.end; d++) {
     const bool in = i <= g.mx - 2 && j <= g.my - 2 && k <= g.mz - 2 && (d == 0 || i >= 1) && (d == 1 || j >= 1) &&
                     (d == 2 || k >= 1);
     if (!in) continue;
@@ -244,7 +245,7 @@ void launch_viscous(const Geom &g, const double *nvert, const double *ucat, cons
   for (int d = 0; d < 3; d++)
     for (int a = 0; a < 3; a++) M.m[d][a] = fm[3 * d + a];
   M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
-  const unsigned nb = blocks_for(g.n(), 128);
+  const dim3 nb(blocks_for(g.n(), 128), face_split(blocks_for(g.n(), 128)));
   if (tame && int_mul_factor(nu)) launch_dep(k_visc_faces<true>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
   else launch_dep(k_visc_faces<false>, nb, 128, 0, s, g, nvert, ucat, M, gram, nu, fp);
   if (visc) launch_dep(k_visc_div, blocks_for(g.n(), 256), 256, 0, s, g, (const double *)fp, visc);
@@ -295,7 +296,7 @@ __global__ void __launch_bounds__(128) k_ff1_rct(const __grid_constant__ Geom g,
   const size_t n = g.n();
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int i = (int)(e % g.mx), j = (int)((e / g.mx) % g.my), k = (int)(e / ((size_t)g.mx * g.my));
+  const int pl = g.mx * g.my, k = (int)e / pl, j = ((int)e - k * pl) / g.mx, i = (int)e - k * pl - j * g.mx;
   double out[3] = {0., 0., 0.};
   if (i >= 1 && i <= g.mx - 2 && j >= 1 && j <= g.my - 2 && k >= 1 && k <= g.mz - 2) {
     double rc[3];
@@ -348,6 +349,22 @@ __device__ __noinline__ void ff_previous(const Geom &g, const double *__restrict
   const long sy = g.mx, sz = (long)g.mx * g.my, Q = ((long)k * g.my + j) * g.mx + i;
   if (!ff_dp(nv, p, Q, sz, sy, j, g.my, de)) de = p[Q + sy] - p[Q];
   dz = p[Q + sz] - p[Q];
+}
+
+// What stands in derivative t of cell P at face d where d's own branch assigns
+// nothing: the sections before it in the cell, then the previous cell.
+__device__ __noinline__ double ff_carried(const Geom &g, const double *__restrict__ nv, const double *__restrict__ p,
+                                          int i, int j, int k, int d, int t) {
+  const long st[3] = {1, g.mx, (long)g.mx * g.my}, P = k * st[2] + j * st[1] + i;
+  const int q = t == 0 ? i : t == 1 ? j : k, m = t == 0 ? g.mx : t == 1 ? g.my : g.mz;
+  for (int b = d - 1; b >= 0; b--) {
+    double v;
+    if (t == b) return p[P + st[b]] - p[P];
+    if (ff_dp(nv, p, P, st[b], st[t], q, m, v)) return v;
+  }
+  double de, dz;
+  ff_previous(g, nv, p, i, j, k, de, dz);
+  return t == 1 ? de : dz;
 }
 
 // The pressure gradient through a face, (dp . gram) aj, with FP64 multiplies.
@@ -414,27 +431,23 @@ __global__ void __launch_bounds__(128, 8) k_ff1_faces(const __grid_constant__ Ge
   const long st[3] = {1, mx, (long)mx * my};
   const size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
   if (e >= n) return;
-  const int i = (int)(e % mx), j = (int)((e / mx) % my), k = (int)(e / ((size_t)mx * my));
+  const int pl = mx * my, k = (int)e / pl, j = ((int)e - k * pl) / mx, i = (int)e - k * pl - j * mx;
   const bool in = i >= 1 && i <= mx - 2 && j >= 1 && j <= my - 2 && k >= 1 && k <= mz - 2;
   if (!CALC && !in) return;
   const long P = (long)e;
   const bool solid = in && gt_01(nv[P]);
-  double dp[3] = {0.0, 0.0, 0.0};
+  const FaceDirs dirs = FaceDirs::of_block();
 #pragma unroll 1
-  for (int d = 0; d < 3; d++) {
+  for (int d = dirs.first; d < dirs.end; d++) {
     const long sd = d == 0 ? st[0] : d == 1 ? st[1] : st[2];
     double v = 0.;
     if (in) {
+      double dp[3];
 #pragma unroll
       for (int t = 0; t < 3; t++) {
-        if (t == d) {
-          dp[t] = p[P + sd] - p[P];
-        } else if (!ff_dp(nv, p, P, sd, st[t], t == 0 ? i : t == 1 ? j : k, t == 0 ? mx : t == 1 ? my : mz, dp[t]) &&
-                   d == 0) {
-          double de, dz;
-          ff_previous(g, nv, p, i, j, k, de, dz);
-          dp[t] = t == 1 ? de : dz;
-        }
+        if (t == d) dp[t] = p[P + sd] - p[P];
+        else if (!ff_dp(nv, p, P, sd, st[t], t == 0 ? i : t == 1 ? j : k, t == 0 ? mx : t == 1 ? my : mz, dp[t]))
+          dp[t] = ff_carried(g, nv, p, i, j, k, d, t);
       }
       // (csi . nd, eta . nd, zet . nd) of face d, from k_face_gram
       const double *gr = gram + (size_t)(3 * d) * n + P;
@@ -501,7 +514,9 @@ void launch_form_function1(const Geom &g, const double *nvert, const double *p, 
   if (calc) A = {calc->ucont, calc->ucont_o, calc->ucont_rm1, calc->bdf2, calc->neg_inv_dt, calc->mz_end};
   const unsigned nb = blocks_for(g.n(), 128);
   launch_dep(k_ff1_rct, nb, 128, 0, s, g, conv, fp, csi, eta, zet, aj, rct);
-  auto go = [&](auto kern) { launch_dep(kern, nb, 128, 0, s, g, nvert, p, (const double *)rct, M, gram, A, rhs); };
+  auto go = [&](auto kern) {
+    launch_dep(kern, dim3(nb, face_split(nb)), 128, 0, s, g, nvert, p, (const double *)rct, M, gram, A, rhs);
+  };
   const bool whole = tame && (!calc || int_mul_factor(calc->neg_inv_dt));
   if (calc) whole ? go(k_ff1_faces<true, true>) : go(k_ff1_faces<false, true>);
   else whole ? go(k_ff1_faces<true, false>) : go(k_ff1_faces<false, false>);
@@ -532,37 +547,34 @@ __global__ void __launch_bounds__(256) k_imp_waxpy(Geom g, double a, const doubl
 // The two infinity norms ImpRK takes after its stages (implicitsolver.c:
 // 7183-7200): |rhs| and |pu - u| (VecWAXPY(dU, -1, u, pu)), or |rhs| alone
 // when pu is null.  The largest |x| is exact in any order; non-negative
-// doubles order as their bit patterns, so blocks combine with an integer
-// atomicMax into out[0..1] (zeroed by the host).  NaN entries are passed
+// doubles order as their bit patterns, so every maximum is an integer one (FP64
+// comparisons took 44 us at 96^3), the blocks' by atomicMax into out[0..1] (zeroed
+// by the host).  NaN entries are passed
 // over, as a comparison-based maximum passes them.
+__device__ __forceinline__ void imp_max(unsigned long long &m, double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x) & 0x7fffffffffffffffULL;
+  if (b > m && b <= 0x7ff0000000000000ULL) m = b;
+}
 __global__ void __launch_bounds__(256) k_imp_norms(size_t n, const double *__restrict__ rhs,
                                                    const double *__restrict__ pu, const double *__restrict__ u,
                                                    unsigned long long *out) {
-  double mf = 0., md = 0.;
+  unsigned long long mf = 0, md = 0;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
-    const double f = fabs(rhs[e]);
-    if (f > mf) mf = f;
-    if (pu) {
-      const double d = fabs(-1. * u[e] + pu[e]);
-      if (d > md) md = d;
-    }
+    imp_max(mf, rhs[e]);
+    if (pu) imp_max(md, -1. * u[e] + pu[e]);
   }
   for (int o = 16; o; o >>= 1) {
-    const double f = __shfl_xor_sync(0xffffffffu, mf, o), d = __shfl_xor_sync(0xffffffffu, md, o);
-    if (f > mf) mf = f;
-    if (d > md) md = d;
+    mf = max(mf, __shfl_xor_sync(0xffffffffu, mf, o));
+    md = max(md, __shfl_xor_sync(0xffffffffu, md, o));
   }
-  __shared__ double sf[8], sd[8];
+  __shared__ unsigned long long sf[8], sd[8];
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
   if (l == 0) { sf[w] = mf; sd[w] = md; }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int q = 1; q < (int)(blockDim.x >> 5); q++) {
-      if (sf[q] > mf) mf = sf[q];
-      if (sd[q] > md) md = sd[q];
-    }
-    atomicMax(out, (unsigned long long)__double_as_longlong(mf));
-    if (pu) atomicMax(out + 1, (unsigned long long)__double_as_longlong(md));
+    for (int q = 1; q < (int)(blockDim.x >> 5); q++) mf = max(mf, sf[q]), md = max(md, sd[q]);
+    atomicMax(out, mf);
+    if (pu) atomicMax(out + 1, md);
   }
 }
 
