@@ -365,31 +365,27 @@ static int build_operators(cvb_ctx *ctx) {
   size_t nmax = 0;
   for (auto &lv : ctx->L) nmax = std::max(nmax, lv.g.n());
   TRY(dalloc(ctx, &g9, 9 * nmax));
+  // which levels have cross-derivative terms (the kernels read 7 points on the
+  // others, with the same results)
+  int *flags = nullptr;
+  TRY(dalloc(ctx, &flags, 2 * (size_t)nl));
+  CK(cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nl, ctx->stream));
   for (int l = 0; l < nl; l++) {
     LevelDev &lv = ctx->L[l];
     const Geom &g = lv.g;
     size_t n = g.n();
     const double *m[9];
     for (int q = 0; q < 9; q++) m[q] = ctx->fm[l][q];
-    launch_gcoef(g, m, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], g9, ctx->stream);
     launch_codes(g, lv.nvert, lv.code, ctx->stream);
+    launch_gcoef(g, m, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], lv.code, g9, lv.gf32, flags + 2 * l, ctx->stream);
     launch_weight32(g, lv.nvert, lv.wgt32, ctx->stream);
-    launch_weights(g, g9, ctx->aj64[l], lv.nvert, lv.code, lv.w64, ctx->stream);
+    launch_weights(g, g9, ctx->aj64[l], lv.code, lv.w64, flags + 2 * l + 1, ctx->stream);
     launch_line_factors(g, lv.w64, lv.line64, lv.line32, ctx->stream);
-    launch_to_f32(g9, lv.gf32, 9 * n, ctx->stream);
-    launch_scale_cross(g, lv.code, lv.gf32, ctx->stream);
     launch_to_f32(ctx->aj64[l], lv.ajf32, n, ctx->stream);
     CKL();
   }
   // g9 is a set-up temporary; return it to the pool
   dfree(ctx, g9);
-  // which levels have cross-derivative terms (the kernels read 7 points on the
-  // others, with the same results)
-  int *flags = nullptr;
-  TRY(dalloc(ctx, &flags, 2 * (size_t)nl));
-  CK(cudaMemsetAsync(flags, 0, sizeof(int) * 2 * nl, ctx->stream));
-  for (int l = 0; l < nl; l++) launch_cross_flags(ctx->L[l].g, ctx->L[l].gf32, ctx->L[l].w64, flags + 2 * l, ctx->stream);
-  CKL();
   std::vector<int> hf(2 * nl);
   CK(cudaMemcpyAsync(hf.data(), flags, sizeof(int) * 2 * nl, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));

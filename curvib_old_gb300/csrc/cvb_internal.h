@@ -144,19 +144,22 @@ constexpr int kMaxFusedRows = 400;
 
 // --- kernel launchers (defined in the .cu files) ---------------------------
 // setup
-void launch_gcoef(const Geom &g, const double *const *metric /*12 Cmpnts fields: I(csi,eta,zet) J.. K..*/,
-                  const double *iaj, const double *jaj, const double *kaj, double *g9 /*[9][N]*/,
-                  cudaStream_t s);
+// The face metrics of a level, by value in a kernel's parameters.
+struct FaceMetrics {
+  const double *m[3][3];  // [face direction][csi, eta, zet] Cmpnts arrays
+  const double *aj[3];    // IAj, JAj, KAj
+};
+// after launch_codes; gf32: the FP32 copies, cross terms scaled by their form's
+// weight; *cross = 1 where one is not zero (zeroed by the caller)
+void launch_gcoef(const Geom &g, const double *const *metric /*9 Cmpnts fields: I(csi,eta,zet) J.. K..*/,
+                  const double *iaj, const double *jaj, const double *kaj, const uint32_t *code, double *g9 /*[9][N]*/,
+                  float *gf32 /*[9][N]*/, int *cross, cudaStream_t s);
 void launch_codes(const Geom &g, const double *nvert, uint32_t *code, cudaStream_t s);
 // wgt32 = (float) max(0, 1 - nvert)
 void launch_weight32(const Geom &g, const double *nvert, float *wgt32, cudaStream_t s);
-// flags[0] |= some FP32 cross coefficient is non-zero, flags[1] |= some FP64
-// edge weight is non-zero (flags zeroed by the caller)
-void launch_cross_flags(const Geom &g, const float *gf32, const double *w64, int *flags, cudaStream_t s);
-// FP32 face coefficients: cross terms pre-scaled by their form's weight (after launch_codes)
-void launch_scale_cross(const Geom &g, const uint32_t *code, float *gf32, cudaStream_t s);
-void launch_weights(const Geom &g, const double *g9, const double *aj, const double *nvert,
-                    const uint32_t *code, double *w64, cudaStream_t s);
+// *cross = 1 where an edge weight is not zero (zeroed by the caller)
+void launch_weights(const Geom &g, const double *g9, const double *aj, const uint32_t *code, double *w64, int *cross,
+                    cudaStream_t s);
 void launch_line_factors(const Geom &g, const double *w64, double *line64, float *line32,
                          cudaStream_t s);
 void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate = nullptr);

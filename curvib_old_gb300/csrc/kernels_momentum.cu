@@ -41,11 +41,6 @@ __device__ __forceinline__ bool lt_01(double v) {
   return b < kBits01 && !(b > kBitsNegInf && b < 0);
 }
 
-struct FaceMetrics {
-  const double *m[3][3];  // [face direction][csi, eta, zet] Cmpnts arrays
-  const double *aj[3];    // IAj, JAj, KAj
-};
-
 }  // namespace
 
 namespace {

@@ -11,38 +11,67 @@ namespace cvb {
 
 static inline unsigned nblk(size_t n, int t) { return (unsigned)((n + t - 1) / t); }
 
-// g11..g33 of PoissonLHSNew (poisson.c:699-735): (metric_b . metric_a) * face Jacobian.
-__global__ void k_gcoef(Geom g, const double *__restrict__ ic, const double *__restrict__ ie,
-                        const double *__restrict__ iz, const double *__restrict__ jc,
-                        const double *__restrict__ je, const double *__restrict__ jz,
-                        const double *__restrict__ kc, const double *__restrict__ ke,
-                        const double *__restrict__ kz, const double *__restrict__ iaj,
-                        const double *__restrict__ jaj, const double *__restrict__ kaj,
-                        double *__restrict__ g9) {
-  size_t n = g.n();
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    const double *a = ic + 3 * p, *b = ie + 3 * p, *c = iz + 3 * p;
-    double j1 = iaj[p];
-    g9[0 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], a[0]), __dmul_rn(a[1], a[1])), __dmul_rn(a[2], a[2])), j1);
-    g9[1 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(b[0], a[0]), __dmul_rn(b[1], a[1])), __dmul_rn(b[2], a[2])), j1);
-    g9[2 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(c[0], a[0]), __dmul_rn(c[1], a[1])), __dmul_rn(c[2], a[2])), j1);
-    a = jc + 3 * p; b = je + 3 * p; c = jz + 3 * p;
-    double j2 = jaj[p];
-    g9[3 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2])), j2);
-    g9[4 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(b[0], b[0]), __dmul_rn(b[1], b[1])), __dmul_rn(b[2], b[2])), j2);
-    g9[5 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(c[0], b[0]), __dmul_rn(c[1], b[1])), __dmul_rn(c[2], b[2])), j2);
-    a = kc + 3 * p; b = ke + 3 * p; c = kz + 3 * p;
-    double j3 = kaj[p];
-    g9[6 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(a[0], c[0]), __dmul_rn(a[1], c[1])), __dmul_rn(a[2], c[2])), j3);
-    g9[7 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(b[0], c[0]), __dmul_rn(b[1], c[1])), __dmul_rn(b[2], c[2])), j3);
-    g9[8 * n + p] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(c[0], c[0]), __dmul_rn(c[1], c[1])), __dmul_rn(c[2], c[2])), j3);
+// g11..g33 of PoissonLHSNew (poisson.c:699-735): (metric_b . metric_a) * face
+// Jacobian, and their FP32 copies, in which each cross term carries the weight of
+// its form (0 none, 1/4 central, 1/2 one-sided), so that the FP32 rows need no
+// per-term selection (powers of two: that scaling is exact).  *cross is set where
+// any FP32 cross term is not zero.
+//
+// Bound by the FP64 pipe: half of the products and the conversions are on the
+// integer pipe (intmul.cuh; values beyond its range take FP64 multiplies).  At 96^3
+// 103 us with all of them in FP64, and 33 us more for the copies made apart.
+__device__ __noinline__ void gcoef_face_fp64(const double *const (&x)[3], const double *r, double j, double (&out)[3]) {
+  for (int t = 0; t < 3; t++)
+    out[t] = __dmul_rn(__dadd_rn(__dadd_rn(__dmul_rn(x[t][0], r[0]), __dmul_rn(x[t][1], r[1])), __dmul_rn(x[t][2], r[2])), j);
+}
+__device__ __forceinline__ void gcoef_face(const double *const (&x)[3], const double *r, double j, double (&out)[3]) {
+  bool wild = false;
+  const double r0 = r[0];
+  const IntMulB r1 = int_split_b(r[1], wild), r2 = int_split_b(r[2], wild), jb = int_split_b(j, wild);
+#pragma unroll
+  for (int t = 0; t < 3; t++) {
+    const double s = __dadd_rn(__dadd_rn(__dmul_rn(x[t][0], r0), int_mul(int_split_a(x[t][1], wild), r1)),
+                               int_mul(int_split_a(x[t][2], wild), r2));
+    out[t] = int_mul(int_split_a(s, wild), jb);
   }
+  if (wild) gcoef_face_fp64(x, r, j, out);
+}
+__global__ void __launch_bounds__(128) k_gcoef(Geom g, const __grid_constant__ FaceMetrics M,
+                                               const uint32_t *__restrict__ code, double *__restrict__ g9,
+                                               float *__restrict__ gf, int *__restrict__ cross) {
+  const size_t n = g.n(), p = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  const bool in = p < n;
+  bool any = false;
+  if (in) {
+    const uint32_t c = code[p];
+    const float wgt[4] = {0.0f, 0.25f, 0.5f, 0.5f};
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+      const double *x[3] = {M.m[d][0] + 3 * p, M.m[d][1] + 3 * p, M.m[d][2] + 3 * p};
+      double v[3];
+      gcoef_face(x, x[d], M.aj[d][p], v);
+#pragma unroll
+      for (int t = 0; t < 3; t++) {
+        const int q = 3 * d + t, other = d == 0 ? t - 1 : d == 1 ? (t == 2) : t;  // the cross direction's place
+        float f = int_narrow(v[t]);
+        if (t != d) {
+          f *= wgt[code_branch(c, d, other)];
+          any = any || f != 0.0f;
+        }
+        g9[(size_t)q * n + p] = v[t];
+        gf[(size_t)q * n + p] = f;
+      }
+    }
+  }
+  if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) *cross = 1;
 }
 
-void launch_gcoef(const Geom &g, const double *const *m, const double *iaj, const double *jaj,
-                  const double *kaj, double *g9, cudaStream_t s) {
-  k_gcoef<<<nblk(g.n(), 256), 256, 0, s>>>(g, m[0], m[1], m[2], m[3], m[4], m[5], m[6], m[7], m[8],
-                                           iaj, jaj, kaj, g9); count_launch();
+void launch_gcoef(const Geom &g, const double *const *m, const double *iaj, const double *jaj, const double *kaj,
+                  const uint32_t *code, double *g9, float *gf32, int *cross, cudaStream_t s) {
+  FaceMetrics M;
+  for (int q = 0; q < 9; q++) M.m[q / 3][q % 3] = m[q];
+  M.aj[0] = iaj; M.aj[1] = jaj; M.aj[2] = kaj;
+  k_gcoef<<<nblk(g.n(), 128), 128, 0, s>>>(g, M, code, g9, gf32, cross); count_launch();
 }
 
 // The cross-derivative form of poisson.c:793-1324 from the nvert sums of the two
@@ -121,45 +150,8 @@ void launch_weight32(const Geom &g, const double *nvert, float *wgt32, cudaStrea
   k_weight32<<<nblk(g.n(), 256) < 4096 ? nblk(g.n(), 256) : 4096, 256, 0, s>>>(g.n(), nvert, wgt32); count_launch();
 }
 
-// Any non-zero cross-derivative coefficient (FP32 flux form, after the form
-// scaling) or edge weight (FP64 rows) on the level.
-__global__ void k_cross_flags(size_t n, const float *__restrict__ gf, const double *__restrict__ w, int *flags) {
-  bool f32 = false, f64 = false;
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    f32 |= gf[1 * n + p] != 0.0f || gf[2 * n + p] != 0.0f || gf[3 * n + p] != 0.0f || gf[5 * n + p] != 0.0f ||
-           gf[6 * n + p] != 0.0f || gf[7 * n + p] != 0.0f;
-    for (int s = NE; s <= BW; s++) f64 |= w[(size_t)s * n + p] != 0.0;
-  }
-  if (__any_sync(0xffffffffu, f32) && (threadIdx.x & 31) == 0) flags[0] = 1;
-  if (__any_sync(0xffffffffu, f64) && (threadIdx.x & 31) == 0) flags[1] = 1;
-}
-void launch_cross_flags(const Geom &g, const float *gf32, const double *w64, int *flags, cudaStream_t s) {
-  k_cross_flags<<<nblk(g.n(), 256) < 4096 ? nblk(g.n(), 256) : 4096, 256, 0, s>>>(g.n(), gf32, w64, flags);
-  count_launch();
-}
-
 void launch_codes(const Geom &g, const double *nvert, uint32_t *code, cudaStream_t s) {
   k_codes<<<nblk(g.n(), 256), 256, 0, s>>>(g, nvert, code); count_launch();
-}
-
-// FP32 flux form: scale each cross-term coefficient by the weight of its form
-// (0 none, 1/4 central, 1/2 one-sided), so the apply needs no per-term
-// coefficient selection.  Powers of two: the scaling itself is exact.
-__global__ void k_scale_cross(Geom g, const uint32_t *__restrict__ code, float *__restrict__ gf) {
-  const size_t n = g.n();
-  const float wgt[4] = {0.0f, 0.25f, 0.5f, 0.5f};
-  for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
-    const uint32_t c = code[p];
-    gf[1 * n + p] *= wgt[code_branch(c, 0, 0)];  // g12 (face E, j-direction term)
-    gf[2 * n + p] *= wgt[code_branch(c, 0, 1)];  // g13 (face E, k)
-    gf[3 * n + p] *= wgt[code_branch(c, 1, 0)];  // g21 (face N, i)
-    gf[5 * n + p] *= wgt[code_branch(c, 1, 1)];  // g23 (face N, k)
-    gf[6 * n + p] *= wgt[code_branch(c, 2, 0)];  // g31 (face T, i)
-    gf[7 * n + p] *= wgt[code_branch(c, 2, 1)];  // g32 (face T, j)
-  }
-}
-void launch_scale_cross(const Geom &g, const uint32_t *code, float *gf32, cudaStream_t s) {
-  k_scale_cross<<<nblk(g.n(), 256) < 4096 ? nblk(g.n(), 256) : 4096, 256, 0, s>>>(g, code, gf32); count_launch();
 }
 
 // The colour-split copies of a level's 7-point coefficients (row32_split).
@@ -203,8 +195,9 @@ __device__ __forceinline__ void add_cross(double *vol, int br, double gg, bool u
 // matrix bit for bit.  Bound by the FP64 pipe, which keeps the sums; the products
 // are on the integer pipe (intmul.cuh).
 __global__ void k_weights(Geom g, const double *__restrict__ g9, const double *__restrict__ aj,
-                          const uint32_t *__restrict__ code, double *__restrict__ w) {
+                          const uint32_t *__restrict__ code, double *__restrict__ w, int *__restrict__ cross) {
   size_t n = g.n();
+  bool any = false;  // an edge weight that is not zero
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x) {
     uint32_t c = code[p];
     if (c & CODE_IDENTITY) {
@@ -260,14 +253,17 @@ __global__ void k_weights(Geom g, const double *__restrict__ g9, const double *_
       for (int m = 0; m < NSLOT; m++) r[m] = __dmul_rn(vol[m], a);
     }
 #pragma unroll
-    for (int m = 0; m < NSLOT; m++) w[(size_t)m * n + p] = r[m];
+    for (int m = 0; m < NSLOT; m++) {
+      w[(size_t)m * n + p] = r[m];
+      if (m >= NE) any = any || (__double_as_longlong(r[m]) << 1) != 0;
+    }
   }
+  if (any) *cross = 1;
 }
 
-void launch_weights(const Geom &g, const double *g9, const double *aj, const double *nvert,
-                    const uint32_t *code, double *w64, cudaStream_t s) {
-  (void)nvert;
-  k_weights<<<nblk(g.n(), 128), 128, 0, s>>>(g, g9, aj, code, w64); count_launch();
+void launch_weights(const Geom &g, const double *g9, const double *aj, const uint32_t *code, double *w64, int *cross,
+                    cudaStream_t s) {
+  k_weights<<<nblk(g.n(), 128), 128, 0, s>>>(g, g9, aj, code, w64, cross); count_launch();
 }
 
 // Thomas factors of the in-line (j) part of each row: a_j = w[SP], m_j, c'_j.
@@ -421,7 +417,7 @@ namespace cvb {
 // unknowns 0.9 ms (3.8 inverted on the host), 990 5.9 ms, 4,096 167 ms (23.2 and
 // 531 ms with one column a step: 2 n launches, n passes over the matrix, and
 // the matrix formed on the host).
-constexpr int kGjThreads = 1024, kGjW = 8, kGjTile = 64;
+constexpr int kGjThreads = 1024, kGjW = 8;
 // Panels of kGjW columns (64 bytes a row) of up to this many rows fit in shared
 // memory; beyond, w shrinks.
 constexpr int kGjSmemRows = 3200;
@@ -448,29 +444,30 @@ __global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A,
                                                          double *__restrict__ B, double *__restrict__ Dinv,
                                                          int *__restrict__ status) {
   extern __shared__ double S[];  // the panel's columns from row c0 down, [w][m | 1]
-  __shared__ unsigned long long sv[kGjThreads / 32];
-  __shared__ int si[kGjThreads / 32];
+  __shared__ unsigned long long sv[32];
+  __shared__ int si[32];
   __shared__ int piv[kGjW];
   __shared__ double rcp[kGjW];
   __shared__ double D[kGjW][2 * kGjW];
   dep_sync();
   if (*status) return;
-  const int t = threadIdx.x, lane = t & 31, wid = t >> 5, m = n - c0, mp = m | 1;
-  for (int e = t; e < m * kGjW; e += kGjThreads) {
+  const int nt = blockDim.x, t = threadIdx.x, lane = t & 31, wid = t >> 5, m = n - c0, mp = m | 1;
+#pragma unroll 4
+  for (int e = t; e < m * kGjW; e += nt) {
     const int r = e / kGjW, q = e % kGjW;
     if (q < w) S[q * mp + r] = A[(size_t)(c0 + r) * n + c0 + q];
   }
   __syncthreads();
   unsigned long long best = 0;
   int row = m;
-  for (int r = t; r < m; r += kGjThreads) gj_better(best, row, gj_magnitude(S[r]), r);
+  for (int r = t; r < m; r += nt) gj_better(best, row, gj_magnitude(S[r]), r);
   for (int s = 0; s < w; s++) {
     gj_warp_best(best, row);
     if (lane == 0) { sv[wid] = best; si[wid] = row; }
     __syncthreads();
     if (wid == 0) {
-      best = sv[lane];
-      row = si[lane];
+      best = lane < nt / 32 ? sv[lane] : 0;
+      row = lane < nt / 32 ? si[lane] : m;
       gj_warp_best(best, row);
       if (lane == 0) {
         piv[s] = best > 0 ? row : -1;
@@ -495,7 +492,7 @@ __global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A,
     best = 0;
     row = m;
     if (s + 1 < w)
-      for (int r = s + 1 + t; r < m; r += kGjThreads) {
+      for (int r = s + 1 + t; r < m; r += nt) {
         const double f = -S[s * mp + r] * rcp[s];
         for (int q = s + 1; q < w; q++) {
           const double v = fma(f, S[q * mp + s], S[q * mp + r]);
@@ -509,7 +506,7 @@ __global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A,
   bool moved = false;
   for (int s = 0; s < w; s++) moved = moved || piv[s] != s;
   if (moved) {
-    for (int q = t; q < n; q += kGjThreads)
+    for (int q = t; q < n; q += nt)
       for (int s = 0; s < w; s++) {
         const int p = piv[s];
         if (p == s) continue;
@@ -519,12 +516,13 @@ __global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A,
       }
     __syncthreads();
   }
-  for (int e = t; e < n * kGjW; e += kGjThreads) {
+#pragma unroll 4
+  for (int e = t; e < n * kGjW; e += nt) {
     const int r = e / kGjW, q = e % kGjW;
     F[e] = q < w ? A[(size_t)r * n + c0 + q] : 0.0;
   }
   for (int s = 0; s < kGjW; s++)
-    for (int q = t; q < n; q += kGjThreads)
+    for (int q = t; q < n; q += nt)
       B[(size_t)s * n + q] =
           q >= c0 && q < c0 + w ? (q - c0 == s ? 1.0 : 0.0) : s < w ? A[(size_t)(c0 + s) * n + q] : 0.0;
   // D and its inverse: Gauss-Jordan beside the unit matrix, in the order of the
@@ -550,22 +548,24 @@ __global__ void __launch_bounds__(kGjThreads) k_gj_panel(double *__restrict__ A,
   if (t < kGjW * kGjW) Dinv[t] = D[t / kGjW][kGjW + t % kGjW];
 }
 
-// A 64 x 64 tile per block, 4 x 4 entries a thread (columns 16 apart).
+// A T x T tile per block, (T / 16)^2 entries a thread (columns 16 apart).
+template <int T>
 __global__ void __launch_bounds__(256) k_gj_update(double *__restrict__ A, int n, int c0, int w,
                                                    const double *__restrict__ F, const double *__restrict__ B,
                                                    const double *__restrict__ Dinv, const int *__restrict__ status) {
-  __shared__ double sR[kGjW][kGjTile], sF[kGjTile][kGjW + 1], sD[kGjW * kGjW];
+  constexpr int E = T / 16;
+  __shared__ double sR[kGjW][T], sF[T][kGjW + 1], sD[kGjW * kGjW];
   dep_sync();
   if (*status) return;
-  const int t = threadIdx.x, q0 = blockIdx.x * kGjTile, r0 = blockIdx.y * kGjTile;
+  const int t = threadIdx.x, q0 = blockIdx.x * T, r0 = blockIdx.y * T;
   if (t < kGjW * kGjW) sD[t] = Dinv[t];
-  for (int e = t; e < kGjTile * kGjW; e += 256) {
+  for (int e = t; e < T * kGjW; e += 256) {
     const int r = e / kGjW;
     sF[r][e % kGjW] = r0 + r < n ? F[(size_t)r0 * kGjW + e] : 0.0;
   }
   __syncthreads();
-  for (int e = t; e < kGjW * kGjTile; e += 256) {
-    const int s = e / kGjTile, q = e % kGjTile;
+  for (int e = t; e < kGjW * T; e += 256) {
+    const int s = e / T, q = e % T;
     double v = 0.0;
     if (q0 + q < n)
       for (int u = 0; u < kGjW; u++) v = fma(sD[s * kGjW + u], B[(size_t)u * n + q0 + q], v);
@@ -573,31 +573,31 @@ __global__ void __launch_bounds__(256) k_gj_update(double *__restrict__ A, int n
   }
   __syncthreads();
   const int tx = t % 16, ty = t / 16;
-  double acc[4][4];
+  double acc[E][E];
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < E; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int r = r0 + ty * 4 + a, q = q0 + tx + 16 * b;
+    for (int b = 0; b < E; b++) {
+      const int r = r0 + ty * E + a, q = q0 + tx + 16 * b;
       acc[a][b] = r < n && q < n && !(q >= c0 && q < c0 + w) ? A[(size_t)r * n + q] : 0.0;
     }
 #pragma unroll
   for (int s = 0; s < kGjW; s++) {
-    double f[4], p[4];
+    double f[E], p[E];
 #pragma unroll
-    for (int a = 0; a < 4; a++) f[a] = sF[ty * 4 + a][s];
+    for (int a = 0; a < E; a++) f[a] = sF[ty * E + a][s];
 #pragma unroll
-    for (int b = 0; b < 4; b++) p[b] = sR[s][tx + 16 * b];
+    for (int b = 0; b < E; b++) p[b] = sR[s][tx + 16 * b];
 #pragma unroll
-    for (int a = 0; a < 4; a++)
+    for (int a = 0; a < E; a++)
 #pragma unroll
-      for (int b = 0; b < 4; b++) acc[a][b] = fma(-f[a], p[b], acc[a][b]);
+      for (int b = 0; b < E; b++) acc[a][b] = fma(-f[a], p[b], acc[a][b]);
   }
 #pragma unroll
-  for (int a = 0; a < 4; a++)
+  for (int a = 0; a < E; a++)
 #pragma unroll
-    for (int b = 0; b < 4; b++) {
-      const int r = r0 + ty * 4 + a, q = q0 + tx + 16 * b;
+    for (int b = 0; b < E; b++) {
+      const int r = r0 + ty * E + a, q = q0 + tx + 16 * b;
       if (r < n && q < n) A[(size_t)r * n + q] = r >= c0 && r < c0 + w ? sR[r - c0][tx + 16 * b] : acc[a][b];
     }
 }
@@ -626,15 +626,24 @@ bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap,
   }
   double *F = work, *B = F + (size_t)kGjW * n, *Dinv = B + (size_t)kGjW * n;
   cudaMemsetAsync(status, 0, sizeof(int), s);
-  const unsigned tiles = (n + kGjTile - 1) / kGjTile;
+  // the largest tile that still gives every SM a block (216 unknowns: 16 blocks of
+  // 64 x 64 12 us a step)
+  const unsigned tile = n >= 64 * 12 ? 64 : n >= 32 * 12 ? 32 : 16, tiles = (n + tile - 1) / tile;
   for (int c0 = 0; c0 < n;) {
     int w = kGjW;
     while (w > 1 && (long long)((n - c0) | 1) * w > (long long)kGjSmemRows * kGjW) w--;
     if (w > n - c0) w = n - c0;
-    launch_dep(k_gj_panel, 1, kGjThreads, sizeof(double) * (size_t)((n - c0) | 1) * w, s, A, n, c0, w, perm, F, B, Dinv,
+    // fewer warps meet at a step's barriers where a row a thread takes fewer
+    const int threads = std::min(kGjThreads, std::max(256, (n - c0 + 31) / 32 * 32));
+    launch_dep(k_gj_panel, 1, threads, sizeof(double) * (size_t)((n - c0) | 1) * w, s, A, n, c0, w, perm, F, B, Dinv,
                status);
-    launch_dep(k_gj_update, dim3(tiles, tiles), 256, 0, s, A, n, c0, w, (const double *)F, (const double *)B,
-               (const double *)Dinv, (const int *)status);
+    auto update = [&](auto k) {
+      launch_dep(k, dim3(tiles, tiles), 256, 0, s, A, n, c0, w, (const double *)F, (const double *)B,
+                 (const double *)Dinv, (const int *)status);
+    };
+    if (tile == 64) update(k_gj_update<64>);
+    else if (tile == 32) update(k_gj_update<32>);
+    else update(k_gj_update<16>);
     c0 += w;
   }
   int h_status = 0;
