@@ -939,6 +939,23 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
   double cs[kMaxRestart], sn[kMaxRestart], gv[kMaxRestart + 1], yv[kMaxRestart];
   int status = CVB_NOT_CONVERGED;
   const double target = std::max(o->rtol * bnorm, o->atol);
+  // z_j = M^-1 v_j and w = A z_j
+  auto direction = [&](int j) -> int {
+    if (mixed) {
+      // ctx->b32 holds V[j] in FP32 (written by the scaling that formed V[j])
+      // FP32 V-cycle; its result is widened once into the FP64 basis so the
+      // FP64 operator and the final update read it without per-use conversions
+      // (the operator on the FP32 vector, widening on the integer pipe and
+      // keeping an FP32 basis, took 73 us at 4.4 M cells against 62 + 9)
+      TRY(vcycle_graph<float>(ctx, o, 0, ctx->b32, ctx->Z32));
+      launch_f32_to_f64(ctx->Z32, ctx->Z64[j], n, s);
+    } else {
+      TRY(vcycle_graph<double>(ctx, o, j, ctx->V[j], ctx->Z64[j]));
+    }
+    launch_apply<double>(F, ctx->Z64[j], ctx->w, s);
+    CKL();
+    return CVB_OK;
+  };
   while (true) {
     if (!std::isfinite(beta)) return fail(ctx, CVB_NAN_DETECTED, "residual became %g", beta);
     if (beta <= target) { status = CVB_OK; break; }
@@ -951,23 +968,10 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
     for (int q = 0; q <= m; q++) gv[q] = 0.0;
     gv[0] = beta;
     int j = 0;
-    double est = beta;
+    double est = beta, rate = 0.01;
+    bool ahead = false;
     for (; j < m && total < o->max_it; j++) {
-      // z_j = M^-1 v_j
-      if (mixed) {
-        // ctx->b32 holds V[j] in FP32 (written by the scaling that formed V[j])
-        // FP32 V-cycle; its result is widened once into the FP64 basis so the
-        // FP64 operator and the final update read it without per-use conversions
-        // (the operator on the FP32 vector, widening on the integer pipe and
-        // keeping an FP32 basis, took 73 us at 4.4 M cells against 62 + 9)
-        TRY(vcycle_graph<float>(ctx, o, 0, ctx->b32, ctx->Z32));
-        launch_f32_to_f64(ctx->Z32, ctx->Z64[j], n, s);
-        launch_apply<double>(F, ctx->Z64[j], ctx->w, s);
-      } else {
-        TRY(vcycle_graph<double>(ctx, o, j, ctx->V[j], ctx->Z64[j]));
-        launch_apply<double>(F, ctx->Z64[j], ctx->w, s);
-      }
-      CKL();
+      if (!ahead) TRY(direction(j));
       // classical Gram-Schmidt (PETSc's default for GMRES/FGMRES), with a second
       // pass only when the first one cancelled most of w (||w|| dropped below
       // half of its length before orthogonalisation).  The projections and the
@@ -978,6 +982,9 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
       // has eroded it is off by far more than rounding, and FGMRES then needed
       // 32 iterations instead of 6 on the channel.
       // The event is recorded before the scaling, so the host works beside it.
+      // Where convergence in this iteration is out of reach (ten times the last
+      // contraction would not do), the next direction is queued before the host
+      // waits, so that the GPU does not; not with a second pass, which needs w.
       double h[kMaxRestart + 2], h2[kMaxRestart + 1], nw2;
       auto gram_schmidt = [&](double *hq) -> int {
         launch_dots(V, j + 1, ctx->w, n, ctx->partial, ctx->red_counter, dev_dots(ctx), s);
@@ -986,6 +993,8 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
         CK(cudaEventRecord(ctx->kry_ev, s));
         launch_scale(ctx->V[j + 1], ctx->w, dev_norm(ctx) + 1, n, in32, s);
         CKL();
+        ahead = !o->cgs_refine && j + 1 < m && total + 1 < o->max_it && 0.1 * std::min(rate, 1.0) * est > target;
+        if (ahead) TRY(direction(j + 1));
         CK(cudaEventSynchronize(ctx->kry_ev));
         std::copy(ctx->kry_host, ctx->kry_host + j + 1, hq);
         nw2 = ctx->kry_host[j + 1];
@@ -1014,6 +1023,7 @@ static int fgmres(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats *st) {
       H[j + 1][j] = 0.0;
       gv[j + 1] = -sn[j] * gv[j];
       gv[j] = cs[j] * gv[j];
+      rate = std::fabs(gv[j + 1]) / est;
       est = std::fabs(gv[j + 1]);
       if (est <= target || hn == 0.0) { j++; break; }
     }
