@@ -130,10 +130,13 @@ __global__ void __launch_bounds__(kSolveThreads, 4) kg_zebra_fused(const __grid_
 template <typename T>
 __global__ void __launch_bounds__(128) kg_resid_color(const __grid_constant__ TaskList tl) {
   dep_sync();
-  const GTask &K = tl.t[find_task(tl, blockIdx.x)];
+  // one colour a launch; the second from the last block to the first, so that it
+  // begins with the coefficients that the first left in the L2 cache
+  const int block = tl.t[0].p0 ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+  const GTask &K = tl.t[find_task(tl, block)];
   if (gated(K.gate)) return;
   const LevelDev L = *K.L;
-  Blk3 q = blk3(K, blockIdx.x);
+  Blk3 q = blk3(K, block);
   if (has_cross<T>(L)) resid_color_body<T, true>(L, (const T *)K.a, (const T *)K.b, (T *)K.c, K.p0, q.x, q.y, q.z);
   else resid_color_body<T, false>(L, (const T *)K.a, (const T *)K.b, (T *)K.c, K.p0, q.x, q.y, q.z);
 }
