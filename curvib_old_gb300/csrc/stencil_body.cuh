@@ -12,6 +12,8 @@
 //       the face is active from P's side.  Reads 9 face coefficients, aj and a
 //       code per cell: ~52 B/cell.
 #pragma once
+#include <type_traits>
+
 #include "cvb_internal.h"
 #include "intmul.cuh"
 #include "launch.cuh"
@@ -689,6 +691,12 @@ __device__ __forceinline__ int tile_line(int bx, int tx, int k, int TW, int colo
   return color < 0 ? bx * TW + tx : 2 * (bx * TW + tx) + ((color + k) & 1);
 }
 
+// Tiles of a line solve: all lines or one color's.
+template <int TW>
+__host__ __device__ inline int solve_tiles_x(const Geom &g, int color) {
+  return color < 0 ? (g.mx + TW - 1) / TW : ((g.mx + 1) / 2 + TW - 1) / TW;
+}
+
 template <typename T>
 struct Vec16;
 template <>
@@ -727,9 +735,11 @@ inline size_t line_solve_smem_rr(const Geom &g, int rr) {
   return sizeof(T) * (reg_factors(sizeof(T), TW, rr) ? 2 : 5) * (size_t)LineLayout::of(g.my).ls * TW;
 }
 // Resident blocks per SM the tile kernels are compiled for: with the factors in
-// registers they fit in 48 registers, ten blocks of 128 threads (R = 8: eight).
+// registers they fit in 48 registers, ten blocks of 128 threads (R = 8: eight;
+// FP64 with the factors of eight rows a lane: six).
 template <typename T, int TW, int RR>
-constexpr int kTileMinBlocks = kRegFactors<T, TW, RR> ? (RR == 8 ? 8 : 10) : 4;
+constexpr int kTileMinBlocks = sizeof(T) == 8 && TW == 4 && RR == 2 ? 6
+                                                                    : kRegFactors<T, TW, RR> ? (RR == 8 ? 8 : 10) : 4;
 
 template <int N>
 __device__ __forceinline__ void ld_run(const float *p, float (&o)[N]) {
@@ -762,13 +772,49 @@ __device__ __forceinline__ void ld_run(const double *p, double (&o)[N]) {
   }
 }
 
+// FP64 tiles of four lines with 33 to 64 rows: one warp solves all four, eight lanes
+// a line and eight rows a lane.  The FP64 pipe bounds these kernels, and a scan over
+// 32 lanes of two rows costs it 40 operations a warp and line where eight lanes of
+// eight rows cost 23.  The line solves of a colour at 66^3 8.1 -> 6.5 us, the 7-point
+// half-sweep at 130 x 66 x 66 18.9 -> 17.6.  Up to 32 rows the same (eight lanes of four)
+// took as long as before: 6.9 us at 34^3.
+template <typename T, int TW, int RR>
+constexpr bool kSegments = sizeof(T) == 8 && TW == 4 && RR == 2;
+template <int RS>
+struct SegFactors {
+  double a[RS], m[RS], c[RS];
+};
 // The factors of the lines one warp solves in a tile: lines warp, warp + NW, ...
 template <typename T, int TW, int RR>
-using TileLaneFactors = LaneFactors<T, TW / (kSolveThreads / 32), (RR > 0 ? RR : 1)>;
+using TileLaneFactors = std::conditional_t<kSegments<T, TW, RR>, SegFactors<4 * (RR > 0 ? RR : 1)>,
+                                           LaneFactors<T, TW / (kSolveThreads / 32), (RR > 0 ? RR : 1)>>;
+// The warp of a block that solves its tile: another one in the blocks that come to
+// the same SM next, since each quarter of an SM has its own FP64 unit.
+__device__ __forceinline__ int segment_warp(int bx, int k, int tiles) { return ((k * tiles + bx) / 152) & 3; }
 
 template <typename T, int TW, int RR>
 __device__ __forceinline__ void lane_factors_load(const LevelDev &L, int bx, int k, int color,
                                                   TileLaneFactors<T, TW, RR> &f) {
+  if constexpr (kSegments<T, TW, RR>) {
+    constexpr int RS = 4 * RR;
+    const Geom &g = L.g;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q0 = (lane & 7) * RS;
+    if (warp != segment_warp(bx, k, solve_tiles_x<TW>(g, color))) return;
+    const int il = tile_line(bx, lane >> 3, k, TW, color);
+    const bool in = k >= 1 && k <= g.mz - 2 && il >= 1 && il <= g.mx - 2;
+    const LineFac F = LineFac::of(g);
+    const T *p = RowOf<T>::fac(L) + (in ? F.line(il, k) : 0) + q0;
+#pragma unroll
+    for (int u = 0; u < RS; u += 4) {
+      double v[3][4] = {};
+      if (in && q0 + u < g.my - 2) {
+#pragma unroll
+        for (int r = 0; r < 3; r++) ld_run<4>(p + (size_t)r * F.Q + u, v[r]);
+      }
+#pragma unroll
+      for (int t = 0; t < 4; t++) f.a[u + t] = v[0][t], f.m[u + t] = v[1][t], f.c[u + t] = v[2][t];
+    }
+  } else {
   constexpr int NW = kSolveThreads / 32, NL = TW / NW, R = RR > 0 ? RR : 1;
   const Geom &g = L.g;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q0 = lane * R;
@@ -787,6 +833,54 @@ __device__ __forceinline__ void lane_factors_load(const LevelDev &L, int bx, int
 #pragma unroll
       for (int t = 0; t < R; t++) f.a_[l][t] = f.m_[l][t] = f.c_[l][t] = T(0);
     }
+  }
+  }
+}
+
+// The four lines of a tile (line l at sr + l ls, laid out as LineLayout) by one warp:
+// the affine recurrences of warp_lines_solve, a lane composing the maps of its RS
+// rows, scans over the eight lanes of a line.
+template <int RR>
+__device__ __forceinline__ void segment_lines_solve(double *sr, const SegFactors<4 * RR> &f, int ls, int nr, int lane) {
+  constexpr int RS = 4 * RR;
+  const int s = lane & 7, q0 = s * RS;
+  double *line = sr + (lane >> 3) * ls;
+  auto at = [&](int t) { return (t % RR) * 33 + (q0 + t) / RR; };
+  double d[RS], B = 1.0, G = 0.0;
+#pragma unroll
+  for (int t = 0; t < RS; t++) {
+    const double beta = -f.m[t] * f.a[t];
+    d[t] = q0 + t < nr ? f.m[t] * line[at(t)] : 0.0;
+    B = beta * B;
+    G = beta * G + d[t];
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const double Bp = __shfl_up_sync(0xffffffffu, B, o, 8), Gp = __shfl_up_sync(0xffffffffu, G, o, 8);
+    if (s >= o) { G = B * Gp + G; B = B * Bp; }
+  }
+  double prev = __shfl_up_sync(0xffffffffu, G, 1, 8);
+  if (s == 0) prev = 0.0;
+#pragma unroll
+  for (int t = 0; t < RS; t++) prev = d[t] = d[t] - f.m[t] * f.a[t] * prev;
+  B = 1.0;
+  G = 0.0;
+#pragma unroll
+  for (int t = RS - 1; t >= 0; t--) {
+    B = -f.c[t] * B;
+    G = d[t] - f.c[t] * G;
+  }
+#pragma unroll
+  for (int o = 1; o < 8; o <<= 1) {
+    const double Bn = __shfl_down_sync(0xffffffffu, B, o, 8), Gn = __shfl_down_sync(0xffffffffu, G, o, 8);
+    if (s + o < 8) { G = B * Gn + G; B = B * Bn; }
+  }
+  prev = __shfl_down_sync(0xffffffffu, G, 1, 8);
+  if (s == 7) prev = 0.0;
+#pragma unroll
+  for (int t = RS - 1; t >= 0; t--) {
+    prev = d[t] - f.c[t] * prev;
+    if (q0 + t < nr) line[at(t)] = prev;
   }
 }
 
@@ -868,7 +962,10 @@ __device__ __forceinline__ void solve_tile_finish(const LevelDev &L, const T *__
   // the interior hold stale shared memory whose results are never read
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = kSolveThreads / 32, NL = TW / NW;
-  if (kin) {
+  if constexpr (kSegments<T, TW, RR>) {
+    if (kin && warp == segment_warp(bx, k, solve_tiles_x<TW>(g, color)))
+      segment_lines_solve<RR>(sr, lf, Lo.ls, Lo.nr, lane);
+  } else if (kin) {
     const int o = warp * Lo.ls;
     if constexpr (kRegFactors<T, TW, RR>) {
       warp_lines_solve<T, NL, RR>(sr + o, lf, NW * Lo.ls, Lo, lane);
@@ -920,12 +1017,6 @@ __device__ __forceinline__ void line_solve_body(const LevelDev &L, const T *__re
   cp_async_wait_all();
   __syncthreads();
   solve_tile_finish<T, TW, RR>(L, x, xnew, omega, bx, k, st, color, lf);
-}
-
-// Tiles of a line solve: all lines or one color's.
-template <int TW>
-__host__ __device__ inline int solve_tiles_x(const Geom &g, int color) {
-  return color < 0 ? (g.mx + TW - 1) / TW : ((g.mx + 1) / 2 + TW - 1) / TW;
 }
 
 // Residual b - A x on the interior cells of one zebra color ((i + k) % 2 ==
