@@ -4,7 +4,7 @@ A hierarchy of one level is solved by the inverse alone, so FGMRES needs one
 iteration, or a few where rounding leaves more than the tolerance: the inverse
 is off by the unit roundoff times the matrix's condition number (below 1e5
 here), so three iterations reach 1e-10.  Sizes at the edges of its panels of 8
-columns and tiles of 64, with a body that leaves rows out, and with face
+columns and tiles of 16, 32 and 64, with a body that leaves rows out, and with face
 Jacobians of random sign and size, whose rows are not diagonally dominant, so
 that pivot rows move."""
 import types
@@ -15,7 +15,8 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("cells", [(2, 2, 2), (3, 3, 3), (4, 4, 4), (5, 13, 2), (3, 8, 8), (6, 6, 6), (9, 10, 11)])
+@pytest.mark.parametrize("cells", [(2, 2, 2), (3, 3, 3), (4, 4, 4), (5, 13, 2), (3, 8, 8), (6, 6, 6), (6, 8, 8), (7, 9, 12),
+                                   (8, 8, 12), (9, 10, 11)])
 @pytest.mark.parametrize("rows", ["dominant", "pivoting", "body"])
 def test_one_level_solve(cells, rows):
     from curvib_old_gb300 import _lib
