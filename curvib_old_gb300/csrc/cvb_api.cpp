@@ -1954,7 +1954,7 @@ static void momentum_rhs(cvb_ctx *ctx, const MomentumTime *calc) {
 // their way in: p, the incoming rhs and calc's fluxes (uo, urm on the host) come
 // in while Contra2Cart, Convection and Viscous run, and ucat goes out beside the
 // last kernels.  CalcRHS at 192^3 from pinned arrays: 11.5 ms with the copies
-// before and after the kernels, 8.2 so (5.3 ms of kernels).
+// before and after the kernels, 7.9 so (5.1 ms of kernels).
 static int momentum_call(cvb_ctx *ctx, double ren, int central, const MomentumTime *calc, const double *uo,
                          const double *urm, const double *p, double *ucat, double *rhs) {
   const size_t n = ctx->L[ctx->nlevels - 1].g.n();

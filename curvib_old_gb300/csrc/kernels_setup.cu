@@ -414,7 +414,7 @@ namespace cvb {
 //
 // The update is bound by the FP64 pipe (n^3 multiply-adds in all), the panel by
 // its n dependent steps on one SM.  Set-up of the coarsest solver, all in: 216
-// unknowns 0.9 ms (3.8 inverted on the host), 990 5.9 ms, 4,096 167 ms (23.2 and
+// unknowns 0.63 ms (3.8 inverted on the host), 1,024 6.6 ms, 4,096 170 ms (24 and
 // 531 ms with one column a step: 2 n launches, n passes over the matrix, and
 // the matrix formed on the host).
 constexpr int kGjThreads = 1024, kGjW = 8;
