@@ -124,32 +124,44 @@ __device__ __noinline__ void c2c_fp64(double q0, double q1, double q2, const dou
 // factors are in intmul.cuh's range) puts the nine products on the integer
 // pipe and divides by the determinant through its reciprocal: 24 FP64
 // operations a cell, where the products and three divisions made about 45
-// (192^3: 0.31 ms, 0.56 ms with them).
+// (192^3: 0.31 ms, 0.56 ms with them).  What a cell needs is loaded at once, before
+// the first test: on small grids one latency is most of the kernel.
+struct C2cCell {
+  double nv, w[3], c[3], f[kC2cFactors];  // nvert; the lower and upper face's flux; the factors
+  __device__ __forceinline__ C2cCell(const Geom &g, const double *__restrict__ fac, const double *__restrict__ nvert,
+                                     const double *uc, size_t p) {
+    const size_t n = g.n();
+    nv = nvert[p];
+    w[0] = uc[3 * (p - 1)];
+    w[1] = uc[3 * (p - g.mx) + 1];
+    w[2] = uc[3 * (p - (size_t)g.mx * g.my) + 2];
+#pragma unroll
+    for (int d = 0; d < 3; d++) c[d] = uc[3 * p + d];
+#pragma unroll
+    for (int q = 0; q < kC2cFactors; q++) f[q] = fac[q * n + p];
+  }
+};
+// the velocity into u, unchanged where the cell is not fluid
 template <bool INT>
-__device__ __forceinline__ void c2c_cell(const Geom &g, const double *__restrict__ fac,
-                                         const double *__restrict__ nvert, const double *uc, double *ucat, size_t p) {
-  const size_t n = g.n();
-  if (!conv_fluid(nvert[p])) return;
-  const size_t pw = p - 1, ps = p - g.mx, pb = p - (size_t)g.mx * g.my;
-  const double q0 = mean2(uc[3 * pw + 0], uc[3 * p + 0]);
-  const double q1 = mean2(uc[3 * ps + 1], uc[3 * p + 1]);
-  const double q2 = mean2(uc[3 * pb + 2], uc[3 * p + 2]);
+__device__ __forceinline__ void c2c_cell(const Geom &g, const C2cCell &in, const double *__restrict__ fac, size_t p,
+                                         double (&u)[3]) {
+  if (!conv_fluid(in.nv)) return;
+  const double q0 = mean2(in.w[0], in.c[0]), q1 = mean2(in.w[1], in.c[1]), q2 = mean2(in.w[2], in.c[2]);
   bool fp64 = !INT;
   if constexpr (INT) {
     const IntMulA a0 = int_split_a(q0, fp64), a1 = int_split_a(q1, fp64), a2 = int_split_a(q2, fp64);
     if (!fp64) {
-      auto f = [&](int q) { return int_split_b(fac[q * n + p]); };
+      auto f = [&](int q) { return int_split_b(in.f[q]); };
       // -q0 f = -(q0 f): the subtraction below adds it
       const double d0 = da(ds(int_mul(a0, f(0)), int_mul(a1, f(3))), int_mul(a2, f(4)));
       const double d1 = ds(ds(int_mul(a1, f(5)), int_mul(a0, f(1))), int_mul(a2, f(6)));
       const double d2 = da(ds(int_mul(a0, f(2)), int_mul(a1, f(7))), int_mul(a2, f(8)));
-      const double det = fac[9 * n + p], rcp = fac[10 * n + p];
-      ucat[3 * p + 0] = quot_known(d0, det, rcp);
-      ucat[3 * p + 1] = quot_known(d1, det, rcp);
-      ucat[3 * p + 2] = quot_known(d2, det, rcp);
+      u[0] = quot_known(d0, in.f[9], in.f[10]);
+      u[1] = quot_known(d1, in.f[9], in.f[10]);
+      u[2] = quot_known(d2, in.f[9], in.f[10]);
     }
   }
-  if (fp64) c2c_fp64(q0, q1, q2, fac + p, n, ucat + 3 * p);
+  if (fp64) c2c_fp64(q0, q1, q2, fac + p, g.n(), u);
 }
 
 template <bool INT>
@@ -161,8 +173,14 @@ __global__ void __launch_bounds__(128) k_contra2cart(Geom g, const double *__res
   const size_t cells = (size_t)ni * nj * nk;
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= cells) return;
-  const int i = 1 + (int)(t % ni), j = 1 + (int)((t / ni) % nj), k = k0 + (int)(t / ((size_t)ni * nj));
-  c2c_cell<INT>(g, fac, nvert, uc, ucat, ((size_t)k * g.my + j) * g.mx + i);
+  const int k = (int)t / (ni * nj), j = ((int)t - k * ni * nj) / ni, i = (int)t - (k * nj + j) * ni;
+  const size_t p = ((size_t)(k0 + k) * g.my + 1 + j) * g.mx + 1 + i;
+  const C2cCell in(g, fac, nvert, uc, p);
+  if (!conv_fluid(in.nv)) return;
+  double u[3];
+  c2c_cell<INT>(g, in, fac, p, u);
+#pragma unroll
+  for (int c = 0; c < 3; c++) ucat[3 * p + c] = u[c];
 }
 
 // Interior cells of the planes k0 .. k0 + nk - 1 (nk < 0: all from k0 on).
@@ -572,23 +590,29 @@ __global__ void __launch_bounds__(128) k_outlet_plane(Geom g, const double *__re
   if (t >= n) return;
   const int i = 1 + t % ni, j = 1 + t / ni;
   const size_t q = ((size_t)(g.mz - 2) * g.my + j) * g.mx + i, qb = q + (size_t)g.mx * g.my;
-  const bool fluid = nv[q] < 0.1;
-  const double *z = zet + 3 * q;
-  double *c = ucat + 3 * q;
+  // every load first: the kernel is one latency after another otherwise (a plane of
+  // 30 x 30 cells with the next terms 6.1 us, 4.2 so)
+  const double z[3] = {zet[3 * q], zet[3 * q + 1], zet[3 * q + 2]};
+  double c[3] = {ucat[3 * q], ucat[3 * q + 1], ucat[3 * q + 2]};
   double a = 0., f = 0.;
-  if (fluid && (APPLY || AREA)) a = __dsqrt_rn(da(da(dm(z[0], z[0]), dm(z[1], z[1])), dm(z[2], z[2])));
-  if (APPLY) {
-    if (fluid) {
-      ub[3 * qb] = c[0];
-      ub[3 * qb + 1] = c[1];
-      ub[3 * qb + 2] = c[2];
-      uc[3 * q + 2] = da(da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2])), dm(ratio, a));
+  if constexpr (APPLY) {
+    C2cCell in(g, F.fac, nv, uc, q);
+    if (in.nv < 0.1) {
+      a = __dsqrt_rn(da(da(dm(z[0], z[0]), dm(z[1], z[1])), dm(z[2], z[2])));
+#pragma unroll
+      for (int d = 0; d < 3; d++) ub[3 * qb + d] = c[d];
+      uc[3 * q + 2] = in.c[2] = da(da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2])), dm(ratio, a));
     }
-    if (F.tame) c2c_cell<true>(g, F.fac, nv, uc, ucat, q);
-    else c2c_cell<false>(g, F.fac, nv, uc, ucat, q);
+    if (F.tame) c2c_cell<true>(g, in, F.fac, q, c);
+    else c2c_cell<false>(g, in, F.fac, q, c);
+#pragma unroll
+    for (int d = 0; d < 3; d++) ucat[3 * q + d] = c[d];
+    if (TERMS && in.nv < 0.1) f = da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2]));
+  } else if (nv[q] < 0.1) {
+    if (AREA) a = __dsqrt_rn(da(da(dm(z[0], z[0]), dm(z[1], z[1])), dm(z[2], z[2])));
+    if (TERMS) f = da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2]));
   }
   if (TERMS) {
-    if (fluid) f = da(da(dm(c[0], z[0]), dm(c[1], z[1])), dm(c[2], z[2]));
     terms[t] = f;
     if (AREA) terms[n + t] = a;
   }
