@@ -94,6 +94,7 @@ inline int batch_reduce_blocks(size_t n) {
 // --- grouped launchers (kernels_batch.cu) ---------------------------------
 // Stencil / V-cycle phases: L = device LevelDev, a/b/c per kernel.
 void glaunch_residual32(const TaskList &tl, cudaStream_t s);   // a = x, b = rhs, c = r
+void glaunch_residual32_flat(const TaskList &tl, cudaStream_t s);  // the same, levels of apply32_flat
 void glaunch_residual64(const TaskList &tl, cudaStream_t s);   // a = x, b = rhs or null (apply), c = y
 void glaunch_restrict(const TaskList &tl, bool f32, cudaStream_t s);     // a = fine, c = coarse
 void glaunch_prolong(const TaskList &tl, bool f32, cudaStream_t s);      // a = coarse, c = fine (added)

@@ -58,7 +58,7 @@ struct Done {
 
 // Sink of the ops of one round, grouped by schedule key and kernel kind.
 enum OpKind {
-  OK_RES32, OK_RES64, OK_RESTRICT, OK_PROLONG, OK_SWEEP, OK_SOLVE, OK_DENSE, OK_COPY,
+  OK_RES32, OK_RES32F, OK_RES64, OK_RESTRICT, OK_PROLONG, OK_SWEEP, OK_SOLVE, OK_DENSE, OK_COPY,
   OK_ZERO, OK_RESC, OK_ZFUSED,
   // line solves of levels whose lines have 1, 2, 4 or 8 rows per lane: one
   // launch each, so each runs the kernel specialised for its layout
@@ -206,7 +206,10 @@ double *lvec<double>(LevelDev &L, int which) {
 template <typename T>
 static void add_residual(VSink &vs, long long key, LevelDev &L, const LevelDev *dLv, const T *x, const T *b, T *r,
                          const int *gate) {
-  if (sizeof(T) == 4) {
+  if (sizeof(T) == 4 && apply32_flat(L.g, L.cross32)) {
+    const int gx = plane_blocks(L.g);
+    vs.add(key, OK_RES32F, task(dLv, x, b, r, gate, gx, 1), gx * L.g.mz);
+  } else if (sizeof(T) == 4) {
     const MarchGrid m = MarchGrid::of(L.g);
     vs.add(key, OK_RES32, task(dLv, x, b, r, gate, m.gx, m.gy), m.blocks());
   } else {
@@ -365,6 +368,7 @@ static void run_program(cvb_batch *bt, std::map<long long, std::array<Lists, OK_
       for (OpBatch &ob : kv.second[k].v) {
         switch (k) {
           case OK_RES32: glaunch_residual32(ob.tl, s); break;
+          case OK_RES32F: glaunch_residual32_flat(ob.tl, s); break;
           case OK_RES64: glaunch_residual64(ob.tl, s); break;
           case OK_RESTRICT: glaunch_restrict(ob.tl, f32, s); break;
           case OK_PROLONG: glaunch_prolong(ob.tl, f32, s); break;

@@ -43,12 +43,22 @@ __global__ void __launch_bounds__(256) kg_apply32(const __grid_constant__ TaskLi
   if (gated(T.gate)) return;
   const LevelDev L = *T.L;
   Blk3 q = blk3(T, blockIdx.x);
+  apply32_march_body(L.g, L.gf32, L.ajf32, L.code, (const float *)T.a, (const float *)T.b, (float *)T.c, q.x, q.y,
+                     q.z);
+}
+__global__ void __launch_bounds__(kFlat) kg_apply32_flat(const __grid_constant__ TaskList tl) {
+  dep_sync();
+  const GTask &T = tl.t[find_task(tl, blockIdx.x)];
+  if (gated(T.gate)) return;
+  const LevelDev L = *T.L;
+  Blk3 q = blk3(T, blockIdx.x);
+  const int idx = q.x * kFlat + threadIdx.x;
   if (L.cross32)
-    apply32_march_body<true>(L.g, L.gf32, L.ajf32, L.code, (const float *)T.a, (const float *)T.b, (float *)T.c, q.x,
-                             q.y, q.z);
+    apply32_flat_body<true>(L.g, L.gf32, L.ajf32, L.code, (const float *)T.a, (const float *)T.b, (float *)T.c, idx,
+                            q.z);
   else
-    apply32_march_body<false>(L.g, L.gf32, L.ajf32, L.code, (const float *)T.a, (const float *)T.b, (float *)T.c,
-                              q.x, q.y, q.z);
+    apply32_flat_body<false>(L.g, L.gf32, L.ajf32, L.code, (const float *)T.a, (const float *)T.b, (float *)T.c, idx,
+                             q.z);
 }
 __global__ void __launch_bounds__(128) kg_apply64(const __grid_constant__ TaskList tl) {
   dep_sync();
@@ -199,6 +209,10 @@ __global__ void kg_elem(const __grid_constant__ TaskList tl) {
     else c[p] = (TD)a[p];
 }
 
+void glaunch_residual32_flat(const TaskList &tl, cudaStream_t s) {
+  if (!tl.n) return;
+  launch_dep(kg_apply32_flat, tl.nblocks, kFlat, 0, s, tl);
+}
 void glaunch_residual32(const TaskList &tl, cudaStream_t s) {
   if (!tl.n) return;
   launch_dep(kg_apply32, tl.nblocks, dim3(32, 8), 0, s, tl);

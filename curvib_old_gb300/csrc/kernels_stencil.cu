@@ -17,13 +17,22 @@ __global__ void __launch_bounds__(128) k_apply64(Geom g, const double *__restric
   apply64_body<TX, X>(g, w, code, x, b, y, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
-template <bool X>
 __global__ void __launch_bounds__(256) k_apply32(Geom g, const float *__restrict__ gf, const float *__restrict__ aj,
                                                  const uint32_t *__restrict__ code, const float *__restrict__ x,
                                                  const float *__restrict__ b, float *__restrict__ y, const int *gate) {
   dep_sync();
   if (gated(gate)) return;
-  apply32_march_body<X>(g, gf, aj, code, x, b, y, blockIdx.x, blockIdx.y, blockIdx.z);
+  apply32_march_body(g, gf, aj, code, x, b, y, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+template <bool X>
+__global__ void __launch_bounds__(kFlat) k_apply32_flat(Geom g, const float *__restrict__ gf,
+                                                        const float *__restrict__ aj,
+                                                        const uint32_t *__restrict__ code,
+                                                        const float *__restrict__ x, const float *__restrict__ b,
+                                                        float *__restrict__ y, const int *gate) {
+  dep_sync();
+  if (gated(gate)) return;
+  apply32_flat_body<X>(g, gf, aj, code, x, b, y, blockIdx.x * kFlat + threadIdx.x, blockIdx.z);
 }
 static dim3 march_grid(const Geom &g) {
   MarchGrid m = MarchGrid::of(g);
@@ -41,10 +50,13 @@ static void apply64(const LevelDev &L, const TX *x, const double *b, double *y, 
   else launch_dep(k_apply64<TX, false>, grd, kFlat, 0, s, L.g, L.w64, L.code, x, b, y, L.gate);
 }
 static void apply32(const LevelDev &L, const float *x, const float *b, float *y, cudaStream_t s) {
-  if (L.cross32)
-    launch_dep(k_apply32<true>, march_grid(L.g), kMarchBlk, 0, s, L.g, L.gf32, L.ajf32, L.code, x, b, y, L.gate);
-  else
-    launch_dep(k_apply32<false>, march_grid(L.g), kMarchBlk, 0, s, L.g, L.gf32, L.ajf32, L.code, x, b, y, L.gate);
+  if (!apply32_flat(L.g, L.cross32)) {
+    launch_dep(k_apply32, march_grid(L.g), kMarchBlk, 0, s, L.g, L.gf32, L.ajf32, L.code, x, b, y, L.gate);
+    return;
+  }
+  const dim3 grd(plane_blocks(L.g), 1, L.g.mz);
+  if (L.cross32) launch_dep(k_apply32_flat<true>, grd, kFlat, 0, s, L.g, L.gf32, L.ajf32, L.code, x, b, y, L.gate);
+  else launch_dep(k_apply32_flat<false>, grd, kFlat, 0, s, L.g, L.gf32, L.ajf32, L.code, x, b, y, L.gate);
 }
 template <>
 void launch_apply<double>(const LevelDev &L, const double *x, double *y, cudaStream_t s) {

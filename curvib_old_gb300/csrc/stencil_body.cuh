@@ -241,6 +241,26 @@ struct MarchGrid {
   __host__ __device__ int blocks() const { return gx * gy * gz; }
 };
 
+// The residual in one thread per cell (row32): all of its loads are in flight at
+// once, against a plane's after another's in the march.  Measured with / without
+// cross terms, us, march then this: 34^3 3.4 2.3 / 2.5 1.8, 66^3 8.6 5.3 / 5.4 3.3,
+// 130^3 41.7 36.9 / 20.9 14.9, 162^3 68.0 67.5 / 36.5 30.3, 194^3 106 114 / 60.8
+// 50.3: the march, which forms a face's flux once, is ahead on large levels with
+// cross terms.
+constexpr size_t kFlatResidualCells = 4200000;
+__host__ __device__ inline bool apply32_flat(const Geom &g, bool cross) { return !cross || g.n() < kFlatResidualCells; }
+template <bool X>
+__device__ __forceinline__ void apply32_flat_body(const Geom &g, const float *__restrict__ gf,
+                                                  const float *__restrict__ aj, const uint32_t *__restrict__ code,
+                                                  const float *__restrict__ x, const float *__restrict__ b,
+                                                  float *__restrict__ y, int idx, int k) {
+  const int pl = g.mx * g.my;
+  if (idx >= pl) return;
+  const int j = idx / g.mx, i = idx - j * g.mx, p = k * pl + idx;
+  const float ax = row32<float, X>(g, gf, aj, code, x, i, j, k, p, (int)g.n());
+  y[p] = b ? b[p] - ax : ax;
+}
+
 // coordinate of x read for column i of a box of m cells (periodic: the ring
 // and beyond fold onto the image; otherwise clamped -- such values are unused)
 __device__ __forceinline__ int wrap_read(int i, int m, int per) {
@@ -252,8 +272,7 @@ __device__ __forceinline__ int wrap_read(int i, int m, int per) {
 }
 
 // y = A x (b == nullptr) or y = b - A x on the tile (bx, by, bz); 32 x 8 threads.
-// X: the level has cross-derivative coefficients (see row32).
-template <bool X = true>
+// Levels with cross-derivative coefficients.
 __device__ __forceinline__ void apply32_march_body(const Geom &g, const float *__restrict__ gf,
                                                    const float *__restrict__ aj, const uint32_t *__restrict__ code,
                                                    const float *__restrict__ x, const float *__restrict__ b,
@@ -278,20 +297,18 @@ __device__ __forceinline__ void apply32_march_body(const Geom &g, const float *_
     const int kb = k0 - 1;
     const int ob = wrap_read(kb, mz, g.pz) * pl, ot = wrap_read(k0, mz, g.pz) * pl;
     P = x[ob + cP]; E = x[ob + cE]; N = x[ob + cN];
-    W = X ? x[ob + cW] : 0.f;
-    S = X ? x[ob + cS] : 0.f;
+    W = x[ob + cW];
+    S = x[ob + cS];
     const float T = x[ot + cP], TE = x[ot + cE], TN = x[ot + cN];
-    const float TW = X ? x[ot + cW] : 0.f, TS = X ? x[ot + cS] : 0.f;
+    const float TW = x[ot + cW], TS = x[ot + cS];
     if (kb >= 0 && col) {
       const int q = kb * pl + cown;
       const float g33 = __ldg(gf + 8 * n + q);
       ftp = g33 * (T - P);
-      if constexpr (X) {
-        const uint32_t c = __ldg(code + q);
-        const float g31 = __ldg(gf + 6 * n + q), g32 = __ldg(gf + 7 * n + q);
-        ftp = ftp + cross32(code_branch(c, 2, 0), g31, E + TE, P + T, W + TW) +
-              cross32(code_branch(c, 2, 1), g32, N + TN, P + T, S + TS);
-      }
+      const uint32_t c = __ldg(code + q);
+      const float g31 = __ldg(gf + 6 * n + q), g32 = __ldg(gf + 7 * n + q);
+      ftp = ftp + cross32(code_branch(c, 2, 0), g31, E + TE, P + T, W + TW) +
+            cross32(code_branch(c, 2, 1), g32, N + TN, P + T, S + TS);
     }
     B = P; BE = E; BN = N;
     P = T; E = TE; N = TN; W = TW; S = TS;
@@ -305,11 +322,8 @@ __device__ __forceinline__ void apply32_march_body(const Geom &g, const float *_
   auto load = [&](int k, Plane &v) {
     const int op = wrap_read(k, mz, g.pz) * pl, ot = wrap_read(k + 1, mz, g.pz) * pl;
     v.T = x[ot + cP]; v.TE = x[ot + cE]; v.TN = x[ot + cN];
-    v.TW = v.TS = v.NE = v.SE = v.NW = 0.f;
-    if constexpr (X) {
-      v.TW = x[ot + cW]; v.TS = x[ot + cS];
-      v.NE = x[op + cNE]; v.SE = x[op + cSE]; v.NW = x[op + cNW];
-    }
+    v.TW = x[ot + cW]; v.TS = x[ot + cS];
+    v.NE = x[op + cNE]; v.SE = x[op + cSE]; v.NW = x[op + cNW];
     v.c = CODE_IDENTITY;
     v.g11 = v.g12 = v.g13 = v.g21 = v.g22 = v.g23 = v.g31 = v.g32 = v.g33 = 0.f;
     v.ajp = v.bp = v.xo = 0.f;
@@ -317,11 +331,9 @@ __device__ __forceinline__ void apply32_march_body(const Geom &g, const float *_
       const int q = k * pl + cown;
       v.c = __ldg(code + q);
       v.g11 = __ldg(gf + q); v.g22 = __ldg(gf + 4 * n + q); v.g33 = __ldg(gf + 8 * n + q);
-      if constexpr (X) {
-        v.g12 = __ldg(gf + n + q); v.g13 = __ldg(gf + 2 * n + q);
-        v.g21 = __ldg(gf + 3 * n + q); v.g23 = __ldg(gf + 5 * n + q);
-        v.g31 = __ldg(gf + 6 * n + q); v.g32 = __ldg(gf + 7 * n + q);
-      }
+      v.g12 = __ldg(gf + n + q); v.g13 = __ldg(gf + 2 * n + q);
+      v.g21 = __ldg(gf + 3 * n + q); v.g23 = __ldg(gf + 5 * n + q);
+      v.g31 = __ldg(gf + 6 * n + q); v.g32 = __ldg(gf + 7 * n + q);
       v.ajp = __ldg(aj + q);
       if (b && out) v.bp = b[q];
       if (out && (i == 0 || i == mx - 1 || j == 0 || j == my - 1 || k == 0 || k == mz - 1)) v.xo = x[q];
@@ -338,14 +350,12 @@ __device__ __forceinline__ void apply32_march_body(const Geom &g, const float *_
     const bool ring = i == 0 || i == mx - 1 || j == 0 || j == my - 1 || k == 0 || k == mz - 1;
     const float xo = ring ? v.xo : P;
     float fe = v.g11 * (E - P), fn = v.g22 * (N - P), ft = v.g33 * (T - P);
-    if constexpr (X) {
-      fe = fe + cross32(code_branch(c, 0, 0), v.g12, N + NE, P + E, S + SE) +
-           cross32(code_branch(c, 0, 1), v.g13, T + TE, P + E, B + BE);
-      fn = fn + cross32(code_branch(c, 1, 0), v.g21, E + NE, P + N, W + NW) +
-           cross32(code_branch(c, 1, 1), v.g23, T + TN, P + N, B + BN);
-      ft = ft + cross32(code_branch(c, 2, 0), v.g31, E + TE, P + T, W + TW) +
-           cross32(code_branch(c, 2, 1), v.g32, N + TN, P + T, S + TS);
-    }
+    fe = fe + cross32(code_branch(c, 0, 0), v.g12, N + NE, P + E, S + SE) +
+         cross32(code_branch(c, 0, 1), v.g13, T + TE, P + E, B + BE);
+    fn = fn + cross32(code_branch(c, 1, 0), v.g21, E + NE, P + N, W + NW) +
+         cross32(code_branch(c, 1, 1), v.g23, T + TN, P + N, B + BN);
+    ft = ft + cross32(code_branch(c, 2, 0), v.g31, E + TE, P + T, W + TW) +
+         cross32(code_branch(c, 2, 1), v.g32, N + TN, P + T, S + TS);
     const float fw = __shfl_up_sync(0xffffffffu, fe, 1);
     shn[k & 1][w][lane] = fn;
     __syncthreads();
