@@ -340,7 +340,7 @@ def roofline(ctx, orthogonal):
     """The dominant kernel: one FP32 zebra half-sweep on the finest level (eight
     per V(2,2) cycle there), in the form the set-up autotuner chose for that
     level -- one kernel, or a residual and a line-solve kernel -- timed live
-    with CUDA events on the context's stream; the FP32 marching residual and
+    with CUDA events on the context's stream; the FP32 residual and
     the FP64 residual beside it."""
     k_ms, k_bytes = ctx.time_kernel("zebra_f32", level=-1, reps=30)
     fine_tune = [t for t in ctx.tuning()["line_sweep"] if t["level"] == ctx.nlevels - 1]
