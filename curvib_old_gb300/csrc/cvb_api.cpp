@@ -113,7 +113,7 @@ static int galloc(cvb_ctx *ctx, Geometry &G, T **p, size_t count) {
   if (count == 0) count = 1;
   if (ctx->device_limit && G.bytes + sizeof(T) * count > ctx->device_limit)
     return fail(ctx, CVB_OOM, "grid allocation of %zu bytes exceeds the context's limit (%zu of %zu bytes in use)",
-                sizeof(T) * count, (size_t)G.bytes, ctx->device_limit);
+                sizeof(T) * count, G.bytes.load(), ctx->device_limit);
   cudaError_t e = cudaMalloc((void **)p, sizeof(T) * count);
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -140,6 +140,8 @@ static void free_all(cvb_ctx *ctx) {
   ctx->iaj.clear(); ctx->jaj.clear(); ctx->kaj.clear(); ctx->aj64.clear();
   ctx->area3 = nullptr;
   ctx->inv_aj = nullptr;
+  ctx->gram = nullptr;
+  ctx->c2c = {};
   ctx->cm[0] = ctx->cm[1] = ctx->cm[2] = nullptr;
   ctx->nvert_tmp = nullptr;
   ctx->Minv = nullptr;
@@ -1708,7 +1710,7 @@ int cvb_projection(cvb_ctx *ctx, const double *phi, double dt, double st, double
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame, F.nvert, F.code,
+  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->gram, ctx->gram_tame, F.nvert, F.code,
                     ctx->w, dt, st, ctx->uc_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(ucont, ctx->uc_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1732,7 +1734,6 @@ static int ghost_types_ok(cvb_ctx *ctx, const int *bc) {
 }
 
 static int ensure_c2c(cvb_ctx *ctx);
-static C2cFactors c2c_factors(const cvb_ctx *ctx) { return {ctx->geo->c2c, ctx->geo->c2c_tame}; }
 static int post_buffers(cvb_ctx *ctx, size_t n) {
   if (!ctx->ucat_dev) TRY(dalloc(ctx, &ctx->ucat_dev, 3 * n));
   if (!ctx->ubcs_dev) TRY(dalloc(ctx, &ctx->ubcs_dev, 3 * n));
@@ -1748,7 +1749,7 @@ int cvb_contra2cart(cvb_ctx *ctx, const double *ucont, double *ucat) {
   TRY(post_buffers(ctx, n));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
+  launch_contra2cart(F.g, ctx->c2c, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(ucat, ctx->ucat_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
@@ -1810,12 +1811,12 @@ int cvb_projection_cart(cvb_ctx *ctx, const double *phi, double dt, double st, d
   TRY(side.begin());  // after the copies in: they would share the link
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame, F.nvert, F.code,
+  launch_projection(F.g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->gram, ctx->gram_tame, F.nvert, F.code,
                     ctx->w, dt, st, ctx->uc_dev, ctx->stream);
   CK(cudaEventRecord(ctx->main_ev, ctx->stream));  // uc_dev is final
   TRY(side.in(ctx->ucat_dev, ucat, 3 * n));
   TRY(side.before_kernels());
-  launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
+  launch_contra2cart(F.g, ctx->c2c, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   TRY(side.in(ctx->ubcs_dev, ubcs, 3 * n));
   TRY(side.before_kernels());
   const bool ubcs_written =
@@ -1854,8 +1855,13 @@ int cvb_convection(cvb_ctx *ctx, const double *ucont, const double *ucat, int ce
 // determinant and its reciprocal of every interior cell), formed on first use and kept with the
 // grid's metrics.
 static int ensure_c2c(cvb_ctx *ctx) {
+  if (ctx->c2c.fac) return CVB_OK;
   Geometry &G = *ctx->geo;
-  if (G.c2c) return CVB_OK;
+  std::lock_guard<std::mutex> lock(G.lazy);
+  if (G.c2c) {
+    ctx->c2c = {G.c2c, G.c2c_tame};
+    return CVB_OK;
+  }
   const int l = ctx->nlevels - 1;
   double *fac = nullptr;
   TRY(galloc(ctx, G, &fac, 11 * ctx->L[l].g.n()));
@@ -1869,6 +1875,7 @@ static int ensure_c2c(cvb_ctx *ctx) {
   CK(cudaStreamSynchronize(ctx->stream));
   G.c2c_tame = h_wild == 0;
   G.c2c = fac;
+  ctx->c2c = {G.c2c, G.c2c_tame};
   return CVB_OK;
 }
 
@@ -1877,8 +1884,14 @@ static int ensure_c2c(cvb_ctx *ctx) {
 // with the grid's metrics; the stream is synchronised once so that contexts
 // sharing the grid on other streams see them.
 static int ensure_face_gram(cvb_ctx *ctx) {
+  if (ctx->gram) return CVB_OK;
   Geometry &G = *ctx->geo;
-  if (G.gram) return CVB_OK;
+  std::lock_guard<std::mutex> lock(G.lazy);
+  if (G.gram) {
+    ctx->gram = G.gram;
+    ctx->gram_tame = G.gram_tame;
+    return CVB_OK;
+  }
   const int l = ctx->nlevels - 1;
   double *gram = nullptr;
   TRY(galloc(ctx, G, &gram, 9 * ctx->L[l].g.n()));
@@ -1894,6 +1907,8 @@ static int ensure_face_gram(cvb_ctx *ctx) {
   CK(cudaStreamSynchronize(ctx->stream));
   G.gram_tame = h_wild == 0;
   G.gram = gram;
+  ctx->gram = G.gram;
+  ctx->gram_tame = G.gram_tame;
   return CVB_OK;
 }
 
@@ -1935,7 +1950,7 @@ static void momentum_faces(cvb_ctx *ctx, double ren, int central, bool cart = tr
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   if (cart)
-    launch_contra2cart(F.g, c2c_factors(ctx), F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
+    launch_contra2cart(F.g, ctx->c2c, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   launch_convection(F.g, ctx->uc_dev, ctx->ucat_dev, F.nvert, central != 0, ctx->conv_fp, ctx->conv_dev, ctx->stream);
   launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
                  ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, nullptr, ctx->stream);
@@ -1946,7 +1961,7 @@ static void momentum_rhs(cvb_ctx *ctx, const MomentumTime *calc) {
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   launch_form_function1(F.g, F.nvert, ctx->p_dev, ctx->conv_dev, ctx->conv_fp, ctx->cm[0], ctx->cm[1], ctx->cm[2],
-                        ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram, ctx->geo->gram_tame,
+                        ctx->aj64[l], fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->gram, ctx->gram_tame,
                         calc, ctx->rct_dev, ctx->rhs_dev, ctx->stream);
 }
 
@@ -2250,7 +2265,7 @@ static int form_bcs_dev(cvb_ctx *ctx, double flux_intp_sum, BcSums &bs) {
   LevelDev &F = ctx->L[ctx->nlevels - 1];
   const Geom &g = F.g;
   const size_t n2 = (size_t)(g.mx - 2) * (g.my - 2);
-  const C2cFactors fac = c2c_factors(ctx);
+  const C2cFactors &fac = ctx->c2c;
   if (ctx->H[ctx->nlevels - 1].d.bctype[5] == 4) {
     auto plane = [&](bool apply, double ratio, bool terms, bool area) -> int {
       launch_outlet_plane(g, ctx->cm[2], fac, F.nvert, apply, ratio, terms, area, ctx->uc_dev, ctx->ubcs_dev,
@@ -2920,7 +2935,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
       case CVB_KERNEL_RESIDUAL_F64: launch_residual<double>(L, L.r64, L.e64, L.t64, ctx->stream); break;
       case CVB_KERNEL_ZEBRA_F32: launch_zebra_half<float>(L, L.r32, L.e32, L.t32 + n, 1.3f, 1, false, ctx->stream); break;
       case CVB_KERNEL_CONTRA2CART:
-        launch_contra2cart(L.g, c2c_factors(ctx), L.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
+        launch_contra2cart(L.g, ctx->c2c, L.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
         break;
       case CVB_KERNEL_GHOST_NODES:
         launch_ghost_node_velocity(L.g, ctx->H[level].d.bctype, ctx->cm[0], ctx->cm[1], ctx->cm[2], ctx->ubcs_dev,
@@ -2933,7 +2948,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
         const double *fm[9];
         for (int q = 0; q < 9; q++) fm[q] = ctx->fm[level][q];
         launch_viscous(L.g, L.nvert, ctx->ucat_dev, fm, ctx->iaj[level], ctx->jaj[level], ctx->kaj[level],
-                       ctx->geo->gram, ctx->geo->gram_tame, 1. / 300., ctx->conv_fp, ctx->visc_dev, ctx->stream);
+                       ctx->gram, ctx->gram_tame, 1. / 300., ctx->conv_fp, ctx->visc_dev, ctx->stream);
         break;
       }
       case CVB_KERNEL_MOMENTUM_RHS: {

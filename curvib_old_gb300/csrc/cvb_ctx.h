@@ -3,8 +3,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -21,11 +23,15 @@ struct LevelHost {
 
 // The grid's resident metrics, shared by every context built on the same grid
 // (cvb_setup_like): problems that differ only in their immersed bodies keep
-// one copy.  Freed with its last context.
+// one copy.  Freed with its last context.  What is formed on first use (gram and
+// c2c, with their places in allocs and bytes) is formed under `lazy` by the first
+// context that needs it, whichever thread that is in; the contexts keep their own
+// copies of the pointers (cvb_ctx::gram, c2c), taken under it.
 struct Geometry {
   int device = 0;
+  std::mutex lazy;
   std::vector<void *> allocs;
-  size_t bytes = 0;
+  std::atomic<size_t> bytes{0};
   std::vector<std::vector<double *>> fm;  // [level][9] raw face metrics (Cmpnts)
   std::vector<double *> iaj, jaj, kaj, aj64;
   double *area3 = nullptr;                // finest: |csi|, |eta|, |zet| per cell ([3][N])
@@ -75,6 +81,9 @@ struct cvb_ctx {
   double *area3 = nullptr;       // finest: |csi|,|eta|,|zet| per cell ([3][N])
   double *cm[3] = {};            // finest: centre metrics csi, eta, zet (Cmpnts)
   double *inv_aj = nullptr;      // finest: 1 / aj (the Geometry's)
+  const double *gram = nullptr;  // finest, once needed: the Geometry's gram
+  bool gram_tame = false;
+  cvb::C2cFactors c2c = {};      // finest, once needed: the Geometry's c2c
   int *cidx = nullptr;           // coarsest level: fluid cells first, then the rest
   double *nvert_tmp = nullptr;
   // coarsest-level solver
