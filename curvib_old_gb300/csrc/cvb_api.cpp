@@ -123,6 +123,13 @@ static int galloc(cvb_ctx *ctx, Geometry &G, T **p, size_t count) {
   G.bytes += sizeof(T) * count;
   return CVB_OK;
 }
+// Gives the latest of them, `count` elements, back.
+template <typename T>
+static void gfree_last(Geometry &G, T *p, size_t count) {
+  G.allocs.pop_back();
+  G.bytes -= sizeof(T) * count;
+  cudaFree(p);
+}
 
 void drop_vcycle_graphs(cvb_ctx *ctx);
 
@@ -1851,6 +1858,14 @@ int cvb_convection(cvb_ctx *ctx, const double *ucont, const double *ucat, int ce
   return CVB_OK;
 }
 
+// The count that a kernel just launched left in *wild.
+static int read_wild(cvb_ctx *ctx, const int *wild, int *out) {
+  CKL();
+  CK(cudaMemcpyAsync(out, wild, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  return CVB_OK;
+}
+
 // The grid's Contra2Cart factors (k_c2c_factors: the metric rows' minors,
 // determinant and its reciprocal of every interior cell), formed on first use and kept with the
 // grid's metrics.
@@ -1863,16 +1878,17 @@ static int ensure_c2c(cvb_ctx *ctx) {
     return CVB_OK;
   }
   const int l = ctx->nlevels - 1;
+  const size_t count = 11 * ctx->L[l].g.n();
   double *fac = nullptr;
-  TRY(galloc(ctx, G, &fac, 11 * ctx->L[l].g.n()));
-  int *wild = nullptr, h_wild = 0;
-  TRY(dalloc(ctx, &wild, 1));
+  TRY(galloc(ctx, G, &fac, count));
+  int *wild = (int *)ctx->sums, h_wild = 0;  // the reductions' scratch
   cudaMemsetAsync(wild, 0, sizeof(int), ctx->stream);
   launch_c2c_factors(ctx->L[l].g, ctx->cm[0], ctx->cm[1], ctx->cm[2], fac, wild, ctx->stream);
-  cudaMemcpyAsync(&h_wild, wild, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-  dfree(ctx, wild);
-  CKL();
-  CK(cudaStreamSynchronize(ctx->stream));
+  const int rc = read_wild(ctx, wild, &h_wild);
+  if (rc != CVB_OK) {
+    gfree_last(G, fac, count);
+    return rc;
+  }
   G.c2c_tame = h_wild == 0;
   G.c2c = fac;
   ctx->c2c = {G.c2c, G.c2c_tame};
@@ -1893,18 +1909,19 @@ static int ensure_face_gram(cvb_ctx *ctx) {
     return CVB_OK;
   }
   const int l = ctx->nlevels - 1;
+  const size_t count = 9 * ctx->L[l].g.n();
   double *gram = nullptr;
-  TRY(galloc(ctx, G, &gram, 9 * ctx->L[l].g.n()));
+  TRY(galloc(ctx, G, &gram, count));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  int *wild = nullptr, h_wild = 0;
-  TRY(dalloc(ctx, &wild, 1));
+  int *wild = (int *)ctx->sums, h_wild = 0;  // the reductions' scratch
   cudaMemsetAsync(wild, 0, sizeof(int), ctx->stream);
   launch_face_gram(ctx->L[l].g, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], gram, wild, ctx->stream);
-  cudaMemcpyAsync(&h_wild, wild, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
-  dfree(ctx, wild);
-  CKL();
-  CK(cudaStreamSynchronize(ctx->stream));
+  const int rc = read_wild(ctx, wild, &h_wild);
+  if (rc != CVB_OK) {
+    gfree_last(G, gram, count);
+    return rc;
+  }
   G.gram_tame = h_wild == 0;
   G.gram = gram;
   ctx->gram = G.gram;

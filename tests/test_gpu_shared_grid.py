@@ -55,3 +55,27 @@ def test_first_projections_at_once():
         finally:
             for c in ctxs:
                 c.close()
+
+
+def test_products_leave_nothing_behind_at_the_limit():
+    """With not a byte left under the context's own limit, Projection's optional grid
+    products are formed once or not at all: a second call takes no more memory."""
+    from curvib_old_gb300 import workload as W
+    from curvib_old_gb300.solver import PoissonContext
+    P = W.make_problem((24, 20, 28), (1.0, 1.0, 1.0), 1.0, True, (False,) * 3, [], nlevels=2)
+    rng = np.random.default_rng(2)
+    phi, u = rng.standard_normal(P.nvert.shape), rng.standard_normal(P.nvert.shape + (3,))
+    free, full = PoissonContext().setup(P), PoissonContext().setup(P)
+    try:
+        want = free.projection(phi, 1e-3, 1.0, u)
+        size, limit = full.geometry_bytes()[0], full.device_bytes()
+        assert limit >= size + 72 * P.nvert.size  # the products themselves fit
+        full.set_device_limit(limit)
+        sizes = []
+        for _ in range(3):
+            assert np.array_equal(full.projection(phi, 1e-3, 1.0, u), want)
+            sizes.append(full.geometry_bytes()[0] - size)
+        assert sizes[0] in (0, 72 * P.nvert.size) and sizes[1:] == [sizes[0]] * 2
+    finally:
+        free.close()
+        full.close()
