@@ -123,6 +123,21 @@ static int galloc(cvb_ctx *ctx, Geometry &G, T **p, size_t count) {
   G.bytes += sizeof(T) * count;
   return CVB_OK;
 }
+// An array that its callers can do without (null then): taken where `rest` bytes
+// that other calls on the grid cannot do without still fit under the limit, and a
+// sixteenth of the device's memory stays free.
+template <typename T>
+static T *galloc_spare(cvb_ctx *ctx, Geometry &G, size_t count, size_t rest) {
+  const size_t bytes = sizeof(T) * count;
+  if (ctx->device_limit && G.bytes + bytes + rest > ctx->device_limit) return nullptr;
+  size_t free = 0, total = 0;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess || free < bytes + rest + total / 16) return nullptr;
+  const std::string err = ctx->err;
+  T *p = nullptr;
+  galloc(ctx, G, &p, count);
+  ctx->err = err;  // no error of the call's
+  return p;
+}
 // Gives the latest of them, `count` elements, back.
 template <typename T>
 static void gfree_last(Geometry &G, T *p, size_t count) {
@@ -1697,19 +1712,13 @@ int cvb_update_pressure(cvb_ctx *ctx, double *p, double *phi) {
   return CVB_OK;
 }
 
-static int ensure_face_gram(cvb_ctx *ctx);
-// The face metric products for the projection, which does without where there is
-// no room for them.
-static int want_face_gram(cvb_ctx *ctx) {
-  const int rc = ensure_face_gram(ctx);
-  return rc == CVB_OOM ? CVB_OK : rc;
-}
+static int face_gram(cvb_ctx *ctx, bool optional);
 
 int cvb_projection(cvb_ctx *ctx, const double *phi, double dt, double st, double *ucont) {
   if (!ctx) return CVB_BAD_INPUT;
   if (!ctx->ready) return fail(ctx, CVB_NOT_SETUP, "cvb_setup_hierarchy has not run");
   if (!phi || !ucont) return fail(ctx, CVB_BAD_INPUT, "phi/ucont is NULL");
-  TRY(want_face_gram(ctx));
+  TRY(face_gram(ctx, true));  // does without where there is no room for them
   int l = ctx->nlevels - 1;
   LevelDev &F = ctx->L[l];
   size_t n = F.g.n();
@@ -1811,7 +1820,7 @@ int cvb_projection_cart(cvb_ctx *ctx, const double *phi, double dt, double st, d
   LevelDev &F = ctx->L[l];
   const size_t n = F.g.n();
   TRY(post_buffers(ctx, n));
-  TRY(want_face_gram(ctx));
+  TRY(face_gram(ctx, true));  // does without where there is no room for them
   SideCopies side(ctx);
   CK(cudaMemcpyAsync(ctx->w, phi, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
@@ -1866,40 +1875,47 @@ static int read_wild(cvb_ctx *ctx, const int *wild, int *out) {
   return CVB_OK;
 }
 
-// The grid's Contra2Cart factors (k_c2c_factors: the metric rows' minors,
-// determinant and its reciprocal of every interior cell), formed on first use and kept with the
-// grid's metrics.
+// The doubles a cell of the arrays that a grid's calls form on first use.
+constexpr size_t kC2cDoubles = 10, kGramDoubles = 9;
+
+// The grid's Contra2Cart factors (k_c2c_factors: the metric rows' minors and
+// determinant of every interior cell, and where there is room its reciprocal, without
+// which the kernel divides), formed on first use and kept with the grid's metrics.
 static int ensure_c2c(cvb_ctx *ctx) {
   if (ctx->c2c.fac) return CVB_OK;
   Geometry &G = *ctx->geo;
   std::lock_guard<std::mutex> lock(G.lazy);
   if (G.c2c) {
-    ctx->c2c = {G.c2c, G.c2c_tame};
+    ctx->c2c = {G.c2c, G.c2c_rcp, G.c2c_tame};
     return CVB_OK;
   }
   const int l = ctx->nlevels - 1;
-  const size_t count = 11 * ctx->L[l].g.n();
+  const size_t n = ctx->L[l].g.n();
   double *fac = nullptr;
-  TRY(galloc(ctx, G, &fac, count));
+  TRY(galloc(ctx, G, &fac, kC2cDoubles * n));
+  double *rcp = galloc_spare<double>(ctx, G, n, G.gram ? 0 : sizeof(double) * kGramDoubles * n);
   int *wild = (int *)ctx->sums, h_wild = 0;  // the reductions' scratch
   cudaMemsetAsync(wild, 0, sizeof(int), ctx->stream);
-  launch_c2c_factors(ctx->L[l].g, ctx->cm[0], ctx->cm[1], ctx->cm[2], fac, wild, ctx->stream);
+  launch_c2c_factors(ctx->L[l].g, ctx->cm[0], ctx->cm[1], ctx->cm[2], fac, rcp, wild, ctx->stream);
   const int rc = read_wild(ctx, wild, &h_wild);
   if (rc != CVB_OK) {
-    gfree_last(G, fac, count);
+    if (rcp) gfree_last(G, rcp, n);
+    gfree_last(G, fac, kC2cDoubles * n);
     return rc;
   }
-  G.c2c_tame = h_wild == 0;
+  G.c2c_tame = h_wild == 0 && rcp;
   G.c2c = fac;
-  ctx->c2c = {G.c2c, G.c2c_tame};
+  G.c2c_rcp = rcp;
+  ctx->c2c = {G.c2c, G.c2c_rcp, G.c2c_tame};
   return CVB_OK;
 }
 
 // --- the momentum right-hand side ------------------------------------------
 // The grid's face metric products (k_face_gram), formed on first use and kept
 // with the grid's metrics; the stream is synchronised once so that contexts
-// sharing the grid on other streams see them.
-static int ensure_face_gram(cvb_ctx *ctx) {
+// sharing the grid on other streams see them.  optional: only where there is room to
+// spare.
+static int face_gram(cvb_ctx *ctx, bool optional) {
   if (ctx->gram) return CVB_OK;
   Geometry &G = *ctx->geo;
   std::lock_guard<std::mutex> lock(G.lazy);
@@ -1909,9 +1925,10 @@ static int ensure_face_gram(cvb_ctx *ctx) {
     return CVB_OK;
   }
   const int l = ctx->nlevels - 1;
-  const size_t count = 9 * ctx->L[l].g.n();
+  const size_t n = ctx->L[l].g.n(), count = kGramDoubles * n;
   double *gram = nullptr;
-  TRY(galloc(ctx, G, &gram, count));
+  if (!optional) TRY(galloc(ctx, G, &gram, count));
+  else if (!(gram = galloc_spare<double>(ctx, G, count, G.c2c ? 0 : sizeof(double) * kC2cDoubles * n))) return CVB_OK;
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   int *wild = (int *)ctx->sums, h_wild = 0;  // the reductions' scratch
@@ -1948,7 +1965,7 @@ static int momentum_prepare(cvb_ctx *ctx, const char *who, const double *ucont, 
   if (!ctx->conv_fp) TRY(dalloc(ctx, &ctx->conv_fp, 9 * n));
   if (!ctx->rct_dev) TRY(dalloc(ctx, &ctx->rct_dev, 3 * n));
   if (!ctx->rhs_dev) TRY(dalloc(ctx, &ctx->rhs_dev, 3 * n));
-  TRY(ensure_face_gram(ctx));
+  TRY(face_gram(ctx, false));
   if (ucont) CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   if (ucat) CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   return CVB_OK;
@@ -2024,7 +2041,7 @@ int cvb_viscous(cvb_ctx *ctx, const double *ucat, double ren, double *visc) {
   if (!ctx->conv_fp) TRY(dalloc(ctx, &ctx->conv_fp, 9 * n));
   if (!ctx->visc_dev) TRY(dalloc(ctx, &ctx->visc_dev, 3 * n));
   if (ucat) CK(cudaMemcpyAsync(ctx->ucat_dev, ucat, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
-  TRY(ensure_face_gram(ctx));
+  TRY(face_gram(ctx, false));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
   launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
@@ -2415,7 +2432,7 @@ int cvb_imp_rk(cvb_ctx *ctx, double *ucont, const double *ucont_o, const double 
   if (!ctx->pu_dev) TRY(dalloc(ctx, &ctx->pu_dev, n3));
   if (!ctx->imp_norms) TRY(dalloc(ctx, &ctx->imp_norms, 2));
   TRY(bc_buffers(ctx));
-  TRY(ensure_face_gram(ctx));
+  TRY(face_gram(ctx, false));
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->uo_dev, ucont_o, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->urm_dev, ucont_rm1, sizeof(double) * n3, cudaMemcpyHostToDevice, ctx->stream));
@@ -3001,7 +3018,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
       CK(cudaMemsetAsync(ctx->rhs_dev, 0, sizeof(double) * 3 * n, ctx->stream));
       CK(cudaMemsetAsync(ctx->uo_dev, 0, sizeof(double) * 3 * n, ctx->stream));
       CK(cudaMemsetAsync(ctx->urm_dev, 0, sizeof(double) * 3 * n, ctx->stream));
-      TRY(ensure_face_gram(ctx));
+      TRY(face_gram(ctx, false));
     }
     // a velocity field of mixed signs in [-1, 1] (zero fluxes would send every
     // face through the full QUICK expression)

@@ -39,8 +39,9 @@ struct Geometry {
   double *inv_aj = nullptr;               // finest: 1 / aj, for the range projection's sum of b / aj
   double *gram = nullptr;                 // finest, on first use: face metric products ([9][N], see k_face_gram)
   bool gram_tame = false;                 // ... and whether they and the face metrics are in intmul.cuh's range
-  double *c2c = nullptr;                  // finest, on first use: Contra2Cart's minors, determinant, reciprocal ([11][N])
-  bool c2c_tame = false;                  // ... and whether they are in intmul.cuh's range
+  double *c2c = nullptr;                  // finest, on first use: Contra2Cart's minors and determinant ([10][N])
+  double *c2c_rcp = nullptr;              // ... the determinant's reciprocal ([N], where there is room)
+  bool c2c_tame = false;                  // ... and whether all are there and in intmul.cuh's range
   ~Geometry() {
     if (allocs.empty()) return;
     cudaSetDevice(device);

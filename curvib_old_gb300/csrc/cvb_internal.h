@@ -298,16 +298,17 @@ struct IbmWork {
 // The search; tmp is one more [mz][my][mx] array.  The result is left in tmp.
 void launch_ibm_search(const IbmArgs &A, const IbmWork &W, double *tmp, cudaStream_t s);
 
-// The grid's Contra2Cart factors (launch_c2c_factors, 11 N doubles) and whether
-// all of them are in intmul.cuh's range
+// The grid's Contra2Cart factors (launch_c2c_factors: 10 N doubles, and the
+// determinants' reciprocals where there was room for them) and whether all of them
+// are there and in intmul.cuh's range
 struct C2cFactors {
-  const double *fac;
+  const double *fac, *rcp;
   bool tame;
 };
 void launch_contra2cart(const Geom &g, const C2cFactors &F, const double *nvert, const double *ucont, double *ucat,
                         cudaStream_t s, int k0 = 1, int nk = -1);
 void launch_c2c_factors(const Geom &g, const double *csi, const double *eta, const double *zet, double *fac,
-                        int *wild, cudaStream_t s);
+                        double *rcp, int *wild, cudaStream_t s);
 // max |div| and its first box index into out_v / out_i (device); pv / pi
 // hold 1024 partial pairs
 void launch_divergence(const Geom &g, const double *ucont, const double *aj, const double *nvert, double *pv,

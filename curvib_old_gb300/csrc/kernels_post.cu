@@ -51,7 +51,7 @@ __device__ __forceinline__ bool conv_fluid(double n) { return conv_below(n, 0.1)
 // do the nine 2 x 2 minors of Cramer's rule, the determinant and its
 // reciprocal: they come from k_c2c_factors' arrays (the same values, bit for
 // bit), and a call forms the three numerators and quotients.
-constexpr int kC2cFactors = 11;  // minors A..I, the determinant, its reciprocal
+constexpr int kC2cFactors = 10;  // minors A..I, the determinant
 
 // The minors b c - d e of the metric rows m, in the order k_contra2cart uses
 // them: A = m11 m22 - m12 m21, B = m10 m22 - m12 m20, C = m10 m21 - m11 m20,
@@ -70,7 +70,6 @@ __device__ __forceinline__ void c2c_minors(const double (&m)[3][3], double (&f)[
   f[7] = mn(m[0][0], m[2][1], m[0][1], m[2][0]);
   f[8] = mn(m[0][0], m[1][1], m[0][1], m[1][0]);
   f[9] = da(ds(dm(m[0][0], f[0]), dm(m[0][1], f[1])), dm(m[0][2], f[2]));
-  f[10] = __ddiv_rn(1.0, f[9]);
 }
 
 __device__ __forceinline__ void c2c_rows(Geom g, const double *__restrict__ csi, const double *__restrict__ eta,
@@ -84,12 +83,13 @@ __device__ __forceinline__ void c2c_rows(Geom g, const double *__restrict__ csi,
   }
 }
 
-// The minors, determinant and its reciprocal of every interior cell into
-// fac[q N + p]; *wild counts those that intmul.cuh's products and quotients do
-// not take.
+// The minors and the determinant of every interior cell into fac[q N + p], its
+// reciprocal into rcp (null: not kept); *wild counts those that intmul.cuh's
+// products and quotients do not take.
 __global__ void __launch_bounds__(256) k_c2c_factors(Geom g, const double *__restrict__ csi,
                                                      const double *__restrict__ eta, const double *__restrict__ zet,
-                                                     double *__restrict__ fac, int *__restrict__ wild) {
+                                                     double *__restrict__ fac, double *__restrict__ rcp,
+                                                     int *__restrict__ wild) {
   const int ni = g.mx - 2, nj = g.my - 2;
   const size_t cells = (size_t)ni * nj * (g.mz - 2), n = g.n();
   const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -104,6 +104,9 @@ __global__ void __launch_bounds__(256) k_c2c_factors(Geom g, const double *__res
   bool out = f[9] == 0.0;
 #pragma unroll
   for (int q = 0; q < kC2cFactors; q++) int_split_a(f[q], out);
+  const double r = __ddiv_rn(1.0, f[9]);
+  int_split_a(r, out);
+  if (rcp) rcp[p] = r;
   if (out) atomicAdd(wild, 1);
 }
 
@@ -127,9 +130,9 @@ __device__ __noinline__ void c2c_fp64(double q0, double q1, double q2, const dou
 // (192^3: 0.31 ms, 0.56 ms with them).  What a cell needs is loaded at once, before
 // the first test: on small grids one latency is most of the kernel.
 struct C2cCell {
-  double nv, w[3], c[3], f[kC2cFactors];  // nvert; the lower and upper face's flux; the factors
-  __device__ __forceinline__ C2cCell(const Geom &g, const double *__restrict__ fac, const double *__restrict__ nvert,
-                                     const double *uc, size_t p) {
+  double nv, w[3], c[3], f[kC2cFactors], rcp;  // nvert; the lower and upper face's flux; the factors
+  __device__ __forceinline__ C2cCell(const Geom &g, const double *__restrict__ fac, const double *__restrict__ rcps,
+                                     const double *__restrict__ nvert, const double *uc, size_t p) {
     const size_t n = g.n();
     nv = nvert[p];
     w[0] = uc[3 * (p - 1)];
@@ -139,6 +142,7 @@ struct C2cCell {
     for (int d = 0; d < 3; d++) c[d] = uc[3 * p + d];
 #pragma unroll
     for (int q = 0; q < kC2cFactors; q++) f[q] = fac[q * n + p];
+    rcp = rcps ? rcps[p] : 0.0;
   }
 };
 // the velocity into u, unchanged where the cell is not fluid
@@ -156,9 +160,9 @@ __device__ __forceinline__ void c2c_cell(const Geom &g, const C2cCell &in, const
       const double d0 = da(ds(int_mul(a0, f(0)), int_mul(a1, f(3))), int_mul(a2, f(4)));
       const double d1 = ds(ds(int_mul(a1, f(5)), int_mul(a0, f(1))), int_mul(a2, f(6)));
       const double d2 = da(ds(int_mul(a0, f(2)), int_mul(a1, f(7))), int_mul(a2, f(8)));
-      u[0] = quot_known(d0, in.f[9], in.f[10]);
-      u[1] = quot_known(d1, in.f[9], in.f[10]);
-      u[2] = quot_known(d2, in.f[9], in.f[10]);
+      u[0] = quot_known(d0, in.f[9], in.rcp);
+      u[1] = quot_known(d1, in.f[9], in.rcp);
+      u[2] = quot_known(d2, in.f[9], in.rcp);
     }
   }
   if (fp64) c2c_fp64(q0, q1, q2, fac + p, g.n(), u);
@@ -166,8 +170,8 @@ __device__ __forceinline__ void c2c_cell(const Geom &g, const C2cCell &in, const
 
 template <bool INT>
 __global__ void __launch_bounds__(128) k_contra2cart(Geom g, const double *__restrict__ fac,
-                                                     const double *__restrict__ nvert, const double *__restrict__ uc,
-                                                     double *__restrict__ ucat, int k0, int nk) {
+                                                     const double *__restrict__ rcp, const double *__restrict__ nvert,
+                                                     const double *__restrict__ uc, double *__restrict__ ucat, int k0, int nk) {
   dep_sync();
   const int ni = g.mx - 2, nj = g.my - 2;
   const size_t cells = (size_t)ni * nj * nk;
@@ -175,7 +179,7 @@ __global__ void __launch_bounds__(128) k_contra2cart(Geom g, const double *__res
   if (t >= cells) return;
   const int k = (int)t / (ni * nj), j = ((int)t - k * ni * nj) / ni, i = (int)t - (k * nj + j) * ni;
   const size_t p = ((size_t)(k0 + k) * g.my + 1 + j) * g.mx + 1 + i;
-  const C2cCell in(g, fac, nvert, uc, p);
+  const C2cCell in(g, fac, rcp, nvert, uc, p);
   if (!conv_fluid(in.nv)) return;
   double u[3];
   c2c_cell<INT>(g, in, fac, p, u);
@@ -189,15 +193,15 @@ void launch_contra2cart(const Geom &g, const C2cFactors &F, const double *nvert,
   if (nk < 0) nk = g.mz - 2;
   const size_t cells = (size_t)(g.mx - 2) * (g.my - 2) * nk;
   if (!cells) return;
-  auto go = [&](auto k) { launch_dep(k, nblk(cells, 128), 128, 0, s, g, F.fac, nvert, ucont, ucat, k0, nk); };
+  auto go = [&](auto k) { launch_dep(k, nblk(cells, 128), 128, 0, s, g, F.fac, F.rcp, nvert, ucont, ucat, k0, nk); };
   F.tame ? go(k_contra2cart<true>) : go(k_contra2cart<false>);
 }
 
 void launch_c2c_factors(const Geom &g, const double *csi, const double *eta, const double *zet, double *fac,
-                        int *wild, cudaStream_t s) {
+                        double *rcp, int *wild, cudaStream_t s) {
   const size_t cells = (size_t)(g.mx - 2) * (g.my - 2) * (g.mz - 2);
   if (!cells) return;
-  k_c2c_factors<<<nblk(cells, 256), 256, 0, s>>>(g, csi, eta, zet, fac, wild);
+  k_c2c_factors<<<nblk(cells, 256), 256, 0, s>>>(g, csi, eta, zet, fac, rcp, wild);
   count_launch();
 }
 
@@ -596,7 +600,7 @@ __global__ void __launch_bounds__(128) k_outlet_plane(Geom g, const double *__re
   double c[3] = {ucat[3 * q], ucat[3 * q + 1], ucat[3 * q + 2]};
   double a = 0., f = 0.;
   if constexpr (APPLY) {
-    C2cCell in(g, F.fac, nv, uc, q);
+    C2cCell in(g, F.fac, F.rcp, nv, uc, q);
     if (in.nv < 0.1) {
       a = __dsqrt_rn(da(da(dm(z[0], z[0]), dm(z[1], z[1])), dm(z[2], z[2])));
 #pragma unroll

@@ -79,3 +79,30 @@ def test_products_leave_nothing_behind_at_the_limit():
     finally:
         free.close()
         full.close()
+
+
+@pytest.mark.parametrize("first", ["contra2cart", "projection"])
+def test_contra2cart_fits_with_its_factors_alone(first):
+    """A limit that leaves room for Contra2Cart's factors (80 bytes a cell) and nothing
+    else on the grid: the arrays that its kernel and Projection's can do without stay
+    away, whichever call comes first, and the results are the same."""
+    from curvib_old_gb300 import workload as W
+    from curvib_old_gb300.solver import PoissonContext
+    P = W.make_problem((24, 20, 28), (1.0, 1.0, 1.0), 1.0, True, (False,) * 3, [], nlevels=1)
+    rng = np.random.default_rng(3)
+    phi, u = rng.standard_normal(P.nvert.shape), rng.standard_normal(P.nvert.shape + (3,))
+    free, full = PoissonContext().setup(P), PoissonContext().setup(P)
+    try:
+        n = P.nvert.size
+        want = free.projection(phi, 1e-3, 1.0, u), free.contra2cart(u, np.zeros_like(u))
+        limit = full.geometry_bytes()[0] + 80 * n
+        assert limit >= full.device_bytes() + 48 * n  # the context's own part of the call
+        full.set_device_limit(limit)
+        if first == "projection":
+            assert np.array_equal(full.projection(phi, 1e-3, 1.0, u), want[0])
+        assert np.array_equal(full.contra2cart(u, np.zeros_like(u)), want[1])
+        assert np.array_equal(full.projection(phi, 1e-3, 1.0, u), want[0])
+        assert full.geometry_bytes()[0] == limit
+    finally:
+        free.close()
+        full.close()
