@@ -231,28 +231,17 @@ void glaunch_prolong(const TaskList &tl, bool f32, cudaStream_t s) {
   if (f32) launch_dep(kg_prolong<float>, tl.nblocks, kFlat, 0, s, tl);
   else launch_dep(kg_prolong<double>, tl.nblocks, kFlat, 0, s, tl);
 }
-template <typename K>
-static void allow_smem(K kernel) {
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-}
 void glaunch_line_sweep(const TaskList &tl, bool f32, float omega32, double omega64, size_t smem, cudaStream_t s) {
   if (!tl.n) return;
-  static bool attr = false;
-  if (!attr) {
-    allow_smem(kg_line_sweep<float, 32>);
-    allow_smem(kg_line_sweep<double, 16>);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, kg_line_sweep<float, 32>, kg_line_sweep<double, 16>);
   if (f32) launch_dep(kg_line_sweep<float, 32>, tl.nblocks, 256, smem, s, tl, omega32);
   else launch_dep(kg_line_sweep<double, 16>, tl.nblocks, 256, smem, s, tl, omega64);
 }
 template <typename T, int TW, int RR>
 static void line_solve_rr(const TaskList &tl, T omega, size_t smem, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    allow_smem(kg_line_solve<T, TW, RR>);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, kg_line_solve<T, TW, RR>);
   launch_dep(kg_line_solve<T, TW, RR>, tl.nblocks, kSolveThreads, smem, s, tl, omega);
 }
 template <typename T, int TW>
@@ -273,12 +262,8 @@ void glaunch_line_solve(const TaskList &tl, bool f32, float omega32, double omeg
 }
 void glaunch_zebra_fused(const TaskList &tl, bool f32, float omega32, double omega64, size_t smem, cudaStream_t s) {
   if (!tl.n) return;
-  static bool attr = false;
-  if (!attr) {
-    allow_smem(kg_zebra_fused<float, kSolveTW32>);
-    allow_smem(kg_zebra_fused<double, kSolveTW64>);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, kg_zebra_fused<float, kSolveTW32>, kg_zebra_fused<double, kSolveTW64>);
   if (f32) launch_dep(kg_zebra_fused<float, kSolveTW32>, tl.nblocks, kSolveThreads, smem, s, tl, omega32);
   else launch_dep(kg_zebra_fused<double, kSolveTW64>, tl.nblocks, kSolveThreads, smem, s, tl, omega64);
 }

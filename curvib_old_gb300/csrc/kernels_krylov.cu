@@ -469,11 +469,8 @@ template <typename T>
 static void dense_apply(const LevelDev &C, const double *Minv, const T *r, T *e, cudaStream_t s, const int *gate) {
   constexpr int kMaxStaged = 8192;  // 64 KB of staged FP64 input
   const int n = (int)C.g.n();
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_dense<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 8 * kMaxStaged);
-    attr = true;
-  }
+  static PerDevice smem;
+  allow_smem(smem, 8 * kMaxStaged, k_dense<T, true>);
   const int rows_per_block = 8, blocks = std::max(1, std::min((n + rows_per_block - 1) / rows_per_block, 4 * sm_count()));
   if (C.cm <= kMaxStaged)
     launch_dep(k_dense<T, true>, blocks, 256, sizeof(double) * (size_t)C.cm, s, Minv, C.cidx, C.cm, n, r, e, gate);

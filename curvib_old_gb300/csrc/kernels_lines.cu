@@ -159,12 +159,8 @@ __global__ void __launch_bounds__(32 * kLineWarps, 4) k_lines(const __grid_const
 
 void launch_lines(const LevelDev &L, bool fused, const double *r, const double *x, double *xnew, double omega, int color,
                   int rsplit, cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_lines<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_lines<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, k_lines<true>, k_lines<false>);
   const dim3 grd(line_tiles_x(L.g), L.g.mz - 2);
   const size_t smem = sizeof(double) * 32 * (size_t)((L.g.my - 2 + kAhead - 1) / kAhead * kAhead);
   const int nt = 32 * kLineWarps;

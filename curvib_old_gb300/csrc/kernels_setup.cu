@@ -619,11 +619,8 @@ size_t dense_inverse_doubles(int n) { return 2 * (size_t)kGjW * n + kGjW * kGjW;
 // matrix).
 bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *work, int *status,
                           cudaStream_t s) {
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_gj_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGjSmemRows * kGjW * 8);
-    attr = true;
-  }
+  static PerDevice smem;
+  allow_smem(smem, kGjSmemRows * kGjW * 8, k_gj_panel);
   double *F = work, *B = F + (size_t)kGjW * n, *Dinv = B + (size_t)kGjW * n;
   cudaMemsetAsync(status, 0, sizeof(int), s);
   // the largest tile that still gives every SM a block (216 unknowns: 16 blocks of

@@ -120,12 +120,8 @@ template <typename T, int TW>
 static void line_sweep(const LevelDev &L, const T *b, const T *x, T *xnew, T omega, int mode, cudaStream_t s) {
   size_t smem = sizeof(T) * 4 * (size_t)L.g.my * TW;
   dim3 grd(nblk(L.g.mx, TW), L.g.mz);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_line_sweep<T, TW, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_line_sweep<T, TW, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, k_line_sweep<T, TW, true>, k_line_sweep<T, TW, false>);
   if (has_cross<T>(L)) launch_dep(k_line_sweep<T, TW, true>, grd, 256, smem, s, L, b, x, xnew, omega, mode);
   else launch_dep(k_line_sweep<T, TW, false>, grd, 256, smem, s, L, b, x, xnew, omega, mode);
 }
@@ -135,11 +131,8 @@ template <typename T, int TW, int RR>
 static void line_solve_r(const LevelDev &L, const T *r, const T *x, T *xnew, T omega, cudaStream_t s, int color,
                          int rsplit) {
   dim3 grd(solve_tiles_x<TW>(L.g, color), L.g.mz);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_line_solve<T, TW, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, k_line_solve<T, TW, RR>);
   launch_dep(k_line_solve<T, TW, RR>, grd, kSolveThreads, line_solve_smem_rr<T, TW>(L.g, RR), s, L, r, x, xnew, omega,
              color, rsplit);
 }
@@ -254,11 +247,8 @@ void launch_line_smooth<double>(const LevelDev &L, const double *b, const double
 template <typename T, int TW, int RR, bool X>
 static void zebra_fused_rx(const LevelDev &L, const T *b, const T *xin, T *xout, T omega, int color, cudaStream_t s) {
   dim3 grd(solve_tiles_x<TW>(L.g, color), L.g.mz);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_zebra_fused<T, TW, RR, X>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, k_zebra_fused<T, TW, RR, X>);
   launch_dep(k_zebra_fused<T, TW, RR, X>, grd, kSolveThreads, line_solve_smem_rr<T, TW>(L.g, RR), s, L, b, xin, xout, omega,
              color);
 }

@@ -280,7 +280,7 @@ static cudaLaunchConfig_t tail_config(cudaLaunchAttribute (&at)[2], cudaStream_t
   return c;
 }
 
-// Whether the device takes these clusters (16 blocks are beyond the portable eight).
+// Whether the current device takes these clusters (16 blocks are beyond the portable eight).
 template <typename T>
 static bool tail_runs() {
   void (*ks[4])(TailArgs<T>) = {k_tail<T, false, false>, k_tail<T, false, true>, k_tail<T, true, false>,
@@ -304,7 +304,8 @@ static bool tail_runs() {
 
 template <typename T>
 int tail_levels(const LevelDev *L, int nlevels) {
-  static const bool runs = tail_runs<T>();
+  static PerDevice attr;
+  const bool runs = attr.get(current_device(), tail_runs<T>);
   int n = 0;
   while (runs && n < kTailLevels && n + 1 < nlevels - 1) {
     const Geom &g = L[n + 1].g;

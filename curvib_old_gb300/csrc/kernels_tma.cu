@@ -272,12 +272,9 @@ static bool zebra_tma_rr(const LevelDev &L, const float *b, float *x, float omeg
       !cached_map(&M.aj, L.ajf32, g.mx, g.my, g.mz, RP + 2) ||
       !cached_map(&M.code, L.code, g.mx, g.my, g.mz, RP + 2))
     return false;
-  static bool attr = false;
+  static PerDevice attr;
   const size_t smem = zebra_tma_smem<RP>(g);
-  if (!attr) {
-    cudaFuncSetAttribute(k_zebra_tma<RP, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr = true;
-  }
+  allow_smem(attr, 200 * 1024, k_zebra_tma<RP, RR>);
   dim3 grd(solve_tiles_x<kTmaLines>(g, color), g.mz);
   launch_dep(k_zebra_tma<RP, RR>, grd, kSolveThreads, smem, s, L, M, x, omega, color);
   return true;

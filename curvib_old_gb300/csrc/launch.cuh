@@ -18,6 +18,7 @@
 #include <utility>
 
 #include "cvb_internal.h"
+#include "per_device.h"
 
 namespace cvb {
 
@@ -45,6 +46,22 @@ inline void launch_dep(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cuda
   c.numAttrs = pdl_enabled() ? 1 : 0;
   cudaLaunchKernelEx(&c, k, std::forward<A>(a)...);
   count_launch();
+}
+
+inline int current_device() {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  return dev;
+}
+// Lets kernels take up to `bytes` of dynamic shared memory on the current device; `on`
+// is the launch site's own, since the attribute holds for one device.
+template <typename... K>
+inline void allow_smem(PerDevice &on, int bytes, K... kernels) {
+  on.get(current_device(), [&] {
+    bool ok = true;
+    ((ok = cudaFuncSetAttribute(kernels, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess && ok), ...);
+    return ok;
+  });
 }
 
 // The face directions a block of the momentum kernels forms: all three of its cells'
