@@ -6,6 +6,7 @@
 
 #include "intmul.cuh"
 #include "launch.cuh"
+#include "row_swaps.h"
 
 namespace cvb {
 
@@ -616,13 +617,14 @@ size_t dense_inverse_doubles(int n) { return 2 * (size_t)kGjW * n + kGjW * kGjW;
 // Inverts the n x n row-major A (device, overwritten) into out (device).
 // perm / colmap are n ints, work dense_inverse_doubles(n) doubles, status one
 // int (device).  Returns false if a pivot column was all zero (a singular
-// matrix).
+// matrix), or a kernel did not run (the CUDA error stays for the caller).
 bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap, double *work, int *status,
                           cudaStream_t s) {
   static PerDevice smem;
   allow_smem(smem, kGjSmemRows * kGjW * 8, k_gj_panel);
   double *F = work, *B = F + (size_t)kGjW * n, *Dinv = B + (size_t)kGjW * n;
   cudaMemsetAsync(status, 0, sizeof(int), s);
+  cudaMemsetAsync(perm, 0xff, sizeof(int) * n, s);  // -1: no row
   // the largest tile that still gives every SM a block (216 unknowns: 16 blocks of
   // 64 x 64 12 us a step)
   const unsigned tile = n >= 64 * 12 ? 64 : n >= 32 * 12 ? 32 : 16, tiles = (n + tile - 1) / tile;
@@ -643,15 +645,13 @@ bool device_dense_inverse(double *A, int n, double *out, int *perm, int *colmap,
     else update(k_gj_update<16>);
     c0 += w;
   }
+  if (cudaPeekAtLastError() != cudaSuccess) return false;  // a launch failed
   int h_status = 0;
   std::vector<int> h_perm(n), map(n);
   cudaMemcpyAsync(&h_status, status, sizeof(int), cudaMemcpyDeviceToHost, s);
   cudaMemcpyAsync(h_perm.data(), perm, sizeof(int) * n, cudaMemcpyDeviceToHost, s);
   if (cudaStreamSynchronize(s) != cudaSuccess || h_status) return false;
-  // row swaps (c, perm[c]) in order become column swaps of the inverse in
-  // reverse order: out[:, q] = A[:, map[q]]
-  for (int q = 0; q < n; q++) map[q] = q;
-  for (int c = n - 1; c >= 0; c--) std::swap(map[c], map[h_perm[c]]);
+  if (!undo_row_swaps(h_perm.data(), n, map.data())) return false;
   cudaMemcpyAsync(colmap, map.data(), sizeof(int) * n, cudaMemcpyHostToDevice, s);
   const unsigned eb = (unsigned)std::min<size_t>(((size_t)n * n + 255) / 256, (size_t)152 * 16);
   k_gj_unpermute<<<eb, 256, 0, s>>>(A, n, colmap, out); count_launch();
