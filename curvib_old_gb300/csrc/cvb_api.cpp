@@ -434,7 +434,7 @@ static int build_operators(cvb_ctx *ctx) {
   // the rows of the one-thread-per-line relaxation
   for (int l = 0; l < nl; l++) {
     LevelDev &lv = ctx->L[l];
-    if (!lines_worth(lv.g)) continue;
+    if (!lines_fit(lv.g)) continue;
     const size_t S = SplitRow::count(lv.g);
     if (!lv.lf64) TRY(dalloc(ctx, &lv.lf64, 3 * S));
     if (lv.cross64 && lv.lw64) {
@@ -469,8 +469,8 @@ bool g_tune_loaded = false;
 
 // With CVB_TUNE_FILE set, measured choices persist in that text file (one
 // shape per line: mx my mz px py pz, the two cross-term flags and the
-// fourteen timings in microseconds; lines of an earlier form, without the last,
-// are passed over and measured again), so a
+// thirteen timings in microseconds; a fourteenth, where a line has one, is the time of
+// the FP64 sweep with one thread per line, 0 for never, in place of lines_pay), so a
 // later process -- a profiler run, say, whose own timings would be distorted --
 // makes the same choices.  Called with g_tune_mu held.
 void tune_file_load() {
@@ -484,10 +484,11 @@ void tune_file_load() {
   cvb_ctx::Tune t;
   char line[1024];
   while (std::fgets(line, sizeof line, f)) {
+    t.zl64 = -1.0;
     if (std::sscanf(line, "%d %d %d %d %d %d %d %d %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf %lf", &k.mx,
                     &k.my, &k.mz, &k.px, &k.py, &k.pz, &k.c32, &k.c64, &t.us32[0], &t.us32[1], &t.us64[0], &t.us64[1],
                     &t.zb32[0], &t.zb32[1], &t.zb64[0], &t.zb64[1], &t.zt32[0], &t.zt32[1], &t.zt32[2], &t.zw32[0],
-                    &t.zw32[1], &t.zl64) != 22)
+                    &t.zw32[1], &t.zl64) < 21)
       continue;
     t.level = 0;
     t.cells = (size_t)k.mx * k.my * k.mz;
@@ -501,9 +502,9 @@ void tune_file_append(const ShapeKey &k, const cvb_ctx::Tune &t) {
   FILE *f = std::fopen(path, "a");
   if (!f) return;
   std::fprintf(f,
-               "%d %d %d %d %d %d %d %d %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f\n",
-               k.mx, k.my, k.mz, k.px, k.py, k.pz, k.c32, k.c64, t.us32[0], t.us32[1], t.us64[0], t.us64[1], t.zb32[0],
-               t.zb32[1], t.zb64[0], t.zb64[1], t.zt32[0], t.zt32[1], t.zt32[2], t.zw32[0], t.zw32[1], t.zl64);
+               "%d %d %d %d %d %d %d %d %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f %.3f\n", k.mx,
+               k.my, k.mz, k.px, k.py, k.pz, k.c32, k.c64, t.us32[0], t.us32[1], t.us64[0], t.us64[1], t.zb32[0],
+               t.zb32[1], t.zb64[0], t.zb64[1], t.zt32[0], t.zt32[1], t.zt32[2], t.zw32[0], t.zw32[1]);
   std::fclose(f);
 }
 }  // namespace
@@ -541,8 +542,9 @@ static int autotune_sweeps(cvb_ctx *ctx) {
       const int rps[3] = {4, 8, 16};
       for (int v = 0; v < 3; v++)
         if (t.zt32[v] > 0.0 && t.zt32[v] < best) { best = t.zt32[v]; L.ztma32 = rps[v]; }
-      // FP64 with one thread per line, on the same rule
-      L.zlines64 = L.lf64 && t.zl64 > 0.0 && t.zl64 < 0.97 * (L.zfuse64 ? t.zb64[1] : t.zb64[0]);
+      // FP64 with one thread per line: by shape, or as the file has it
+      L.zlines64 = L.lf64 && (t.zl64 < 0.0 ? lines_pay(L.g)
+                                           : t.zl64 > 0.0 && t.zl64 < 0.97 * (L.zfuse64 ? t.zb64[1] : t.zb64[0]));
     };
     {
       std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -559,6 +561,7 @@ static int autotune_sweeps(cvb_ctx *ctx) {
     cvb_ctx::Tune t;
     t.level = l;
     t.cells = n;
+    t.zl64 = -1.0;
     CK(cudaMemsetAsync(L.r32, 0, sizeof(float) * n, ctx->stream));
     CK(cudaMemsetAsync(L.e32, 0, sizeof(float) * n, ctx->stream));
     CK(cudaMemsetAsync(L.r64, 0, sizeof(double) * n, ctx->stream));
@@ -618,23 +621,6 @@ static int autotune_sweeps(cvb_ctx *ctx) {
       t.zw32[v] = 1e3 * ms / reps;
     }
     L.ztw32 = 0;
-    // the FP64 zebra sweep with one thread per line
-    t.zl64 = 0.0;
-    if (L.lf64) {
-      L.zlines64 = 1;
-      const int reps = 5;
-      for (int q = 0; q <= reps; q++) {
-        if (q == 1) CK(cudaEventRecord(ctx->ev0, ctx->stream));
-        launch_zebra_sweep<double>(L, L.r64, L.e64, L.t64, L.t64 + n, 1.3, false, ctx->stream);
-      }
-      CK(cudaEventRecord(ctx->ev1, ctx->stream));
-      CK(cudaEventSynchronize(ctx->ev1));
-      CKL();
-      float ms = 0;
-      CK(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-      t.zl64 = 1e3 * ms / reps;
-      L.zlines64 = 0;
-    }
     // the FP32 zebra sweep with TMA-staged tiles, each chunk size
     for (int v = 0; v < 3; v++) {
       t.zt32[v] = 0.0;
@@ -2900,11 +2886,11 @@ int cvb_tuning_report(cvb_ctx *ctx, char *buf, int len) {
              "\"f64\": {\"fused_us\": %.2f, \"split_us\": %.2f, \"choice\": \"%s\"}, "
              "\"zebra_f32\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"split4_us\": %.2f, \"fused4_us\": %.2f, "
              "\"tma4_us\": %.2f, \"tma8_us\": %.2f, \"tma16_us\": %.2f, \"choice\": \"%s\"}, "
-             "\"zebra_f64\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"lines_us\": %.2f, \"choice\": \"%s\"}}",
+             "\"zebra_f64\": {\"split_us\": %.2f, \"fused_us\": %.2f, \"choice\": \"%s\"}}",
              q ? ", " : "", t.level, t.cells, t.us32[0], t.us32[1], L.sweep32 ? "split" : "fused", t.us64[0],
              t.us64[1], L.sweep64 ? "split" : "fused", t.zb32[0], t.zb32[1], t.zw32[0], t.zw32[1], t.zt32[0],
              t.zt32[1], t.zt32[2], z32,
-             t.zb64[0], t.zb64[1], t.zl64, L.zlines64 ? "lines" : L.zfuse64 ? "fused" : "split");
+             t.zb64[0], t.zb64[1], L.zlines64 ? "lines" : L.zfuse64 ? "fused" : "split");
     o += row;
   }
   o += "]}";

@@ -141,7 +141,8 @@ struct cvb_ctx {
   std::map<int, cvb::VGraph> vgraphs;  // captured V-cycles by (precision, basis slot)
   // measured sweep times (us): line sweeps fused / split, zebra sweeps two-kernel /
   // one-kernel, and the FP32 zebra sweep with TMA-staged tiles of 4, 8, 16 row
-  // pairs (0: not run on this level), 4-line tiles, and FP64 with one thread per line
+  // pairs (0: not run on this level), 4-line tiles, and what the tuning file has for FP64
+  // with one thread per line (-1: nothing)
   struct Tune { int level; size_t cells; double us32[2], us64[2], zb32[2], zb64[2], zt32[3], zw32[2], zl64; };
   std::vector<Tune> tune;
 };

@@ -97,8 +97,8 @@ struct LevelDev {
   float *cs32;           // levels without FP32 cross terms: g11, g22, g33, aj and the code (its bits)
                          // in colour-split rows ([5][SplitRow::count]) for the zebra residual; else null
   double *line64;        // ... in FP64
-  // colour-split rows for the one-thread-per-line relaxation (kernels_lines.cu; null: the level does not
-  // try it): m, beta, -c of each row, and without cross terms the seven weights times -m
+  // colour-split rows for the one-thread-per-line relaxation (kernels_lines.cu; null: the level cannot
+  // take it): m, beta, -c of each row, and without cross terms the seven weights times -m
   double *lf64, *lw64;
   // work vectors of this level (the finest level's b/x live in the solver)
   double *r64, *e64, *t64;  // FP64 V-cycle vectors
@@ -371,11 +371,36 @@ void launch_imp_norms(size_t n, const double *rhs, const double *pu, const doubl
 
 // --- FP64 y-line relaxation, one thread per line (kernels_lines.cu)
 // Tiles of 32 lines of one colour in a plane, and the fewest tiles of a colour
-// in a level that tries it: two for each of 152 SMs.
+// in a level that can take it: two for each of 152 SMs.
 inline int line_tiles_x(const Geom &g) { return ((g.mx - 1) / 2 + 31) / 32; }
-constexpr int kLineTiles = 304;
-inline bool lines_worth(const Geom &g) {
+constexpr int kLineTiles = 304, kLineBlocks = 4, kLineAhead = 8;
+inline bool lines_fit(const Geom &g) {
   return g.my - 2 <= kMaxFusedRows && (long long)line_tiles_x(g) * (g.mz - 2) >= kLineTiles;
+}
+// A block's shared memory: a tile's rows, in steps of kLineAhead.
+inline size_t lines_smem(const Geom &g) {
+  return sizeof(double) * 32 * (size_t)((g.my - 2 + kLineAhead - 1) / kLineAhead * kLineAhead);
+}
+// Whether a level that can take it does.  A rule on the shape, not a time: its results
+// differ from the tile kernels' by rounding, and a solve's bits must not depend on what
+// else ran while the set-up timed its kernels.  What decides is how much of the blocks
+// that run at a time have a line for every lane (fill): a tile takes as long for one
+// line as for 32, and a second round of blocks as long as the first.  The shorter the
+// lines, the more the tile kernels' scans cost them, up to 56 rows because the scans take
+// 64 rows' time.  A sweep's time against the faster tile form's, 7- and 19-point levels
+// of 304 to 1,840 tiles where the rule takes it and where not: 16 to 32 rows 0.22 ..
+// 0.89 and 0.70 .. 1.07, 40 to 56 rows 0.55 .. 1.00 and 1.00 .. 1.01, 64 and more 0.68 ..
+// 1.03 (median 0.91; 1.07 at 392 rows in two rounds) and 0.90 .. 1.44 (median 1.07).
+inline bool lines_pay(const Geom &g) {
+  const long long tiles = (long long)line_tiles_x(g) * (g.mz - 2), lines = (long long)((g.mx - 1) / 2) * (g.mz - 2);
+  const long long per_sm = 228 * 1024 / (long long)(lines_smem(g) + 1024);
+  const long long blocks = (per_sm < kLineBlocks ? per_sm : kLineBlocks) * sm_count();
+  const long long rounds = (tiles + blocks - 1) / blocks;
+  const double fill = (double)lines / (32.0 * blocks * rounds);
+  const int rows = g.my - 2;
+  if (rows <= 32) return fill >= 0.2;
+  if (rows <= 56) return fill >= 0.35;
+  return fill >= 0.6 || (rounds == 1 && fill >= 0.5);
 }
 // lf (and, with lw, the scaled weights of a level without cross terms) from
 // the level's weights and Thomas factors

@@ -1,7 +1,7 @@
 // Krylov support: dots with the basis, orthogonalisation with the norm, null-space
 // removal and the coarsest-level dense solve.  Every reduction is two-stage with
-// a block count fixed by the size and a fixed summation tree, so a solve's result
-// does not depend on timing or on what else shares the GPU.
+// a block count fixed by the size and a fixed summation tree, so their results do
+// not depend on timing or on what else shares the GPU.
 #include <algorithm>
 
 #include "intmul.cuh"

@@ -17,8 +17,8 @@
 // tiles, 4.4 M cells) took 153 us against 216 (one kernel with scans), of the
 // distorted 192^3 box (576 tiles, after a residual kernel) 508 against 663; at
 // 96^3 (192 tiles) it took 109 against 96, and on smaller levels twice as long.
-// Levels with fewer than kLineTiles tiles do not try it, the others choose by
-// time.  In FP32, whose pipe does not bound the sweep, it was slower everywhere
+// Levels with fewer than kLineTiles tiles cannot take it, lines_pay says which
+// others do.  In FP32, whose pipe does not bound the sweep, it was slower everywhere
 // (95 against 62 us on the channel's finest level).  Eight warps and four blocks
 // per SM (64 registers): four warps 165 us, three blocks 226, six blocks 244.
 //
@@ -62,7 +62,7 @@ constexpr int kLineWarps = 8;
 // d, then the solution; np rows, the nr of the lines rounded up to a multiple
 // of kAhead, zero beyond.  be and cn: the lane's beta and -c, `pitch` apart row
 // to row, in flight kAhead rows before they are used (nx: the first beta's).
-constexpr int kAhead = 8;
+constexpr int kAhead = kLineAhead;
 __device__ __forceinline__ void rows_ahead(double (&nx)[kAhead], const double *__restrict__ f, int pitch, int j0, int nr) {
 #pragma unroll
   for (int u = 0; u < kAhead; u++) nx[u] = j0 + u >= 0 && j0 + u < nr ? __ldg(f + (size_t)(j0 + u) * pitch) : 0.0;
@@ -96,7 +96,7 @@ __device__ __forceinline__ void lanes_solve(double *sr, double (&nx)[kAhead], co
 // of the residual r (rsplit: in colour-split rows, else in the caller's
 // layout), xnew = x + omega d on the colour's lines, or omega d with x null.
 template <bool FUSED>
-__global__ void __launch_bounds__(32 * kLineWarps, 4) k_lines(const __grid_constant__ LevelDev L,
+__global__ void __launch_bounds__(32 * kLineWarps, kLineBlocks) k_lines(const __grid_constant__ LevelDev L,
                                                               const double *__restrict__ r, const double *x,
                                                               double *xnew, double omega, int color, int rsplit) {
   dep_sync();
@@ -162,7 +162,7 @@ void launch_lines(const LevelDev &L, bool fused, const double *r, const double *
   static PerDevice attr;
   allow_smem(attr, 200 * 1024, k_lines<true>, k_lines<false>);
   const dim3 grd(line_tiles_x(L.g), L.g.mz - 2);
-  const size_t smem = sizeof(double) * 32 * (size_t)((L.g.my - 2 + kAhead - 1) / kAhead * kAhead);
+  const size_t smem = lines_smem(L.g);
   const int nt = 32 * kLineWarps;
   if (fused) launch_dep(k_lines<true>, grd, nt, smem, s, L, r, x, xnew, omega, color, rsplit);
   else launch_dep(k_lines<false>, grd, nt, smem, s, L, r, x, xnew, omega, color, rsplit);
