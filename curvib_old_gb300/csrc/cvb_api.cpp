@@ -75,16 +75,21 @@ static void ensure_pool(int dev) {
   done[dev] = true;
 }
 
+static bool drop_lines(cvb_ctx *ctx);
+
 template <typename T>
 static int dalloc(cvb_ctx *ctx, T **p, size_t count) {
   *p = nullptr;
   if (count == 0) count = 1;
-  if (ctx->device_limit && ctx->device_bytes + sizeof(T) * count > ctx->device_limit)
+  if (ctx->device_limit && ctx->device_bytes + sizeof(T) * count > ctx->device_limit) {
+    if (drop_lines(ctx)) return dalloc(ctx, p, count);
     return fail(ctx, CVB_OOM, "device allocation of %zu bytes exceeds the context's limit (%zu of %zu bytes in use)",
                 sizeof(T) * count, ctx->device_bytes, ctx->device_limit);
+  }
   cudaError_t e = cudaMallocAsync((void **)p, sizeof(T) * count, ctx->stream);
   if (e != cudaSuccess) {
     cudaGetLastError();
+    if (drop_lines(ctx)) return dalloc(ctx, p, count);
     return fail(ctx, CVB_OOM, "device allocation of %zu bytes failed: %s", sizeof(T) * count,
                 cudaGetErrorString(e));
   }
@@ -431,20 +436,7 @@ static int build_operators(cvb_ctx *ctx) {
     launch_split_coef(lv.g, lv.gf32, lv.ajf32, lv.code, lv.cs32, ctx->stream);
     CKL();
   }
-  // the rows of the one-thread-per-line relaxation
-  for (int l = 0; l < nl; l++) {
-    LevelDev &lv = ctx->L[l];
-    if (!lines_fit(lv.g)) continue;
-    const size_t S = SplitRow::count(lv.g);
-    if (!lv.lf64) TRY(dalloc(ctx, &lv.lf64, 3 * S));
-    if (lv.cross64 && lv.lw64) {
-      dfree(ctx, lv.lw64);
-      lv.lw64 = nullptr;
-    }
-    if (!lv.cross64 && !lv.lw64) TRY(dalloc(ctx, &lv.lw64, 7 * S));
-    launch_line_rows(lv.g, lv.w64, lv.line64, lv.lf64, lv.lw64, ctx->stream);
-    CKL();
-  }
+  ctx->lines_formed = false;
   CK(cudaStreamSynchronize(ctx->stream));
   return CVB_OK;
 }
@@ -543,8 +535,8 @@ static int autotune_sweeps(cvb_ctx *ctx) {
       for (int v = 0; v < 3; v++)
         if (t.zt32[v] > 0.0 && t.zt32[v] < best) { best = t.zt32[v]; L.ztma32 = rps[v]; }
       // FP64 with one thread per line: by shape, or as the file has it
-      L.zlines64 = L.lf64 && (t.zl64 < 0.0 ? lines_pay(L.g)
-                                           : t.zl64 > 0.0 && t.zl64 < 0.97 * (L.zfuse64 ? t.zb64[1] : t.zb64[0]));
+      L.zlines64 = lines_fit(L.g) && (t.zl64 < 0.0 ? lines_pay(L.g)
+                                                   : t.zl64 > 0.0 && t.zl64 < 0.97 * (L.zfuse64 ? t.zb64[1] : t.zb64[0]));
     };
     {
       std::lock_guard<std::mutex> lock(g_tune_mu);
@@ -664,6 +656,75 @@ static void face_areas(const std::vector<double> &csi, const std::vector<double>
       const double *v = &(*src[d])[3 * p];
       a3[d * n + p] = std::sqrt(v[0] * v[0] + v[1] * v[1] + v[2] * v[2]);
     }
+}
+
+// The rows of the one-thread-per-line relaxation (24 bytes a cell of the levels that
+// take it, 80 without cross terms): formed by the first FP64 zebra solve after a set-up,
+// since no other call reads them, and only where they fit.  A level that does without
+// takes the tile kernels until the next set-up.
+static void drop_fp64_graphs(cvb_ctx *ctx) {
+  for (auto it = ctx->vgraphs.begin(); it != ctx->vgraphs.end() && it->first < kFp32Graphs;) {
+    if (it->second.exec) cudaGraphExecDestroy(it->second.exec);
+    it = ctx->vgraphs.erase(it);
+  }
+}
+static void drop_level_lines(cvb_ctx *ctx, LevelDev &L) {
+  for (double **p : {&L.lf64, &L.lw64}) {
+    if (*p) dfree(ctx, *p);
+    *p = nullptr;
+  }
+}
+// Gives them back for an allocation that a call cannot do without; false: there are none.
+static bool drop_lines(cvb_ctx *ctx) {
+  bool any = false;
+  for (LevelDev &L : ctx->L) {
+    if (!L.lf64) continue;
+    drop_level_lines(ctx, L);
+    L.zlines64 = 0;
+    any = true;
+  }
+  if (any) drop_fp64_graphs(ctx);
+  return any;
+}
+// Whether an allocation that can be done without fits: under the limit, with a
+// sixteenth of the device's memory left free.
+static bool spare_room(const cvb_ctx *ctx, size_t bytes) {
+  if (ctx->device_limit && ctx->device_bytes + bytes > ctx->device_limit) return false;
+  size_t free = 0, total = 0;
+  uint64_t reserved = 0, used = 0;  // what the pool keeps cached is free too
+  cudaMemPool_t pool;
+  if (cudaMemGetInfo(&free, &total) != cudaSuccess) return false;
+  if (cudaDeviceGetDefaultMemPool(&pool, ctx->device) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+      cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess && reserved > used)
+    free += reserved - used;
+  return free >= bytes + total / 16;
+}
+static int form_lines(cvb_ctx *ctx) {
+  if (ctx->lines_formed) return CVB_OK;
+  const std::string err = ctx->err;
+  bool changed = false;
+  for (LevelDev &L : ctx->L) {
+    const bool kept = L.zlines64 && L.lf64 && (L.lw64 != nullptr) == !L.cross64;
+    if (!kept) {
+      changed = changed || L.lf64 || L.zlines64;
+      drop_level_lines(ctx, L);
+      if (!L.zlines64) continue;
+      const size_t S = SplitRow::count(L.g);
+      if (!spare_room(ctx, sizeof(double) * S * (L.cross64 ? 3 : 10)) || dalloc(ctx, &L.lf64, 3 * S) != CVB_OK ||
+          (!L.cross64 && dalloc(ctx, &L.lw64, 7 * S) != CVB_OK)) {
+        drop_level_lines(ctx, L);
+        L.zlines64 = 0;
+        ctx->err = err;  // no error of the call's
+        continue;
+      }
+    }
+    launch_line_rows(L.g, L.w64, L.line64, L.lf64, L.lw64, ctx->stream);
+    CKL();
+  }
+  if (changed) drop_fp64_graphs(ctx);
+  ctx->lines_formed = true;
+  return CVB_OK;
 }
 
 // ------------------------------------------------------------------ V-cycle
@@ -817,7 +878,7 @@ void drop_vcycle_graphs(cvb_ctx *ctx) {
 
 template <typename T>
 static int vcycle_graph(cvb_ctx *ctx, const cvb_solve_opts *o, int slot, const T *b, T *out) {
-  const int key = (sizeof(T) == 4 ? 1000 : 0) + slot;
+  const int key = (sizeof(T) == 4 ? kFp32Graphs : 0) + slot;
   VGraph &g = ctx->vgraphs[key];
   const bool same = g.omega == o->omega && g.pre == o->pre_sweeps && g.post == o->post_sweeps && g.b == (const void *)b &&
                     g.out == (void *)out && g.smoother == o->smoother;
@@ -1074,6 +1135,7 @@ static int solve_resident(cvb_ctx *ctx, const cvb_solve_opts *o, cvb_solve_stats
   cvb_solve_stats local;
   if (!st) st = &local;
   std::memset(st, 0, sizeof(*st));
+  if (o->precision == CVB_PRECISION_FP64 && o->smoother == CVB_SMOOTHER_ZEBRA) TRY(form_lines(ctx));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
   int rc = fgmres(ctx, o, st);
   cudaEventRecord(ctx->ev1, ctx->stream);
@@ -2980,6 +3042,7 @@ int cvb_time_kernel(cvb_ctx *ctx, int kernel, int level, int reps, double *avg_m
       default: launch_zebra_half<double>(L, L.r64, L.e64, L.t64 + n, 1.3, 1, false, ctx->stream); break;
     }
   };
+  if (kernel == CVB_KERNEL_ZEBRA_F64 || kernel == CVB_KERNEL_VCYCLE_F64) TRY(form_lines(ctx));
   if (kernel == CVB_KERNEL_VCYCLE_F32 || kernel == CVB_KERNEL_VCYCLE_F64) return time_vcycle(ctx, kernel, level, reps, avg_ms, bytes);
   const bool momentum = kernel == CVB_KERNEL_VISCOUS || kernel == CVB_KERNEL_MOMENTUM_RHS;
   if (kernel == CVB_KERNEL_CONTRA2CART || kernel == CVB_KERNEL_GHOST_NODES || kernel == CVB_KERNEL_CONVECTION ||

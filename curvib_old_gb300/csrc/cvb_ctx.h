@@ -15,7 +15,7 @@
 
 namespace cvb {
 
-constexpr int kMaxRestart = 64;
+constexpr int kMaxRestart = 64, kFp32Graphs = 1000;
 
 struct LevelHost {
   cvb_level_desc d;  // shapes / flags only (pointers are not kept)
@@ -138,7 +138,8 @@ struct cvb_ctx {
   // wall-clock ms of the last set-up's phases: metrics upload (0 when the grid
   // was shared), level arrays, operators, autotuner, coarsest solver
   double setup_ms[5] = {};
-  std::map<int, cvb::VGraph> vgraphs;  // captured V-cycles by (precision, basis slot)
+  std::map<int, cvb::VGraph> vgraphs;  // captured V-cycles by basis slot, FP32 from kFp32Graphs on
+  bool lines_formed = false;           // the levels' lf64 / lw64 are of the operators as they are (form_lines)
   // measured sweep times (us): line sweeps fused / split, zebra sweeps two-kernel /
   // one-kernel, and the FP32 zebra sweep with TMA-staged tiles of 4, 8, 16 row
   // pairs (0: not run on this level), 4-line tiles, and what the tuning file has for FP64

@@ -97,8 +97,8 @@ struct LevelDev {
   float *cs32;           // levels without FP32 cross terms: g11, g22, g33, aj and the code (its bits)
                          // in colour-split rows ([5][SplitRow::count]) for the zebra residual; else null
   double *line64;        // ... in FP64
-  // colour-split rows for the one-thread-per-line relaxation (kernels_lines.cu; null: the level cannot
-  // take it): m, beta, -c of each row, and without cross terms the seven weights times -m
+  // colour-split rows for the one-thread-per-line relaxation (kernels_lines.cu; null: not formed): m, beta,
+  // -c of each row, and without cross terms the seven weights times -m
   double *lf64, *lw64;
   // work vectors of this level (the finest level's b/x live in the solver)
   double *r64, *e64, *t64;  // FP64 V-cycle vectors

@@ -278,7 +278,7 @@ static void zebra_fused(const LevelDev &L, const T *b, const T *xin, T *xout, T 
 }
 template <typename T>
 static bool lines_chosen(const LevelDev &L) {
-  return sizeof(T) == 8 && L.zlines64 != 0;
+  return sizeof(T) == 8 && L.zlines64 != 0 && L.lf64;
 }
 template <typename T>
 static bool fused_ok(const LevelDev &L) {
