@@ -106,8 +106,9 @@ __global__ void __launch_bounds__(256, 2) kg_line_sweep(const __grid_constant__ 
     line_sweep_body<T, TW, false>(L, (const T *)K.a, (const T *)K.b, (T *)K.c, omega, K.p0, lb % K.gx, lb / K.gx,
                                   smem_raw);
 }
-// RR: rows per lane of every task's level (0: each task's own, at run time)
-template <typename T, int TW, int RR>
+// RR: rows per lane of every task's level (0: each task's own, at run time); a batch's
+// tasks are all of zebra sweeps (SEG where it has segments) or all of Jacobi sweeps
+template <typename T, int TW, int RR, bool SEG>
 __global__ void __launch_bounds__(kSolveThreads, 4) kg_line_solve(const __grid_constant__ TaskList tl, T omega) {
   dep_sync();
   const GTask &K = tl.t[find_task(tl, blockIdx.x)];
@@ -116,7 +117,7 @@ __global__ void __launch_bounds__(kSolveThreads, 4) kg_line_solve(const __grid_c
   const LevelDev L = *K.L;
   int lb = blockIdx.x - K.block0;
   // p1: colour + 1 (0: all lines), plus 16 when the residual is colour-split
-  line_solve_body<T, TW, RR>(L, (const T *)K.a, (const T *)K.b, (T *)K.c, omega, lb % K.gx, lb / K.gx, smem_raw,
+  line_solve_body<T, TW, RR, SEG>(L, (const T *)K.a, (const T *)K.b, (T *)K.c, omega, lb % K.gx, lb / K.gx, smem_raw,
                              (K.p1 & 15) - 1, (K.p1 >> 4) != 0);
 }
 // zebra half-sweep in one kernel: b = a, x from b into c (in place when b == c),
@@ -238,11 +239,16 @@ void glaunch_line_sweep(const TaskList &tl, bool f32, float omega32, double omeg
   if (f32) launch_dep(kg_line_sweep<float, 32>, tl.nblocks, 256, smem, s, tl, omega32);
   else launch_dep(kg_line_sweep<double, 16>, tl.nblocks, 256, smem, s, tl, omega64);
 }
+template <typename T, int TW, int RR, bool SEG>
+static void line_solve_seg(const TaskList &tl, T omega, size_t smem, cudaStream_t s) {
+  static PerDevice attr;
+  allow_smem(attr, 200 * 1024, kg_line_solve<T, TW, RR, SEG>);
+  launch_dep(kg_line_solve<T, TW, RR, SEG>, tl.nblocks, kSolveThreads, smem, s, tl, omega);
+}
 template <typename T, int TW, int RR>
 static void line_solve_rr(const TaskList &tl, T omega, size_t smem, cudaStream_t s) {
-  static PerDevice attr;
-  allow_smem(attr, 200 * 1024, kg_line_solve<T, TW, RR>);
-  launch_dep(kg_line_solve<T, TW, RR>, tl.nblocks, kSolveThreads, smem, s, tl, omega);
+  if (kSegments<T, TW, RR> && (tl.t[0].p1 & 15)) line_solve_seg<T, TW, RR, kSegments<T, TW, RR>>(tl, omega, smem, s);
+  else line_solve_seg<T, TW, RR, false>(tl, omega, smem, s);
 }
 template <typename T, int TW>
 static void line_solve_r(const TaskList &tl, T omega, size_t smem, int rr, cudaStream_t s) {

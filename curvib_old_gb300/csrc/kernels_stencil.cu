@@ -85,13 +85,13 @@ __global__ void __launch_bounds__(256, 3) k_line_sweep(LevelDev L, const T *__re
 }
 
 // RR: the line layout's rows per lane fixed at compile time (0: read from my)
-template <typename T, int TW, int RR>
-__global__ void __launch_bounds__(kSolveThreads, kTileMinBlocks<T, TW, RR>) k_line_solve(LevelDev L, const T *__restrict__ r, const T *x,
+template <typename T, int TW, int RR, bool SEG>
+__global__ void __launch_bounds__(kSolveThreads, kTileMinBlocks<T, TW, RR, SEG>) k_line_solve(LevelDev L, const T *__restrict__ r, const T *x,
                                                                  T *xnew, T omega, int color, int rsplit) {
   dep_sync();
   if (gated(L.gate)) return;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  line_solve_body<T, TW, RR>(L, r, x, xnew, omega, blockIdx.x, blockIdx.y, smem_raw, color, rsplit != 0);
+  line_solve_body<T, TW, RR, SEG>(L, r, x, xnew, omega, blockIdx.x, blockIdx.y, smem_raw, color, rsplit != 0);
 }
 
 template <typename T, int TW, int RR, bool X>
@@ -127,14 +127,21 @@ static void line_sweep(const LevelDev &L, const T *b, const T *x, T *xnew, T ome
 }
 
 
-template <typename T, int TW, int RR>
-static void line_solve_r(const LevelDev &L, const T *r, const T *x, T *xnew, T omega, cudaStream_t s, int color,
+template <typename T, int TW, int RR, bool SEG>
+static void line_solve_seg(const LevelDev &L, const T *r, const T *x, T *xnew, T omega, cudaStream_t s, int color,
                          int rsplit) {
   dim3 grd(solve_tiles_x<TW>(L.g, color), L.g.mz);
   static PerDevice attr;
-  allow_smem(attr, 200 * 1024, k_line_solve<T, TW, RR>);
-  launch_dep(k_line_solve<T, TW, RR>, grd, kSolveThreads, line_solve_smem_rr<T, TW>(L.g, RR), s, L, r, x, xnew, omega,
-             color, rsplit);
+  allow_smem(attr, 200 * 1024, k_line_solve<T, TW, RR, SEG>);
+  launch_dep(k_line_solve<T, TW, RR, SEG>, grd, kSolveThreads, line_solve_smem_rr<T, TW>(L.g, RR), s, L, r, x, xnew,
+             omega, color, rsplit);
+}
+template <typename T, int TW, int RR>
+static void line_solve_r(const LevelDev &L, const T *r, const T *x, T *xnew, T omega, cudaStream_t s, int color,
+                         int rsplit) {
+  if (kSegments<T, TW, RR> && color >= 0)
+    line_solve_seg<T, TW, RR, kSegments<T, TW, RR>>(L, r, x, xnew, omega, s, color, rsplit);
+  else line_solve_seg<T, TW, RR, false>(L, r, x, xnew, omega, s, color, rsplit);
 }
 template <typename T, int TW>
 static void line_solve(const LevelDev &L, const T *r, const T *x, T *xnew, T omega, cudaStream_t s, int color = -1,

@@ -747,9 +747,8 @@ inline size_t line_solve_smem_rr(const Geom &g, int rr) {
 // Resident blocks per SM the tile kernels are compiled for: with the factors in
 // registers they fit in 48 registers, ten blocks of 128 threads (R = 8: eight;
 // FP64 with the factors of eight rows a lane: six).
-template <typename T, int TW, int RR>
-constexpr int kTileMinBlocks = sizeof(T) == 8 && TW == 4 && RR == 2 ? 6
-                                                                    : kRegFactors<T, TW, RR> ? (RR == 8 ? 8 : 10) : 4;
+template <typename T, int TW, int RR, bool SEG = sizeof(T) == 8 && TW == 4 && RR == 2>
+constexpr int kTileMinBlocks = SEG ? 6 : kRegFactors<T, TW, RR> ? (RR == 8 ? 8 : 10) : 4;
 
 template <int N>
 __device__ __forceinline__ void ld_run(const float *p, float (&o)[N]) {
@@ -787,7 +786,9 @@ __device__ __forceinline__ void ld_run(const double *p, double (&o)[N]) {
 // 32 lanes of two rows costs it 40 operations a warp and line where eight lanes of
 // eight rows cost 23.  The line solves of a colour at 66^3 8.1 -> 6.5 us, the 7-point
 // half-sweep at 130 x 66 x 66 18.9 -> 17.6.  Up to 32 rows the same (eight lanes of four)
-// took as long as before: 6.9 us at 34^3.
+// took as long as before: 6.9 us at 34^3.  The zebra kernels alone (SEG below): the sums
+// differ from the scans' by rounding, and of the Jacobi sweep's two forms, which the
+// set-up chooses between by time, one has the scan of line_sweep_body.
 template <typename T, int TW, int RR>
 constexpr bool kSegments = sizeof(T) == 8 && TW == 4 && RR == 2;
 template <int RS>
@@ -795,17 +796,17 @@ struct SegFactors {
   double a[RS], m[RS], c[RS];
 };
 // The factors of the lines one warp solves in a tile: lines warp, warp + NW, ...
-template <typename T, int TW, int RR>
-using TileLaneFactors = std::conditional_t<kSegments<T, TW, RR>, SegFactors<4 * (RR > 0 ? RR : 1)>,
+template <typename T, int TW, int RR, bool SEG = kSegments<T, TW, RR>>
+using TileLaneFactors = std::conditional_t<SEG, SegFactors<4 * (RR > 0 ? RR : 1)>,
                                            LaneFactors<T, TW / (kSolveThreads / 32), (RR > 0 ? RR : 1)>>;
 // The warp of a block that solves its tile: another one in the blocks that come to
 // the same SM next, since each quarter of an SM has its own FP64 unit.
 __device__ __forceinline__ int segment_warp(int bx, int k, int tiles) { return ((k * tiles + bx) / 152) & 3; }
 
-template <typename T, int TW, int RR>
+template <typename T, int TW, int RR, bool SEG = kSegments<T, TW, RR>>
 __device__ __forceinline__ void lane_factors_load(const LevelDev &L, int bx, int k, int color,
-                                                  TileLaneFactors<T, TW, RR> &f) {
-  if constexpr (kSegments<T, TW, RR>) {
+                                                  TileLaneFactors<T, TW, RR, SEG> &f) {
+  if constexpr (SEG) {
     constexpr int RS = 4 * RR;
     const Geom &g = L.g;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, q0 = (lane & 7) * RS;
@@ -954,10 +955,10 @@ __device__ __forceinline__ void solve_tile_load(const LevelDev &L, const T *__re
 
 // Solve the tile's lines in shared memory and write it out (the tile's copies
 // have landed and the block is synchronised when this is entered).
-template <typename T, int TW, int RR = 0>
+template <typename T, int TW, int RR = 0, bool SEG = kSegments<T, TW, RR>>
 __device__ __forceinline__ void solve_tile_finish(const LevelDev &L, const T *__restrict__ x, T *__restrict__ xnew,
                                                   T omega, int bx, int k, T *st, int color,
-                                                  const TileLaneFactors<T, TW, RR> &lf) {
+                                                  const TileLaneFactors<T, TW, RR, SEG> &lf) {
   const Geom &g = L.g;
   const int my = g.my, mx = g.mx;
   const LineLayout Lo = LineLayout::fixed<RR>(my);
@@ -972,7 +973,7 @@ __device__ __forceinline__ void solve_tile_finish(const LevelDev &L, const T *__
   // the interior hold stale shared memory whose results are never read
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int NW = kSolveThreads / 32, NL = TW / NW;
-  if constexpr (kSegments<T, TW, RR>) {
+  if constexpr (SEG) {
     if (kin && warp == segment_warp(bx, k, solve_tiles_x<TW>(g, color)))
       segment_lines_solve<RR>(sr, lf, Lo.ls, Lo.nr, lane);
   } else if (kin) {
@@ -1016,17 +1017,17 @@ __device__ __forceinline__ void solve_tile_finish(const LevelDev &L, const T *__
 // with x == nullptr, written on those lines only (the caller zeroed the rest).
 // rsplit: r is in the colour-split row layout (a zebra residual), else in the
 // level's own layout.
-template <typename T, int TW, int RR = 0>
+template <typename T, int TW, int RR = 0, bool SEG = kSegments<T, TW, RR>>
 __device__ __forceinline__ void line_solve_body(const LevelDev &L, const T *__restrict__ r, const T *x, T *xnew,
                                                 T omega, int bx, int k, unsigned char *smem_raw, int color = -1,
                                                 bool rsplit = false) {
   T *st = reinterpret_cast<T *>(smem_raw);
-  TileLaneFactors<T, TW, RR> lf;
+  TileLaneFactors<T, TW, RR, SEG> lf;
   solve_tile_load<T, TW, RR>(L, r, x, bx, k, st, color, rsplit, true, !kRegFactors<T, TW, RR>);
-  if constexpr (kRegFactors<T, TW, RR>) lane_factors_load<T, TW, RR>(L, bx, k, color, lf);
+  if constexpr (kRegFactors<T, TW, RR>) lane_factors_load<T, TW, RR, SEG>(L, bx, k, color, lf);
   cp_async_wait_all();
   __syncthreads();
-  solve_tile_finish<T, TW, RR>(L, x, xnew, omega, bx, k, st, color, lf);
+  solve_tile_finish<T, TW, RR, SEG>(L, x, xnew, omega, bx, k, st, color, lf);
 }
 
 // Residual b - A x on the interior cells of one zebra color ((i + k) % 2 ==
