@@ -1727,14 +1727,15 @@ int cvb_poisson_solver_mg(cvb_ctx *ctx, double *ucont, double fis, int immersed,
   SideCopies side(ctx);
   CK(cudaMemcpyAsync(ctx->uc_dev, ucont, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, ctx->stream));
   TRY(volume_flux_dev(ctx, fis, immersed));
-  // the corrected fluxes go out while the solve runs
   TRY(side.begin());
-  TRY(side.out(ucont, ctx->uc_dev, 3 * n));
   launch_poisson_rhs(F.g, ctx->uc_dev, ctx->aj64[ctx->nlevels - 1], F.nvert, dt, st, ctx->b, nullptr, ctx->stream);
   CKL();
   cvb_solve_opts def;
   if (!o) { cvb_solve_opts_default(&def); o = &def; }
   if (o->warm_start) CK(cudaMemcpyAsync(ctx->x, phi, sizeof(double) * n, cudaMemcpyHostToDevice, ctx->stream));
+  // the corrected fluxes go out while the solve runs (pinned arrays: the copy of a
+  // pageable one holds the host, which queues the solve's kernels)
+  TRY(side.out(ucont, ctx->uc_dev, 3 * n));
   int rc = cvb_solve_resident(ctx, o, stats);
   if (rc == CVB_OK || rc == CVB_NOT_CONVERGED)
     CK(cudaMemcpyAsync(phi, ctx->x, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
