@@ -246,6 +246,8 @@ static int check_desc(cvb_ctx *ctx, const cvb_level_desc &d, int level, bool fin
 // Largest coarsest box (ring included) solved by a dense inverse unless the
 // options say otherwise: 18^3 = 5832 holds a 16^3-cell coarsest level.
 constexpr int kCoarseDenseMaxDefault = 6000;
+// Unknowns up to which an inversion's temporaries (1.2 MB) are outside the limit.
+constexpr int kUncountedInverse = 384;
 
 // Rows of the coarsest operator, made nonsingular: M = A + sum_r u_r v_r^T with
 // v_r the indicator of fluid region r and u_r = s v_r.  A's left null vector on
@@ -334,22 +336,33 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
   if (!ctx->cidx) TRY(dalloc(ctx, &ctx->cidx, n));
   CK(cudaMemcpyAsync(ctx->cidx, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice, ctx->stream));
   if (m > 0) {
+    // the matrix and the work arrays, in one piece that is given back before the set-up
+    // ends; towards the context's limit it counts as the matrix, two columns and the
+    // pivot tables, and where the block is small as nothing
+    const size_t nd = (size_t)m * m + dense_inverse_doubles(m), ni = tab.size() + 2 * (size_t)m + 1;
+    const size_t counted = m > kUncountedInverse ? sizeof(double) * ((size_t)m * m + 2 * m) + sizeof(int) * (2 * m + 1) : 0;
+    auto over = [&] { return ctx->device_limit && ctx->device_bytes + counted > ctx->device_limit; };
+    if (over() && !(drop_lines(ctx) && !over()))
+      return fail(ctx, CVB_OOM, "the coarsest inverse's %zu bytes exceed the context's limit (%zu of %zu bytes in use)",
+                  counted, ctx->device_bytes, ctx->device_limit);
     double *dA = nullptr;
-    int *dtab = nullptr, *iwork = nullptr;
-    const size_t nd = dense_inverse_doubles(m);
-    int rc = dalloc(ctx, &dA, (size_t)m * m + nd);
-    if (rc == CVB_OK) rc = dalloc(ctx, &dtab, tab.size());
-    if (rc == CVB_OK) rc = dalloc(ctx, &iwork, 2 * (size_t)m + 1);
+    cudaError_t e = cudaMallocAsync((void **)&dA, sizeof(double) * nd + sizeof(int) * ni, ctx->stream);
+    if (e != cudaSuccess && drop_lines(ctx)) {
+      cudaGetLastError();
+      e = cudaMallocAsync((void **)&dA, sizeof(double) * nd + sizeof(int) * ni, ctx->stream);
+    }
+    if (e != cudaSuccess) {
+      cudaGetLastError();
+      return fail(ctx, CVB_OOM, "device allocation of %zu bytes failed: %s", sizeof(double) * nd + sizeof(int) * ni,
+                  cudaGetErrorString(e));
+    }
+    int *dtab = (int *)(dA + nd), *iwork = dtab + tab.size();
     bool ok = false;
-    if (rc == CVB_OK && cudaMemcpyAsync(dtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice,
-                                        ctx->stream) == cudaSuccess) {
+    if (cudaMemcpyAsync(dtab, tab.data(), sizeof(int) * tab.size(), cudaMemcpyHostToDevice, ctx->stream) == cudaSuccess) {
       launch_coarse_matrix(m, (int)n, dtab, dtab + n, dtab + n + m, sv[0], sv[1], C.w64, dA, ctx->stream);
       ok = device_dense_inverse(dA, m, ctx->Minv, iwork, iwork + m, dA + (size_t)m * m, iwork + 2 * m, ctx->stream);
     }
-    if (iwork) dfree(ctx, iwork);
-    if (dtab) dfree(ctx, dtab);
-    if (dA) dfree(ctx, dA);
-    if (rc != CVB_OK) return rc;
+    cudaFreeAsync(dA, ctx->stream);
     CK(cudaGetLastError());
     if (!ok) return fail(ctx, CVB_BAD_INPUT, "coarsest operator is singular after regularisation");
   }
