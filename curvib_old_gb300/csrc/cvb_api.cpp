@@ -322,10 +322,10 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
   double sv[2] = {0.0, 0.0};
   for (int q = 0; q < 2; q++)
     if (cnt[q]) sv[q] = diag_sum / nfl / cnt[q];
-  // the inverse stays where it was while it fits, so that captured V-cycles
+  // the inverse stays where it was while its size does, so that captured V-cycles
   // stay valid when a body moves
   const size_t need = std::max((size_t)m * m, (size_t)1);
-  if (ctx->Minv && ctx->minv_len < need) {
+  if (ctx->Minv && ctx->minv_len != need) {
     dfree(ctx, ctx->Minv);
     ctx->Minv = nullptr;
   }

@@ -89,7 +89,7 @@ struct cvb_ctx {
   double *nvert_tmp = nullptr;
   // coarsest-level solver
   double *Minv = nullptr;
-  size_t minv_len = 0;           // doubles it has room for
+  size_t minv_len = 0;           // its doubles
   int ncoarse = 0;
   bool coarse_dense = false;
   int multinullspace = 0;

@@ -33,3 +33,23 @@ def test_inverse_at_the_limit(cells):
     finally:
         free.close()
         full.close()
+
+
+def test_a_smaller_inverse_takes_less():
+    """A body that blocks coarse cells leaves a smaller inverse, and no more memory than
+    a context set up with it holds."""
+    from curvib_old_gb300 import workload as W
+    from curvib_old_gb300.solver import PoissonContext
+    P = W.make_problem((24, 16, 20), (1.0, 1.0, 1.0), 2.0, True, (False,) * 3, [], nlevels=2)
+    ctx = PoissonContext().setup(P)
+    try:
+        for r in (0.45, 0.2, 0.45):
+            P.nvert = W.sphere_nvert(P.metrics[-1]["Cent"], [(0.5, 0.5, 0.5, r)])
+            ctx.set_nvert(P.nvert)
+            fresh = PoissonContext().setup(P)
+            try:
+                assert ctx.device_bytes() == fresh.device_bytes()
+            finally:
+                fresh.close()
+    finally:
+        ctx.close()
