@@ -261,8 +261,8 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
   size_t n = C.g.n();
   ctx->ncoarse = (int)n;
   int dense_max = opt ? opt->coarse_dense_max : kCoarseDenseMaxDefault;
-  ctx->coarse_dense = (int)n <= dense_max;
-  if (!ctx->coarse_dense) return CVB_OK;
+  ctx->coarse_dense = false;  // until there is an inverse: a set-up that fails leaves none
+  if ((int)n > dense_max) return CVB_OK;
   std::vector<double> w(n * NSLOT), nv(n);
   CK(cudaMemcpyAsync(w.data(), C.w64, sizeof(double) * n * NSLOT, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaMemcpyAsync(nv.data(), C.nvert, sizeof(double) * n, cudaMemcpyDeviceToHost, ctx->stream));
@@ -369,6 +369,7 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
   CK(cudaStreamSynchronize(ctx->stream));
   C.cidx = ctx->cidx;
   C.cm = m;
+  ctx->coarse_dense = true;
   return CVB_OK;
 }
 

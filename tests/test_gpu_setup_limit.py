@@ -53,3 +53,33 @@ def test_a_smaller_inverse_takes_less():
                 fresh.close()
     finally:
         ctx.close()
+
+
+def test_a_set_nvert_without_room_for_its_inverse():
+    """set_nvert that fails on the inverse leaves a context that solves without one (the
+    coarsest level smoothed), and sets up again once there is room."""
+    from curvib_old_gb300 import workload as W
+    from curvib_old_gb300._lib import STATUS_NAMES, CvbError
+    from curvib_old_gb300.solver import PoissonContext
+    P = W.make_problem((24, 16, 20), (1.0, 1.0, 1.0), 2.0, True, (False,) * 3, [], nlevels=2)
+    small, large = (W.sphere_nvert(P.metrics[-1]["Cent"], [(0.5, 0.5, 0.5, r)]) for r in (0.2, 0.45))
+    P.nvert = large
+    ctx = PoissonContext().setup(P)
+    P.nvert = small
+    fresh = PoissonContext().setup(P)
+    try:
+        uc, _, _ = fresh.volume_flux_rev(P.ucont)
+        b, _ = fresh.poisson_rhs(uc, 1e-3, 1.0)
+        ctx.solve(b, check=False, max_it=3)  # the basis
+        ctx.set_device_limit(ctx.device_bytes() + 72 * P.nvert.size)  # the operators', not the larger inverse
+        with pytest.raises(CvbError) as e:
+            ctx.set_nvert(small)
+        assert STATUS_NAMES[e.value.status] == "OOM"
+        phi, st = ctx.solve(b, check=False, max_it=3)
+        assert st["iterations"] == 3 and np.isfinite(phi).all()
+        ctx.set_device_limit(0)
+        ctx.set_nvert(small)
+        assert np.array_equal(ctx.solve(b)[0], fresh.solve(b)[0])
+    finally:
+        ctx.close()
+        fresh.close()
