@@ -2049,8 +2049,8 @@ static void momentum_faces(cvb_ctx *ctx, double ren, int central, bool cart = tr
   if (cart)
     launch_contra2cart(F.g, ctx->c2c, F.nvert, ctx->uc_dev, ctx->ucat_dev, ctx->stream);
   launch_convection(F.g, ctx->uc_dev, ctx->ucat_dev, F.nvert, central != 0, ctx->conv_fp, ctx->conv_dev, ctx->stream);
-  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
-                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, nullptr, ctx->stream);
+  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->gram,
+                 ctx->gram_tame, 1. / ren, ctx->conv_fp, nullptr, ctx->stream);
 }
 static void momentum_rhs(cvb_ctx *ctx, const MomentumTime *calc) {
   const int l = ctx->nlevels - 1;
@@ -2107,8 +2107,8 @@ int cvb_viscous(cvb_ctx *ctx, const double *ucat, double ren, double *visc) {
   TRY(face_gram(ctx, false));
   const double *fm[9];
   for (int q = 0; q < 9; q++) fm[q] = ctx->fm[l][q];
-  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->geo->gram,
-                 ctx->geo->gram_tame, 1. / ren, ctx->conv_fp, ctx->visc_dev, ctx->stream);
+  launch_viscous(F.g, F.nvert, ctx->ucat_dev, fm, ctx->iaj[l], ctx->jaj[l], ctx->kaj[l], ctx->gram,
+                 ctx->gram_tame, 1. / ren, ctx->conv_fp, ctx->visc_dev, ctx->stream);
   CKL();
   CK(cudaMemcpyAsync(visc, ctx->visc_dev, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
