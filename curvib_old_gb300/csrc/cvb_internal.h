@@ -162,7 +162,7 @@ void launch_weights(const Geom &g, const double *g9, const double *aj, const uin
                     cudaStream_t s);
 void launch_line_factors(const Geom &g, const double *w64, double *line64, float *line32,
                          cudaStream_t s);
-void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate = nullptr);
+void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s);
 void launch_nvert_restrict(const Geom &fine, const double *nvf, const Geom &coarse, int isc, int jsc,
                            int ksc, double *nvc, double *tmp, cudaStream_t s);
 

@@ -67,10 +67,10 @@ __global__ void __launch_bounds__(128) kg_apply64(const __grid_constant__ TaskLi
   const LevelDev L = *T.L;
   Blk3 q = blk3(T, blockIdx.x);
   if (L.cross64)
-    apply64_body<double, true>(L.g, L.w64, L.code, (const double *)T.a, (const double *)T.b, (double *)T.c, q.x, q.y,
+    apply64_body<true>(L.g, L.w64, L.code, (const double *)T.a, (const double *)T.b, (double *)T.c, q.x, q.y,
                                q.z);
   else
-    apply64_body<double, false>(L.g, L.w64, L.code, (const double *)T.a, (const double *)T.b, (double *)T.c, q.x, q.y,
+    apply64_body<false>(L.g, L.w64, L.code, (const double *)T.a, (const double *)T.b, (double *)T.c, q.x, q.y,
                                 q.z);
 }
 template <typename T>

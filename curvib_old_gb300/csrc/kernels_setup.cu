@@ -326,14 +326,13 @@ void launch_line_factors(const Geom &g, const double *w64, double *line64, float
   k_line_factors<<<nblk(lines, 32), 32, 0, s>>>(g, w64, line64, line32); count_launch();
 }
 
-__global__ void k_to_f32(const double *__restrict__ a, float *__restrict__ b, size_t n, const int *gate) {
+__global__ void k_to_f32(const double *__restrict__ a, float *__restrict__ b, size_t n) {
   dep_sync();
-  if (gated(gate)) return;
   for (size_t p = blockIdx.x * (size_t)blockDim.x + threadIdx.x; p < n; p += (size_t)gridDim.x * blockDim.x)
     b[p] = (float)a[p];
 }
-void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s, const int *gate) {
-  launch_dep(k_to_f32, dim3(nblk(n, 256) < 4096 ? nblk(n, 256) : 4096), 256, 0, s, a, b, n, gate);
+void launch_to_f32(const double *a, float *b, size_t n, cudaStream_t s) {
+  launch_dep(k_to_f32, dim3(nblk(n, 256) < 4096 ? nblk(n, 256) : 4096), 256, 0, s, a, b, n);
 }
 // The FP32 V-cycle's result as the FP64 basis vector: the widening on the integer
 // pipe, four cells a thread (17 + 35 MB on 4.4 M cells).

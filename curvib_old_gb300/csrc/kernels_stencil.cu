@@ -8,13 +8,13 @@ static inline unsigned nblk(size_t n, int t) { return (unsigned)((n + t - 1) / t
 
 // X (every operator kernel): the level has cross-derivative terms; kernels for
 // an orthogonal level (X false) read the seven face points only.
-template <typename TX, bool X>
+template <bool X>
 __global__ void __launch_bounds__(128) k_apply64(Geom g, const double *__restrict__ w, const uint32_t *__restrict__ code,
-                                                 const TX *__restrict__ x, const double *__restrict__ b,
+                                                 const double *__restrict__ x, const double *__restrict__ b,
                                                  double *__restrict__ y, const int *gate) {
   dep_sync();
   if (gated(gate)) return;
-  apply64_body<TX, X>(g, w, code, x, b, y, blockIdx.x, blockIdx.y, blockIdx.z);
+  apply64_body<X>(g, w, code, x, b, y, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 __global__ void __launch_bounds__(256) k_apply32(Geom g, const float *__restrict__ gf, const float *__restrict__ aj,
@@ -43,11 +43,10 @@ static const dim3 kMarchBlk(32, 8, 1);
 static dim3 grid3(const Geom &g) { return dim3(nblk(g.mx, 32), nblk(g.my, 4), g.mz); }
 static const dim3 kBlk(32, 4, 1);
 
-template <typename TX>
-static void apply64(const LevelDev &L, const TX *x, const double *b, double *y, cudaStream_t s) {
+static void apply64(const LevelDev &L, const double *x, const double *b, double *y, cudaStream_t s) {
   const dim3 grd(plane_blocks(L.g), 1, L.g.mz);
-  if (L.cross64) launch_dep(k_apply64<TX, true>, grd, kFlat, 0, s, L.g, L.w64, L.code, x, b, y, L.gate);
-  else launch_dep(k_apply64<TX, false>, grd, kFlat, 0, s, L.g, L.w64, L.code, x, b, y, L.gate);
+  if (L.cross64) launch_dep(k_apply64<true>, grd, kFlat, 0, s, L.g, L.w64, L.code, x, b, y, L.gate);
+  else launch_dep(k_apply64<false>, grd, kFlat, 0, s, L.g, L.w64, L.code, x, b, y, L.gate);
 }
 static void apply32(const LevelDev &L, const float *x, const float *b, float *y, cudaStream_t s) {
   if (!apply32_flat(L.g, L.cross32)) {
@@ -60,11 +59,11 @@ static void apply32(const LevelDev &L, const float *x, const float *b, float *y,
 }
 template <>
 void launch_apply<double>(const LevelDev &L, const double *x, double *y, cudaStream_t s) {
-  apply64<double>(L, x, nullptr, y, s);
+  apply64(L, x, nullptr, y, s);
 }
 template <>
 void launch_residual<double>(const LevelDev &L, const double *b, const double *x, double *r, cudaStream_t s) {
-  apply64<double>(L, x, b, r, s);
+  apply64(L, x, b, r, s);
 }
 template <>
 void launch_apply<float>(const LevelDev &L, const float *x, float *y, cudaStream_t s) {

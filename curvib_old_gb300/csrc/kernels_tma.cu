@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kSolveThreads) k_zebra_tma(const __grid_consta
       const float g22 = at(AG22, j, i), s22 = at(AG22, j - 1, i);
       const float g33 = at(AG33, j, i), b33 = at(AG33B, j, i);
       const float ajp = at(AAJ, j, i), bp = at(ARHS, j, i);
-      // row32<float, false>: the same flux form in the same order
+      // row32<false>: the same flux form in the same order
       const float fe = g11 * (E - P), fw = w11 * (P - W), fn = g22 * (N - P);
       const float fs = s22 * (P - Sv), ft = g33 * (T - P), fb = b33 * (P - B);
       const float acc = act(c, CODE_ACT_E) * fe - act(c, CODE_ACT_W) * fw + act(c, CODE_ACT_N) * fn -

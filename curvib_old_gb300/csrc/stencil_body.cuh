@@ -57,15 +57,15 @@ template <typename T>
 struct Star {
   T P, E, W, N, S, Tt, B, NE, SE, NW, SW, TN, BN, TS, BS, TE, BE, TW, BW;
 };
-template <typename T, typename TX>
-__device__ __forceinline__ Star<T> load_star(const TX *__restrict__ x, int p, const Off &o) {
+template <typename T>
+__device__ __forceinline__ Star<T> load_star(const T *__restrict__ x, int p, const Off &o) {
   Star<T> s;
-  s.P = (T)x[p];
-  s.E = (T)x[p + o.e]; s.W = (T)x[p + o.w]; s.N = (T)x[p + o.n]; s.S = (T)x[p + o.s];
-  s.Tt = (T)x[p + o.t]; s.B = (T)x[p + o.b];
-  s.NE = (T)x[p + o.e + o.n]; s.SE = (T)x[p + o.e + o.s]; s.NW = (T)x[p + o.w + o.n]; s.SW = (T)x[p + o.w + o.s];
-  s.TN = (T)x[p + o.t + o.n]; s.BN = (T)x[p + o.b + o.n]; s.TS = (T)x[p + o.t + o.s]; s.BS = (T)x[p + o.b + o.s];
-  s.TE = (T)x[p + o.t + o.e]; s.BE = (T)x[p + o.b + o.e]; s.TW = (T)x[p + o.t + o.w]; s.BW = (T)x[p + o.b + o.w];
+  s.P = x[p];
+  s.E = x[p + o.e]; s.W = x[p + o.w]; s.N = x[p + o.n]; s.S = x[p + o.s];
+  s.Tt = x[p + o.t]; s.B = x[p + o.b];
+  s.NE = x[p + o.e + o.n]; s.SE = x[p + o.e + o.s]; s.NW = x[p + o.w + o.n]; s.SW = x[p + o.w + o.s];
+  s.TN = x[p + o.t + o.n]; s.BN = x[p + o.b + o.n]; s.TS = x[p + o.t + o.s]; s.BS = x[p + o.b + o.s];
+  s.TE = x[p + o.t + o.e]; s.BE = x[p + o.b + o.e]; s.TW = x[p + o.t + o.w]; s.BW = x[p + o.b + o.w];
   return s;
 }
 
@@ -76,10 +76,10 @@ __device__ __forceinline__ Star<T> load_star(const TX *__restrict__ x, int p, co
 // X: the level has cross-derivative weights; without them (an orthogonal grid,
 // the 12 edge slots all zero) only the seven face slots are read, which gives
 // the same sum: every skipped term is an fma with a zero weight.
-template <typename TX, bool X = true>
+template <bool X = true>
 __device__ __forceinline__ double row64(const Geom &g, const double *__restrict__ w, const uint32_t *__restrict__ code,
-                                        const TX *__restrict__ x, int i, int j, int k, int p, int n) {
-  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return (double)x[p];
+                                        const double *__restrict__ x, int i, int j, int k, int p, int n) {
+  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return x[p];
   Off o = offsets(g, i, j, k);
   uint32_t c = __ldg(code + p);
   Star<double> s = load_star<double>(x, p, o);
@@ -118,11 +118,11 @@ __device__ __forceinline__ float act(uint32_t c, uint32_t bit) { return (c & bit
 // X: the level has cross-derivative coefficients; without them (an orthogonal
 // grid) each face flux is its normal term alone and only the seven face
 // values of x are read.
-template <typename TX, bool X = true>
+template <bool X = true>
 __device__ __forceinline__ float row32(const Geom &g, const float *__restrict__ gf, const float *__restrict__ aj,
-                                       const uint32_t *__restrict__ code, const TX *__restrict__ x, int i, int j,
+                                       const uint32_t *__restrict__ code, const float *__restrict__ x, int i, int j,
                                        int k, int p, int n) {
-  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return (float)x[p];
+  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return x[p];
   Off o = offsets(g, i, j, k);
   const int pw = p - 1, ps = p - g.mx, pb = p - g.mx * g.my;  // lower neighbours (never wrapped)
   const uint32_t c = __ldg(code + p), cw = __ldg(code + pw), cs = __ldg(code + ps), cb = __ldg(code + pb);
@@ -160,7 +160,7 @@ __device__ __forceinline__ float row32(const Geom &g, const float *__restrict__ 
 // the cells of one zebra colour sit side by side there, so a half-sweep, which
 // needs the coefficients of one colour's cells, reads whole sectors of them
 // instead of every other value.  The same operands, flux form and order as
-// row32<TX, false>; the W, S and B faces are the E, N and T faces of the
+// row32<false>; the W, S and B faces are the E, N and T faces of the
 // neighbours i - 1, j - 1, k - 1 (never wrapped).  Interior cells only (the
 // zebra kernels' cells): their split positions follow from the cell's own, q,
 // with the row of the other colour h away -- i - 1 and k - 1 are of the other
@@ -194,9 +194,9 @@ __device__ __forceinline__ float row32_split(const Geom &g, const float *__restr
 // Bodies take the block's coordinates explicitly so that the grouped (batched)
 // kernels can run them for any problem of a work-list: (bx, bz) = (block of the
 // plane, plane), kFlat threads.
-template <typename TX, bool X = true>
+template <bool X = true>
 __device__ __forceinline__ void apply64_body(const Geom &g, const double *__restrict__ w,
-                                             const uint32_t *__restrict__ code, const TX *__restrict__ x,
+                                             const uint32_t *__restrict__ code, const double *__restrict__ x,
                                              const double *__restrict__ b, double *__restrict__ y, int bx, int by,
                                              int bz) {
   (void)by;
@@ -204,7 +204,7 @@ __device__ __forceinline__ void apply64_body(const Geom &g, const double *__rest
   if (idx >= pl) return;
   const int j = idx / g.mx, i = idx - j * g.mx, k = bz;
   const int n = (int)g.n(), p = k * pl + idx;
-  double ax = row64<TX, X>(g, w, code, x, i, j, k, p, n);
+  double ax = row64<X>(g, w, code, x, i, j, k, p, n);
   y[p] = b ? b[p] - ax : ax;
 }
 
@@ -257,7 +257,7 @@ __device__ __forceinline__ void apply32_flat_body(const Geom &g, const float *__
   const int pl = g.mx * g.my;
   if (idx >= pl) return;
   const int j = idx / g.mx, i = idx - j * g.mx, p = k * pl + idx;
-  const float ax = row32<float, X>(g, gf, aj, code, x, i, j, k, p, (int)g.n());
+  const float ax = row32<X>(g, gf, aj, code, x, i, j, k, p, (int)g.n());
   y[p] = b ? b[p] - ax : ax;
 }
 
@@ -388,7 +388,7 @@ template <>
 struct RowOf<float> {
   template <bool X = true>
   __device__ static float r(const Geom &g, const LevelDev &L, const float *x, int i, int j, int k, int p, int n) {
-    return row32<float, X>(g, L.gf32, L.ajf32, L.code, x, i, j, k, p, n);
+    return row32<X>(g, L.gf32, L.ajf32, L.code, x, i, j, k, p, n);
   }
   __device__ static const float *fac(const LevelDev &L) { return L.line32; }
 };
@@ -396,7 +396,7 @@ template <>
 struct RowOf<double> {
   template <bool X = true>
   __device__ static double r(const Geom &g, const LevelDev &L, const double *x, int i, int j, int k, int p, int n) {
-    return row64<double, X>(g, L.w64, L.code, x, i, j, k, p, n);
+    return row64<X>(g, L.w64, L.code, x, i, j, k, p, n);
   }
   __device__ static const double *fac(const LevelDev &L) { return L.line64; }
 };
@@ -1042,14 +1042,14 @@ struct ColorRow<float> {
     if constexpr (!X) {
       if (L.cs32) return row32_split(g, L.cs32, x, i, j, k, p);
     }
-    return row32<float, X>(g, L.gf32, L.ajf32, L.code, x, i, j, k, p, n);
+    return row32<X>(g, L.gf32, L.ajf32, L.code, x, i, j, k, p, n);
   }
 };
 template <>
 struct ColorRow<double> {
   template <bool X>
   __device__ static double r(const Geom &g, const LevelDev &L, const double *x, int i, int j, int k, int p, int n) {
-    return row64<double, X>(g, L.w64, L.code, x, i, j, k, p, n);
+    return row64<X>(g, L.w64, L.code, x, i, j, k, p, n);
   }
 };
 template <typename T, bool X = true>
@@ -1152,8 +1152,6 @@ template <int K>
 __device__ __forceinline__ double down(double x) { return scale_down<K>(x); }
 template <int K>
 __device__ __forceinline__ float down(float x) { return __fmul_rn(x, 1.0f / (1 << K)); }
-__device__ __forceinline__ double div_rn(double a, double b) { return __ddiv_rn(a, b); }
-__device__ __forceinline__ float div_rn(float a, float b) { return __fdiv_rn(a, b); }
 // Restriction weight of a fine cell, max(0, 1 - nvert): FP64 from nvert (as the
 // reference), FP32 from the set-up copy of the same value rounded to float.
 __device__ __forceinline__ const double *restrict_weights(const LevelDev &F, double) { return F.nvert; }
