@@ -375,6 +375,7 @@ static int build_coarse(cvb_ctx *ctx, const cvb_solve_opts *opt) {
 
 // nvert restriction down the hierarchy and the operator build of every level.
 static int build_operators(cvb_ctx *ctx) {
+  ctx->lines_formed = false;  // also where what follows fails half-way
   int nl = ctx->nlevels;
   for (int l = nl - 2; l >= 0; l--) {
     LevelDev &F = ctx->L[l + 1], &C = ctx->L[l];
@@ -450,7 +451,6 @@ static int build_operators(cvb_ctx *ctx) {
     launch_split_coef(lv.g, lv.gf32, lv.ajf32, lv.code, lv.cs32, ctx->stream);
     CKL();
   }
-  ctx->lines_formed = false;
   CK(cudaStreamSynchronize(ctx->stream));
   return CVB_OK;
 }
